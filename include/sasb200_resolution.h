@@ -24,6 +24,13 @@
  *                              162-175): np.average over the oversampling
  *                              bins, theory laid out bin-major [nbins][nq],
  *                              wsum = the sum of the bin weights.
+ *   sasb200_pinhole_weights,   the weights of a pinhole or slit resolution
+ *   sasb200_slit_weights       formed once (the reference's weight_matrix, its
+ *                              bands only): those of q i at w[off[i] + j -
+ *                              lo[i]] for lo[i] <= j < hi[i], to be divided
+ *                              by norm[i];
+ *   sasb200_band_apply         apply_resolution_matrix with them, for n_sets
+ *                              curves.
  * All arrays are device pointers; the calls are asynchronous on *stream*.
  * Return 0, -1 for a bad argument, -3 for a launch error;
  * sasb200_resolution_last_error() describes the last failure.
@@ -61,6 +68,20 @@ int32_t sasb200_slit_smear(int32_t nq, int32_t n_calc, const double *q, const do
 int32_t sasb200_pinhole2d_average(int32_t nq, int32_t nbins, const double *theory,
                                   const double *weights, double wsum, double *out,
                                   void *stream);
+
+int32_t sasb200_pinhole_weights(int32_t nq, const double *q, const double *width,
+                                const int32_t *lo, const int32_t *hi, const int64_t *off,
+                                const double *edges, double *w, double *norm, void *stream);
+
+int32_t sasb200_slit_weights(int32_t nq, const double *q, const double *width,
+                             const double *length, int32_t n_length, const double *q_calc,
+                             const double *edges, const int32_t *lo, const int32_t *hi,
+                             const int64_t *off, double *w, double *norm, void *stream);
+
+int32_t sasb200_band_apply(int32_t n_sets, int32_t nq, int32_t n_calc, const int32_t *lo,
+                           const int32_t *hi, const int64_t *off, const double *w,
+                           const double *norm, const double *theory, int64_t theory_stride,
+                           double *out, int64_t out_stride, void *stream);
 
 #ifdef __cplusplus
 }

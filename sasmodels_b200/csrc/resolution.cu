@@ -15,6 +15,9 @@
 //                       and per step across the slit width, the bins between
 //                       |q| and sqrt(q^2 + l^2) found by binary search, the
 //                       u-substituted bin widths formed on the fly.
+//   pinhole_weights,    the same weights formed once per resolution object, and
+//   slit_weights,       their banded product with one curve or many.
+//   band_apply(_sets)
 //   nllf_sets           the fit objective of every curve of a population
 //                       against one data set (bumps_model.py:263-282).
 //   pinhole2d_average   2D pinhole (sasmodels/resolution2d.py:162-175): the
@@ -31,6 +34,11 @@
 namespace res {
 
 constexpr unsigned FULL = 0xffffffffu;
+
+// band_apply (a warp per q and curve) up to this many (q, curve) pairs, then
+// band_apply_sets: 181 q x 61 curves 3.8 against 6.2 us and 400 x 61 5.7 against
+// 6.6, but 181 x 200 7.3 against 6.3 and 1000 x 61 12.1 against 8.4.
+constexpr long long BAND_WARP_LIMIT = 28000;
 constexpr double SQRT2 = 1.4142135623730951;     // numpy sqrt(2.0), correctly rounded
 
 // One curve per blockIdx.y: theory + y*theory_stride -> out + y*out_stride.
@@ -59,6 +67,23 @@ pinhole_smear(int nq, const double *__restrict__ q, const double *__restrict__ w
         wsum += __shfl_xor_sync(FULL, wsum, off);
     }
     if (lane == 0) out[i] = acc/wsum;
+}
+
+// 8 bytes global -> shared, asynchronously; zeros where !valid (src is not read)
+__device__ __forceinline__ void copy8(double *dst, const double *src, bool valid = true)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;"
+                 :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 8 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_commit()
+{
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void copy_wait()
+{
+    asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory");
 }
 
 __global__ void __launch_bounds__(256)
@@ -137,6 +162,255 @@ slit_smear(int nq, int n_calc, const double *__restrict__ q, const double *__res
     #pragma unroll
     for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(FULL, acc, off);
     if (lane == 0) out[i] = acc;
+}
+
+// ------------------------------------------------- banded weights (plans) --
+// A resolution object is applied to new theory curves at every step of a fit
+// while its weights never change, so they are formed once (pinhole_weights,
+// slit_weights) and each application is a banded product.  Weights of q i:
+// w[off[i] + j - lo[i]] for the calculated points lo[i] <= j < hi[i], divided
+// by norm[i] after the sum.
+
+// One warp per q: the bin masses of pinhole_smear and their sum, in its order.
+__global__ void __launch_bounds__(256)
+pinhole_weights(int nq, const double *__restrict__ q, const double *__restrict__ width,
+                const int32_t *__restrict__ lo, const int32_t *__restrict__ hi,
+                const int64_t *__restrict__ off, const double *__restrict__ edges,
+                double *__restrict__ w, double *__restrict__ norm)
+{
+    const int i = (int)((blockIdx.x*(size_t)blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
+    if (i >= nq) return;
+    const double qi = q[i];
+    const double s = SQRT2*width[i];
+    double *wi = w + off[i];
+    const int a = lo[i], b = hi[i];
+    double wsum = 0.0;
+    for (int j = a + lane; j < b; j += 32) {
+        const double m = erf((edges[j + 1] - qi)/s) - erf((edges[j] - qi)/s);
+        wi[j - a] = m;
+        wsum += m;
+    }
+    #pragma unroll
+    for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(FULL, wsum, o);
+    if (lane == 0) norm[i] = wsum;
+}
+
+// One block per q (bound by the square roots: 61 per edge of the band, 199 us
+// per application of 251 q when slit_smear forms them, now once per plan and
+// 3 us per application), the steps across the slit (qk and its upper limit) in
+// shared memory.  A warp takes 31 bins at a time: lane L forms sqrt(u) at edge
+// L of the group and gets the next edge's from lane L + 1, so each (edge,
+// step) costs one square root instead of slit_smear's two and its two binary
+// searches per step.  A step that does not reach a bin has equal u at both of
+// its edges and adds 0.
+constexpr int SLIT_BATCH = 128;
+__global__ void __launch_bounds__(256)
+slit_weights(const double *__restrict__ q, const double *__restrict__ width,
+             const double *__restrict__ length, int n_length, const double *__restrict__ q_calc,
+             const double *__restrict__ edges, const int32_t *__restrict__ lo,
+             const int32_t *__restrict__ hi, const int64_t *__restrict__ off,
+             double *__restrict__ w, double *__restrict__ norm)
+{
+    __shared__ double sq[SLIT_BATCH], sl[SLIT_BATCH];
+    const int i = blockIdx.x, t = threadIdx.x;
+    const int warp = t >> 5, lane = t & 31, warps = (int)blockDim.x >> 5;
+    const double qi = q[i], wi = width[i], li = length[i];
+    const int a = lo[i], b = hi[i];
+    double *out = w + off[i];
+    if (wi == 0.0 && li == 0.0) {
+        // perfect resolution: the theory at q_calc == q
+        if (t == 0) norm[i] = 1.0;
+        for (int j = a + t; j < b; j += (int)blockDim.x) out[j - a] = q_calc[j] == qi ? 1.0 : 0.0;
+        return;
+    }
+    const int kmax = wi == 0.0 ? 0 : n_length;
+    const int steps = 2*kmax + 1;
+    if (t == 0) norm[i] = (double)steps;
+    for (int k0 = 0; k0 < steps; k0 += SLIT_BATCH) {
+        const int nk = min(SLIT_BATCH, steps - k0);
+        __syncthreads();
+        for (int k = t; k < nk; k += (int)blockDim.x) {
+            const double qk = kmax ? qi + ((k0 + k - kmax)*wi)/n_length : qi;
+            sq[k] = qk;
+            sl[k] = sqrt(__dadd_rn(__dmul_rn(qk, qk), __dmul_rn(li, li)));
+        }
+        __syncthreads();
+        for (int j0 = a + 31*warp; j0 < b; j0 += 31*warps) {
+            const double edge = edges[min(j0 + lane, b)];
+            double acc = 0.0;
+            #pragma unroll 4
+            for (int k = 0; k < nk; ++k) {
+                const double r = sqrt(slit_u(edge, sq[k], sl[k]));
+                acc += __dsub_rn(__shfl_down_sync(FULL, r, 1), r);
+            }
+            const int j = j0 + lane;
+            if (lane < 31 && j < b) {
+                const double part = acc/li;
+                out[j - a] = k0 == 0 ? part : out[j - a] + part;
+            }
+        }
+    }
+}
+
+// One warp per (q, curve): bound by latency and the two streams of doubles;
+// taken for one curve and for few (see sasb200_band_apply).
+__global__ void __launch_bounds__(128)
+band_apply(int nq, const int32_t *__restrict__ lo, const int32_t *__restrict__ hi,
+           const int64_t *__restrict__ off, const double *__restrict__ w,
+           const double *__restrict__ norm, const double *__restrict__ theory,
+           size_t theory_stride, double *__restrict__ out, size_t out_stride)
+{
+    const int i = (int)((blockIdx.x*(size_t)blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
+    if (i >= nq) return;
+    const int a = lo[i], n = hi[i] - a;
+    const double *wi = w + off[i], *th = theory + blockIdx.y*theory_stride + a;
+    double acc = 0.0;
+    #pragma unroll 4
+    for (int j = lane; j < n; j += 32) acc += wi[j]*th[j];
+    #pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
+    if (lane == 0) out[blockIdx.y*out_stride + i] = acc/norm[i];
+}
+
+// x/d from r = 1/d: one Newton step on the quotient's residual, which rounds as
+// the division does for the normal range that sr_of admits; an infinite
+// quotient has no residual and r = 0 marks the divisors that sr_of refuses.
+__device__ __forceinline__ double sr_of(double d)
+{
+    return fabs(d) > 1e-290 && fabs(d) < 1e290 ? 1.0/d : 0.0;
+}
+__device__ __forceinline__ double quotient(double x, double d, double r)
+{
+    const double q = x*r;
+    return r == 0.0 || !isfinite(q) ? x/d : fma(fma(-q, d, x), r, q);
+}
+
+// Many curves: a block takes 32 q and 64 curves; a warp holds 8 of the q, a
+// lane two of the curves, so one theory value in a register serves 8 sums and
+// one weight (read as a broadcast) serves 64: 16 multiply-adds per 6
+// shared-memory reads, the point where both pipes are as busy.  The points of
+// the 32 bands pass through shared memory 16 at a time, the next 16 on their
+// way meanwhile.  Sums over 16 points are added to the totals, which keeps the
+// rounding error below that of one long sum.  A warp runs over the union of its
+// 8 bands with weight 0 outside each; a sum that this leaves infinite or
+// undefined is formed again over its own band alone, so that such a theory value
+// reaches only the q that see it.  4096 curves of 1000 q, 5 % width: 48 us; with
+// the weights formed for every curve (pinhole_smear) 2868 us.
+constexpr int BQ = 32, BQW = 8, BJ = 16, BS = 64, BWARPS = BQ/BQW, BTHREADS = 32*BWARPS;
+constexpr int BW_LD = BQ + 2;                // even: pairs of weights are read as double2
+constexpr int BT_LD = BS + 1;                // odd: spreads a row of points over the banks
+
+__global__ void __launch_bounds__(BTHREADS, 4)
+band_apply_sets(int n_sets, int nq, const int32_t *__restrict__ lo,
+                const int32_t *__restrict__ hi, const int64_t *__restrict__ off,
+                const double *__restrict__ w, const double *__restrict__ norm,
+                const double *__restrict__ theory, size_t theory_stride,
+                double *__restrict__ out, size_t out_stride)
+{
+    constexpr int TH = 2*BJ*BT_LD, OUT = BS*(BQ + 1);
+    __shared__ double th[TH > OUT ? TH : OUT];
+    __shared__ __align__(16) double ws[2*BJ*BW_LD];
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int q0 = blockIdx.x*BQ, s0 = blockIdx.y*BS;
+    const int qs = q0 + lane;
+    const int my_lo = qs < nq ? lo[qs] : 0x7fffffff, my_hi = qs < nq ? hi[qs] : 0;
+    const int jmin = __reduce_min_sync(FULL, my_lo), jmax = __reduce_max_sync(FULL, my_hi);
+    const int chunks = jmax > jmin ? (jmax - jmin + BJ - 1)/BJ : 0;
+    // the union of this warp's bands
+    const bool mine = lane/BQW == warp;
+    const int ulo = __reduce_min_sync(FULL, mine ? my_lo : 0x7fffffff);
+    const int uhi = __reduce_max_sync(FULL, mine ? my_hi : 0);
+    // staging: thread t copies point t % 16 of a chunk, of eight curves and of
+    // four q
+    const int js = t & (BJ - 1), rs = t/BJ;
+    const double *tsrc = theory + (size_t)min(s0 + rs, n_sets - 1)*theory_stride + jmin + js;
+    const int t_rows = n_sets - s0 - rs;
+    int wlo[4], whi[4];
+    const double *wsrc[4];
+    #pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int iq = q0 + rs + 8*r;
+        wlo[r] = iq < nq ? lo[iq] : 0;
+        whi[r] = iq < nq ? hi[iq] : 0;
+        wsrc[r] = w + (iq < nq ? off[iq] : 0) - wlo[r];
+    }
+    auto stage = [&](int c) {
+        const int j = jmin + c*BJ + js;
+        double *tb = th + (c & 1)*BJ*BT_LD + js*BT_LD + rs;
+        double *wb = ws + (c & 1)*BJ*BW_LD + js*BW_LD + rs;
+        const double *src = tsrc + c*BJ;
+        #pragma unroll
+        for (int r = 0; r < BS/8; ++r) {
+            const bool ok = 8*r < t_rows && j < jmax;
+            copy8(tb + 8*r, ok ? src : theory, ok);
+            src += 8*theory_stride;
+        }
+        #pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const bool ok = j >= wlo[r] && j < whi[r];
+            copy8(wb + 8*r, ok ? wsrc[r] + j : w, ok);
+        }
+        copy_commit();
+    };
+    double acc[BQW][2], part[BQW][2];
+    #pragma unroll
+    for (int u = 0; u < BQW; ++u) acc[u][0] = acc[u][1] = part[u][0] = part[u][1] = 0.0;
+    if (chunks > 0) stage(0);
+    for (int c = 0; c < chunks; ++c) {
+        if (c + 1 < chunks) {
+            stage(c + 1);
+            copy_wait<1>();
+        } else {
+            copy_wait<0>();
+        }
+        __syncthreads();
+        const int jc = jmin + c*BJ;
+        const int first = max(ulo - jc, 0), last = min(BJ, uhi - jc);
+        const double *tb = th + (c & 1)*BJ*BT_LD + lane;
+        const double *wb = ws + (c & 1)*BJ*BW_LD + BQW*warp;
+        #pragma unroll 4
+        for (int jj = first; jj < last; ++jj) {
+            const double x0 = tb[jj*BT_LD], x1 = tb[jj*BT_LD + 32];
+            const double2 *wp = reinterpret_cast<const double2 *>(wb + jj*BW_LD);
+            #pragma unroll
+            for (int u = 0; u < BQW; u += 2) {
+                const double2 y = wp[u/2];
+                part[u][0] = fma(y.x, x0, part[u][0]);
+                part[u][1] = fma(y.x, x1, part[u][1]);
+                part[u + 1][0] = fma(y.y, x0, part[u + 1][0]);
+                part[u + 1][1] = fma(y.y, x1, part[u + 1][1]);
+            }
+        }
+        #pragma unroll
+        for (int u = 0; u < BQW; ++u) {
+            acc[u][0] += part[u][0];
+            acc[u][1] += part[u][1];
+            part[u][0] = part[u][1] = 0.0;
+        }
+        __syncthreads();
+    }
+    // through shared memory, so that rows of 32 q leave together
+    #pragma unroll
+    for (int u = 0; u < BQW; ++u) {
+        th[lane*(BQ + 1) + BQW*warp + u] = acc[u][0];
+        th[(32 + lane)*(BQ + 1) + BQW*warp + u] = acc[u][1];
+    }
+    __syncthreads();
+    if (qs < nq) {
+        const double d = norm[qs], r = sr_of(d);
+        const int64_t o = off[qs];
+        for (int k = warp; k < BS && s0 + k < n_sets; k += BWARPS) {
+            double v = th[k*(BQ + 1) + lane];
+            if (!isfinite(v)) {
+                v = 0.0;
+                const double *src = theory + (s0 + k)*theory_stride;
+                for (int j = my_lo; j < my_hi; ++j) v = fma(w[o + (j - my_lo)], src[j], v);
+            }
+            out[(s0 + k)*out_stride + qs] = quotient(v, d, r);
+        }
+    }
 }
 
 // Negative log-likelihood of each curve against one data set
@@ -221,6 +495,66 @@ int32_t sasb200_pinhole_smear_sets(int32_t n_sets, int32_t nq, int32_t n_calc, c
     res::pinhole_smear<<<grid, threads, 0, (cudaStream_t)stream>>>(
         nq, q, width, lo, hi, edges, theory, out, (size_t)theory_stride, (size_t)out_stride);
     return res::status("pinhole_smear_sets");
+}
+
+// The weights of a pinhole resolution for sasb200_band_apply: w[off[i] .. off[i]
+// + hi[i] - lo[i]) and norm[nq], from the arrays of sasb200_pinhole_smear.
+int32_t sasb200_pinhole_weights(int32_t nq, const double *q, const double *width,
+                                const int32_t *lo, const int32_t *hi, const int64_t *off,
+                                const double *edges, double *w, double *norm, void *stream)
+{
+    res::errbuf()[0] = 0;
+    if (nq < 0 || (nq > 0 && (!q || !width || !lo || !hi || !off || !edges || !w || !norm)))
+        return (std::snprintf(res::errbuf(), 256, "bad arguments"), -1);
+    if (nq == 0) return 0;
+    const unsigned blocks = (unsigned)(((long long)nq*32 + 255)/256);
+    res::pinhole_weights<<<blocks, 256, 0, (cudaStream_t)stream>>>(nq, q, width, lo, hi, off,
+                                                                    edges, w, norm);
+    return res::status("pinhole_weights");
+}
+
+// The weights of a slit resolution for sasb200_band_apply; lo/hi: the bins
+// that any step across the slit reaches.
+int32_t sasb200_slit_weights(int32_t nq, const double *q, const double *width,
+                             const double *length, int32_t n_length, const double *q_calc,
+                             const double *edges, const int32_t *lo, const int32_t *hi,
+                             const int64_t *off, double *w, double *norm, void *stream)
+{
+    res::errbuf()[0] = 0;
+    if (nq < 0 || n_length < 1 || (nq > 0 && (!q || !width || !length || !q_calc || !edges || !lo
+                                               || !hi || !off || !w || !norm)))
+        return (std::snprintf(res::errbuf(), 256, "bad arguments"), -1);
+    if (nq == 0) return 0;
+    res::slit_weights<<<nq, 256, 0, (cudaStream_t)stream>>>(q, width, length, n_length, q_calc,
+                                                             edges, lo, hi, off, w, norm);
+    return res::status("slit_weights");
+}
+
+// out[s*out_stride + i] = sum_j w[off[i] + j - lo[i]] theory[s*theory_stride + j]/norm[i]
+// over lo[i] <= j < hi[i], for n_sets curves.
+int32_t sasb200_band_apply(int32_t n_sets, int32_t nq, int32_t n_calc, const int32_t *lo,
+                           const int32_t *hi, const int64_t *off, const double *w,
+                           const double *norm, const double *theory, int64_t theory_stride,
+                           double *out, int64_t out_stride, void *stream)
+{
+    res::errbuf()[0] = 0;
+    if (n_sets < 0 || n_sets > 65535 || nq < 0 || n_calc < 0 || theory_stride < n_calc
+        || out_stride < nq || (nq > 0 && n_sets > 0 && (!lo || !hi || !off || !w || !norm
+                                                          || !theory || !out)))
+        return (std::snprintf(res::errbuf(), 256, "bad arguments"), -1);
+    if (nq == 0 || n_sets == 0) return 0;
+    cudaStream_t st = (cudaStream_t)stream;
+    const size_t ts = (size_t)theory_stride, os = (size_t)out_stride;
+    const unsigned qb = (unsigned)((nq + res::BQ - 1)/res::BQ);
+    if ((long long)nq*n_sets <= res::BAND_WARP_LIMIT) {
+        const dim3 grid((unsigned)((nq + 3)/4), (unsigned)n_sets);
+        res::band_apply<<<grid, 128, 0, st>>>(nq, lo, hi, off, w, norm, theory, ts, out, os);
+    } else {
+        const dim3 grid(qb, (unsigned)((n_sets + res::BS - 1)/res::BS));
+        res::band_apply_sets<<<grid, res::BTHREADS, 0, st>>>(n_sets, nq, lo, hi, off, w, norm,
+                                                             theory, ts, out, os);
+    }
+    return res::status("band_apply");
 }
 
 // out[s] = 0.5 sum_i ((theory[s*theory_stride + i] - y[i])/dy[i])^2.

@@ -12,9 +12,9 @@ returns the same kind, so theory and smearing stay on the device.
 
 The 1D smearing never forms the dense n_calc x nq weight matrix: each
 measured q only sees the calculated points inside its +2.5/-3 sigma window
-(``resolution.py:206-216``), found here once by binary search, and the GPU
-forms the gaussian bin weights of that band on the fly
-(``csrc/resolution.cu``).  ``weight_matrix`` is still available for callers
+(``resolution.py:206-216``) or slit, found here once by binary search, and
+the GPU forms the weights of those bands once per object and applies them to
+every theory (``csrc/resolution.cu``).  ``weight_matrix`` is still available for callers
 that read it, built on the host on first access.
 """
 
@@ -57,6 +57,12 @@ def _lib():
         lib.sasb200_nllf_sets.argtypes = [I, I, P, L, P, P, P, P]
         lib.sasb200_nllf_sets.restype = I
         lib.sasb200_pinhole2d_average.restype = I
+        lib.sasb200_pinhole_weights.argtypes = [I] + [P]*9
+        lib.sasb200_pinhole_weights.restype = I
+        lib.sasb200_slit_weights.argtypes = [I, P, P, P, I] + [P]*8
+        lib.sasb200_slit_weights.restype = I
+        lib.sasb200_band_apply.argtypes = [I, I, I, P, P, P, P, P, P, L, P, L, P]
+        lib.sasb200_band_apply.restype = I
         lib.sasb200_resolution_last_error.restype = ct.c_char_p
         _LIB = lib
     return _LIB
@@ -155,6 +161,39 @@ def _device(device):
     return dev
 
 
+#: most weights that a resolution object keeps (256 MB); beyond it they are
+#: formed in every application
+MAX_WEIGHTS = 1 << 25
+
+
+def _band_plan(lo, hi, dev, form):
+    """Weights of the bands [lo, hi) on the device, formed once by *form*
+    (lo, hi, off, w, norm, stream), or None when they are too many.  Complete
+    on return, so that any stream may use them."""
+    import torch
+    off = np.hstack([0, np.cumsum(np.maximum(hi.astype(np.int64) - lo, 0))])
+    if off[-1] > MAX_WEIGHTS:
+        return None
+    n = len(lo)
+    index = np.concatenate([off[:-1].view(np.int32), lo, hi])
+    with torch.cuda.device(dev):
+        st = torch.cuda.current_stream(dev)
+        index = torch.as_tensor(index, device=dev)
+        weights = torch.empty(int(off[-1]) + n, dtype=torch.float64, device=dev)
+        plan = dict(hold=(index, weights), off=index.data_ptr(), lo=index[2*n:].data_ptr(),
+                    hi=index[3*n:].data_ptr(), norm=weights.data_ptr(),
+                    w=weights[n:].data_ptr())
+        form(plan["lo"], plan["hi"], plan["off"], plan["w"], plan["norm"], st.cuda_stream)
+        st.synchronize()
+    return plan
+
+
+def _band_apply(plan, n_sets, nq, n_calc, theory, stride, out, stream):
+    _check(_lib().sasb200_band_apply(
+        n_sets, nq, n_calc, plan["lo"], plan["hi"], plan["off"], plan["w"], plan["norm"],
+        theory.data_ptr(), stride, out.data_ptr(), nq, stream.cuda_stream), "band_apply")
+
+
 class Perfect1D:
     """No smearing (``resolution.py:52-63``)."""
 
@@ -201,12 +240,21 @@ class Pinhole1D:
     def _upload(self):
         if self._dev is None:
             import torch
-            d = dict(device=self.device)
-            self._dev = dict(
-                q=torch.as_tensor(np.ascontiguousarray(self.q, 'd'), **d),
-                width=torch.as_tensor(self._width, **d),
-                lo=torch.as_tensor(self.band_lo, **d), hi=torch.as_tensor(self.band_hi, **d),
-                edges=torch.as_tensor(self.edges, **d))
+            dev = self.device
+            d = dict(
+                q=torch.as_tensor(np.ascontiguousarray(self.q, 'd'), device=dev),
+                width=torch.as_tensor(self._width, device=dev),
+                edges=torch.as_tensor(self.edges, device=dev))
+
+            def form(lo, hi, off, w, norm, stream):
+                _check(_lib().sasb200_pinhole_weights(
+                    len(d["q"]), d["q"].data_ptr(), d["width"].data_ptr(), lo, hi, off,
+                    d["edges"].data_ptr(), w, norm, stream), "pinhole_weights")
+            d["plan"] = _band_plan(self.band_lo, self.band_hi, dev, form)
+            if d["plan"] is None:
+                d.update(lo=torch.as_tensor(self.band_lo, device=dev),
+                         hi=torch.as_tensor(self.band_hi, device=dev))
+            self._dev = d
         return self._dev
 
     def apply(self, theory, stream=None):
@@ -224,10 +272,13 @@ class Pinhole1D:
         st = stream if stream is not None else torch.cuda.current_stream(self.device)
         with torch.cuda.device(self.device), torch.cuda.stream(st):
             out = torch.empty(len(d["q"]), dtype=torch.float64, device=self.device)
-            _check(_lib().sasb200_pinhole_smear(
-                len(d["q"]), t.numel(), d["q"].data_ptr(), d["width"].data_ptr(),
-                d["lo"].data_ptr(), d["hi"].data_ptr(), d["edges"].data_ptr(), t.data_ptr(),
-                out.data_ptr(), st.cuda_stream), "pinhole_smear")
+            if d["plan"] is not None:
+                _band_apply(d["plan"], 1, len(d["q"]), t.numel(), t, t.numel(), out, st)
+            else:
+                _check(_lib().sasb200_pinhole_smear(
+                    len(d["q"]), t.numel(), d["q"].data_ptr(), d["width"].data_ptr(),
+                    d["lo"].data_ptr(), d["hi"].data_ptr(), d["edges"].data_ptr(), t.data_ptr(),
+                    out.data_ptr(), st.cuda_stream), "pinhole_smear")
         if on_device:
             return out
         st.synchronize()
@@ -244,11 +295,14 @@ class Pinhole1D:
         nq = len(d["q"])
         with torch.cuda.device(self.device), torch.cuda.stream(stream):
             out = torch.empty((n_sets, nq), dtype=torch.float64, device=self.device)
-            _check(_lib().sasb200_pinhole_smear_sets(
-                n_sets, nq, n_calc, d["q"].data_ptr(), d["width"].data_ptr(),
-                d["lo"].data_ptr(), d["hi"].data_ptr(), d["edges"].data_ptr(),
-                theory.data_ptr(), theory.stride(0), out.data_ptr(), nq, stream.cuda_stream),
-                "pinhole_smear_sets")
+            if d["plan"] is not None:
+                _band_apply(d["plan"], n_sets, nq, n_calc, theory, theory.stride(0), out, stream)
+            else:
+                _check(_lib().sasb200_pinhole_smear_sets(
+                    n_sets, nq, n_calc, d["q"].data_ptr(), d["width"].data_ptr(),
+                    d["lo"].data_ptr(), d["hi"].data_ptr(), d["edges"].data_ptr(),
+                    theory.data_ptr(), theory.stride(0), out.data_ptr(), nq, stream.cuda_stream),
+                    "pinhole_smear_sets")
         return out
 
     @property
@@ -305,6 +359,43 @@ class Slit1D:
     def device(self):
         return _device(self._device_arg)
 
+    def _bands(self):
+        """[lo, hi) of the bins that any step across the slit reaches: from the
+        last edge below the smallest |qk| to the first edge above the largest
+        limit sqrt(qk^2 + l^2); with neither length nor width, the points of
+        q_calc equal to q."""
+        q, w, l = self.q, self._width, self._length
+        k = np.arange(-self.N_LENGTH, self.N_LENGTH + 1)
+        qk = np.abs(q[:, None] + (k[None, :]*w[:, None])/self.N_LENGTH)
+        qc = self._signed_q_calc
+        first = np.maximum(np.searchsorted(self.edges, qk.min(1), side="left") - 1, 0)
+        top = qk.max(1)
+        last = np.minimum(np.searchsorted(self.edges, np.sqrt(top*top + l*l), side="right"),
+                          len(qc))
+        perfect = (w == 0) & (l == 0)
+        lo = np.where(perfect, np.searchsorted(qc, q, side="left"), first)
+        hi = np.where(perfect, np.searchsorted(qc, q, side="right"), last)
+        return lo.astype(np.int32), hi.astype(np.int32)
+
+    def _upload(self):
+        if self._dev is None:
+            import torch
+            dev = self.device
+            d = dict(q=torch.as_tensor(self.q, device=dev),
+                     w=torch.as_tensor(self._width, device=dev),
+                     l=torch.as_tensor(self._length, device=dev),
+                     qc=torch.as_tensor(np.ascontiguousarray(self._signed_q_calc), device=dev),
+                     e=torch.as_tensor(self.edges, device=dev))
+
+            def form(lo, hi, off, w, norm, stream):
+                _check(_lib().sasb200_slit_weights(
+                    len(self.q), d["q"].data_ptr(), d["w"].data_ptr(), d["l"].data_ptr(),
+                    self.N_LENGTH, d["qc"].data_ptr(), d["e"].data_ptr(), lo, hi, off, w, norm,
+                    stream), "slit_weights")
+            d["plan"] = _band_plan(*self._bands(), dev, form)
+            self._dev = d
+        return self._dev
+
     def apply(self, theory, stream=None):
         """Smeared I(q) from I(q_calc); CUDA tensor in -> CUDA tensor out,
         host array in -> host array out."""
@@ -315,20 +406,17 @@ class Slit1D:
         t = t.to(torch.float64).contiguous()
         if t.numel() != len(self.q_calc):
             raise ValueError("theory has %d points, q_calc %d" % (t.numel(), len(self.q_calc)))
-        if self._dev is None:
-            d = dict(device=self.device)
-            self._dev = dict(q=torch.as_tensor(self.q, **d), w=torch.as_tensor(self._width, **d),
-                             l=torch.as_tensor(self._length, **d),
-                             qc=torch.as_tensor(np.ascontiguousarray(self._signed_q_calc), **d),
-                             e=torch.as_tensor(self.edges, **d))
-        d = self._dev
+        d = self._upload()
         st = stream if stream is not None else torch.cuda.current_stream(self.device)
         with torch.cuda.device(self.device), torch.cuda.stream(st):
             out = torch.empty(len(self.q), dtype=torch.float64, device=self.device)
-            _check(_lib().sasb200_slit_smear(
-                len(self.q), t.numel(), d["q"].data_ptr(), d["w"].data_ptr(),
-                d["l"].data_ptr(), self.N_LENGTH, d["qc"].data_ptr(), d["e"].data_ptr(),
-                t.data_ptr(), out.data_ptr(), st.cuda_stream), "slit_smear")
+            if d["plan"] is not None:
+                _band_apply(d["plan"], 1, len(self.q), t.numel(), t, t.numel(), out, st)
+            else:
+                _check(_lib().sasb200_slit_smear(
+                    len(self.q), t.numel(), d["q"].data_ptr(), d["w"].data_ptr(),
+                    d["l"].data_ptr(), self.N_LENGTH, d["qc"].data_ptr(), d["e"].data_ptr(),
+                    t.data_ptr(), out.data_ptr(), st.cuda_stream), "slit_smear")
         if on_device:
             return out
         st.synchronize()

@@ -1,0 +1,84 @@
+"""
+The banded-weight plans of the resolution classes (csrc/resolution.cu:
+pinhole_weights, slit_weights, band_apply, band_apply_sets) against the dense-matrix oracle, at the edges of their tiles
+(8 and 32 q, 32 points, 64 and 128 curves) and of their dispatch rules.
+"""
+
+import numpy as np
+import pytest
+
+from oracle import resolution_ref
+
+
+def _grid(nq, shuffle=False):
+    q = np.linspace(0.01, 0.3, nq) if nq > 1 else np.array([0.05])
+    qc = np.linspace(0.004, 0.4, 3*nq + 40)
+    if shuffle:
+        np.random.default_rng(1).shuffle(q)
+    return q, qc
+
+
+@pytest.mark.parametrize("length, width", [(0.05, 0.0), (0.05, 0.004), (0.02, 0.05)])
+def test_slit_bands_hold_the_matrix(length, width):
+    """The host's bands hold every nonzero weight of the dense slit matrix."""
+    from sasmodels_b200.resolution import Slit1D
+    q, qc = _grid(60)
+    r = Slit1D(q, q_length=length, q_width=width, q_calc=qc)
+    W = resolution_ref.slit_matrix(r._signed_q_calc, q, r._length, r._width)
+    lo, hi = r._bands()
+    for i in range(len(q)):
+        nz = np.flatnonzero(W[:, i])
+        assert nz[0] >= lo[i] and nz[-1] < hi[i]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nq, sets, shuffle", [(1, 1, False), (31, 3, False), (33, 64, True),
+                                               (200, 129, False), (257, 400, False),
+                                               (700, 65, True), (1000, 1300, False)])
+def test_band_apply_matches_matrix(cuda, nq, sets, shuffle):
+    """One curve, few and many, against the dense matrix (the 1e-12 bar of the
+    smearing tests), with rows of theory wider than the grid."""
+    import torch
+    from sasmodels_b200.resolution import Pinhole1D
+    q, qc = _grid(nq, shuffle)
+    r = Pinhole1D(q, 0.05*q, q_calc=qc)
+    rng = np.random.default_rng(nq)
+    th = rng.uniform(0.5, 2.0, (sets, len(qc) + 3))
+    dev = torch.as_tensor(th, device="cuda")[:, :len(qc)]
+    out = r.apply_sets(dev, torch.cuda.current_stream()).cpu().numpy()
+    want = th[:, :len(qc)] @ r.weight_matrix
+    np.testing.assert_allclose(out, want, rtol=1e-12, atol=0)
+    one = r.apply(dev[0].contiguous()).cpu().numpy()
+    np.testing.assert_allclose(one, want[0], rtol=1e-12, atol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sets", [1, 700])
+def test_infinite_theory_reaches_only_its_bands(cuda, sets):
+    """A point where a model is undefined spoils the q that see it, no other."""
+    import torch
+    from sasmodels_b200.resolution import Pinhole1D
+    q, qc = _grid(200)
+    r = Pinhole1D(q, 0.05*q, q_calc=qc)
+    at = len(qc)//2
+    th = torch.ones((sets, len(qc)), dtype=torch.float64, device="cuda")
+    th[:, at] = float("inf")
+    out = r.apply_sets(th, torch.cuda.current_stream()).cpu().numpy()
+    sees = (r.band_lo <= at) & (at < r.band_hi)
+    assert sees.any() and not sees.all()
+    assert (np.isfinite(out) == ~sees[None, :]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length, width", [(0.05, 0.0), (0.05, 0.004), (0.0, 0.0)])
+@pytest.mark.parametrize("nq", [2, 31, 250])
+def test_slit_plan_matches_formed_weights(cuda, monkeypatch, nq, length, width):
+    """The plan against the kernel that forms the weights in every call."""
+    from sasmodels_b200 import resolution as R
+    q, qc = _grid(nq)
+    qc = np.union1d(q, qc)
+    th = np.random.default_rng(3).uniform(0.5, 2.0, len(qc))
+    a = R.Slit1D(q, q_length=length, q_width=width, q_calc=qc).apply(th)
+    monkeypatch.setattr(R, "MAX_WEIGHTS", -1)
+    b = R.Slit1D(q, q_length=length, q_width=width, q_calc=qc).apply(th)
+    np.testing.assert_allclose(a, b, rtol=1e-12, atol=0)
