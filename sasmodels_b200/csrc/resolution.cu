@@ -39,6 +39,11 @@ constexpr unsigned FULL = 0xffffffffu;
 // band_apply_sets: 181 q x 61 curves 3.8 against 6.2 us and 400 x 61 5.7 against
 // 6.6, but 181 x 200 7.3 against 6.3 and 1000 x 61 12.1 against 8.4.
 constexpr long long BAND_WARP_LIMIT = 28000;
+
+// nllf_sets (a block per curve) up to this many curves, then nllf_rows: 800
+// curves of 1000 points 4.3 against 6.2 us, 1600 of 1000 6.8 against 6.7, 1600
+// of 400 4.8 against 3.9, 4096 of 1000 14.3 against 8.6.
+constexpr int NLLF_BLOCKS = 1200;
 constexpr double SQRT2 = 1.4142135623730951;     // numpy sqrt(2.0), correctly rounded
 
 // One curve per blockIdx.y: theory + y*theory_stride -> out + y*out_stride.
@@ -435,6 +440,49 @@ nllf_sets(int nq, const double *__restrict__ theory, size_t theory_stride,
     if (threadIdx.x == 0) out[blockIdx.x] = 0.5*red[0];
 }
 
+// The same for many curves: a warp per curve, eight curves per block sharing y,
+// dy and 1/dy of 256 points in shared memory, so the block divides once per
+// point instead of once per (curve, point); each lane's 8 theory values are on
+// their way meanwhile.
+constexpr int NL_POINTS = 256, NL_CURVES = 8;
+__global__ void __launch_bounds__(32*NL_CURVES)
+nllf_rows(int n_sets, int nq, const double *__restrict__ theory, size_t theory_stride,
+          const double *__restrict__ y, const double *__restrict__ dy, double *__restrict__ out)
+{
+    __shared__ double sy[NL_POINTS], sd[NL_POINTS], sr[NL_POINTS];
+    const int t = threadIdx.x, lane = t & 31;
+    const int s = blockIdx.x*NL_CURVES + (t >> 5);
+    const double *th = theory + (size_t)min(s, n_sets - 1)*theory_stride;
+    double acc = 0.0;
+    for (int i0 = 0; i0 < nq; i0 += NL_POINTS) {
+        const int n = min(NL_POINTS, nq - i0);
+        // this lane's points of the curve, on their way while y and dy are staged
+        double x[NL_POINTS/32];
+        #pragma unroll
+        for (int k = 0; k < NL_POINTS/32; ++k)
+            x[k] = 32*k + lane < n ? th[i0 + 32*k + lane] : 0.0;
+        __syncthreads();
+        for (int i = t; i < n; i += 32*NL_CURVES) {
+            const double d = dy[i0 + i];
+            sy[i] = y[i0 + i];
+            sd[i] = d;
+            sr[i] = sr_of(d);
+        }
+        __syncthreads();
+        #pragma unroll
+        for (int k = 0; k < NL_POINTS/32; ++k) {
+            const int i = 32*k + lane;
+            if (i < n) {
+                const double z = quotient(x[k] - sy[i], sd[i], sr[i]);
+                acc += z*z;
+            }
+        }
+    }
+    #pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
+    if (lane == 0 && s < n_sets) out[s] = 0.5*acc;
+}
+
 inline char *errbuf()
 {
     static thread_local char buf[256] = "";
@@ -567,8 +615,14 @@ int32_t sasb200_nllf_sets(int32_t n_sets, int32_t nq, const double *theory,
         || (n_sets > 0 && (!theory || !y || !dy || !out)))
         return (std::snprintf(res::errbuf(), 256, "bad arguments"), -1);
     if (n_sets == 0) return 0;
-    res::nllf_sets<<<n_sets, 256, 0, (cudaStream_t)stream>>>(nq, theory, (size_t)theory_stride,
-                                                              y, dy, out);
+    if (n_sets > res::NLLF_BLOCKS)
+        res::nllf_rows<<<(n_sets + res::NL_CURVES - 1)/res::NL_CURVES, 32*res::NL_CURVES, 0,
+                         (cudaStream_t)stream>>>(n_sets, nq, theory, (size_t)theory_stride, y, dy,
+                                                 out);
+    else
+        res::nllf_sets<<<n_sets, 256, 0, (cudaStream_t)stream>>>(nq, theory,
+                                                                  (size_t)theory_stride, y, dy,
+                                                                  out);
     return res::status("nllf_sets");
 }
 

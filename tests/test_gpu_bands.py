@@ -1,6 +1,7 @@
 """
 The banded-weight plans of the resolution classes (csrc/resolution.cu:
-pinhole_weights, slit_weights, band_apply, band_apply_sets) against the dense-matrix oracle, at the edges of their tiles
+pinhole_weights, slit_weights, band_apply, band_apply_sets) and the
+many-curve nllf against the dense-matrix oracle, at the edges of their tiles
 (8 and 32 q, 32 points, 64 and 128 curves) and of their dispatch rules.
 """
 
@@ -82,3 +83,24 @@ def test_slit_plan_matches_formed_weights(cuda, monkeypatch, nq, length, width):
     monkeypatch.setattr(R, "MAX_WEIGHTS", -1)
     b = R.Slit1D(q, q_length=length, q_width=width, q_calc=qc).apply(th)
     np.testing.assert_allclose(a, b, rtol=1e-12, atol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nq", [1, 511, 513, 1000])
+@pytest.mark.parametrize("sets", [1, 4097])
+def test_nllf_matches_numpy(cuda, nq, sets):
+    """One curve and many; points of dy where 1/dy is not a normal number
+    (their terms vanish) and an infinite theory value."""
+    import torch
+    from sasmodels_b200.resolution import nllf_sets
+    rng = np.random.default_rng(nq)
+    th = rng.uniform(0.5, 2.0, (sets, nq))
+    y, dy = rng.uniform(0.5, 2.0, nq), rng.uniform(0.01, 0.1, nq)
+    dy[::7] = 1e300
+    th[-1, nq//2] = np.inf
+    dy[nq//2] = 0.5
+    got = nllf_sets(torch.as_tensor(th, device="cuda"), y, dy,
+                    torch.cuda.current_stream()).cpu().numpy()
+    want = 0.5*np.sum(((th - y)/dy)**2, axis=1)
+    assert np.isinf(got[-1])
+    np.testing.assert_allclose(got[:-1], want[:-1], rtol=1e-12, atol=0)
