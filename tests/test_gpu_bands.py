@@ -104,3 +104,23 @@ def test_nllf_matches_numpy(cuda, nq, sets):
     want = 0.5*np.sum(((th - y)/dy)**2, axis=1)
     assert np.isinf(got[-1])
     np.testing.assert_allclose(got[:-1], want[:-1], rtol=1e-12, atol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nbins", [1, 7, 8, 9, 40, 48, 200])
+@pytest.mark.parametrize("nq", [1, 63, 65, 4097])
+def test_pinhole2d_average_keeps_the_order(cuda, nq, nbins):
+    """The 2D average is numpy's axis-0 reduction bit for bit."""
+    import torch
+    from sasmodels_b200.resolution import _check, _lib
+    rng = np.random.default_rng(nbins)
+    th, w = rng.uniform(-1, 2, (nbins, nq)), rng.uniform(0.1, 1.0, nbins)
+    d = [torch.as_tensor(a, device="cuda") for a in (th, w)]
+    out = torch.empty(nq, dtype=torch.float64, device="cuda")
+    _check(_lib().sasb200_pinhole2d_average(nq, nbins, d[0].data_ptr(), d[1].data_ptr(), 3.0,
+                                            out.data_ptr(),
+                                            torch.cuda.current_stream().cuda_stream), "average")
+    num = th[0]*w[0]
+    for b in range(1, nbins):
+        num = num + th[b]*w[b]
+    np.testing.assert_array_equal(out.cpu().numpy(), num/3.0)
