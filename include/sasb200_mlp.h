@@ -90,6 +90,30 @@ int32_t sasb200_adam(int32_t size, int32_t splits, const float *grad, float *p, 
                      float *v, float lr, float b1, float b2, float eps, int32_t step, void *w,
                      void *wt, int32_t rows, int32_t cols, void *stream);
 
+/* a training step on tiled planes, [4 layers][n_pad/128 tiles][32 groups][128
+ * rows][8] bf16 (group g holds columns 8g .. 8g + 7): the forward with the loss
+ * gradient dout[n_pad] of the mean Huber loss (delta <= 0: squared error)
+ * against y[n] and row_sums[2][n_pad/32] (loss and dout summed over 32 rows
+ * each); the backward from dout; every gradient as partial sums over splits of
+ * the rows (dw[l]: [splits][256 x (16 or 256)], db: [4][splits][256], dw_out:
+ * [splits][256]), the mean loss and db_out as scalars; and outs[k][i] = sum of
+ * parts[k][s*sizes[k] + i] over s for n <= 16 tensors (host arrays). */
+int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const void *x_lo,
+                                  const void *img, const float *const *b, const float *w_out,
+                                  const float *b_out, const float *y, float delta, float *out,
+                                  float *dout, float *row_sums, void *z, void *h, int32_t *err,
+                                  void *stream);
+int32_t sasb200_mlp_train_backward(int32_t n_pad, const void *img_t, const float *w_out,
+                                   const float *dout, const void *z, void *dz, int32_t *err,
+                                   void *stream);
+int32_t sasb200_mlp_weight_grads(int32_t n, int32_t n_pad, int32_t splits, const void *x,
+                                 const void *h, const void *dz, const float *dout,
+                                 const float *row_sums, float *const *dw, float *db,
+                                 float *dw_out, float *loss, float *db_out, int32_t *err,
+                                 void *stream);
+int32_t sasb200_sum_partials(int32_t n, const int32_t *sizes, const int32_t *splits,
+                             const float *const *parts, float *const *outs, void *stream);
+
 /* the learning rate and Adam bias corrections of a training step, on the
  * device: counters = {schedule step s, Adam step count t} (int32), sched =
  * {lr, 1 - b1^t, 1 - b2^t} with lr = lr0 min(1, (s + 1)/warmup)

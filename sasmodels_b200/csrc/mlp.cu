@@ -23,10 +23,10 @@
 //   mlp_serve      the forward with the tensor core and the epilogue working
 //                  at once (a dedicated MMA warp, two TMEM accumulators,
 //                  layer l+1's MMAs under layer l's epilogue chunk by chunk);
-//                  serves inference and, with the planes, the training
-//                  forward.
-//   gemm_nt        C_split = A[M x K] B[N x K]^T over a K range (split-K):
-//                  weight gradients dW = dZ^T H with the batch as K.
+//                  serves inference and the training forward.
+//   mlp_backward_t, mlp_weight_grads   the training step's backward and weight
+//                  gradients on tiled planes (mlp_train.cuh).
+//   gemm_nt        C_split = A[M x K] B[N x K]^T over a K range (split-K).
 //   + transpose, column sums (bias gradients), loss gradient, the learning
 //     rate schedule, Adam (one tensor, or every tensor in one launch),
 //     feature packing.
@@ -507,14 +507,8 @@ __global__ void col_sum_final(int nparts, int cols, const float *__restrict__ pa
 // per-row loss: squared error for delta <= 0, else Huber with threshold
 // delta (quadratic inside, linear outside), which keeps the few points
 // near form-factor minima from dominating the fit.
-__global__ void loss_grad(int n, int n_pad, const float *__restrict__ out,
-                          const float *__restrict__ y, float delta, float *__restrict__ dout,
-                          float *__restrict__ loss)
+__device__ __forceinline__ void loss_of(float d, float delta, float &g, float &l)
 {
-    const int i = blockIdx.x*blockDim.x + threadIdx.x;
-    if (i >= n_pad) return;
-    const float d = i < n ? out[i] - y[i] : 0.0f;
-    float g, l;
     if (delta <= 0.0f || fabsf(d) <= delta) {
         g = 2.0f*d;
         l = d*d;
@@ -522,6 +516,16 @@ __global__ void loss_grad(int n, int n_pad, const float *__restrict__ out,
         g = 2.0f*delta*copysignf(1.0f, d);
         l = delta*(2.0f*fabsf(d) - delta);
     }
+}
+
+__global__ void loss_grad(int n, int n_pad, const float *__restrict__ out,
+                          const float *__restrict__ y, float delta, float *__restrict__ dout,
+                          float *__restrict__ loss)
+{
+    const int i = blockIdx.x*blockDim.x + threadIdx.x;
+    if (i >= n_pad) return;
+    float g, l;
+    loss_of(i < n ? out[i] - y[i] : 0.0f, delta, g, l);
     dout[i] = i < n ? g/(float)n : 0.0f;
     loss[i] = l;
 }
@@ -701,6 +705,11 @@ struct InferParams {
     const float *b_out;
     __nv_bfloat16 *z_save;        // optional [4][n_pad x 256] pre-activations (training)
     __nv_bfloat16 *h_save;        // optional [4][n_pad x 256] activations (training)
+    // training step (tiled planes): targets, Huber threshold, the loss gradient
+    // [n_pad], and [2][4 n_tiles] sums over 32 rows of the loss and of dout
+    const float *y;
+    float delta;
+    float *dout, *row_sums;
 };
 
 // W_l [out][in] bf16 -> the chunk image: W0 as one 256 x 16 canonical tile,
@@ -923,6 +932,24 @@ mlp_infer(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
     if (warp == 0) tc::tmem_dealloc(tmem, HID);
 }
 
+// -------------------------------------------------------- training planes --
+// The pre-activations z, the activations h and the gradients dZ of a
+// training step live in tiled planes [4 layers][n_tiles][32 groups][128 rows][8]
+// bf16: the 128 x 256 tile of a CTA is one 64 KB image, the 8 columns of a group
+// 16 contiguous bytes per row.  A warp whose lanes hold consecutive rows reads
+// and writes 512 contiguous bytes (of row-major planes 32 separate 16-byte
+// pieces: the forward of 8192 rows took 50 us with them and takes 28), and the
+// image is at the same time the canonical MN-major operand of dW = dZ^T H, whose
+// K dimension is the rows, so nothing is transposed on the way.
+constexpr int TILE_ELEMS = TM*HID;
+constexpr int GROUP_ELEMS = TM*8;
+
+// Element of a tiled plane: tile `tile` of layer `l`, column group kg, row.
+__device__ __forceinline__ size_t tiled_at(int l, int n_tiles, int tile, int kg, int row)
+{
+    return ((size_t)l*n_tiles + tile)*TILE_ELEMS + (size_t)kg*GROUP_ELEMS + 8*row;
+}
+
 // ------------------------------------------------------------------ serve --
 // mlp_serve: the forward pass (inference, or training with the z/h planes)
 // with the tensor core and the epilogue busy at the same time.  Arithmetic per element as mlp_infer
@@ -1005,7 +1032,10 @@ __device__ __forceinline__ void save8(__nv_bfloat16 *dst, const float (&v)[8])
     *reinterpret_cast<uint4 *>(dst) = u;
 }
 
-template <int RND>
+// PLANES: none (inference), row-major z/h planes, or a training step's tiled
+// planes with the loss gradient of every row.
+enum { PLANES_NONE, PLANES_ROWS, PLANES_TILED };
+template <int RND, int PLANES>
 __global__ void __launch_bounds__(SV_THREADS, 1)
 mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
           const __nv_bfloat16 *__restrict__ x_lo, InferParams prm, float *__restrict__ out,
@@ -1222,9 +1252,10 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                         const int c = RND*j + r;
                         float z[8], h[8];
                         sv_silu8(ra[r], bias + KCI*c, z, h);
-                        if (prm.z_save != nullptr) {   // training: the planes of every layer
-                            const size_t at = (size_t)l*plane + (size_t)(row0 + row)*HID
-                                            + KCI*c + cs;
+                        if (PLANES != PLANES_NONE) {   // the planes of every layer
+                            const size_t at = PLANES == PLANES_TILED
+                                ? tiled_at(l, n_tiles, row0/TM, 4*c + slot, row)
+                                : (size_t)l*plane + (size_t)(row0 + row)*HID + KCI*c + cs;
                             save8(prm.z_save + at, z);
                             save8(prm.h_save + at, h);
                         }
@@ -1278,9 +1309,26 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                     } else {
                         if (!(ok = warp_wait(&dot_bar[quad], (uint32_t)(k & 1))))
                             break;
-                        if (row0 + row < n)
-                            out[row0 + row] = ((dot + dot_part[0][row]) + dot_part[1][row])
-                                              + dot_part[2][row] + b_out;
+                        const bool valid = row0 + row < n;
+                        const float o = ((dot + dot_part[0][row]) + dot_part[1][row])
+                                        + dot_part[2][row] + b_out;
+                        if (valid) out[row0 + row] = o;
+                        if (PLANES == PLANES_TILED) {
+                            float g, loss;
+                            loss_of(valid ? o - prm.y[row0 + row] : 0.0f, prm.delta, g, loss);
+                            g = valid ? g/(float)n : 0.0f;
+                            prm.dout[row0 + row] = g;
+                            #pragma unroll
+                            for (int o2 = 16; o2 > 0; o2 >>= 1) {
+                                g += __shfl_xor_sync(0xffffffffu, g, o2);
+                                loss += __shfl_xor_sync(0xffffffffu, loss, o2);
+                            }
+                            if (lane == 0) {
+                                float *sums = prm.row_sums + 4*(row0/TM) + quad;
+                                sums[0] = loss;
+                                sums[4*n_tiles] = g;
+                            }
+                        }
                     }
                 }
             }
@@ -1291,6 +1339,8 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, 2*HID);
 }
+
+#include "mlp_train.cuh"
 
 // ---------------------------------------------------------------- backward --
 // mlp_backward_p: the backward pass through the three 256 x 256 layers as a
@@ -1588,11 +1638,142 @@ int32_t sasb200_mlp_serve(int32_t n, int32_t n_pad, const void *x, const void *x
         blocks = sms > 0 ? sms : 1;
     }
     if (blocks > n_tiles) blocks = n_tiles;
-    cudaFuncSetAttribute(mlp_serve<SV_ROUND>, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
-    mlp_serve<SV_ROUND><<<blocks, SV_THREADS, SV_SMEM, (cudaStream_t)stream>>>(
+    const auto kernel = z_save ? mlp_serve<SV_ROUND, PLANES_ROWS> : mlp_serve<SV_ROUND, PLANES_NONE>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
+    kernel<<<blocks, SV_THREADS, SV_SMEM, (cudaStream_t)stream>>>(
         n, n_tiles, static_cast<const __nv_bfloat16 *>(x),
         static_cast<const __nv_bfloat16 *>(x_lo), prm, out, err);
     return status("mlp_serve");
+}
+
+// One CTA per SM, or per tile where there are fewer.
+static int tile_blocks(int n_tiles)
+{
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return n_tiles < sms || sms <= 0 ? n_tiles : sms;
+}
+
+// The forward of a training step: out[n] as sasb200_mlp_serve, the tiled z and
+// h planes ([4][n_pad x 256] bf16 each), dout[n_pad] of the mean Huber loss
+// (threshold delta; squared error for delta <= 0) against y[n], 0 on padding,
+// and row_sums[2][n_pad/32]: the loss and dout summed over 32 rows each.
+int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const void *x_lo,
+                                  const void *img, const float *const *b, const float *w_out,
+                                  const float *b_out, const float *y, float delta, float *out,
+                                  float *dout, float *row_sums, void *z, void *h, int32_t *err,
+                                  void *stream)
+{
+    errbuf()[0] = 0;
+    if (n < 0 || n_pad % TM || n > n_pad || !x || !x_lo || !img || !b || !w_out || !b_out || !y
+        || !out || !dout || !row_sums || !z || !h || !err)
+        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
+    if (reinterpret_cast<uintptr_t>(img) % 16)
+        return (std::snprintf(errbuf(), 256, "weight image must be 16-byte aligned"), -1);
+    InferParams prm = {};
+    prm.img = static_cast<const uint8_t *>(img);
+    for (int l = 0; l < 4; ++l) {
+        if (!b[l]) return (std::snprintf(errbuf(), 256, "bad bias pointer"), -1);
+        prm.b[l] = b[l];
+    }
+    if (n_pad == 0) return 0;
+    prm.w_out = w_out;
+    prm.b_out = b_out;
+    prm.z_save = static_cast<__nv_bfloat16 *>(z);
+    prm.h_save = static_cast<__nv_bfloat16 *>(h);
+    prm.y = y;
+    prm.delta = delta;
+    prm.dout = dout;
+    prm.row_sums = row_sums;
+    const int n_tiles = n_pad/TM;
+    const auto kernel = mlp_serve<SV_ROUND, PLANES_TILED>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
+    kernel<<<tile_blocks(n_tiles), SV_THREADS, SV_SMEM, (cudaStream_t)stream>>>(
+        n, n_tiles, static_cast<const __nv_bfloat16 *>(x),
+        static_cast<const __nv_bfloat16 *>(x_lo), prm, out, err);
+    return status("mlp_train_forward");
+}
+
+// The backward of a training step: tiled dZ planes from dout[n_pad] and the
+// tiled z planes.
+int32_t sasb200_mlp_train_backward(int32_t n_pad, const void *img_t, const float *w_out,
+                                   const float *dout, const void *z, void *dz, int32_t *err,
+                                   void *stream)
+{
+    errbuf()[0] = 0;
+    if (n_pad < 0 || n_pad % TM || !img_t || !w_out || !dout || !z || !dz || !err)
+        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
+    if (reinterpret_cast<uintptr_t>(img_t) % 16 || reinterpret_cast<uintptr_t>(w_out) % 16)
+        return (std::snprintf(errbuf(), 256, "weights must be 16-byte aligned"), -1);
+    if (n_pad == 0) return 0;
+    const int n_tiles = n_pad/TM;
+    cudaFuncSetAttribute(mlp_backward_t, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM);
+    mlp_backward_t<<<tile_blocks(n_tiles), SV_THREADS, BT_SMEM, (cudaStream_t)stream>>>(
+        n_tiles, static_cast<const uint8_t *>(img_t), w_out, dout,
+        static_cast<const __nv_bfloat16 *>(z), static_cast<__nv_bfloat16 *>(dz), err);
+    return status("mlp_train_backward");
+}
+
+// Every gradient of a training step from its planes: dw[0..3] [splits][256 x (16
+// or 256)], db [4][splits][256] and dw_out [splits][256] as partial sums over
+// splits of the rows; the mean loss over n rows and db_out as scalars.
+int32_t sasb200_mlp_weight_grads(int32_t n, int32_t n_pad, int32_t splits, const void *x,
+                                 const void *h, const void *dz, const float *dout,
+                                 const float *row_sums, float *const *dw, float *db,
+                                 float *dw_out, float *loss, float *db_out, int32_t *err,
+                                 void *stream)
+{
+    errbuf()[0] = 0;
+    if (n < 0 || n > n_pad || n_pad <= 0 || n_pad % TM || splits <= 0 || splits > 4096 || !x || !h
+        || !dz || !dout || !row_sums || !dw || !db || !dw_out || !loss || !db_out || !err)
+        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
+    if ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(dz)
+         | reinterpret_cast<uintptr_t>(x)) % 16)
+        return (std::snprintf(errbuf(), 256, "planes must be 16-byte aligned"), -1);
+    WeightGrads prm;
+    prm.x = static_cast<const __nv_bfloat16 *>(x);
+    prm.h = static_cast<const __nv_bfloat16 *>(h);
+    prm.dz = static_cast<const __nv_bfloat16 *>(dz);
+    prm.dout = dout;
+    prm.row_sums = row_sums;
+    for (int l = 0; l < 4; ++l) {
+        if (!dw[l] || reinterpret_cast<uintptr_t>(dw[l]) % 16)
+            return (std::snprintf(errbuf(), 256, "bad gradient pointer"), -1);
+        prm.dw[l] = dw[l];
+    }
+    prm.db = db;
+    prm.dw_out = dw_out;
+    prm.loss = loss;
+    prm.db_out = db_out;
+    prm.n = (float)n;
+    cudaFuncSetAttribute(mlp_weight_grads, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
+    mlp_weight_grads<<<(WG_BIG + 2)*splits, WG_THREADS, WG_SMEM, (cudaStream_t)stream>>>(
+        n_pad/TM, splits, prm, err);
+    return status("mlp_weight_grads");
+}
+
+// outs[k][i] = sum over s < splits[k] of parts[k][s*sizes[k] + i] for n (<= 16)
+// tensors (host arrays of device pointers).
+int32_t sasb200_sum_partials(int32_t n, const int32_t *sizes, const int32_t *splits,
+                             const float *const *parts, float *const *outs, void *stream)
+{
+    errbuf()[0] = 0;
+    if (n <= 0 || n > SUM_TENSORS || !sizes || !splits || !parts || !outs)
+        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
+    SumTensors T = {};
+    int most = 0;
+    for (int k = 0; k < n; ++k) {
+        if (sizes[k] <= 0 || splits[k] <= 0 || !parts[k] || !outs[k])
+            return (std::snprintf(errbuf(), 256, "bad tensor"), -1);
+        T.size[k] = sizes[k];
+        T.splits[k] = splits[k];
+        T.part[k] = parts[k];
+        T.out[k] = outs[k];
+        most = sizes[k] > most ? sizes[k] : most;
+    }
+    sum_partials<<<dim3((most + 255)/256, n), 256, 0, (cudaStream_t)stream>>>(T);
+    return status("sum_partials");
 }
 
 // out[n] (and z/h planes [4][n_pad x 256] when non-null) for x[n_pad x 16];

@@ -1,0 +1,476 @@
+// The training step's kernels after the forward: the backward pass, the weight
+// gradients and their reduction.  Included by mlp.cu.
+#pragma once
+
+// Sum over the 32 lanes of each of a lane's 8 values in 9 shuffles: halves of
+// the set are exchanged while the set shrinks to one value per lane.  Lane L
+// returns the sum of value L/4 (every fourth lane's is the one to use).
+__device__ __forceinline__ float warp_sum8(float (&v)[8], int lane)
+{
+    #pragma unroll
+    for (int half = 4; half >= 1; half >>= 1) {
+        const bool up = (lane & (4*half)) != 0;
+        #pragma unroll
+        for (int j = 0; j < half; ++j) {
+            const float mine = up ? v[j + half] : v[j], other = up ? v[j] : v[j + half];
+            v[j] = mine + __shfl_xor_sync(0xffffffffu, other, 4*half);
+        }
+    }
+    float s = v[0];
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    return s;
+}
+
+// ---------------------------------------------------------------- backward --
+// mlp_backward_t: dZ3 = dout w_out silu'(z3), then dZ(l-1) = (dZl W_l)
+// silu'(z(l-1)) for l = 3, 2, 1, from tiled z to tiled dZ planes; the values of
+// mlp_backward.  Built as mlp_serve: sixteen epilogue warps (quadrant w % 4, 8
+// columns of every 32-column chunk at 8(w / 4)), one MMA warp, a bulk-copy
+// producer and a waiter, two TMEM accumulators, so that the MMAs of the next
+// layer start on the first chunk while the epilogue works on the last.  A
+// training batch of 8192 rows is one tile for 64 CTAs, so the kernel is bound by
+// the latency of one tile's chain: the ring holds a whole layer of weights
+// (fetched while dZ3 forms), and each warp loads the z of its eight chunks one
+// layer ahead.  8192 rows: 18.5 us (mlp_backward_p 38 us).
+constexpr int BT_STAGES = 8;
+constexpr int BT_SMEM = ACT_BYTES + BT_STAGES*CHUNK_BYTES;
+
+__global__ void __launch_bounds__(SV_THREADS, 1)
+mlp_backward_t(int n_tiles, const uint8_t *__restrict__ img_t, const float *__restrict__ w_out,
+               const float *__restrict__ dout, const __nv_bfloat16 *__restrict__ z_save,
+               __nv_bfloat16 *__restrict__ dz_save, int *__restrict__ err)
+{
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t *act = smem;
+    uint8_t *ring = smem + ACT_BYTES;
+    __shared__ __align__(8) uint64_t full[BT_STAGES], empty[BT_STAGES];
+    __shared__ __align__(8) uint64_t act_ready[CHUNKS_PER_LAYER], acc_full[2], acc_empty[2], drain;
+    __shared__ uint32_t tmem_slot, ready_seq;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int my_tiles = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x)/gridDim.x + 1 : 0;
+
+    if (warp == 0) {
+        tc::tmem_alloc(&tmem_slot, 2*HID);
+        tc::tmem_relinquish();
+    }
+    if (t == 0) {
+        for (int s = 0; s < BT_STAGES; ++s) {
+            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&empty[s], 1);
+        }
+        for (int c = 0; c < CHUNKS_PER_LAYER; ++c) tc::mbar_init(&act_ready[c], SV_EPI_WARPS);
+        for (int a = 0; a < 2; ++a) {
+            tc::mbar_init(&acc_full[a], 1);
+            tc::mbar_init(&acc_empty[a], SV_EPI_WARPS);
+        }
+        tc::mbar_init(&drain, 1);
+        ready_seq = 0;
+        tc::mbar_fence_init();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == SV_PROD_WARP) {
+        if (lane == 0) {
+            bool ok = true;
+            const int total = my_tiles*CHUNKS_PER_TILE;
+            int i = 0;
+            for (; i < total; ++i) {
+                const int s = i % BT_STAGES, use = i/BT_STAGES;
+                if (use > 0 && !tc::mbar_wait(&empty[s], (uint32_t)((use - 1) & 1))) {
+                    ok = false;
+                    break;
+                }
+                tc::mbar_arrive_expect_tx(&full[s], CHUNK_BYTES);
+                tc::bulk_load(ring + s*CHUNK_BYTES,
+                              img_t + (size_t)(i % CHUNKS_PER_TILE)*CHUNK_BYTES,
+                              CHUNK_BYTES, &full[s]);
+            }
+            for (int j = (i > BT_STAGES ? i - BT_STAGES : 0); j < i; ++j)
+                ok = tc::mbar_wait(&full[j % BT_STAGES], (uint32_t)((j/BT_STAGES) & 1)) && ok;
+            if (!ok) atomicExch(err, 2);
+        }
+    } else if (warp == SV_WAIT_WARP) {
+        // step g = 3 k + s accumulates in acc[g & 1]; its previous reader is the
+        // epilogue of step g - 2 (completion (g - 2)/2 of acc_empty), and the
+        // inputs of its chunks are completion g of act_ready.  No barrier can
+        // run two phases ahead: each next completion needs what is published
+        // here first.
+        bool ok = true;
+        int chunk = 0;
+        for (int g = 0; g < 3*my_tiles && ok; ++g) {
+            if (g >= 2 && !(ok = warp_wait(&acc_empty[g & 1], (uint32_t)(((g - 2) >> 1) & 1))))
+                break;
+            for (int c = 0; c < CHUNKS_PER_LAYER; ++c, ++chunk) {
+                if (!(ok = warp_wait(&act_ready[c], (uint32_t)(g & 1))
+                           && warp_wait(&full[chunk % BT_STAGES],
+                                        (uint32_t)((chunk/BT_STAGES) & 1))))
+                    break;
+                if (lane == 0) tc::st_release_shared(&ready_seq, (uint32_t)(chunk + 1));
+            }
+        }
+        if (!ok && lane == 0) atomicExch(err, 4);
+    } else if (warp == SV_MMA_WARP) {
+        bool ok = true;
+        if (lane == 0) {
+            constexpr uint32_t idesc = tc::idesc_bf16(TM, HID);
+            const uint32_t a_addr = tc::smem_u32(act);
+            int chunk = 0;
+            for (int g = 0; g < 3*my_tiles && ok; ++g) {
+                const uint32_t d = tmem + (uint32_t)(HID*(g & 1));
+                for (int c = 0; c < CHUNKS_PER_LAYER; ++c, ++chunk) {
+                    if (!(ok = tc::spin_acquire_ge(&ready_seq, (uint32_t)(chunk + 1)))) break;
+                    tc::fence_after_sync();
+                    const int s = chunk % BT_STAGES;
+                    const uint32_t b_addr = tc::smem_u32(ring + s*CHUNK_BYTES);
+                    #pragma unroll
+                    for (int st = 0; st < KCI/16; ++st)
+                        tc::mma_bf16(d, tc::kmajor_desc<TM>(a_addr, c*(KCI/16) + st),
+                                     tc::kmajor_desc<HID>(b_addr, st), idesc,
+                                     (c > 0 || st > 0) ? 1u : 0u);
+                    tc::mma_commit(&empty[s]);
+                }
+                if (ok) tc::mma_commit(&acc_full[g & 1]);
+            }
+            // every MMA issued has completed before TMEM is released
+            tc::mma_commit(&drain);
+            ok = tc::mbar_wait(&drain, 0u) && ok;
+            if (!ok) atomicExch(err, 3);
+        }
+        __syncwarp();
+    } else {
+        const int quad = warp & 3, slot = warp >> 2;
+        const int row = 32*quad + lane;
+        const uint32_t lane_base = (uint32_t)(32*quad) << 16;
+        bool ok = true;
+        for (int k = 0; k < my_tiles && ok; ++k) {
+            const int tile = blockIdx.x + k*gridDim.x;
+            const float d = dout[tile*TM + row];
+            const uint4 *z0 = reinterpret_cast<const uint4 *>(z_save + tiled_at(0, n_tiles, tile, slot, row));
+            const size_t plane16 = (size_t)n_tiles*TILE_ELEMS/8;   // a plane in 16-byte units
+            constexpr int CHUNK16 = 4*GROUP_ELEMS/8;               // four groups
+            uint4 *dz0 = reinterpret_cast<uint4 *>(dz_save + tiled_at(0, n_tiles, tile, slot, row));
+            uint4 z[CHUNKS_PER_LAYER];
+            #pragma unroll
+            for (int c = 0; c < CHUNKS_PER_LAYER; ++c) z[c] = z0[3*plane16 + c*CHUNK16];
+            // s = -1: dZ3 from dout; s = 0, 1, 2: the epilogues of W3, W2, W1
+            #pragma unroll 1
+            for (int s = -1; s < 3; ++s) {
+                const int g = 3*k + s, l = 2 - s, a = g & 1;
+                uint32_t ra[8], rb[8];
+                const uint32_t acc = tmem + lane_base + (uint32_t)(HID*a + 8*slot);
+                if (s >= 0) {
+                    if (!(ok = warp_wait(&acc_full[a], (uint32_t)((g >> 1) & 1)))) break;
+                    tc::fence_after_sync();
+                    tc::tmem_ld8(acc, ra);
+                    tc::tmem_wait_ld8(ra);
+                }
+                #pragma unroll
+                for (int c = 0; c < CHUNKS_PER_LAYER; ++c) {
+                    const bool more = c + 1 < CHUNKS_PER_LAYER;
+                    if (s >= 0) {
+                        if (more) {
+                            tc::tmem_ld8(acc + (uint32_t)(KCI*(c + 1)), rb);
+                        } else {
+                            tc::fence_before_sync();
+                            __syncwarp();
+                            if (lane == 0) tc::mbar_arrive(&acc_empty[a]);
+                        }
+                    } else {
+                        const float4 *wp = reinterpret_cast<const float4 *>(w_out + KCI*c + 8*slot);
+                        const float4 w0 = __ldg(wp), w1 = __ldg(wp + 1);
+                        const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+                        #pragma unroll
+                        for (int e = 0; e < 8; ++e) ra[e] = __float_as_uint(d*w[e]);
+                    }
+                    const uint32_t zu[4] = {z[c].x, z[c].y, z[c].z, z[c].w};
+                    uint4 o;
+                    uint32_t *op = &o.x;
+                    #pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        op[e] = pack2(__uint_as_float(ra[2*e])*dsilu(bf_lo(zu[e])),
+                                      __uint_as_float(ra[2*e + 1])*dsilu(bf_hi(zu[e])));
+                    if (s < 2) {
+                        *reinterpret_cast<uint4 *>(act + tc::kmajor_offset<TM>(row, KCI*c + 8*slot)) = o;
+                        tc::fence_async_smem();
+                        __syncwarp();
+                        if (lane == 0) tc::mbar_arrive(&act_ready[c]);
+                        // the next layer's z, in use one epilogue from now
+                        z[c] = z0[(size_t)(l - 1)*plane16 + c*CHUNK16];
+                    }
+                    dz0[(size_t)l*plane16 + c*CHUNK16] = o;
+                    if (s >= 0 && more) {
+                        tc::tmem_wait_ld8(rb);
+                        #pragma unroll
+                        for (int e = 0; e < 8; ++e) ra[e] = rb[e];
+                    }
+                }
+            }
+        }
+        if (!ok && lane == 0) atomicExch(err, 1);
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, 2*HID);
+}
+
+// -------------------------------------------------------- weight gradients --
+// mlp_weight_grads: every gradient of a step from the tiled planes in one
+// launch.  With S splits of the tiles, block b is
+//   b < 12 S        layer 1 + (b % 12)/4, M half (b/2) % 2 (columns of dZ), N half
+//                   b % 2 (columns of h), split b/12: dW_l += dZ_l^T h_{l-1} over
+//                   the split's tiles (M 128, N 128, K 128 per tile); the blocks
+//                   of N half 0 also sum their columns of dZ_l (bias gradients);
+//   next S blocks   layer 0: all of dZ_0 against the 16 features, and its sums;
+//   next S blocks   the output weights, columns of h_3 weighted by dout; block 0
+//                   of them also adds the loss and dout sums of the forward.
+// The rows are the K dimension of both operands, so the 32 KB halves of the tile
+// images are MN-major operands as they lie in memory: each half is one bulk
+// copy into a three-stage ring.  Bound by those copies (64 KB per 512-cycle
+// tile of MMAs); eight warps add the columns from the same stages meanwhile.
+// 14 S <= 148 blocks are one wave: S = 10.  Partial sums leave per split, added
+// by whoever reads them (Adam, sum_partials).  8192 rows: 14 us with cold caches,
+// for eight transposes, four split-K GEMMs (28 us the larger) and five column
+// sums on four streams.
+constexpr int WG_STAGES = 3;
+constexpr int WG_HALF = ACT_BYTES/2;                   // 32 KB: 128 columns of a tile
+constexpr int WG_STAGE_BYTES = 2*WG_HALF;
+constexpr int WG_SUM_WARPS = 8;
+constexpr int WG_THREADS = 32*(WG_SUM_WARPS + 2);      // + producer, MMA
+constexpr int WG_SMEM = WG_STAGES*(WG_STAGE_BYTES + X_BYTES);
+constexpr int WG_BIG = 12;
+
+struct WeightGrads {
+    const __nv_bfloat16 *x;          // [n_pad x 16] features (high halves)
+    const __nv_bfloat16 *h, *dz;     // tiled planes
+    const float *dout;               // [n_pad]
+    const float *row_sums;           // [2][4 n_tiles]: loss and dout sums of 32 rows each
+    float *dw[4];                    // [S][256 x (16 or 256)]
+    float *db;                       // [4][S][256]
+    float *dw_out;                   // [S][256]
+    float *loss, *db_out;            // scalars
+    float n;                         // rows of the mean loss
+};
+
+__global__ void __launch_bounds__(WG_THREADS, 1)
+mlp_weight_grads(int n_tiles, int splits, WeightGrads prm, int *__restrict__ err)
+{
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t *xs = smem + WG_STAGES*WG_STAGE_BYTES;
+    __shared__ __align__(8) uint64_t full[WG_STAGES], empty[WG_STAGES], x_full[WG_STAGES], done;
+    __shared__ uint32_t tmem_slot;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int b = blockIdx.x;
+    const bool big = b < WG_BIG*splits, first = !big && b < (WG_BIG + 1)*splits;
+    const int split = big ? b/WG_BIG : (first ? b - WG_BIG*splits : b - (WG_BIG + 1)*splits);
+    const int layer = big ? 1 + (b % WG_BIG)/4 : (first ? 0 : 4);
+    const int mh = big ? (b >> 1) & 1 : 0, nh = big ? b & 1 : 0;
+    const bool mma = layer < 4, sums = !big || nh == 0;
+    const int t0 = (int)((long long)n_tiles*split/splits);
+    const int tiles = (int)((long long)n_tiles*(split + 1)/splits) - t0;
+
+    if (warp == 0) {
+        tc::tmem_alloc(&tmem_slot, 128);
+        tc::tmem_relinquish();
+    }
+    if (t == 0) {
+        for (int s = 0; s < WG_STAGES; ++s) {
+            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&empty[s], (mma ? 1 : 0) + (sums ? WG_SUM_WARPS : 0));
+            tc::mbar_init(&x_full[s], WG_SUM_WARPS);
+        }
+        tc::mbar_init(&done, 1);
+        tc::mbar_fence_init();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+    bool ok = true;
+
+    if (warp == WG_SUM_WARPS) {
+        // ---- producer ----
+        if (lane == 0) {
+            int i = 0;
+            for (; i < tiles; ++i) {
+                const int s = i % WG_STAGES, use = i/WG_STAGES;
+                if (use > 0 && !(ok = tc::mbar_wait(&empty[s], (uint32_t)((use - 1) & 1)))) break;
+                uint8_t *to = smem + s*WG_STAGE_BYTES;
+                tc::mbar_arrive_expect_tx(&full[s], 2*WG_HALF);
+                const size_t own = (size_t)(t0 + i)*TILE_ELEMS, plane = (size_t)n_tiles*TILE_ELEMS;
+                if (big) {
+                    tc::bulk_load(to, prm.dz + layer*plane + own + mh*(TILE_ELEMS/2), WG_HALF,
+                                  &full[s]);
+                    tc::bulk_load(to + WG_HALF, prm.h + (layer - 1)*plane + own + nh*(TILE_ELEMS/2),
+                                  WG_HALF, &full[s]);
+                } else {
+                    tc::bulk_load(to, (first ? prm.dz : prm.h + 3*plane) + own, 2*WG_HALF, &full[s]);
+                }
+            }
+            // every issued copy has landed before the CTA may exit
+            for (int j = (i > WG_STAGES ? i - WG_STAGES : 0); j < i; ++j)
+                ok = tc::mbar_wait(&full[j % WG_STAGES], (uint32_t)((j/WG_STAGES) & 1)) && ok;
+            if (!ok) atomicExch(err, 2);
+        }
+    } else if (warp == WG_SUM_WARPS + 1) {
+        // ---- MMA issue ----
+        if (lane == 0) {
+            if (mma) {
+                for (int i = 0; i < tiles; ++i) {
+                    const int s = i % WG_STAGES;
+                    const uint32_t parity = (uint32_t)((i/WG_STAGES) & 1);
+                    if (!(ok = tc::mbar_wait(&full[s], parity)
+                               && (big || tc::mbar_wait(&x_full[s], parity))))
+                        break;
+                    tc::fence_after_sync();
+                    const uint32_t a = tc::smem_u32(smem + s*WG_STAGE_BYTES);
+                    if (big) {
+                        constexpr uint32_t idesc = tc::idesc_bf16_mn(TM, 128);
+                        #pragma unroll
+                        for (int st = 0; st < TM/16; ++st)
+                            tc::mma_bf16(tmem, tc::mnmajor_desc<TM>(a, st),
+                                         tc::mnmajor_desc<TM>(a + WG_HALF, st), idesc,
+                                         (i > 0 || st > 0) ? 1u : 0u);
+                    } else {
+                        constexpr uint32_t idesc = tc::idesc_bf16_mn(TM, NIN);
+                        const uint32_t bx = tc::smem_u32(xs + s*X_BYTES);
+                        #pragma unroll
+                        for (int st = 0; st < TM/16; ++st) {
+                            const uint64_t bd = tc::mnmajor_desc<TM>(bx, st);
+                            const uint32_t acc = (i > 0 || st > 0) ? 1u : 0u;
+                            tc::mma_bf16(tmem, tc::mnmajor_desc<TM>(a, st), bd, idesc, acc);
+                            tc::mma_bf16(tmem + 64u, tc::mnmajor_desc<TM>(a + WG_HALF, st), bd,
+                                         idesc, acc);
+                        }
+                    }
+                    tc::mma_commit(&empty[s]);
+                }
+            }
+            tc::mma_commit(&done);
+            ok = tc::mbar_wait(&done, 0u) && ok;
+            if (!ok) atomicExch(err, 3);
+        }
+        __syncwarp();
+    } else {
+        // ---- column sums: lane = row (mod 32), a warp 2 or 4 groups of 8 columns ----
+        const int groups = big ? 2 : 4;
+        float acc[4][8];
+        #pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            #pragma unroll
+            for (int e = 0; e < 8; ++e) acc[q][e] = 0.0f;
+        }
+        if (sums) {
+            for (int i = 0; i < tiles && ok; ++i) {
+                const int s = i % WG_STAGES;
+                if (first) {
+                    // the features of the tile: one 16-byte unit per thread
+                    if (i >= WG_STAGES
+                        && !(ok = warp_wait(&empty[s], (uint32_t)((i/WG_STAGES - 1) & 1))))
+                        break;
+                    const int r = t >> 1, c = (t & 1)*8;
+                    *reinterpret_cast<uint4 *>(xs + s*X_BYTES + tc::kmajor_offset<TM>(r, c)) =
+                        *reinterpret_cast<const uint4 *>(prm.x + ((size_t)(t0 + i)*TM + r)*NIN + c);
+                    tc::fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&x_full[s]);
+                }
+                float w[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+                if (layer == 4) {
+                    #pragma unroll
+                    for (int r = 0; r < 4; ++r) w[r] = prm.dout[(t0 + i)*TM + 32*r + lane];
+                }
+                if (!(ok = warp_wait(&full[s], (uint32_t)((i/WG_STAGES) & 1)))) break;
+                const uint8_t *from = smem + s*WG_STAGE_BYTES + warp*groups*(2*GROUP_ELEMS) + 16*lane;
+                #pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (q >= groups) break;
+                    #pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const uint4 u = *reinterpret_cast<const uint4 *>(from + q*(2*GROUP_ELEMS)
+                                                                         + 512*r);
+                        const uint32_t v[4] = {u.x, u.y, u.z, u.w};
+                        #pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            acc[q][2*e] = fmaf(bf_lo(v[e]), w[r], acc[q][2*e]);
+                            acc[q][2*e + 1] = fmaf(bf_hi(v[e]), w[r], acc[q][2*e + 1]);
+                        }
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&empty[s]);
+            }
+            float *to = layer == 4 ? prm.dw_out + (size_t)split*HID
+                                   : prm.db + ((size_t)layer*splits + split)*HID + mh*128;
+            #pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (q >= groups) break;
+                const float v = warp_sum8(acc[q], lane);
+                if ((lane & 3) == 0) to[8*(warp*groups + q) + (lane >> 2)] = v;
+            }
+        }
+        if (layer == 4 && split == 0 && warp < 2) {
+            // warp 0 the loss, warp 1 the output bias: sums of 4 n_tiles partials
+            const float *part = prm.row_sums + (size_t)warp*4*n_tiles;
+            float v = 0.0f;
+            for (int j = lane; j < 4*n_tiles; j += 32) v += part[j];
+            #pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) *(warp == 0 ? prm.loss : prm.db_out) = warp == 0 ? v/prm.n : v;
+        }
+        // ---- the accumulators: warps 0-3 the first 64 columns, 4-7 the rest ----
+        if (mma && ok) {
+            ok = warp_wait(&done, 0u);
+            tc::fence_after_sync();
+            const int quad = warp & 3, part = warp >> 2;
+            const uint32_t at = tmem + ((uint32_t)(32*quad) << 16) + (uint32_t)(64*part);
+            const int m = 32*quad + lane;
+            const int ld = big ? HID : NIN;
+            float *crow = prm.dw[layer] + (size_t)split*HID*ld
+                        + (big ? (size_t)(mh*128 + m)*HID + nh*128 + 64*part
+                               : (size_t)(128*part + m)*NIN);
+            for (int c0 = 0; c0 < (big ? 64 : NIN); c0 += 16) {
+                uint32_t r[16];
+                tc::tmem_ld16(at + (uint32_t)c0, r);
+                tc::tmem_wait_ld();
+                #pragma unroll
+                for (int j = 0; j < 16; j += 4) {
+                    float4 v = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
+                                           __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
+                    if (tiles == 0) v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    *reinterpret_cast<float4 *>(crow + c0 + j) = v;
+                }
+            }
+            tc::fence_before_sync();
+        }
+        if (!ok && lane == 0) atomicExch(err, 1);
+    }
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, 128);
+}
+
+// out[k][i] = the sum over its splits of part[k][s*size + i], in split order, for
+// up to 16 tensors in one launch (blockIdx.y = tensor): a step's gradients as
+// one set of plain tensors.  Bound by the bytes of the partials (8 MB, in L2).
+constexpr int SUM_TENSORS = 16;
+struct SumTensors {
+    int size[SUM_TENSORS], splits[SUM_TENSORS];
+    const float *part[SUM_TENSORS];
+    float *out[SUM_TENSORS];
+};
+
+__global__ void __launch_bounds__(256)
+sum_partials(SumTensors T)
+{
+    const int k = blockIdx.y, size = T.size[k], splits = T.splits[k];
+    const int i = blockIdx.x*256 + threadIdx.x;
+    if (i >= size) return;
+    const float *p = T.part[k] + i;
+    float v = 0.0f;
+    #pragma unroll 8
+    for (int s = 0; s < splits; ++s) v += p[(size_t)s*size];
+    T.out[k][i] = v;
+}

@@ -215,6 +215,13 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n)
          | ((uint32_t)(m >> 4) << 24);            // M / 16
 }
 
+// The same with both operands MN-major (stored with the M or N index
+// contiguous, as mnmajor_desc describes): D = A^T B of two row-major blocks.
+__host__ __device__ constexpr uint32_t idesc_bf16_mn(int m, int n)
+{
+    return idesc_bf16(m, n) | (1u << 15) | (1u << 16);
+}
+
 // D[tmem] (+)= A * B^T, issued by a single thread.
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                          uint32_t idesc, uint32_t accumulate)
@@ -245,6 +252,17 @@ template <int ROWS>
 __device__ __forceinline__ uint64_t kmajor_desc(uint32_t tile_addr, int s)
 {
     return smem_desc(tile_addr + (uint32_t)(2*s*ROWS*16), ROWS*16, 128);
+}
+
+// Descriptor of MMA step s (K = 16 rows) of a no-swizzle MN-major tile of ROWS
+// rows: the same bytes as above with rows as K, i.e. core matrices of 8 rows x 8
+// contiguous columns, 128 bytes from one 8-row group to the next (the K
+// stride, LBO) and ROWS*16 bytes from one 8-column group to the next (the MN
+// stride, SBO).
+template <int ROWS>
+__device__ __forceinline__ uint64_t mnmajor_desc(uint32_t tile_addr, int s)
+{
+    return smem_desc(tile_addr + (uint32_t)(s*256), 128, ROWS*16);
 }
 
 }  // namespace tc

@@ -67,7 +67,13 @@ def _lib():
     lib.sasb200_mlp_serve.argtypes = [I, I, P, P, P, P, P, P, P, P, P, P, I, P]
     lib.sasb200_mlp_pack_t.argtypes = [P, P, P, P, P]
     lib.sasb200_mlp_backward_p.argtypes = [I, I, P, P, P, P, P, P, I, P]
-    for name in ("sasb200_mlp_forward", "sasb200_mlp_backward", "sasb200_gemm_nt",
+    lib.sasb200_mlp_train_forward.argtypes = [I, I] + [P]*7 + [F] + [P]*7
+    lib.sasb200_mlp_train_backward.argtypes = [I] + [P]*7
+    lib.sasb200_mlp_weight_grads.argtypes = [I, I, I] + [P]*12
+    lib.sasb200_sum_partials.argtypes = [I] + [P]*5
+    for name in ("sasb200_mlp_train_forward", "sasb200_mlp_train_backward",
+                 "sasb200_mlp_weight_grads", "sasb200_sum_partials",
+                 "sasb200_mlp_forward", "sasb200_mlp_backward", "sasb200_gemm_nt",
                  "sasb200_transpose_bf16", "sasb200_loss_grad",
                  "sasb200_adam", "sasb200_mlp_features", "sasb200_mlp_pack",
                  "sasb200_mlp_infer", "sasb200_mlp_serve", "sasb200_mlp_image_bytes",
@@ -94,7 +100,6 @@ class MLP:
             self.device = torch.device("cuda", torch.cuda.current_device())
         self.lib = _lib()
         self.stream = stream if stream is not None else torch.cuda.Stream(self.device)
-        self._side = [torch.cuda.Stream(self.device) for _ in range(4)]
         rng = np.random.default_rng(seed)
         shapes = [(HID, NIN), (HID, HID), (HID, HID), (HID, HID)]
         f32 = dict(dtype=torch.float32, device=self.device)
@@ -113,6 +118,9 @@ class MLP:
         self.m = [torch.zeros_like(p) for p in self.params]
         self.v = [torch.zeros_like(p) for p in self.params]
         self.step_count = 0
+        #: partial sums of each weight gradient (see mlp_weight_grads: 14 blocks
+        #: per split, one wave of blocks)
+        self.splits = 10
         #: Huber threshold of the training loss (<= 0: squared error)
         self.huber = 0.0
         self.err = torch.zeros(1, dtype=torch.int32, device=self.device)
@@ -147,21 +155,18 @@ class MLP:
             return
         bf = dict(dtype=torch.bfloat16, device=self.device)
         f32 = dict(dtype=torch.float32, device=self.device)
+        # planes of a training step (tiled) and of forward(save=True)
         self.z_save = torch.empty(4*n_pad*HID, **bf)
         self.h_save = torch.empty(4*n_pad*HID, **bf)
         self.dz_save = torch.empty(4*n_pad*HID, **bf)
-        # per layer (the four weight-gradient chains run concurrently):
-        # transposed dZ, transposed h / x, column-sum partials
-        self.t_a = [torch.empty(HID*n_pad, **bf) for _ in range(4)]
-        self.t_b = [torch.empty(HID*n_pad, **bf) for _ in range(4)]
         self.out = torch.empty(n_pad, **f32)
         self.dout = torch.empty(n_pad, **f32)
-        self.sq = torch.empty(n_pad, **f32)
-        parts = self.lib.sasb200_col_sum_parts(n_pad)*HID
-        self.cs_part = [torch.empty(parts, **f32) for _ in range(5)]
-        self.splits = 32     # split-K of the weight gradients: 64+ CTAs at batch 8192
+        self.row_sums = torch.empty(2*(n_pad//32), **f32)
+        # gradients as partial sums over splits of the rows
         self.gW = [torch.empty(self.splits*HID*(NIN if l == 0 else HID), **f32)
                    for l in range(4)]
+        self.gb_part = torch.empty((4, self.splits*HID), **f32)
+        self.gw_part = torch.empty(self.splits*HID, **f32)
         self.gb = [torch.empty(HID, **f32) for _ in range(4)]
         self.gw = torch.empty(HID, **f32)
         self.gbo = torch.empty(1, **f32)
@@ -232,75 +237,49 @@ class MLP:
     def gradients(self, x, x_lo, y, n):
         """Loss and gradients of one batch, all on self.stream: returns
         (loss, dW split partials [4], db [4], dw_out, db_out)."""
+        torch = self.torch
         self._scratch(x.shape[0])
         self._pack()
-        return self._gradient_kernels(x, x_lo, y, n)
+        with torch.cuda.stream(self.stream):
+            loss = torch.empty((), dtype=torch.float32, device=self.device)
+        self._gradient_kernels(x, x_lo, y, n, loss, self.gbo)
+        self._sum_partials(list(zip(self._vector_partials(), self.gb + [self.gw])))
+        return loss, self.gW, self.gb, self.gw, self.gbo
 
-    def _gradient_kernels(self, x, x_lo, y, n):
-        torch = self.torch
+    def _vector_partials(self):
+        """Partial sums of the four bias gradients and the output weights'."""
+        return [self.gb_part[l] for l in range(4)] + [self.gw_part]
+
+    def _sum_partials(self, pairs):
+        """Every (partials, out) pair summed over the splits, in one launch."""
+        n = len(pairs)
+        I32, VP = ct.c_int32*n, ct.c_void_p*n
+        self._check(self.lib.sasb200_sum_partials(
+            n, I32(*[o.numel() for _, o in pairs]), I32(*[self.splits]*n),
+            VP(*[p.data_ptr() for p, _ in pairs]), VP(*[o.data_ptr() for _, o in pairs]),
+            self.stream.cuda_stream), "sum_partials")
+
+    def _gradient_kernels(self, x, x_lo, y, n, loss, db_out):
+        """Forward, backward and weight gradients of one batch: the loss and
+        db_out as scalars, the other gradients as partial sums over
+        self.splits (gW, gb_part, gw_part)."""
         n_pad = x.shape[0]
         st = self.stream.cuda_stream
         lib = self.lib
-        # forward with the z/h planes through the overlapped kernel, backward
-        # through the pipelined persistent kernel (weights streamed from the
-        # packed images)
-        self._check(lib.sasb200_mlp_serve(
+        err = self.err.data_ptr()
+        z, h, dz = (t.data_ptr() for t in (self.z_save, self.h_save, self.dz_save))
+        dout, sums = self.dout.data_ptr(), self.row_sums.data_ptr()
+        self._check(lib.sasb200_mlp_train_forward(
             n, n_pad, x.data_ptr(), x_lo.data_ptr(), self.img.data_ptr(), self._ptrs(self.b),
-            self.w_out.data_ptr(), self.b_out.data_ptr(), self.out.data_ptr(),
-            self.z_save.data_ptr(), self.h_save.data_ptr(), self.err.data_ptr(), 0, st),
-            "forward")
-        self._check(lib.sasb200_loss_grad(n, n_pad, self.out.data_ptr(), y.data_ptr(),
-                                          float(self.huber), self.dout.data_ptr(),
-                                          self.sq.data_ptr(), st), "loss")
-        self._check(lib.sasb200_mlp_backward_p(n, n_pad, self.img_t.data_ptr(),
-                                               self.w_out.data_ptr(), self.dout.data_ptr(),
-                                               self.z_save.data_ptr(), self.dz_save.data_ptr(),
-                                               self.err.data_ptr(), 0, st), "backward")
-        # the weight-gradient chain of each layer (transposes, split-K GEMM,
-        # bias column sums) depends only on the planes: the four chains run on
-        # side streams forked from self.stream and joined before it goes on,
-        # so together they fill the SMs that one chain leaves idle
-        plane = n_pad*HID
-        fork = torch.cuda.Event()
-        fork.record(self.stream)
-        joins = []
-        for l in range(4):
-            side = self._side[l]
-            side.wait_event(fork)
-            ss = side.cuda_stream
-            nb = NIN if l == 0 else HID
-            dz = self.dz_save[l*plane:(l + 1)*plane]
-            t_a, t_b = self.t_a[l], self.t_b[l]
-            self._check(lib.sasb200_transpose_bf16(n_pad, HID, dz.data_ptr(), t_a.data_ptr(), ss),
-                        "transpose")
-            if l == 0:
-                src, cols = x, NIN
-            else:
-                src, cols = self.h_save[(l - 1)*plane:l*plane], HID
-            self._check(lib.sasb200_transpose_bf16(n_pad, cols, src.data_ptr(), t_b.data_ptr(), ss),
-                        "transpose")
-            self._check(lib.sasb200_gemm_nt(HID, nb, n_pad, n_pad, n_pad, t_a.data_ptr(),
-                                            t_b.data_ptr(), self.splits,
-                                            self.gW[l].data_ptr(), self.err.data_ptr(), ss),
-                        "gemm_nt")
-            # bias gradient: column sums of the dZ plane (zero on padding rows)
-            self._check(lib.sasb200_col_sums(n_pad, HID, dz.data_ptr(), None,
-                                             self.cs_part[l].data_ptr(), self.gb[l].data_ptr(), ss),
-                        "col_sums")
-            done = torch.cuda.Event()
-            done.record(side)
-            joins.append(done)
-        # output weights: columns of the last h plane weighted by dout
-        h3 = self.h_save[3*plane:4*plane]
-        self._check(lib.sasb200_col_sums(n_pad, HID, h3.data_ptr(), self.dout.data_ptr(),
-                                         self.cs_part[4].data_ptr(), self.gw.data_ptr(), st),
-                    "col_sums")
-        for done in joins:
-            self.stream.wait_event(done)
-        with torch.cuda.stream(self.stream):
-            self.gbo.copy_(self.dout[:n_pad].sum().reshape(1))
-            loss = self.sq[:n].mean()
-        return loss, self.gW, self.gb, self.gw, self.gbo
+            self.w_out.data_ptr(), self.b_out.data_ptr(), y.data_ptr(), float(self.huber),
+            self.out.data_ptr(), dout, sums, z, h, err, st), "forward")
+        self._check(lib.sasb200_mlp_train_backward(n_pad, self.img_t.data_ptr(),
+                                                   self.w_out.data_ptr(), dout, z, dz, err, st),
+                    "backward")
+        self._check(lib.sasb200_mlp_weight_grads(
+            n, n_pad, self.splits, x.data_ptr(), h, dz, dout, sums, self._ptrs(self.gW),
+            self.gb_part.data_ptr(), self.gw_part.data_ptr(), loss.data_ptr(), db_out.data_ptr(),
+            err, st), "weight_grads")
 
     def train_step(self, x, x_lo, y, n, lr, b1=0.9, b2=0.999, eps=1e-8, reduce=None):
         """One Adam step on one batch; returns the loss (a device scalar).
@@ -324,10 +303,16 @@ class MLP:
         """[loss (1 element), dW_1..dW_4, db_1..db_4, dw_out, db_out] of one
         batch as fp32 device tensors, the weight gradients summed over their
         split-K partials: the ≈200k numbers a data-parallel step exchanges."""
-        loss, dW, db, gw, gbo = self.gradients(x, x_lo, y, n)
-        with self.torch.cuda.stream(self.stream):
-            dW = [g.view(self.splits, -1).sum(0) for g in dW]
-            return [loss.reshape(1).clone()] + dW + [g.clone() for g in db + [gw, gbo]]
+        torch = self.torch
+        self._scratch(x.shape[0])
+        self._pack()
+        sizes = [p.numel() for p in self.params]
+        with torch.cuda.stream(self.stream):
+            flat = torch.empty(sum(sizes) + 1, dtype=torch.float32, device=self.device)
+        parts = flat.split(sizes + [1])
+        self._gradient_kernels(x, x_lo, y, n, parts[-1], parts[9])
+        self._sum_partials(list(zip(self.gW + self._vector_partials(), parts)))
+        return [parts[-1]] + list(parts[:-1])
 
     def capture_training(self, x_all, x_lo_all, y_all, batch, lr, total, step0, warmup=200,
                          b1=0.9, b2=0.999, eps=1e-8):
@@ -548,6 +533,7 @@ class TrainingGraph:
         self.xb = torch.empty((batch, x_all.shape[1]), dtype=x_all.dtype, device=dev)
         self.xlb = torch.empty_like(self.xb)
         self.yb = torch.empty(batch, dtype=y_all.dtype, device=dev)
+        self.loss = torch.zeros((), dtype=torch.float32, device=dev)
         net._scratch(batch)
         lib, st = net.lib, net.stream.cuda_stream
         net.stream.synchronize()
@@ -560,12 +546,12 @@ class TrainingGraph:
                                                int(total), int(warmup), float(lr), b1, b2, st),
                        "lr_schedule")
             net._pack_kernels()
-            self.loss, dW, db, gw, gbo = net._gradient_kernels(self.xb, self.xlb, self.yb, batch)
-            grads = dW + db + [gw, gbo]
+            net._gradient_kernels(self.xb, self.xlb, self.yb, batch, self.loss, net.gbo)
+            grads = net.gW + net._vector_partials() + [net.gbo]
             nt = len(net.params)
             I32, VP = ct.c_int32*nt, ct.c_void_p*nt
             sizes = [p.numel() for p in net.params]
-            splits = [net.splits if k < 4 else 1 for k in range(nt)]
+            splits = [net.splits if k < 9 else 1 for k in range(nt)]
             shape = [(HID, NIN if k == 0 else HID) if k < 4 else (0, 0) for k in range(nt)]
             net._check(lib.sasb200_adam_multi(
                 nt, I32(*sizes), I32(*splits), VP(*[g.data_ptr() for g in grads]),
