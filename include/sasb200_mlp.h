@@ -114,6 +114,25 @@ int32_t sasb200_mlp_weight_grads(int32_t n, int32_t n_pad, int32_t splits, const
 int32_t sasb200_sum_partials(int32_t n, const int32_t *sizes, const int32_t *splits,
                              const float *const *parts, float *const *outs, void *stream);
 
+/* a captured step's batch and schedule in one launch: rows idx[n] of the data set
+ * (x_all, x_lo_all [rows x 16] bf16, y_all[rows]) into x, x_lo, y, and the step
+ * of sasb200_lr_schedule; an index outside the set leaves zeros and *err = 5. */
+int32_t sasb200_gather_batch(int32_t n, int64_t rows, const int64_t *idx, const void *x_all,
+                             const void *x_lo_all, const float *y_all, void *x, void *x_lo,
+                             float *y, int32_t *counters, float *sched, int32_t total,
+                             int32_t warmup, float lr0, float b1, float b2, int32_t *err,
+                             void *stream);
+
+/* Adam for the whole network in one launch (host arrays of 10 device pointers:
+ * W0..W3, b0..b3, w_out, b_out, with splits[k] partial gradients each) with the
+ * bf16 weights w[4], transposes wt[4] and both weight images; lr and the bias
+ * corrections from sched (sasb200_lr_schedule), or from lr and step when it is
+ * NULL. */
+int32_t sasb200_adam_pack(const float *const *grads, const int32_t *splits, float *const *p,
+                          float *const *m, float *const *v, void *const *w, void *const *wt,
+                          void *img, void *img_t, const float *sched, float lr, int32_t step,
+                          float b1, float b2, float eps, void *stream);
+
 /* the learning rate and Adam bias corrections of a training step, on the
  * device: counters = {schedule step s, Adam step count t} (int32), sched =
  * {lr, 1 - b1^t, 1 - b2^t} with lr = lr0 min(1, (s + 1)/warmup)

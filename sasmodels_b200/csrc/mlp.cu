@@ -530,6 +530,17 @@ __global__ void loss_grad(int n, int n_pad, const float *__restrict__ out,
     loss[i] = l;
 }
 
+__device__ __forceinline__ void adam_update(float g, float &p, float &m, float &v, float lr,
+                                            float b1, float b2, float eps, float bc1, float bc2)
+{
+    // the contractions are spelled out, so that every kernel rounds alike
+    const float mi = fmaf(b1, m, (1.0f - b1)*g);
+    const float vi = fmaf(b2, v, (1.0f - b2)*g*g);
+    m = mi;
+    v = vi;
+    p = p - lr*(mi/bc1)/(sqrtf(vi/bc2) + eps);
+}
+
 // Adam on one FP32 master tensor; grad = sum of `splits` partial gradients.
 // Writes the BF16 copy (and its transpose if wt != nullptr, rows x cols).
 // Adam update of element i: the gradient summed over its `splits` split-K
@@ -544,11 +555,8 @@ __device__ __forceinline__ void adam_element(int i, int size, int splits,
 {
     float g = 0.0f;
     for (int s = 0; s < splits; ++s) g += grad[(size_t)s*size + i];
-    const float mi = b1*m[i] + (1.0f - b1)*g;
-    const float vi = b2*v[i] + (1.0f - b2)*g*g;
-    m[i] = mi;
-    v[i] = vi;
-    const float pi = p[i] - lr*(mi/bc1)/(sqrtf(vi/bc2) + eps);
+    float pi = p[i];
+    adam_update(g, pi, m[i], v[i], lr, b1, b2, eps, bc1, bc2);
     p[i] = pi;
     if (w) w[i] = __float2bfloat16_rn(pi);
     if (wt) {
@@ -596,10 +604,10 @@ __global__ void adam_multi(AdamTensors T, float b1, float b2, float eps,
 // device counters {schedule step s, Adam step count t}, then s and t advance:
 // lr = lr0 min(1, (s + 1)/warmup) (1 + cos(pi s/total))/2 (linear warm-up,
 // cosine decay), bc1 = 1 - b1^(t+1), bc2 = 1 - b2^(t+1).  One thread.
-__global__ void lr_schedule(int *__restrict__ counters, float *__restrict__ sched, int total,
-                            int warmup, float lr0, float b1, float b2)
+__device__ __forceinline__ void schedule_step(int *__restrict__ counters,
+                                              float *__restrict__ sched, int total, int warmup,
+                                              float lr0, float b1, float b2)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const int s = counters[0], t = counters[1] + 1;
     const double frac = (double)s/(double)total;
     const double rate = (double)lr0*fmin(1.0, (double)(s + 1)/(double)warmup)
@@ -609,6 +617,13 @@ __global__ void lr_schedule(int *__restrict__ counters, float *__restrict__ sche
     sched[2] = 1.0f - powf(b2, (float)t);
     counters[0] = s + 1;
     counters[1] = t;
+}
+
+__global__ void lr_schedule(int *__restrict__ counters, float *__restrict__ sched, int total,
+                            int warmup, float lr0, float b1, float b2)
+{
+    if (threadIdx.x == 0 && blockIdx.x == 0)
+        schedule_step(counters, sched, total, warmup, lr0, b1, b2);
 }
 
 // Surrogate input features, each mapped to about [-1, 1]: the seven model
@@ -1751,6 +1766,74 @@ int32_t sasb200_mlp_weight_grads(int32_t n, int32_t n_pad, int32_t splits, const
     mlp_weight_grads<<<(WG_BIG + 2)*splits, WG_THREADS, WG_SMEM, (cudaStream_t)stream>>>(
         n_pad/TM, splits, prm, err);
     return status("mlp_weight_grads");
+}
+
+// The batch of a captured training step: rows idx[n] of the data set (x_all,
+// x_lo_all [rows x 16] bf16, y_all[rows]) into x, x_lo, y, and the schedule
+// step of sasb200_lr_schedule; err receives 5 for an index outside the set.
+int32_t sasb200_gather_batch(int32_t n, int64_t rows, const int64_t *idx, const void *x_all,
+                             const void *x_lo_all, const float *y_all, void *x, void *x_lo,
+                             float *y, int32_t *counters, float *sched, int32_t total,
+                             int32_t warmup, float lr0, float b1, float b2, int32_t *err,
+                             void *stream)
+{
+    errbuf()[0] = 0;
+    if (n <= 0 || rows < 0 || !idx || !x_all || !x_lo_all || !y_all || !x || !x_lo || !y
+        || !counters || !sched || total <= 0 || warmup <= 0 || !err)
+        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
+    if ((reinterpret_cast<uintptr_t>(x_all) | reinterpret_cast<uintptr_t>(x_lo_all)
+         | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(x_lo)) % 16)
+        return (std::snprintf(errbuf(), 256, "features must be 16-byte aligned"), -1);
+    gather_batch<<<(unsigned)((4ll*n + 255)/256), 256, 0, (cudaStream_t)stream>>>(
+        n, rows, idx, static_cast<const uint4 *>(x_all), static_cast<const uint4 *>(x_lo_all),
+        y_all, static_cast<uint4 *>(x), static_cast<uint4 *>(x_lo), y, counters, sched, total,
+        warmup, lr0, b1, b2, err);
+    return status("gather_batch");
+}
+
+// Adam for the whole network (host arrays of 10 device pointers, in the order
+// W0..W3, b0..b3, w_out, b_out; splits partial gradients each) refreshing the
+// bf16 weights w[4], their transposes wt[4] and both weight images; lr and the
+// bias corrections from sched when it is not NULL, else lr and step (>= 1).
+int32_t sasb200_adam_pack(const float *const *grads, const int32_t *splits, float *const *p,
+                          float *const *m, float *const *v, void *const *w, void *const *wt,
+                          void *img, void *img_t, const float *sched, float lr, int32_t step,
+                          float b1, float b2, float eps, void *stream)
+{
+    errbuf()[0] = 0;
+    if (!grads || !splits || !p || !m || !v || !w || !wt || !img || !img_t || (!sched && step < 1))
+        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
+    AdamPack A;
+    uintptr_t bits = reinterpret_cast<uintptr_t>(img) | reinterpret_cast<uintptr_t>(img_t);
+    for (int k = 0; k < 10; ++k) {
+        if (!grads[k] || splits[k] <= 0 || !p[k] || !m[k] || !v[k])
+            return (std::snprintf(errbuf(), 256, "bad tensor"), -1);
+        A.grad[k] = grads[k];
+        A.splits[k] = splits[k];
+        A.p[k] = p[k];
+        A.m[k] = m[k];
+        A.v[k] = v[k];
+        if (k < 4) {
+            if (!w[k] || !wt[k]) return (std::snprintf(errbuf(), 256, "bad tensor"), -1);
+            A.w[k] = static_cast<__nv_bfloat16 *>(w[k]);
+            A.wt[k] = static_cast<__nv_bfloat16 *>(wt[k]);
+            bits |= reinterpret_cast<uintptr_t>(grads[k]) | reinterpret_cast<uintptr_t>(p[k])
+                  | reinterpret_cast<uintptr_t>(m[k]) | reinterpret_cast<uintptr_t>(v[k])
+                  | reinterpret_cast<uintptr_t>(w[k]) | reinterpret_cast<uintptr_t>(wt[k]);
+        }
+    }
+    if (bits % 16) return (std::snprintf(errbuf(), 256, "tensors must be 16-byte aligned"), -1);
+    A.img = static_cast<uint8_t *>(img);
+    A.img_t = static_cast<uint8_t *>(img_t);
+    A.sched = sched;
+    A.lr = lr;
+    A.bc1 = sched ? 0.0f : 1.0f - powf(b1, (float)step);
+    A.bc2 = sched ? 0.0f : 1.0f - powf(b2, (float)step);
+    A.b1 = b1;
+    A.b2 = b2;
+    A.eps = eps;
+    adam_pack<<<AP_BLOCKS, 256, 0, (cudaStream_t)stream>>>(A);
+    return status("adam_pack");
 }
 
 // outs[k][i] = sum over s < splits[k] of parts[k][s*sizes[k] + i] for n (<= 16)

@@ -474,3 +474,143 @@ sum_partials(SumTensors T)
     for (int s = 0; s < splits; ++s) v += p[(size_t)s*size];
     T.out[k][i] = v;
 }
+
+// ------------------------------------------------------ batch and schedule --
+// One launch at the head of a captured training step: the batch's rows of the
+// data set (idx, 32 bytes of x and of x_lo and one target each) and, by one
+// thread, the schedule.  Bound by the random 32-byte reads (0.8 MB of 8192 rows);
+// 5.6 us with cold caches, where three index_select launches and lr_schedule took
+// 29.  A row outside the data set leaves zeros and err = 5.
+__global__ void __launch_bounds__(256)
+gather_batch(int n, long long rows, const int64_t *__restrict__ idx,
+             const uint4 *__restrict__ x_all, const uint4 *__restrict__ xlo_all,
+             const float *__restrict__ y_all, uint4 *__restrict__ x, uint4 *__restrict__ x_lo,
+             float *__restrict__ y, int *__restrict__ counters, float *__restrict__ sched,
+             int total, int warmup, float lr0, float b1, float b2, int *__restrict__ err)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        schedule_step(counters, sched, total, warmup, lr0, b1, b2);
+    const int i = blockIdx.x*256 + threadIdx.x, row = i >> 2, part = i & 3;
+    if (row >= n) return;
+    const long long src = idx[row];
+    const bool in = src >= 0 && src < rows;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (in) v = (part < 2 ? x_all : xlo_all)[2*src + (part & 1)];
+    (part < 2 ? x : x_lo)[2*row + (part & 1)] = v;
+    if (part == 0) {
+        y[row] = in ? y_all[src] : 0.0f;
+        if (!in) atomicExch(err, 5);
+    }
+}
+
+// -------------------------------------------------------------------- Adam --
+// adam_pack: the update of every parameter and everything that is kept of the
+// weights in bf16 -- W, W^T and the chunk images that the forward and the
+// backward stream -- in one launch.  A block owns a 32 x 32 tile of a hidden
+// weight, so that the partial gradients, masters and moments are read and
+// written in 16-byte units along the rows, and W^T and both images from the
+// tile in shared memory as whole 16-byte units too.  Bound by the bytes (8 MB of
+// partials, 6 MB of state): 7.1 us with cold caches, where adam_multi and the two
+// packing kernels took 14.6.
+// Blocks: 64 per hidden layer, 4 for W0 (64 rows each), one per vector.
+struct AdamPack {
+    const float *grad[10];           // W0..W3, b0..b3, w_out, b_out
+    int splits[10];
+    float *p[10], *m[10], *v[10];
+    __nv_bfloat16 *w[4], *wt[4];
+    uint8_t *img, *img_t;
+    const float *sched;              // {lr, bc1, bc2}, or null and the values below
+    float lr, bc1, bc2, b1, b2, eps;
+};
+constexpr int AP_TILES = (HID/32)*(HID/32);
+constexpr int AP_W0 = 4;
+constexpr int AP_BLOCKS = 3*AP_TILES + AP_W0 + 6;
+constexpr int AP_LD = 40;            // bf16 per row of the tile: 16-byte units stay aligned
+
+__device__ __forceinline__ float4 adam4(const AdamPack &A, int k, int i, int size, float lr,
+                                        float bc1, float bc2)
+{
+    const float *grad = A.grad[k] + i;
+    const int splits = A.splits[k];
+    float g[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    #pragma unroll 5
+    for (int s = 0; s < splits; ++s) {
+        const float4 u = *reinterpret_cast<const float4 *>(grad + (size_t)s*size);
+        g[0] += u.x;
+        g[1] += u.y;
+        g[2] += u.z;
+        g[3] += u.w;
+    }
+    float4 p = *reinterpret_cast<float4 *>(A.p[k] + i), m = *reinterpret_cast<float4 *>(A.m[k] + i),
+           v = *reinterpret_cast<float4 *>(A.v[k] + i);
+    float *pp = &p.x, *mp = &m.x, *vp = &v.x;
+    #pragma unroll
+    for (int e = 0; e < 4; ++e) adam_update(g[e], pp[e], mp[e], vp[e], lr, A.b1, A.b2, A.eps, bc1, bc2);
+    *reinterpret_cast<float4 *>(A.p[k] + i) = p;
+    *reinterpret_cast<float4 *>(A.m[k] + i) = m;
+    *reinterpret_cast<float4 *>(A.v[k] + i) = v;
+    return p;
+}
+
+__global__ void __launch_bounds__(256)
+adam_pack(AdamPack A)
+{
+    __shared__ __align__(16) __nv_bfloat16 tile[32*AP_LD];
+    const int t = threadIdx.x, b = blockIdx.x;
+    const float lr = A.sched ? A.sched[0] : A.lr, bc1 = A.sched ? A.sched[1] : A.bc1,
+                bc2 = A.sched ? A.sched[2] : A.bc2;
+    if (b < 3*AP_TILES) {
+        const int l = 1 + b/AP_TILES, tr = (b % AP_TILES)/(HID/32), tc_ = b % (HID/32);
+        const int r = t >> 3, c = 4*(t & 7);
+        const int at = (32*tr + r)*HID + 32*tc_ + c;
+        const float4 p = adam4(A, l, at, HID*HID, lr, bc1, bc2);
+        uint2 h;
+        h.x = pack2(p.x, p.y);
+        h.y = pack2(p.z, p.w);
+        *reinterpret_cast<uint2 *>(A.w[l] + at) = h;
+        *reinterpret_cast<uint2 *>(tile + r*AP_LD + c) = h;
+        __syncthreads();
+        const int j = t & 31, g = (t >> 5) & 3;
+        if (t < 128) {
+            // row j of the tile, input group g
+            *reinterpret_cast<uint4 *>(A.img + W0_BYTES
+                                       + (size_t)((l - 1)*CHUNKS_PER_LAYER + tc_)*CHUNK_BYTES
+                                       + tc::kmajor_offset<HID>(32*tr + j, 8*g)) =
+                *reinterpret_cast<const uint4 *>(tile + j*AP_LD + 8*g);
+        } else {
+            // column j of the tile, output group g
+            uint4 u;
+            uint32_t *up = &u.x;
+            #pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const __nv_bfloat162 two = __halves2bfloat162(tile[(8*g + 2*e)*AP_LD + j],
+                                                              tile[(8*g + 2*e + 1)*AP_LD + j]);
+                up[e] = *reinterpret_cast<const uint32_t *>(&two);
+            }
+            *reinterpret_cast<uint4 *>(A.wt[l] + (32*tc_ + j)*HID + 32*tr + 8*g) = u;
+            *reinterpret_cast<uint4 *>(A.img_t + (size_t)((3 - l)*CHUNKS_PER_LAYER + tr)*CHUNK_BYTES
+                                       + tc::kmajor_offset<HID>(32*tc_ + j, 8*g)) = u;
+        }
+    } else if (b < 3*AP_TILES + AP_W0) {
+        const int r = 64*(b - 3*AP_TILES) + (t >> 2), c = 4*(t & 3);
+        const float4 p = adam4(A, 0, r*NIN + c, HID*NIN, lr, bc1, bc2);
+        uint2 h;
+        h.x = pack2(p.x, p.y);
+        h.y = pack2(p.z, p.w);
+        *reinterpret_cast<uint2 *>(A.w[0] + r*NIN + c) = h;
+        *reinterpret_cast<uint2 *>(A.img + tc::kmajor_offset<HID>(r, c)) = h;
+        const float *pp = &p.x;
+        #pragma unroll
+        for (int e = 0; e < 4; ++e) A.wt[0][(c + e)*HID + r] = __float2bfloat16_rn(pp[e]);
+    } else {
+        const int k = 4 + b - 3*AP_TILES - AP_W0, size = k < 9 ? HID : 1;
+        if (t >= size) return;
+        float g = 0.0f;
+        for (int s = 0; s < A.splits[k]; ++s) g += A.grad[k][s*size + t];
+        float p = A.p[k][t], m = A.m[k][t], v = A.v[k][t];
+        adam_update(g, p, m, v, lr, A.b1, A.b2, A.eps, bc1, bc2);
+        A.p[k][t] = p;
+        A.m[k][t] = m;
+        A.v[k][t] = v;
+    }
+}

@@ -71,7 +71,10 @@ def _lib():
     lib.sasb200_mlp_train_backward.argtypes = [I] + [P]*7
     lib.sasb200_mlp_weight_grads.argtypes = [I, I, I] + [P]*12
     lib.sasb200_sum_partials.argtypes = [I] + [P]*5
-    for name in ("sasb200_mlp_train_forward", "sasb200_mlp_train_backward",
+    lib.sasb200_gather_batch.argtypes = [I, ct.c_int64] + [P]*9 + [I, I, F, F, F, P, P]
+    lib.sasb200_adam_pack.argtypes = [P]*10 + [F, I, F, F, F, P]
+    for name in ("sasb200_gather_batch", "sasb200_adam_pack",
+                 "sasb200_mlp_train_forward", "sasb200_mlp_train_backward",
                  "sasb200_mlp_weight_grads", "sasb200_sum_partials",
                  "sasb200_mlp_forward", "sasb200_mlp_backward", "sasb200_gemm_nt",
                  "sasb200_transpose_bf16", "sasb200_loss_grad",
@@ -137,8 +140,14 @@ class MLP:
     def _sync_bf16(self):
         torch = self.torch
         self._wversion = getattr(self, "_wversion", 0) + 1
-        self.Wb = [w.to(torch.bfloat16).contiguous() for w in self.W]
-        self.WTb = [w.t().contiguous().to(torch.bfloat16) for w in self.W]
+        if not hasattr(self, "Wb"):
+            self.Wb = [torch.empty_like(w, dtype=torch.bfloat16) for w in self.W]
+            self.WTb = [torch.empty_like(w.t(), dtype=torch.bfloat16,
+                                         memory_format=torch.contiguous_format) for w in self.W]
+        # in place: a captured training step holds their addresses
+        for w, wb, wtb in zip(self.W, self.Wb, self.WTb):
+            wb.copy_(w)
+            wtb.copy_(w.t())
 
     def _ptrs(self, tensors):
         arr = (ct.c_void_p*len(tensors))(*[t.data_ptr() for t in tensors])
@@ -327,22 +336,22 @@ class MLP:
     def apply_gradients(self, grads, lr, splits, b1=0.9, b2=0.999, eps=1e-8):
         """Adam update from [dW_1..dW_4 (each `splits` partials), db_1..db_4,
         dw_out, db_out], refreshing the bf16 weight copies; on self.stream."""
-        dW, rest = grads[:4], grads[4:]
         self.step_count += 1
-        st = self.stream.cuda_stream
-        lib = self.lib
-        for l in range(4):
-            nb = NIN if l == 0 else HID
-            self._check(lib.sasb200_adam(HID*nb, splits, dW[l].data_ptr(), self.W[l].data_ptr(),
-                                         self.m[l].data_ptr(), self.v[l].data_ptr(), lr, b1, b2, eps,
-                                         self.step_count, self.Wb[l].data_ptr(),
-                                         self.WTb[l].data_ptr(), HID, nb, st), "adam")
-        for k, g in enumerate(rest):
-            p = self.params[4 + k]
-            self._check(lib.sasb200_adam(p.numel(), 1, g.data_ptr(), p.data_ptr(),
-                                         self.m[4 + k].data_ptr(), self.v[4 + k].data_ptr(), lr,
-                                         b1, b2, eps, self.step_count, None, None, 0, 0, st),
-                        "adam")
+        self._adam(grads, [splits]*4 + [1]*6, None, lr, b1, b2, eps)
+        # the update refreshed the weight images as well
+        self._packed = (self.step_count, self._wversion)
+
+    def _adam(self, grads, splits, sched, lr, b1, b2, eps):
+        # the kernel reads the weights' gradients in 16-byte units
+        with self.torch.cuda.stream(self.stream):
+            grads = [g if k >= 4 or g.data_ptr() % 16 == 0 else g.clone()
+                     for k, g in enumerate(grads)]
+        self._check(self.lib.sasb200_adam_pack(
+            self._ptrs(grads), (ct.c_int32*10)(*splits), self._ptrs(self.params),
+            self._ptrs(self.m), self._ptrs(self.v), self._ptrs(self.Wb), self._ptrs(self.WTb),
+            self.img.data_ptr(), self.img_t.data_ptr(),
+            None if sched is None else sched.data_ptr(), lr, self.step_count, b1, b2, eps,
+            self.stream.cuda_stream), "adam_pack")
 
     def features(self, radius, length, rpd, lpd, contrast, q, flag):
         """Compensated bf16 features (hi, lo) [n_pad x 16] on the device from
@@ -511,12 +520,10 @@ def gate_thresholds(r, err, tols, alpha):
 
 class TrainingGraph:
     """One training step of an :class:`MLP` captured as a CUDA graph: the
-    batch gather (rows named by ``idx``), the weight images, forward,
-    loss, backward, weight gradients, the learning-rate schedule and Adam
-    for every parameter; the schedule's counters live on the device, so a
-    replay needs only the new row indices.  Launching the ~30 kernels of a
-    step from Python costs more host time than their device time at batch
-    8192; a replay costs one graph launch."""
+    batch gather (rows named by ``idx``) and the learning-rate schedule,
+    forward and loss, backward, weight gradients, and Adam for every
+    parameter with the bf16 weights and their images; the schedule's counters
+    live on the device, so a replay needs only the new row indices."""
 
     def __init__(self, net, x_all, x_lo_all, y_all, batch, lr, total, step0, warmup,
                  b1, b2, eps):
@@ -536,41 +543,49 @@ class TrainingGraph:
         self.loss = torch.zeros((), dtype=torch.float32, device=dev)
         net._scratch(batch)
         lib, st = net.lib, net.stream.cuda_stream
+        # the gather kernel takes 32-byte rows of bf16 and float targets, as
+        # MLP.features and the surrogate lay them out
+        direct = (all(t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[1] == NIN
+                      for t in (x_all, x_lo_all))
+                  and y_all.dtype == torch.float32 and y_all.dim() == 1
+                  and len(x_all) == len(x_lo_all) == len(y_all)
+                  and all(t.is_contiguous() and t.data_ptr() % 16 == 0
+                          for t in (x_all, x_lo_all, y_all)))
+        schedule = (self.counters.data_ptr(), self.sched.data_ptr(), int(total), int(warmup),
+                    float(lr), b1, b2)
         net.stream.synchronize()
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph, stream=net.stream):
-            torch.index_select(x_all, 0, self.idx, out=self.xb)
-            torch.index_select(x_lo_all, 0, self.idx, out=self.xlb)
-            torch.index_select(y_all, 0, self.idx, out=self.yb)
-            net._check(lib.sasb200_lr_schedule(self.counters.data_ptr(), self.sched.data_ptr(),
-                                               int(total), int(warmup), float(lr), b1, b2, st),
-                       "lr_schedule")
-            net._pack_kernels()
+            if direct:
+                net._check(lib.sasb200_gather_batch(
+                    batch, len(y_all), self.idx.data_ptr(), x_all.data_ptr(),
+                    x_lo_all.data_ptr(), y_all.data_ptr(), self.xb.data_ptr(),
+                    self.xlb.data_ptr(), self.yb.data_ptr(), *schedule,
+                    net.err.data_ptr(), st), "gather_batch")
+            else:
+                torch.index_select(x_all, 0, self.idx, out=self.xb)
+                torch.index_select(x_lo_all, 0, self.idx, out=self.xlb)
+                torch.index_select(y_all, 0, self.idx, out=self.yb)
+                net._check(lib.sasb200_lr_schedule(*schedule, st), "lr_schedule")
             net._gradient_kernels(self.xb, self.xlb, self.yb, batch, self.loss, net.gbo)
-            grads = net.gW + net._vector_partials() + [net.gbo]
-            nt = len(net.params)
-            I32, VP = ct.c_int32*nt, ct.c_void_p*nt
-            sizes = [p.numel() for p in net.params]
-            splits = [net.splits if k < 9 else 1 for k in range(nt)]
-            shape = [(HID, NIN if k == 0 else HID) if k < 4 else (0, 0) for k in range(nt)]
-            net._check(lib.sasb200_adam_multi(
-                nt, I32(*sizes), I32(*splits), VP(*[g.data_ptr() for g in grads]),
-                VP(*[p.data_ptr() for p in net.params]), VP(*[m.data_ptr() for m in net.m]),
-                VP(*[v.data_ptr() for v in net.v]),
-                VP(*[net.Wb[k].data_ptr() if k < 4 else None for k in range(nt)]),
-                VP(*[net.WTb[k].data_ptr() if k < 4 else None for k in range(nt)]),
-                I32(*[r for r, _ in shape]), I32(*[c for _, c in shape]),
-                self.sched.data_ptr(), b1, b2, eps, st), "adam_multi")
+            net._adam(net.gW + net._vector_partials() + [net.gbo], [net.splits]*9 + [1],
+                      self.sched, lr, b1, b2, eps)
+        # what the graph reads and writes outlives the network's next, larger
+        # scratch
+        self._held = (x_all, x_lo_all, y_all, net.z_save, net.h_save, net.dz_save, net.out,
+                      net.dout, net.row_sums, net.gW, net.gb_part, net.gw_part, net.gbo)
 
     def step(self, idx):
         """One training step on rows `idx` (int64 device tensor of `batch`
         entries); returns the loss (a device scalar, overwritten by the
         next step)."""
         net = self.net
+        net._pack()          # current unless the weights were set from outside
         with net.torch.cuda.stream(net.stream):
             self.idx.copy_(idx)
             self.graph.replay()
         net.step_count += 1
+        net._packed = (net.step_count, net._wversion)
         return self.loss
 
 
@@ -672,8 +687,10 @@ class Surrogate:
             if log:
                 log("%s epoch %d loss %.3e" % (what, ep, losses[-1]))
         graph = None
-        if net.errors():
-            raise RuntimeError("tensor-core kernel reported a timeout")
+        code = net.errors()
+        if code:
+            raise RuntimeError("a row index outside the training data" if code == 5 else
+                               "tensor-core kernel reported a timeout")
         return losses
 
     def fit(self, cols, y, epochs=8, batch=8192, lr=2e-3, seed=0, log=None, huber=0.05,

@@ -79,3 +79,94 @@ def test_training_step_kernels(cuda, n):
         assert torch.equal(red[5 + l], db[l])
         close(red[1 + l], dW[l].view(net.splits, -1).double().sum(0),
               dW[l].view(net.splits, -1).double().abs().sum(0))
+
+
+def test_adam_pack_matches_adam_and_pack(cuda):
+    """One launch for every tensor, the bf16 copies and both weight images
+    against the per-tensor Adam and the packing kernels, bit for bit."""
+    import torch
+    from sasmodels_b200.surrogate import HID, NIN
+    rng = np.random.default_rng(7)
+    (a, *_), (b, *_) = _gpu_net(np.random.default_rng(8)), _gpu_net(np.random.default_rng(8))
+    g = torch.Generator(device="cuda").manual_seed(3)
+    lib, st = b.lib, b.stream.cuda_stream
+    for step in range(1, 3):
+        splits = 3
+        grads = [torch.randn(splits*p.numel() if k < 4 else p.numel(), device="cuda", generator=g)
+                 for k, p in enumerate(a.params)]
+        torch.cuda.synchronize()
+        a.apply_gradients(grads, 1e-2, splits)
+        for k, p in enumerate(b.params):
+            nb = NIN if k == 0 else HID
+            b._check(lib.sasb200_adam(
+                p.numel(), splits if k < 4 else 1, grads[k].data_ptr(), p.data_ptr(),
+                b.m[k].data_ptr(), b.v[k].data_ptr(), 1e-2, 0.9, 0.999, 1e-8, step,
+                b.Wb[k].data_ptr() if k < 4 else None, b.WTb[k].data_ptr() if k < 4 else None,
+                HID if k < 4 else 0, nb if k < 4 else 0, st), "adam")
+        b._pack_kernels()
+        a.stream.synchronize()
+        b.stream.synchronize()
+        for u, v in zip(a.params + a.m + a.v + a.Wb + a.WTb + [a.img, a.img_t],
+                        b.params + b.m + b.v + b.Wb + b.WTb + [b.img, b.img_t]):
+            assert torch.equal(u, v)
+
+
+def test_captured_batch_gather(cuda):
+    """The gather kernel and index_select (taken for strided data) give the
+    same step; rows past the data set are refused through the error flag."""
+    import torch
+    from sasmodels_b200.surrogate import MLP
+    n, B = 1000, 256
+    wide = torch.rand((n, 32), device="cuda").to(torch.bfloat16)
+    y = torch.randn(n, device="cuda")
+    idx = torch.randperm(n, device="cuda")[:B]
+    nets = []
+    for x in (wide[:, :16], wide[:, :16].contiguous()):
+        net = MLP(seed=6)
+        lo = torch.zeros_like(x)
+        torch.cuda.synchronize()
+        net.train_step(x[:B].contiguous(), lo[:B].contiguous(), y[:B], B, 1e-3)
+        graph = net.capture_training(x, lo, y, B, 1e-3, 100, 1)
+        for _ in range(3):
+            loss = graph.step(idx)
+        net.stream.synchronize()
+        assert net.errors() == 0
+        nets.append((net, float(loss.item()), graph))
+    assert nets[0][1] == nets[1][1]
+    for u, v in zip(nets[0][0].params, nets[1][0].params):
+        assert torch.equal(u, v)
+    bad = idx.clone()
+    bad[5] = n
+    net, _, graph = nets[1]
+    torch.cuda.synchronize()
+    graph.step(bad)
+    net.stream.synchronize()
+    assert net.errors() == 5
+
+
+def test_captured_step_follows_load_state(cuda):
+    """Weights set from outside after the capture are the ones it trains."""
+    import torch
+    from sasmodels_b200.surrogate import MLP
+    B = 128
+    x = torch.rand((B, 16), device="cuda").to(torch.bfloat16)
+    lo, y = torch.zeros_like(x), torch.randn(B, device="cuda")
+    idx = torch.arange(B, device="cuda")
+    a, b = MLP(seed=1), MLP(seed=2)
+    torch.cuda.synchronize()
+    out = []
+    for net, late in ((a, True), (b, False)):
+        if not late:
+            net.load_state(a_state)
+            torch.cuda.synchronize()
+        graph = net.capture_training(x, lo, y, B, 1e-3, 100, 1)
+        if late:
+            a_state = MLP(seed=9).state()
+            net.load_state(a_state)
+            torch.cuda.synchronize()
+        loss = graph.step(idx)
+        net.stream.synchronize()
+        out.append((float(loss.item()), [p.clone() for p in net.params]))
+    assert out[0][0] == out[1][0]
+    for u, v in zip(out[0][1], out[1][1]):
+        assert torch.equal(u, v)
