@@ -24,6 +24,8 @@
 //                  at once (a dedicated MMA warp, two TMEM accumulators,
 //                  layer l+1's MMAs under layer l's epilogue chunk by chunk);
 //                  serves inference and the training forward.
+//   mlp_serve_pairs   inference over many tiles: pairs of SMs (cta_group::2), two
+//                  tiles in flight on each (mlp_pairs.cuh).
 //   mlp_backward_t, mlp_weight_grads   the training step's backward and weight
 //                  gradients on tiled planes (mlp_train.cuh).
 //   gemm_nt        C_split = A[M x K] B[N x K]^T over a K range (split-K).
@@ -1356,6 +1358,7 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
 }
 
 #include "mlp_train.cuh"
+#include "mlp_pairs.cuh"
 
 // ---------------------------------------------------------------- backward --
 // mlp_backward_p: the backward pass through the three 256 x 256 layers as a
@@ -1591,7 +1594,7 @@ int32_t sasb200_mlp_infer(int32_t n, int32_t n_pad, const void *x, const void *x
     if (reinterpret_cast<uintptr_t>(img) % 16)
         return (std::snprintf(errbuf(), 256, "weight image must be 16-byte aligned"), -1);
     if (n_pad == 0) return 0;
-    InferParams prm;
+    InferParams prm = {};
     prm.img = static_cast<const uint8_t *>(img);
     for (int l = 0; l < 4; ++l) prm.b[l] = b[l];
     prm.w_out = w_out;
@@ -1616,7 +1619,8 @@ int32_t sasb200_mlp_infer(int32_t n, int32_t n_pad, const void *x, const void *x
 }
 
 // out[n] for x, x_lo [n_pad x 16] with the packed weights through the
-// overlapped kernel (mlp_serve), and, when z_save/h_save are given, the
+// overlapped kernels (mlp_serve; mlp_serve_pairs where a CTA has several tiles
+// and no planes are wanted: the same values), and, when z_save/h_save are given, the
 // pre-activations and activations of all four layers ([4][n_pad x 256] bf16
 // each, those of mlp_infer) for training; persistent grid of at most
 // `blocks` CTAs (0 = one per SM).  err receives 1, 2, 3 or 4 if a pipeline
@@ -1636,7 +1640,7 @@ int32_t sasb200_mlp_serve(int32_t n, int32_t n_pad, const void *x, const void *x
         if (!b[l] || reinterpret_cast<uintptr_t>(b[l]) % 4)
             return (std::snprintf(errbuf(), 256, "bad bias pointer"), -1);
     if (n_pad == 0) return 0;
-    InferParams prm;
+    InferParams prm = {};
     prm.img = static_cast<const uint8_t *>(img);
     for (int l = 0; l < 4; ++l) prm.b[l] = b[l];
     prm.w_out = w_out;
@@ -1653,9 +1657,14 @@ int32_t sasb200_mlp_serve(int32_t n, int32_t n_pad, const void *x, const void *x
         blocks = sms > 0 ? sms : 1;
     }
     if (blocks > n_tiles) blocks = n_tiles;
-    const auto kernel = z_save ? mlp_serve<SV_ROUND, PLANES_ROWS> : mlp_serve<SV_ROUND, PLANES_NONE>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
-    kernel<<<blocks, SV_THREADS, SV_SMEM, (cudaStream_t)stream>>>(
+    // by pairs of CTAs, two tiles in flight, where a CTA has several tiles
+    const bool in_pairs = !z_save && blocks > 1 && n_tiles > SP_TILES*blocks;
+    if (in_pairs) blocks &= ~1;
+    const auto kernel = z_save ? mlp_serve<SV_ROUND, PLANES_ROWS>
+                               : (in_pairs ? mlp_serve_pairs : mlp_serve<SV_ROUND, PLANES_NONE>);
+    const int bytes = in_pairs ? SP_SMEM : SV_SMEM, threads = in_pairs ? SP_THREADS : SV_THREADS;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    kernel<<<blocks, threads, bytes, (cudaStream_t)stream>>>(
         n, n_tiles, static_cast<const __nv_bfloat16 *>(x),
         static_cast<const __nv_bfloat16 *>(x_lo), prm, out, err);
     return status("mlp_serve");

@@ -54,6 +54,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
     return done != 0;
 }
 
+// Whether the phase with the given parity is complete, without suspending.
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return done != 0;
+}
+
 // Bounded wait for the phase with the given parity to complete.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity)
 {
@@ -77,6 +88,29 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(bar)) : "memory");
 }
 
+// ---- CTA pairs (clusters of two) -----------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// All threads of both CTAs (converged warps): arrive and wait.
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Arrive once on the barrier at this offset in CTA `rank` of the cluster.
+// Relaxed: see mlp_serve_pairs for what the count stands for.
+__device__ __forceinline__ void mbar_arrive_relaxed_cta(uint64_t *bar, uint32_t rank)
+{
+    asm volatile("{\n\t.reg .b32 remote;\n\t"
+                 "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
+                 "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [remote];\n\t}"
+                 :: "r"(smem_u32(bar)), "r"(rank) : "memory");
+}
+
 // ---- release/acquire flags in shared memory ------------------------------
 __device__ __forceinline__ uint32_t ld_acquire_shared(const uint32_t *p)
 {
@@ -88,12 +122,17 @@ __device__ __forceinline__ void st_release_shared(uint32_t *p, uint32_t v)
 {
     asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" :: "r"(smem_u32(p)), "r"(v) : "memory");
 }
-// Bounded spin until *p >= target (acquire).
+// Bounded spin until *p >= target (acquire); returns the value, below target when
+// the limit ran out.
+__device__ __forceinline__ uint32_t spin_acquire_until(const uint32_t *p, uint32_t target)
+{
+    uint32_t v = 0;
+    for (uint32_t i = 0; i < WAIT_LIMIT && v < target; ++i) v = ld_acquire_shared(p);
+    return v;
+}
 __device__ __forceinline__ bool spin_acquire_ge(const uint32_t *p, uint32_t target)
 {
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
-        if (ld_acquire_shared(p) >= target) return true;
-    return false;
+    return spin_acquire_until(p, target) >= target;
 }
 
 // ---- bulk copy (TMA engine, untiled, no multicast) --------------------------
@@ -159,6 +198,19 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
                  :: "r"(taddr), "r"(ncols) : "memory");
 }
 
+// The same for a CTA pair (one warp of each CTA).
+__device__ __forceinline__ void tmem_alloc2(uint32_t *slot, uint32_t ncols)
+{
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n\t"
+                 "tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;"
+                 :: "r"(smem_u32(slot)), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols)
+{
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;"
+                 :: "r"(taddr), "r"(ncols) : "memory");
+}
+
 // 32 TMEM lanes x 16 consecutive 32-bit columns into 16 registers (one row
 // per thread of the warp); pair with tmem_wait_ld before use.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
@@ -173,6 +225,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
 __device__ __forceinline__ void tmem_wait_ld()
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// A wait for loads into these registers: they are operands, so that no use of
+// them can be scheduled before it (a statement takes 30 of them at most).
+__device__ __forceinline__ void tmem_tie16(uint32_t (&a)[16])
+{
+    asm volatile("" : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]),
+                      "+r"(a[6]), "+r"(a[7]), "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]),
+                      "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15]) :: "memory");
 }
 
 // 32 TMEM lanes x 8 columns; tmem_wait_ld8 on the same registers completes
@@ -231,6 +292,27 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                  :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
                  : "memory");
+}
+
+// The same over a CTA pair, issued by the CTA of rank 0: M rows, half of them in
+// each CTA's A tile and TMEM, half of the N rows of B in each CTA's shared
+// memory, at the same offsets in both.
+__device__ __forceinline__ void mma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                              uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+                 : "memory");
+}
+// Arrive on the barrier at this offset in both CTAs of the pair once every pair
+// MMA this thread issued so far has completed.
+__device__ __forceinline__ void mma_commit_pair(uint64_t *bar)
+{
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster"
+                 ".multicast::cluster.b64 [%0], %1;"
+                 :: "r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
 // Arrive on *bar once every MMA this thread issued so far has completed.

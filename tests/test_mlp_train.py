@@ -170,3 +170,29 @@ def test_captured_step_follows_load_state(cuda):
     assert out[0][0] == out[1][0]
     for u, v in zip(out[0][1], out[1][1]):
         assert torch.equal(u, v)
+
+
+@pytest.mark.parametrize("n, blocks", [(128*3, 2), (128*4 - 5, 2), (128*5, 2), (128*9 + 1, 4),
+                                       (128*149, 0), (128*297 + 1, 0), (128*1500, 5)])
+def test_serve_pairs_is_serve(cuda, n, blocks):
+    """Pairs of CTAs with two tiles in flight against one tile at a time, bit
+    for bit: one and several double tiles per cluster, odd counts of tiles and
+    of double tiles, an odd limit of blocks; rows beyond n are not written."""
+    import torch
+    from sasmodels_b200.surrogate import pad128
+    rng = np.random.default_rng(n)
+    net, *_ = _gpu_net(rng)
+    x, xlo, _, _ = _inputs(rng, n, pad128(n))
+    torch.cuda.synchronize()
+    net.serve(x, xlo, n, blocks=blocks)
+    net._infer_out.fill_(float("nan"))
+    torch.cuda.synchronize()
+    a = net.serve(x, xlo, n, blocks=blocks)
+    net.stream.synchronize()
+    a = a.clone()
+    torch.cuda.synchronize()
+    b = net.serve(x, xlo, n, blocks=pad128(n)//128)     # one tile per CTA
+    net.stream.synchronize()
+    assert net.errors() == 0
+    assert torch.equal(a[:n], b[:n])
+    assert torch.isnan(a[n:]).all()
