@@ -967,6 +967,94 @@ __device__ __forceinline__ size_t tiled_at(int l, int n_tiles, int tile, int kg,
     return ((size_t)l*n_tiles + tile)*TILE_ELEMS + (size_t)kg*GROUP_ELEMS + 8*row;
 }
 
+// ------------------------------------------------------- paired arithmetic --
+// Two FP32 lanes in one register pair: each half rounded to nearest.
+__device__ __forceinline__ uint64_t f2_pack(float a, float b)
+{
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// silu of two accumulator columns plus bias (see silu())
+__device__ __forceinline__ uint64_t silu2(uint32_t a0, uint32_t a1, uint64_t bias)
+{
+    const uint64_t z = f2_add(f2_pack(__uint_as_float(a0), __uint_as_float(a1)), bias);
+    const uint64_t hz = f2_mul(z, f2_pack(0.5f, 0.5f));
+    float x0, x1, t0, t1;
+    f2_unpack(hz, x0, x1);
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t0) : "f"(x0));
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t1) : "f"(x1));
+    return f2_fma(hz, f2_pack(t0, t1), hz);
+}
+
+// 8 columns of a row, from the accumulators r[at ..]: silu, then the hi and lo
+// halves (one 16-byte unit each)
+__device__ __forceinline__ void silu_columns(const uint32_t (&r)[16], int at, const float *bias,
+                                             uint4 &hi, uint4 &lo)
+{
+    const ulonglong2 *b2 = reinterpret_cast<const ulonglong2 *>(bias + at);
+    const uint64_t minus1 = f2_pack(-1.0f, -1.0f);
+    uint32_t *hp = &hi.x, *lp = &lo.x;
+    #pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const ulonglong2 b = b2[e];
+        #pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const uint64_t h = silu2(r[at + 4*e + 2*q], r[at + 4*e + 2*q + 1], q ? b.y : b.x);
+            float x, y, dx, dy;
+            f2_unpack(h, x, y);
+            const uint32_t u = pack2(x, y);
+            f2_unpack(f2_fma(f2_pack(bf_lo(u), bf_hi(u)), minus1, h), dx, dy);
+            hp[2*e + q] = u;
+            lp[2*e + q] = pack2(dx, dy);
+        }
+    }
+}
+
+// dot + sum over 8 columns of silu(acc + bias) wo, in column order
+__device__ __forceinline__ float dot8(const uint32_t (&r)[8], const float *bias, const float *wo,
+                                      float dot)
+{
+    const ulonglong2 *b2 = reinterpret_cast<const ulonglong2 *>(bias);
+    const float4 *w4 = reinterpret_cast<const float4 *>(wo);
+    #pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const ulonglong2 b = b2[e];
+        const float4 w = w4[e];
+        float h0, h1, h2, h3;
+        f2_unpack(silu2(r[4*e], r[4*e + 1], b.x), h0, h1);
+        f2_unpack(silu2(r[4*e + 2], r[4*e + 3], b.y), h2, h3);
+        dot = fmaf(h0, w.x, dot);
+        dot = fmaf(h1, w.y, dot);
+        dot = fmaf(h2, w.z, dot);
+        dot = fmaf(h3, w.w, dot);
+    }
+    return dot;
+}
+
 // ------------------------------------------------------------------ serve --
 // mlp_serve: the forward pass (inference, or training with the z/h planes)
 // with the tensor core and the epilogue busy at the same time.  Arithmetic per element as mlp_infer
@@ -976,27 +1064,27 @@ __device__ __forceinline__ size_t tiled_at(int l, int n_tiles, int tile, int kg,
 //
 // Roles, 19 warps per CTA (one CTA per SM, persistent over 128-row tiles):
 //   warps 0-15  epilogue.  Warp w reads the TMEM lanes of its quadrant
-//               (rows 32(w%4) .. +31) and, of every 32-column chunk, the 8
-//               columns at 8(w/4).  Chunk by chunk: bias + SiLU + split into
-//               the activation tile, then one arrive per warp on
-//               act_ready[chunk].
+//               (rows 32(w%4) .. +31) and the 16 columns at 16(w/4) of every 64,
+//               all of them before the first is used (which frees the
+//               accumulator); 64 by 64 columns: bias + SiLU + split into the
+//               activation tile, then one arrive per warp on act_ready[64 columns];
+//               but for the first and the last it comes behind the arithmetic
+//               of the next 64, under which the stores land.  In the last layer the 8 columns at 8(w/4) of every 32.
 //   warp 16     lane 0 issues every MMA; all lanes load the next tile's
 //               features while the tensor core runs the last layer.  An MMA
 //               issue holds its thread for about the tensor core's time for
 //               the previous MMA, so this lane does no barrier waits of its
 //               own for layers 1-3: it spins on a counter of ready chunks.
 //   warp 17     the bulk-copy producer of the weight ring (as mlp_infer).
-//   warp 18     the waiter: for every chunk of layers 1-3 in MMA order, waits
-//               for the accumulator to be free, the activations and the
-//               weights, then publishes the chunk (release store of the
-//               count of ready chunks).
+//   warps 18,   one lane each: count the chunks whose input is written (and whose
+//        19     accumulator is free), and those whose weights have landed
+//               (release stores), so that neither wait is behind the other.
 // Two TMEM accumulators (columns [0, 256) and [256, 512)): layer l of a tile
-// accumulates into acc[l & 1], so layer l+1's MMAs start on chunk c of its
-// input as soon as the epilogue of layer l has written that chunk, while the
-// epilogue still drains acc[l & 1].  The activations are rewritten in place:
-// the epilogue of layer l starts only after every MMA of layer l (the
-// readers of the old activations) has completed.  acc_empty[a] tells the MMA
-// warp that all sixteen epilogue warps have finished their TMEM loads of
+// accumulates into acc[l & 1], so layer l+1's MMAs start on the first columns of
+// its input as soon as the epilogue of layer l has written them.  The activations
+// are rewritten in place: the epilogue of layer l starts only after every MMA of
+// layer l (the readers of the old activations) has completed.  acc_empty[a] tells
+// the MMA warp that all sixteen epilogue warps have finished their TMEM loads of
 // acc[a], before the next layer that accumulates there.
 //
 // Barrier phases (all parity waits, bounded): per tile acc_full[a] and
@@ -1004,16 +1092,22 @@ __device__ __forceinline__ size_t tiled_at(int l, int n_tiles, int tile, int kg,
 // (inputs of layers 1-3), dot_bar[quadrant] once; none can run two phases
 // ahead of its waiter because each completion needs the waiter's previous
 // step (argued at each wait below).
+//
+// One tile per CTA: 17.5 us (19.0 with one warp waiting for a chunk's three barriers
+// in turn, an arrival per 32 columns, and the features loaded 16 bytes at a time).
+// Bound by the chain of one tile: 4 x (commit, 16 columns of epilogue, hand-over,
+// 8 chunks of MMA at 540-690 cycles).
 constexpr int SV_EPI_WARPS = 16;
 constexpr int SV_EPI = 32*SV_EPI_WARPS;                    // 512 epilogue threads
 constexpr int SV_MMA_WARP = SV_EPI_WARPS;
 constexpr int SV_PROD_WARP = SV_EPI_WARPS + 1;
-constexpr int SV_WAIT_WARP = SV_EPI_WARPS + 2;
-constexpr int SV_THREADS = SV_EPI + 96;
+constexpr int SV_ACT_WARP = SV_EPI_WARPS + 2;
+constexpr int SV_WEIGHT_WARP = SV_EPI_WARPS + 3;
+constexpr int SV_THREADS = SV_EPI + 128;
 constexpr int SV_COLS = KCI/(SV_EPI_WARPS/4);              // 8 columns of a chunk per warp
 constexpr int SV_PARAMS = 5*HID;                           // b[0..3], w_out (floats)
 constexpr int SV_SMEM = 2*ACT_BYTES + STAGES*CHUNK_BYTES + W0_BYTES + 4*X_BYTES + 4*SV_PARAMS;
-constexpr int SV_ROUND = 1;                                // chunks per epilogue round
+constexpr int SV_UNITS = HID/64;                           // 64 columns per hand-over
 static_assert(SV_COLS == 8, "the epilogue moves one 16-byte unit per row and chunk");
 
 // Bounded wait by every lane of a warp on one mbarrier phase; the warp agrees
@@ -1024,17 +1118,30 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity)
     return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity)) != 0;
 }
 
-// z = acc + bias and h = silu(z) for 8 columns.
-__device__ __forceinline__ void sv_silu8(const uint32_t (&a)[8], const float *bias, float (&z)[8],
-                                         float (&h)[8])
+// z = acc + bias and h = silu(z) for 8 columns, accumulators r[at ..].
+template <int N>
+__device__ __forceinline__ void sv_silu8(const uint32_t (&r)[N], int at, const float *bias,
+                                         float (&z)[8], float (&h)[8])
 {
-    const float4 b0 = *reinterpret_cast<const float4 *>(bias);
-    const float4 b1 = *reinterpret_cast<const float4 *>(bias + 4);
+    const float4 b0 = *reinterpret_cast<const float4 *>(bias + at);
+    const float4 b1 = *reinterpret_cast<const float4 *>(bias + at + 4);
     const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
     #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        z[j] = __uint_as_float(a[j]) + bb[j];
+        z[j] = __uint_as_float(r[at + j]) + bb[j];
         h[j] = silu(z[j]);
+    }
+}
+
+// hi = bf16(h), lo = bf16(h - hi) of 8 columns, one 16-byte unit each
+__device__ __forceinline__ void split8(const float (&h)[8], uint4 &hi, uint4 &lo)
+{
+    uint32_t *hp = &hi.x, *lp = &lo.x;
+    #pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const uint32_t u = pack2(h[2*e], h[2*e + 1]);
+        hp[e] = u;
+        lp[e] = pack2(h[2*e] - bf_lo(u), h[2*e + 1] - bf_hi(u));
     }
 }
 
@@ -1049,10 +1156,38 @@ __device__ __forceinline__ void save8(__nv_bfloat16 *dst, const float (&v)[8])
     *reinterpret_cast<uint4 *>(dst) = u;
 }
 
+// An MMA lane's view of a count of ready units: covers(n) waits until n are ready
+// (bounded), reading the count only when the last value does not cover n.
+struct ReadyCount {
+    const uint32_t *at;
+    uint32_t known = 0;
+    __device__ explicit ReadyCount(const uint32_t *p) : at(p) {}
+    __device__ __forceinline__ bool covers(uint32_t n)
+    {
+        if (known < n) known = tc::spin_acquire_until(at, n);
+        return known >= n;
+    }
+};
+// The same of two counts, each kept by a warp of its own: chunks whose input is
+// written (x) and chunks whose weights have landed (y).
+struct ReadyCounts {
+    const uint2 *at;
+    uint32_t known = 0;
+    __device__ explicit ReadyCounts(const uint2 *p) : at(p) {}
+    __device__ __forceinline__ bool covers(uint32_t n)
+    {
+        for (uint32_t i = 0; i < tc::WAIT_LIMIT && known < n; ++i) {
+            const uint2 v = tc::ld_acquire_shared2(at);
+            known = min(v.x, v.y);
+        }
+        return known >= n;
+    }
+};
+
 // PLANES: none (inference), row-major z/h planes, or a training step's tiled
 // planes with the loss gradient of every row.
 enum { PLANES_NONE, PLANES_ROWS, PLANES_TILED };
-template <int RND, int PLANES>
+template <int PLANES>
 __global__ void __launch_bounds__(SV_THREADS, 1)
 mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
           const __nv_bfloat16 *__restrict__ x_lo, InferParams prm, float *__restrict__ out,
@@ -1065,9 +1200,10 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
     uint8_t *w0 = ring + STAGES*CHUNK_BYTES;
     uint8_t *xs = w0 + W0_BYTES;                  // [2 buffers][hi, lo] x X_BYTES
     float *par = reinterpret_cast<float *>(xs + 4*X_BYTES);
-    __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], act_ready[CHUNKS_PER_LAYER];
+    __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], act_ready[SV_UNITS];
     __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], dot_bar[4], w0_bar, drain;
-    __shared__ uint32_t tmem_slot, ready_seq;
+    __shared__ uint32_t tmem_slot;
+    __shared__ __align__(8) uint2 ready_seq;
     __shared__ float dot_part[3][TM];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int my_tiles = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x)/gridDim.x + 1 : 0;
@@ -1081,7 +1217,7 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             tc::mbar_init(&full[s], 1);
             tc::mbar_init(&empty[s], 1);
         }
-        for (int c = 0; c < CHUNKS_PER_LAYER; ++c) tc::mbar_init(&act_ready[c], SV_EPI_WARPS);
+        for (int c = 0; c < SV_UNITS; ++c) tc::mbar_init(&act_ready[c], SV_EPI_WARPS);
         for (int a = 0; a < 2; ++a) {
             tc::mbar_init(&acc_full[a], 1);
             tc::mbar_init(&acc_empty[a], SV_EPI_WARPS);
@@ -1089,7 +1225,7 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         for (int q = 0; q < 4; ++q) tc::mbar_init(&dot_bar[q], SV_EPI_WARPS/4 - 1);
         tc::mbar_init(&w0_bar, 1);
         tc::mbar_init(&drain, 1);
-        ready_seq = 0;
+        ready_seq = make_uint2(0u, 0u);
         tc::mbar_fence_init();
     }
     tc::fence_before_sync();
@@ -1121,33 +1257,43 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             ok = tc::mbar_wait(&w0_bar, 0u) && ok;
             if (!ok) atomicExch(err, 2);
         }
-    } else if (warp == SV_WAIT_WARP) {
-        // ---- waiter: readiness of every chunk of layers 1-3, in MMA order ----
-        // A chunk is ready when its accumulator is free (chunk 0 of a layer),
-        // its input activations are written and its weights have landed;
-        // the count of ready chunks is published with a release store that
-        // the MMA lane reads with acquire loads.
-        bool ok = true;
-        int chunk = 0;
-        for (int k = 0; k < my_tiles && ok; ++k) {
-            for (int l = 1; l < 4 && ok; ++l) {
-                const int a = l & 1;
-                // previous reader of acc[a]: layer 3 of tile k-1 for l = 1
-                // (completion 2k-1), layer l-2 of this tile for l = 2, 3
-                // (completion 2k); the next completion needs this layer's
-                // MMAs, which wait for what is published here
-                if ((l >= 2 || k > 0) && !(ok = warp_wait(&acc_empty[a], l >= 2 ? 0u : 1u)))
-                    break;
-                for (int c = 0; c < CHUNKS_PER_LAYER; ++c, ++chunk) {
-                    // chunk c of this layer's input: completion 3k + l - 1
-                    if (!(ok = warp_wait(&act_ready[c], (uint32_t)((3*k + l - 1) & 1))
-                               && warp_wait(&full[chunk % STAGES], (uint32_t)((chunk/STAGES) & 1))))
+    } else if (warp == SV_ACT_WARP) {
+        // ---- inputs: chunks of layers 1-3 whose accumulator is free and whose
+        // activations are written, in MMA order ----
+        if (lane == 0) {
+            bool ok = true;
+            uint32_t chunk = 0;
+            for (int k = 0; k < my_tiles && ok; ++k) {
+                for (int l = 1; l < 4 && ok; ++l) {
+                    // previous reader of acc[l & 1]: layer 3 of tile k-1 for l = 1
+                    // (completion 2k-1), layer l-2 of this tile for l = 2, 3
+                    // (completion 2k); the next completion needs this layer's
+                    // MMAs, which wait for what is published here
+                    if ((l >= 2 || k > 0)
+                        && !(ok = tc::mbar_wait(&acc_empty[l & 1], l >= 2 ? 0u : 1u)))
                         break;
-                    if (lane == 0) tc::st_release_shared(&ready_seq, (uint32_t)(chunk + 1));
+                    for (int q = 0; q < SV_UNITS; ++q) {
+                        // 64 columns of this layer's input: completion 3k + l - 1
+                        if (!(ok = tc::mbar_wait(&act_ready[q], (uint32_t)((3*k + l - 1) & 1)))) break;
+                        chunk += CHUNKS_PER_LAYER/SV_UNITS;
+                        tc::st_release_shared(&ready_seq.x, chunk);
+                    }
                 }
             }
+            if (!ok) atomicExch(err, 4);
         }
-        if (!ok && lane == 0) atomicExch(err, 4);
+        __syncwarp();
+    } else if (warp == SV_WEIGHT_WARP) {
+        // ---- weights: chunks that have landed ----
+        if (lane == 0) {
+            bool ok = true;
+            const uint32_t total = (uint32_t)(my_tiles*CHUNKS_PER_TILE);
+            for (uint32_t i = 0; i < total && ok; ++i)
+                if ((ok = tc::mbar_wait(&full[i % STAGES], (i/STAGES) & 1u)))
+                    tc::st_release_shared(&ready_seq.y, i + 1);
+            if (!ok) atomicExch(err, 4);
+        }
+        __syncwarp();
     } else if (warp == SV_MMA_WARP) {
         // ---- MMA issue (lane 0) and feature loads (all lanes) ----
         constexpr uint32_t idesc = tc::idesc_bf16(TM, HID);
@@ -1155,19 +1301,27 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         auto load_x = [&](int k) {
             uint8_t *xb = xs + (k & 1)*2*X_BYTES;
             const int row0 = (blockIdx.x + k*gridDim.x)*TM;
-            for (int i = lane; i < 2*TM; i += 32) {
-                const int r = i >> 1, c = (i & 1)*8;
-                const size_t g = (size_t)(row0 + r)*NIN + c;
-                *reinterpret_cast<uint4 *>(xb + tc::kmajor_offset<TM>(r, c)) =
-                    *reinterpret_cast<const uint4 *>(x + g);
-                *reinterpret_cast<uint4 *>(xb + X_BYTES + tc::kmajor_offset<TM>(r, c)) =
-                    *reinterpret_cast<const uint4 *>(x_lo + g);
+            uint4 hi[2*TM/32], lo[2*TM/32];          // every load in flight at once
+            #pragma unroll
+            for (int j = 0; j < 2*TM/32; ++j) {
+                const int i = lane + 32*j;
+                const size_t g = (size_t)(row0 + (i >> 1))*NIN + (i & 1)*8;
+                hi[j] = *reinterpret_cast<const uint4 *>(x + g);
+                lo[j] = *reinterpret_cast<const uint4 *>(x_lo + g);
+            }
+            #pragma unroll
+            for (int j = 0; j < 2*TM/32; ++j) {
+                const int i = lane + 32*j;
+                const uint32_t at = tc::kmajor_offset<TM>(i >> 1, (i & 1)*8);
+                *reinterpret_cast<uint4 *>(xb + at) = hi[j];
+                *reinterpret_cast<uint4 *>(xb + X_BYTES + at) = lo[j];
             }
             tc::fence_async_smem();
             __syncwarp();
         };
         bool ok = true;
         int chunk = 0;
+        ReadyCounts count(&ready_seq);
         if (my_tiles > 0) load_x(0);
         ok = warp_wait(&w0_bar, 0u);
         for (int k = 0; k < my_tiles && ok; ++k) {
@@ -1182,14 +1336,14 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 tc::mma_bf16(tmem, tc::kmajor_desc<TM>(xb, 0), bdesc, idesc, 0u);
                 tc::mma_bf16(tmem, tc::kmajor_desc<TM>(xb + X_BYTES, 0), bdesc, idesc, 1u);
                 tc::mma_commit(&acc_full[0]);
-                // layers 1-3: each chunk as soon as the waiter has published
+                // layers 1-3: each chunk as soon as both counts cover
                 // it.  An MMA issue holds this thread about as long as the
                 // tensor core takes for the previous one, so nothing else
                 // runs on this thread between chunks.
                 for (int l = 1; l < 4 && ok; ++l) {
                     const uint32_t d = tmem + (uint32_t)(HID*(l & 1));
                     for (int c = 0; c < CHUNKS_PER_LAYER; ++c, ++chunk) {
-                        if (!(ok = tc::spin_acquire_ge(&ready_seq, (uint32_t)(chunk + 1)))) break;
+                        if (!(ok = count.covers((uint32_t)(chunk + 1)))) break;
                         tc::fence_after_sync();
                         const int s = chunk % STAGES;
                         const uint32_t b_addr = tc::smem_u32(ring + s*CHUNK_BYTES);
@@ -1240,78 +1394,84 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 if (!(ok = warp_wait(&acc_full[a], (uint32_t)(l >> 1))))
                     break;
                 tc::fence_after_sync();
-                const uint32_t acc = tmem + lane_base + (uint32_t)(HID*a + cs);
-                const float *bias = par + l*HID + cs;
                 float dot = 0.0f;
-                // RND chunks per round: their TMEM loads are issued together,
-                // one round ahead of the arithmetic, and one proxy fence
-                // covers their stores
-                uint32_t ra[RND][8], rb[RND][8];
-                #pragma unroll
-                for (int r = 0; r < RND; ++r) tc::tmem_ld8(acc + (uint32_t)(KCI*r), ra[r]);
-                #pragma unroll
-                for (int r = 0; r < RND; ++r) tc::tmem_wait_ld8(ra[r]);
-                #pragma unroll
-                for (int j = 0; j < CHUNKS_PER_LAYER/RND; ++j) {
-                    const bool more = j + 1 < CHUNKS_PER_LAYER/RND;
-                    if (more) {
-                        #pragma unroll
-                        for (int r = 0; r < RND; ++r)
-                            tc::tmem_ld8(acc + (uint32_t)(KCI*(RND*(j + 1) + r)), rb[r]);
-                    } else {
-                        // all TMEM loads of acc[a] have completed
-                        tc::fence_before_sync();
-                        __syncwarp();
-                        if (lane == 0) tc::mbar_arrive(&acc_empty[a]);
-                    }
+                // 8 columns of a plane of this layer, for this row
+                auto plane_at = [&](int col) {
+                    return PLANES == PLANES_TILED ? tiled_at(l, n_tiles, row0/TM, col/8, row)
+                                                  : (size_t)l*plane + (size_t)(row0 + row)*HID + col;
+                };
+                if (l < 3) {
+                    // 16 columns of every 64
+                    const uint32_t acc = tmem + lane_base + (uint32_t)(HID*a + 16*slot);
+                    const float *bias = par + l*HID + 16*slot;
+                    uint32_t r[SV_UNITS][16];
                     #pragma unroll
-                    for (int r = 0; r < RND; ++r) {
-                        const int c = RND*j + r;
-                        float z[8], h[8];
-                        sv_silu8(ra[r], bias + KCI*c, z, h);
-                        if (PLANES != PLANES_NONE) {   // the planes of every layer
-                            const size_t at = PLANES == PLANES_TILED
-                                ? tiled_at(l, n_tiles, row0/TM, 4*c + slot, row)
-                                : (size_t)l*plane + (size_t)(row0 + row)*HID + KCI*c + cs;
+                    for (int q = 0; q < SV_UNITS; ++q) tc::tmem_ld16(acc + (uint32_t)(64*q), r[q]);
+                    tc::tmem_wait_ld();
+                    #pragma unroll
+                    for (int q = 0; q < SV_UNITS; ++q) tc::tmem_tie16(r[q]);
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&acc_empty[a]);
+                    #pragma unroll
+                    for (int q = 0; q < SV_UNITS; ++q) {
+                        uint4 hi[2], lo[2];
+                        #pragma unroll
+                        for (int g = 0; g < 2; ++g) {
+                            if (PLANES == PLANES_NONE) {
+                                silu_columns(r[q], 8*g, bias + 64*q, hi[g], lo[g]);
+                            } else {
+                                float z[8], h[8];
+                                sv_silu8(r[q], 8*g, bias + 64*q, z, h);
+                                split8(h, hi[g], lo[g]);
+                                const size_t at = plane_at(64*q + 16*slot + 8*g);
+                                save8(prm.z_save + at, z);
+                                *reinterpret_cast<uint4 *>(prm.h_save + at) = hi[g];
+                            }
+                            // the stores of the 64 columns before have had time to land
+                            if (g == 0 && q > 1) {
+                                tc::fence_async_smem();
+                                __syncwarp();
+                                if (lane == 0) tc::mbar_arrive(&act_ready[q - 1]);
+                            }
+                        }
+                        #pragma unroll
+                        for (int g = 0; g < 2; ++g) {
+                            const uint32_t off = tc::kmajor_offset<TM>(row, 64*q + 16*slot + 8*g);
+                            *reinterpret_cast<uint4 *>(act + off) = hi[g];
+                            *reinterpret_cast<uint4 *>(act_lo + off) = lo[g];
+                        }
+                        // the tensor core is waiting for the first and the last
+                        if (q == 0 || q == SV_UNITS - 1) {
+                            tc::fence_async_smem();
+                            __syncwarp();
+                            if (lane == 0) tc::mbar_arrive(&act_ready[q]);
+                        }
+                    }
+                } else {
+                    // the output dot: 8 columns of every 32
+                    const uint32_t acc = tmem + lane_base + (uint32_t)(HID*a + cs);
+                    const float *bias = par + 3*HID + cs, *wo = par + 4*HID + cs;
+                    uint32_t r[CHUNKS_PER_LAYER][8];
+                    #pragma unroll
+                    for (int c = 0; c < CHUNKS_PER_LAYER; ++c) tc::tmem_ld8(acc + (uint32_t)(KCI*c), r[c]);
+                    #pragma unroll
+                    for (int c = 0; c < CHUNKS_PER_LAYER; ++c) tc::tmem_wait_ld8(r[c]);
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&acc_empty[a]);
+                    #pragma unroll
+                    for (int c = 0; c < CHUNKS_PER_LAYER; ++c) {
+                        if (PLANES == PLANES_NONE) {
+                            dot = dot8(r[c], bias + KCI*c, wo + KCI*c, dot);
+                        } else {
+                            float z[8], h[8];
+                            sv_silu8(r[c], 0, bias + KCI*c, z, h);
+                            const size_t at = plane_at(KCI*c + cs);
                             save8(prm.z_save + at, z);
                             save8(prm.h_save + at, h);
-                        }
-                        if (l < 3) {
-                            uint4 hi, lo;
-                            uint32_t *hp = &hi.x, *lp = &lo.x;
                             #pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const uint32_t u = pack2(h[2*e], h[2*e + 1]);
-                                hp[e] = u;
-                                lp[e] = pack2(h[2*e] - bf_lo(u), h[2*e + 1] - bf_hi(u));
-                            }
-                            const uint32_t off = tc::kmajor_offset<TM>(row, KCI*c + cs);
-                            *reinterpret_cast<uint4 *>(act + off) = hi;
-                            *reinterpret_cast<uint4 *>(act_lo + off) = lo;
-                        } else {
-                            const float *wp = par + 4*HID + KCI*c + cs;
-                            const float4 w0v = *reinterpret_cast<const float4 *>(wp);
-                            const float4 w1v = *reinterpret_cast<const float4 *>(wp + 4);
-                            const float wo[8] = {w0v.x, w0v.y, w0v.z, w0v.w,
-                                                 w1v.x, w1v.y, w1v.z, w1v.w};
-                            #pragma unroll
-                            for (int e = 0; e < 8; ++e) dot = fmaf(h[e], wo[e], dot);
-                        }
-                    }
-                    if (l < 3) {
-                        tc::fence_async_smem();
-                        __syncwarp();
-                        if (lane == 0) {
-                            #pragma unroll
-                            for (int r = 0; r < RND; ++r) tc::mbar_arrive(&act_ready[RND*j + r]);
-                        }
-                    }
-                    if (more) {
-                        #pragma unroll
-                        for (int r = 0; r < RND; ++r) {
-                            tc::tmem_wait_ld8(rb[r]);
-                            #pragma unroll
-                            for (int e = 0; e < 8; ++e) ra[r][e] = rb[r][e];
+                            for (int e = 0; e < 8; ++e) dot = fmaf(h[e], wo[KCI*c + e], dot);
                         }
                     }
                 }
@@ -1660,8 +1820,8 @@ int32_t sasb200_mlp_serve(int32_t n, int32_t n_pad, const void *x, const void *x
     // by pairs of CTAs, two tiles in flight, where a CTA has several tiles
     const bool in_pairs = !z_save && blocks > 1 && n_tiles > SP_TILES*blocks;
     if (in_pairs) blocks &= ~1;
-    const auto kernel = z_save ? mlp_serve<SV_ROUND, PLANES_ROWS>
-                               : (in_pairs ? mlp_serve_pairs : mlp_serve<SV_ROUND, PLANES_NONE>);
+    const auto kernel = z_save ? mlp_serve<PLANES_ROWS>
+                               : (in_pairs ? mlp_serve_pairs : mlp_serve<PLANES_NONE>);
     const int bytes = in_pairs ? SP_SMEM : SV_SMEM, threads = in_pairs ? SP_THREADS : SV_THREADS;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     kernel<<<blocks, threads, bytes, (cudaStream_t)stream>>>(
@@ -1711,7 +1871,7 @@ int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const
     prm.dout = dout;
     prm.row_sums = row_sums;
     const int n_tiles = n_pad/TM;
-    const auto kernel = mlp_serve<SV_ROUND, PLANES_TILED>;
+    const auto kernel = mlp_serve<PLANES_TILED>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
     kernel<<<tile_blocks(n_tiles), SV_THREADS, SV_SMEM, (cudaStream_t)stream>>>(
         n, n_tiles, static_cast<const __nv_bfloat16 *>(x),

@@ -32,8 +32,7 @@
 //   warp 16     CTA 0, lane 0: issues the MMAs, a "unit" (a chunk, or a layer 0) as
 //               soon as the count of ready units covers it.  An issue holds the
 //               thread for about the time of the MMA before, so nothing else is
-//               waited for here, and the count is read only when the last value
-//               does not cover the unit.
+//               waited for here.
 //   warp 17     producer of this CTA's half of the weight ring.
 //   warp 18     CTA 0: polls the barriers of the current step's units, one per lane,
 //               and publishes how many are ready in order.  (Waiting for a chunk's
@@ -64,83 +63,17 @@
 // 32 inputs: 2.18 ms, of 128: 2.42 ms.
 #pragma once
 
-// Two FP32 lanes in one register pair: each half rounded to nearest.
-__device__ __forceinline__ uint64_t f2_pack(float a, float b)
-{
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
-    return v;
-}
-__device__ __forceinline__ void f2_unpack(uint64_t v, float &a, float &b)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
-// silu of two accumulator columns plus bias (see silu())
-__device__ __forceinline__ uint64_t silu2(uint32_t a0, uint32_t a1, uint64_t bias)
-{
-    const uint64_t z = f2_add(f2_pack(__uint_as_float(a0), __uint_as_float(a1)), bias);
-    const uint64_t hz = f2_mul(z, f2_pack(0.5f, 0.5f));
-    float x0, x1, t0, t1;
-    f2_unpack(hz, x0, x1);
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t0) : "f"(x0));
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t1) : "f"(x1));
-    return f2_fma(hz, f2_pack(t0, t1), hz);
-}
-
-// 8 columns of a row, from the accumulators r[at ..]: silu, then the hi and lo
-// halves (one 16-byte unit each)
-__device__ __forceinline__ void silu_columns(const uint32_t (&r)[16], int at, const float *bias,
-                                             uint4 &hi, uint4 &lo)
-{
-    const ulonglong2 *b2 = reinterpret_cast<const ulonglong2 *>(bias + at);
-    const uint64_t minus1 = f2_pack(-1.0f, -1.0f);
-    uint32_t *hp = &hi.x, *lp = &lo.x;
-    #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const ulonglong2 b = b2[e];
-        #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const uint64_t h = silu2(r[at + 4*e + 2*q], r[at + 4*e + 2*q + 1], q ? b.y : b.x);
-            float x, y, dx, dy;
-            f2_unpack(h, x, y);
-            const uint32_t u = pack2(x, y);
-            f2_unpack(f2_fma(f2_pack(bf_lo(u), bf_hi(u)), minus1, h), dx, dy);
-            hp[2*e + q] = u;
-            lp[2*e + q] = pack2(dx, dy);
-        }
-    }
-}
-
-constexpr int SP_X_WARP = SV_WAIT_WARP + 1;
-constexpr int SP_THREADS = SV_THREADS + 32;
+constexpr int SP_POLL_WARP = SV_EPI_WARPS + 2;
+constexpr int SP_X_WARP = SV_EPI_WARPS + 3;
+constexpr int SP_THREADS = SV_EPI + 128;
 constexpr int SP_K = 64;                           // inputs of a chunk
 constexpr int SP_CHUNKS = HID/SP_K;                // of a step, and of the weight ring
 constexpr int SP_SIDE = SP_CHUNKS/2;               // chunk before which a layer 0 goes
 constexpr int SP_GROUP = HID/2*16;                 // 8 inputs of this CTA's 128 outputs: 2 KB
 constexpr int SP_HALF = SP_K/8*SP_GROUP;           // this CTA's weights of a chunk
 constexpr int SP_SMEM = 2*ACT_BYTES + SP_CHUNKS*SP_HALF + W0_BYTES/2 + 4*X_BYTES + 4*SV_PARAMS;
-// Tiles per CTA up to which mlp_serve is taken: its chunk-by-chunk hand-over has
-// one tile done earlier (20.5 us against two and a half layers more of waiting
-// for B), while 157 tiles on 148 CTAs already take 32.7 us here and 35.0 there.
+// Tiles per CTA up to which mlp_serve is taken: 8 tiles 17.5 us there and 18.9 here,
+// 148 tiles 18.6 and 20.2; but 157 tiles on 148 CTAs 35.0 and 32.7.
 constexpr int SP_TILES = 1;
 
 // Turn j (from SP_FIRST on) of the epilogues, for `mine` tiles (A the even ones,
@@ -264,7 +197,7 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             if (!ok) atomicExch(err, 2);
         }
         __syncwarp();
-    } else if (warp == SV_WAIT_WARP) {
+    } else if (warp == SP_POLL_WARP) {
         bool ok = true;
         if (rank == 0) {
             // ---- poll: the units of every step ----
@@ -372,12 +305,12 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             constexpr uint32_t idesc = tc::idesc_bf16(2*TM, HID);
             const uint32_t a_hi = tc::smem_u32(act), a_lo = tc::smem_u32(act_lo);
             bool ok = true;
-            uint32_t unit = 0, ready = 0;
+            uint32_t unit = 0;
+            ReadyCount count(&ready_seq);
             auto next_unit = [&]() {
-                ++unit;
-                if (ready < unit) ready = tc::spin_acquire_until(&ready_seq, unit);
+                const bool there = count.covers(++unit);
                 tc::fence_after_sync();
-                return ready >= unit;
+                return there;
             };
             auto layer0 = [&](int z) {
                 const uint32_t dz = tmem + (uint32_t)(HID*z);
@@ -493,22 +426,7 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 __syncwarp();
                 if (lane == 0) arrive0(&acc_empty[p]);
                 #pragma unroll
-                for (int c = 0; c < CHUNKS_PER_LAYER; ++c) {
-                    const ulonglong2 *b2 = reinterpret_cast<const ulonglong2 *>(bias + KCI*c);
-                    const float4 *w4 = reinterpret_cast<const float4 *>(wo + KCI*c);
-                    #pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const ulonglong2 b = b2[e];
-                        const float4 w = w4[e];
-                        float h0, h1, h2, h3;
-                        f2_unpack(silu2(r[c][4*e], r[c][4*e + 1], b.x), h0, h1);
-                        f2_unpack(silu2(r[c][4*e + 2], r[c][4*e + 3], b.y), h2, h3);
-                        dot = fmaf(h0, w.x, dot);
-                        dot = fmaf(h1, w.y, dot);
-                        dot = fmaf(h2, w.z, dot);
-                        dot = fmaf(h3, w.w, dot);
-                    }
-                }
+                for (int c = 0; c < CHUNKS_PER_LAYER; ++c) dot = dot8(r[c], bias + KCI*c, wo + KCI*c, dot);
                 // four partial sums per row; slot 0 adds them.  Slots 1-3
                 // write dot_part[p] again in the last layer of p's next
                 // tile, which needs slot 0's activations of that tile.

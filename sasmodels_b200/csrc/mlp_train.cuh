@@ -25,10 +25,10 @@ __device__ __forceinline__ float warp_sum8(float (&v)[8], int lane)
 // ---------------------------------------------------------------- backward --
 // mlp_backward_t: dZ3 = dout w_out silu'(z3), then dZ(l-1) = (dZl W_l)
 // silu'(z(l-1)) for l = 3, 2, 1, from tiled z to tiled dZ planes; the values of
-// mlp_backward.  Built as mlp_serve: sixteen epilogue warps (quadrant w % 4, 8
-// columns of every 32-column chunk at 8(w / 4)), one MMA warp, a bulk-copy
-// producer and a waiter, two TMEM accumulators, so that the MMAs of the next
-// layer start on the first chunk while the epilogue works on the last.  A
+// mlp_backward.  Built as mlp_serve: sixteen epilogue warps (quadrant w % 4, 16
+// columns of every 64 at 16(w / 4)), one MMA warp, a bulk-copy producer and the two
+// counting warps, two TMEM accumulators, so that the MMAs of the next layer start on the
+// first columns while the epilogue works on the last.  A
 // training batch of 8192 rows is one tile for 64 CTAs, so the kernel is bound by
 // the latency of one tile's chain: the ring holds a whole layer of weights
 // (fetched while dZ3 forms), and each warp loads the z of its eight chunks one
@@ -45,8 +45,9 @@ mlp_backward_t(int n_tiles, const uint8_t *__restrict__ img_t, const float *__re
     uint8_t *act = smem;
     uint8_t *ring = smem + ACT_BYTES;
     __shared__ __align__(8) uint64_t full[BT_STAGES], empty[BT_STAGES];
-    __shared__ __align__(8) uint64_t act_ready[CHUNKS_PER_LAYER], acc_full[2], acc_empty[2], drain;
-    __shared__ uint32_t tmem_slot, ready_seq;
+    __shared__ __align__(8) uint64_t act_ready[SV_UNITS], acc_full[2], acc_empty[2], drain;
+    __shared__ uint32_t tmem_slot;
+    __shared__ __align__(8) uint2 ready_seq;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int my_tiles = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x)/gridDim.x + 1 : 0;
 
@@ -59,13 +60,13 @@ mlp_backward_t(int n_tiles, const uint8_t *__restrict__ img_t, const float *__re
             tc::mbar_init(&full[s], 1);
             tc::mbar_init(&empty[s], 1);
         }
-        for (int c = 0; c < CHUNKS_PER_LAYER; ++c) tc::mbar_init(&act_ready[c], SV_EPI_WARPS);
+        for (int c = 0; c < SV_UNITS; ++c) tc::mbar_init(&act_ready[c], SV_EPI_WARPS);
         for (int a = 0; a < 2; ++a) {
             tc::mbar_init(&acc_full[a], 1);
             tc::mbar_init(&acc_empty[a], SV_EPI_WARPS);
         }
         tc::mbar_init(&drain, 1);
-        ready_seq = 0;
+        ready_seq = make_uint2(0u, 0u);
         tc::mbar_fence_init();
     }
     tc::fence_before_sync();
@@ -93,36 +94,47 @@ mlp_backward_t(int n_tiles, const uint8_t *__restrict__ img_t, const float *__re
                 ok = tc::mbar_wait(&full[j % BT_STAGES], (uint32_t)((j/BT_STAGES) & 1)) && ok;
             if (!ok) atomicExch(err, 2);
         }
-    } else if (warp == SV_WAIT_WARP) {
+    } else if (warp == SV_ACT_WARP) {
         // step g = 3 k + s accumulates in acc[g & 1]; its previous reader is the
-        // epilogue of step g - 2 (completion (g - 2)/2 of acc_empty), and the
-        // inputs of its chunks are completion g of act_ready.  No barrier can
-        // run two phases ahead: each next completion needs what is published
-        // here first.
-        bool ok = true;
-        int chunk = 0;
-        for (int g = 0; g < 3*my_tiles && ok; ++g) {
-            if (g >= 2 && !(ok = warp_wait(&acc_empty[g & 1], (uint32_t)(((g - 2) >> 1) & 1))))
-                break;
-            for (int c = 0; c < CHUNKS_PER_LAYER; ++c, ++chunk) {
-                if (!(ok = warp_wait(&act_ready[c], (uint32_t)(g & 1))
-                           && warp_wait(&full[chunk % BT_STAGES],
-                                        (uint32_t)((chunk/BT_STAGES) & 1))))
+        // epilogue of step g - 2 (completion (g - 2)/2 of acc_empty), and its input
+        // is completion g of act_ready.  No barrier can run two phases ahead: each
+        // next completion needs what is published here first.
+        if (lane == 0) {
+            bool ok = true;
+            uint32_t chunk = 0;
+            for (int g = 0; g < 3*my_tiles && ok; ++g) {
+                if (g >= 2 && !(ok = tc::mbar_wait(&acc_empty[g & 1], (uint32_t)(((g - 2) >> 1) & 1))))
                     break;
-                if (lane == 0) tc::st_release_shared(&ready_seq, (uint32_t)(chunk + 1));
+                for (int q = 0; q < SV_UNITS; ++q) {
+                    if (!(ok = tc::mbar_wait(&act_ready[q], (uint32_t)(g & 1)))) break;
+                    chunk += CHUNKS_PER_LAYER/SV_UNITS;
+                    tc::st_release_shared(&ready_seq.x, chunk);
+                }
             }
+            if (!ok) atomicExch(err, 4);
         }
-        if (!ok && lane == 0) atomicExch(err, 4);
+        __syncwarp();
+    } else if (warp == SV_WEIGHT_WARP) {
+        if (lane == 0) {
+            bool ok = true;
+            const uint32_t total = (uint32_t)(my_tiles*CHUNKS_PER_TILE);
+            for (uint32_t i = 0; i < total && ok; ++i)
+                if ((ok = tc::mbar_wait(&full[i % BT_STAGES], (i/BT_STAGES) & 1u)))
+                    tc::st_release_shared(&ready_seq.y, i + 1);
+            if (!ok) atomicExch(err, 4);
+        }
+        __syncwarp();
     } else if (warp == SV_MMA_WARP) {
         bool ok = true;
         if (lane == 0) {
             constexpr uint32_t idesc = tc::idesc_bf16(TM, HID);
             const uint32_t a_addr = tc::smem_u32(act);
             int chunk = 0;
+            ReadyCounts count(&ready_seq);
             for (int g = 0; g < 3*my_tiles && ok; ++g) {
                 const uint32_t d = tmem + (uint32_t)(HID*(g & 1));
                 for (int c = 0; c < CHUNKS_PER_LAYER; ++c, ++chunk) {
-                    if (!(ok = tc::spin_acquire_ge(&ready_seq, (uint32_t)(chunk + 1)))) break;
+                    if (!(ok = count.covers((uint32_t)(chunk + 1)))) break;
                     tc::fence_after_sync();
                     const int s = chunk % BT_STAGES;
                     const uint32_t b_addr = tc::smem_u32(ring + s*CHUNK_BYTES);
@@ -149,63 +161,90 @@ mlp_backward_t(int n_tiles, const uint8_t *__restrict__ img_t, const float *__re
         for (int k = 0; k < my_tiles && ok; ++k) {
             const int tile = blockIdx.x + k*gridDim.x;
             const float d = dout[tile*TM + row];
-            const uint4 *z0 = reinterpret_cast<const uint4 *>(z_save + tiled_at(0, n_tiles, tile, slot, row));
+            // this thread's 16 columns of every 64: two groups of 8
+            const size_t at0 = tiled_at(0, n_tiles, tile, 2*slot, row);
+            const uint4 *z0 = reinterpret_cast<const uint4 *>(z_save + at0);
+            uint4 *dz0 = reinterpret_cast<uint4 *>(dz_save + at0);
             const size_t plane16 = (size_t)n_tiles*TILE_ELEMS/8;   // a plane in 16-byte units
-            constexpr int CHUNK16 = 4*GROUP_ELEMS/8;               // four groups
-            uint4 *dz0 = reinterpret_cast<uint4 *>(dz_save + tiled_at(0, n_tiles, tile, slot, row));
-            uint4 z[CHUNKS_PER_LAYER];
+            constexpr int GROUP16 = GROUP_ELEMS/8;
+            uint4 z[SV_UNITS][2];
             #pragma unroll
-            for (int c = 0; c < CHUNKS_PER_LAYER; ++c) z[c] = z0[3*plane16 + c*CHUNK16];
+            for (int q = 0; q < SV_UNITS; ++q) {
+                z[q][0] = z0[3*plane16 + 8*q*GROUP16];
+                z[q][1] = z0[3*plane16 + (8*q + 1)*GROUP16];
+            }
             // s = -1: dZ3 from dout; s = 0, 1, 2: the epilogues of W3, W2, W1
             #pragma unroll 1
             for (int s = -1; s < 3; ++s) {
                 const int g = 3*k + s, l = 2 - s, a = g & 1;
-                uint32_t ra[8], rb[8];
-                const uint32_t acc = tmem + lane_base + (uint32_t)(HID*a + 8*slot);
+                const uint32_t acc = tmem + lane_base + (uint32_t)(HID*a + 16*slot);
+                uint32_t ra[16], rb[16];
                 if (s >= 0) {
                     if (!(ok = warp_wait(&acc_full[a], (uint32_t)((g >> 1) & 1)))) break;
                     tc::fence_after_sync();
-                    tc::tmem_ld8(acc, ra);
-                    tc::tmem_wait_ld8(ra);
+                    tc::tmem_ld16(acc, ra);
+                    tc::tmem_wait_ld();
+                    tc::tmem_tie16(ra);
                 }
                 #pragma unroll
-                for (int c = 0; c < CHUNKS_PER_LAYER; ++c) {
-                    const bool more = c + 1 < CHUNKS_PER_LAYER;
+                for (int q = 0; q < SV_UNITS; ++q) {
+                    const bool more = q + 1 < SV_UNITS;
                     if (s >= 0) {
                         if (more) {
-                            tc::tmem_ld8(acc + (uint32_t)(KCI*(c + 1)), rb);
+                            tc::tmem_ld16(acc + (uint32_t)(64*(q + 1)), rb);
                         } else {
                             tc::fence_before_sync();
                             __syncwarp();
                             if (lane == 0) tc::mbar_arrive(&acc_empty[a]);
                         }
                     } else {
-                        const float4 *wp = reinterpret_cast<const float4 *>(w_out + KCI*c + 8*slot);
-                        const float4 w0 = __ldg(wp), w1 = __ldg(wp + 1);
-                        const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+                        const float4 *wp = reinterpret_cast<const float4 *>(w_out + 64*q + 16*slot);
                         #pragma unroll
-                        for (int e = 0; e < 8; ++e) ra[e] = __float_as_uint(d*w[e]);
+                        for (int e = 0; e < 4; ++e) {
+                            const float4 w = __ldg(wp + e);
+                            ra[4*e] = __float_as_uint(d*w.x);
+                            ra[4*e + 1] = __float_as_uint(d*w.y);
+                            ra[4*e + 2] = __float_as_uint(d*w.z);
+                            ra[4*e + 3] = __float_as_uint(d*w.w);
+                        }
                     }
-                    const uint32_t zu[4] = {z[c].x, z[c].y, z[c].z, z[c].w};
-                    uint4 o;
-                    uint32_t *op = &o.x;
+                    uint4 o[2];
                     #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        op[e] = pack2(__uint_as_float(ra[2*e])*dsilu(bf_lo(zu[e])),
-                                      __uint_as_float(ra[2*e + 1])*dsilu(bf_hi(zu[e])));
-                    if (s < 2) {
-                        *reinterpret_cast<uint4 *>(act + tc::kmajor_offset<TM>(row, KCI*c + 8*slot)) = o;
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t zu[4] = {z[q][h].x, z[q][h].y, z[q][h].z, z[q][h].w};
+                        uint32_t *op = &o[h].x;
+                        #pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            op[e] = pack2(__uint_as_float(ra[8*h + 2*e])*dsilu(bf_lo(zu[e])),
+                                          __uint_as_float(ra[8*h + 2*e + 1])*dsilu(bf_hi(zu[e])));
+                        // the stores of the 64 columns before have had time to land
+                        if (h == 0 && q > 1 && s < 2) {
+                            tc::fence_async_smem();
+                            __syncwarp();
+                            if (lane == 0) tc::mbar_arrive(&act_ready[q - 1]);
+                        }
+                    }
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (s < 2) {
+                            *reinterpret_cast<uint4 *>(
+                                act + tc::kmajor_offset<TM>(row, 64*q + 16*slot + 8*h)) = o[h];
+                            // the next layer's z, in use one epilogue from now
+                            z[q][h] = z0[(size_t)(l - 1)*plane16 + (8*q + h)*GROUP16];
+                        }
+                        dz0[(size_t)l*plane16 + (8*q + h)*GROUP16] = o[h];
+                    }
+                    // the tensor core is waiting for the first and the last
+                    if (s < 2 && (q == 0 || !more)) {
                         tc::fence_async_smem();
                         __syncwarp();
-                        if (lane == 0) tc::mbar_arrive(&act_ready[c]);
-                        // the next layer's z, in use one epilogue from now
-                        z[c] = z0[(size_t)(l - 1)*plane16 + c*CHUNK16];
+                        if (lane == 0) tc::mbar_arrive(&act_ready[q]);
                     }
-                    dz0[(size_t)l*plane16 + c*CHUNK16] = o;
                     if (s >= 0 && more) {
-                        tc::tmem_wait_ld8(rb);
+                        tc::tmem_wait_ld();
+                        tc::tmem_tie16(rb);
                         #pragma unroll
-                        for (int e = 0; e < 8; ++e) ra[e] = rb[e];
+                        for (int e = 0; e < 16; ++e) ra[e] = rb[e];
                     }
                 }
             }

@@ -122,6 +122,12 @@ __device__ __forceinline__ void st_release_shared(uint32_t *p, uint32_t v)
 {
     asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" :: "r"(smem_u32(p)), "r"(v) : "memory");
 }
+__device__ __forceinline__ uint2 ld_acquire_shared2(const uint2 *p)
+{
+    uint64_t v;
+    asm volatile("ld.acquire.cta.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(smem_u32(p)) : "memory");
+    return make_uint2((uint32_t)v, (uint32_t)(v >> 32));
+}
 // Bounded spin until *p >= target (acquire); returns the value, below target when
 // the limit ran out.
 __device__ __forceinline__ uint32_t spin_acquire_until(const uint32_t *p, uint32_t target)
