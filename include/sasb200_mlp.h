@@ -33,6 +33,19 @@ int32_t sasb200_mlp_features(int32_t n, int32_t n_pad, const double *radius,
                              const double *drho, const double *q, const double *flag,
                              void *x, void *x_lo, void *stream);
 
+/* the same for n points in runs that share a parameter set: run r covers starts[r] <=
+ * i < starts[r + 1] (starts[0] = 0, the last run ends at n), table[runs x 7] =
+ * (radius, length, radius pd, length pd, contrast, flag, inside the domain); and, from
+ * the networks' outputs there, I = exp(out y_std + y_mean + 2 log|contrast|) and
+ * accept (inside, q in [q_lo, q_hi] and gate g_std + g_mean <= thr; gate NULL: 0). */
+int32_t sasb200_features_runs(int32_t n, int32_t n_pad, int32_t runs, const int32_t *starts,
+                              const double *table, const double *q, void *x, void *x_lo,
+                              void *stream);
+int32_t sasb200_finish_runs(int32_t n, int32_t runs, const int32_t *starts, const double *table,
+                            const double *q, const float *out, const float *gate, double y_std,
+                            double y_mean, double g_std, double g_mean, double thr, double q_lo,
+                            double q_hi, double *I, uint8_t *accept, void *stream);
+
 /* pipelined forward: the weights packed once by sasb200_mlp_pack into an
  * image of sasb200_mlp_image_bytes() bytes (16-byte aligned); out[n], and
  * for training the z/h planes [4][n_pad x 256] bf16 (both NULL for

@@ -636,6 +636,44 @@ __global__ void lr_schedule(int *__restrict__ counters, float *__restrict__ sche
 // dispersity damping log(1 + R_pd qR), log(1 + L_pd qL/2), and the damped
 // oscillations cos/sin(2qR) exp(-2 (R_pd qR)^2), cos/sin(qL) exp(-2 (L_pd qL/2)^2).
 // Slot 15 is zero.
+__device__ __forceinline__ void feature_row(double radius, double length, double rpd, double lpd,
+                                            double drho, double q, double flag, float (&f)[16])
+{
+    f[0] = (float)(2.0*(log(radius) - log(10.0))/(log(300.0) - log(10.0)) - 1.0);
+    f[1] = (float)(2.0*(log(length) - log(20.0))/(log(3000.0) - log(20.0)) - 1.0);
+    f[2] = (float)(2.0*rpd/0.3 - 1.0);
+    f[3] = (float)(2.0*lpd/0.3 - 1.0);
+    f[4] = (float)(drho/5.0);
+    f[5] = (float)(2.0*(log(q) - log(1e-3))/(log(0.5) - log(1e-3)) - 1.0);
+    f[6] = (float)(2.0*flag - 1.0);
+    const double qr = q*radius, qh = 0.5*q*length;
+    f[7] = (float)(log(qr)/4.0);
+    f[8] = (float)(log(qh)/4.0);
+    f[9] = (float)(log1p(rpd*qr)/2.0);
+    f[10] = (float)(log1p(lpd*qh)/2.0);
+    // oscillation of the cross-section and length factors (period pi in
+    // qR and qL/2), damped as a gaussian size distribution damps them
+    const double ar = exp(-2.0*(rpd*qr)*(rpd*qr));
+    const double al = exp(-2.0*(lpd*qh)*(lpd*qh));
+    double sr, cr, sh, ch;
+    sincos(2.0*qr, &sr, &cr);
+    sincos(2.0*qh, &sh, &ch);
+    f[11] = (float)(ar*cr);
+    f[12] = (float)(ar*sr);
+    f[13] = (float)(al*ch);
+    f[14] = (float)(al*sh);
+}
+
+__device__ __forceinline__ void save_features(const float (&f)[16], __nv_bfloat16 *x,
+                                              __nv_bfloat16 *x_lo, int i)
+{
+    float lo[16];
+    #pragma unroll
+    for (int j = 0; j < 16; ++j) lo[j] = f[j] - __bfloat162float(__float2bfloat16_rn(f[j]));
+    save16(x + (size_t)i*NIN, f);
+    save16(x_lo + (size_t)i*NIN, lo);
+}
+
 __global__ void features(int n, int n_pad, const double *__restrict__ radius,
                          const double *__restrict__ length, const double *__restrict__ rpd,
                          const double *__restrict__ lpd, const double *__restrict__ drho,
@@ -647,33 +685,62 @@ __global__ void features(int n, int n_pad, const double *__restrict__ radius,
     float f[16];
     #pragma unroll
     for (int j = 0; j < 16; ++j) f[j] = 0.0f;
-    if (i < n) {
-        f[0] = (float)(2.0*(log(radius[i]) - log(10.0))/(log(300.0) - log(10.0)) - 1.0);
-        f[1] = (float)(2.0*(log(length[i]) - log(20.0))/(log(3000.0) - log(20.0)) - 1.0);
-        f[2] = (float)(2.0*rpd[i]/0.3 - 1.0);
-        f[3] = (float)(2.0*lpd[i]/0.3 - 1.0);
-        f[4] = (float)(drho[i]/5.0);
-        f[5] = (float)(2.0*(log(q[i]) - log(1e-3))/(log(0.5) - log(1e-3)) - 1.0);
-        f[6] = (float)(2.0*flag[i] - 1.0);
-        const double qr = q[i]*radius[i], qh = 0.5*q[i]*length[i];
-        f[7] = (float)(log(qr)/4.0);
-        f[8] = (float)(log(qh)/4.0);
-        f[9] = (float)(log1p(rpd[i]*qr)/2.0);
-        f[10] = (float)(log1p(lpd[i]*qh)/2.0);
-        // oscillation of the cross-section and length factors (period pi in
-        // qR and qL/2), damped as a gaussian size distribution damps them
-        const double ar = exp(-2.0*(rpd[i]*qr)*(rpd[i]*qr));
-        const double al = exp(-2.0*(lpd[i]*qh)*(lpd[i]*qh));
-        f[11] = (float)(ar*cos(2.0*qr));
-        f[12] = (float)(ar*sin(2.0*qr));
-        f[13] = (float)(al*cos(2.0*qh));
-        f[14] = (float)(al*sin(2.0*qh));
+    if (i < n) feature_row(radius[i], length[i], rpd[i], lpd[i], drho[i], q[i], flag[i], f);
+    save_features(f, x, x_lo, i);
+}
+
+// Points that come as runs sharing a parameter set: run r covers the points
+// starts[r] <= i < starts[r + 1] (starts[0] = 0), its row of `table` is (radius,
+// length, radius pd, length pd, contrast, flag, inside the domain).
+__device__ __forceinline__ int run_of(const int *__restrict__ starts, int runs, int i)
+{
+    int lo = 0, hi = runs;                 // starts[lo] <= i < starts[hi]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (starts[mid] <= i) lo = mid; else hi = mid;
     }
-    float lo[16];
+    return lo;
+}
+
+constexpr int RUN_COLS = 7;
+// The features of such points, without the seven columns of n doubles in between
+// (56 bytes a point written and read again, by eight launches).
+__global__ void __launch_bounds__(256)
+features_runs(int n, int n_pad, int runs, const int *__restrict__ starts,
+              const double *__restrict__ table, const double *__restrict__ q,
+              __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ x_lo)
+{
+    const int i = blockIdx.x*blockDim.x + threadIdx.x;
+    if (i >= n_pad) return;
+    float f[16];
     #pragma unroll
-    for (int j = 0; j < 16; ++j) lo[j] = f[j] - __bfloat162float(__float2bfloat16_rn(f[j]));
-    save16(x + (size_t)i*NIN, f);
-    save16(x_lo + (size_t)i*NIN, lo);
+    for (int j = 0; j < 16; ++j) f[j] = 0.0f;
+    if (i < n) {
+        const double *row = table + (size_t)RUN_COLS*run_of(starts, runs, i);
+        feature_row(row[0], row[1], row[2], row[3], row[4], q[i], row[5], f);
+    }
+    save_features(f, x, x_lo, i);
+}
+
+// I = exp(out y_std + y_mean + 2 log|contrast|) of every point, and whether the
+// network is trusted there: inside the domain, q inside its range and the gate's
+// prediction at most thr (gate null: nowhere).  Every operation rounds on its own.
+__global__ void __launch_bounds__(256)
+finish_runs(int n, int runs, const int *__restrict__ starts, const double *__restrict__ table,
+            const double *__restrict__ q, const float *__restrict__ out,
+            const float *__restrict__ gate, double y_std, double y_mean, double g_std,
+            double g_mean, double thr, double q_lo, double q_hi, double *__restrict__ I,
+            uint8_t *__restrict__ accept)
+{
+    const int i = blockIdx.x*blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double *row = table + (size_t)RUN_COLS*run_of(starts, runs, i);
+    const double y = __dadd_rn(__dmul_rn((double)out[i], y_std), y_mean);
+    I[i] = exp(__dadd_rn(y, __dmul_rn(2.0, log(fabs(row[4])))));
+    bool ok = row[6] > 0.5 && q[i] >= q_lo && q[i] <= q_hi;
+    if (ok) ok = gate != nullptr
+                 && __dadd_rn(__dmul_rn((double)gate[i], g_std), g_mean) <= thr;
+    accept[i] = ok ? 1 : 0;
 }
 
 inline char *errbuf()
@@ -2202,6 +2269,38 @@ int32_t sasb200_mlp_features(int32_t n, int32_t n_pad, const double *radius, con
         n, n_pad, radius, length, rpd, lpd, drho, q, flag, static_cast<__nv_bfloat16 *>(x),
         static_cast<__nv_bfloat16 *>(x_lo));
     return status("features");
+}
+
+// Features of n points in runs of equal parameters: run r covers starts[r] <= i <
+// starts[r + 1] (starts[0] = 0; the last run ends at n), table[runs x 7] = (radius,
+// length, radius pd, length pd, contrast, flag, inside).
+int32_t sasb200_features_runs(int32_t n, int32_t n_pad, int32_t runs, const int32_t *starts,
+                              const double *table, const double *q, void *x, void *x_lo,
+                              void *stream)
+{
+    errbuf()[0] = 0;
+    if (n <= 0 || n > n_pad || runs <= 0 || runs > n || !starts || !table || !q || !x || !x_lo)
+        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
+    features_runs<<<(n_pad + 255)/256, 256, 0, (cudaStream_t)stream>>>(
+        n, n_pad, runs, starts, table, q, static_cast<__nv_bfloat16 *>(x),
+        static_cast<__nv_bfloat16 *>(x_lo));
+    return status("features_runs");
+}
+
+// I[n] and accept[n] from the networks' outputs at those points; gate may be
+// NULL (nothing accepted).
+int32_t sasb200_finish_runs(int32_t n, int32_t runs, const int32_t *starts, const double *table,
+                            const double *q, const float *out, const float *gate, double y_std,
+                            double y_mean, double g_std, double g_mean, double thr, double q_lo,
+                            double q_hi, double *I, uint8_t *accept, void *stream)
+{
+    errbuf()[0] = 0;
+    if (n <= 0 || runs <= 0 || runs > n || !starts || !table || !q || !out || !I || !accept)
+        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
+    finish_runs<<<(n + 255)/256, 256, 0, (cudaStream_t)stream>>>(
+        n, runs, starts, table, q, out, gate, y_std, y_mean, g_std, g_mean, thr, q_lo, q_hi, I,
+        accept);
+    return status("finish_runs");
 }
 
 }  // extern "C"

@@ -73,7 +73,11 @@ def _lib():
     lib.sasb200_sum_partials.argtypes = [I] + [P]*5
     lib.sasb200_gather_batch.argtypes = [I, ct.c_int64] + [P]*9 + [I, I, F, F, F, P, P]
     lib.sasb200_adam_pack.argtypes = [P]*10 + [F, I, F, F, F, P]
-    for name in ("sasb200_gather_batch", "sasb200_adam_pack",
+    D = ct.c_double
+    lib.sasb200_features_runs.argtypes = [I, I, I] + [P]*6
+    lib.sasb200_finish_runs.argtypes = [I, I] + [P]*5 + [D]*7 + [P]*3
+    for name in ("sasb200_features_runs", "sasb200_finish_runs",
+                 "sasb200_gather_batch", "sasb200_adam_pack",
                  "sasb200_mlp_train_forward", "sasb200_mlp_train_backward",
                  "sasb200_mlp_weight_grads", "sasb200_sum_partials",
                  "sasb200_mlp_forward", "sasb200_mlp_backward", "sasb200_gemm_nt",
@@ -813,43 +817,53 @@ class Surrogate:
 
     def _device_eval(self, cols, tol):
         """(I, accepted mask) of the network at every point, computed on the
-        device: only q, a run index and one row per run of points sharing a
-        parameter set cross to the GPU (points of a set are contiguous, as
-        flatten() lays them out); the domain check, the gate threshold and
-        exp(log I) run there too."""
+        device: only q and one row per run of points sharing a parameter set
+        cross to the GPU (points of a set are contiguous, as flatten() lays
+        them out); the gate threshold and exp(log I) run there too."""
         torch = self.torch
-        dev = self.net.device
+        net, dev = self.net, self.net.device
         sid = np.asarray(cols["set"])
         n = len(sid)
-        new = np.r_[True, sid[1:] != sid[:-1]] if n else np.zeros(0, bool)
-        starts = np.flatnonzero(new)
-        run = (np.cumsum(new) - 1).astype(np.int32)
+        if n == 0:
+            return np.zeros(0), np.zeros(0, bool)
+        starts = np.concatenate([[0], np.flatnonzero(sid[1:] != sid[:-1]) + 1])
         keys = ("radius", "length", "rpd", "lpd", "contrast", "flag")
-        table = np.stack([np.asarray(cols[k], float)[starts] for k in keys], axis=1)
+        runs = len(starts)
+        # one upload for the rows and, behind them, the runs' first points
+        table = np.zeros((runs, 8))
+        for j, k in enumerate(keys):
+            table[:, j] = np.asarray(cols[k])[starts]
         ok = np.abs(table[:, 4]) > 0
         for j, key in enumerate(keys[:5]):
             lo, hi = DOMAIN[key]
             ok &= (table[:, j] >= lo) & (table[:, j] <= hi)
-        table = np.concatenate([table, ok[:, None].astype(float)], axis=1)
+        table[:, 6] = ok
+        rows = np.concatenate([table[:, :7].ravel(),
+                               np.pad(starts, (0, runs % 2)).astype(np.int32).view(float)])
         thr = self._accept_log_threshold(tol)
         qlo, qhi = DOMAIN["q"]
-        with torch.cuda.stream(self.net.stream):
-            T = torch.as_tensor(table, device=dev).index_select(
-                0, torch.as_tensor(run, device=dev))
+        n_pad = pad128(n)
+        with torch.cuda.stream(net.stream):
+            rows = torch.as_tensor(rows, device=dev)
             q = torch.as_tensor(np.ascontiguousarray(cols["q"], 'd'), device=dev)
-            x, x_lo, _ = self.net.features(T[:, 0], T[:, 1], T[:, 2], T[:, 3], T[:, 4], q,
-                                           T[:, 5])
-            logi = (self.net.serve(x, x_lo, n)[:n].double()*self.y_std + self.y_mean
-                    + 2.0*torch.log(T[:, 4].abs()))
-            accept = (T[:, 6] > 0.5) & (q >= qlo) & (q <= qhi)
-            if np.isfinite(thr):
-                g = self.gate.serve(x, x_lo, n)[:n].double()*self.g_std + self.g_mean
-                accept &= g <= thr
-            else:
-                accept &= False
-            I = torch.exp(logi).cpu().numpy()
-            acc = accept.cpu().numpy()
-        return I, acc
+            feats = torch.empty((2, n_pad, NIN), dtype=torch.bfloat16, device=dev)
+            result = torch.empty(n + (n + 7)//8, dtype=torch.float64, device=dev)
+            st = net.stream.cuda_stream
+            table_ptr = rows.data_ptr()
+            starts_ptr = table_ptr + 8*7*runs
+            x, x_lo = feats[0], feats[1]
+            net._check(net.lib.sasb200_features_runs(
+                n, n_pad, runs, starts_ptr, table_ptr, q.data_ptr(), x.data_ptr(),
+                x_lo.data_ptr(), st), "features_runs")
+            out = net.serve(x, x_lo, n)
+            g = self.gate.serve(x, x_lo, n) if np.isfinite(thr) else None
+            net._check(net.lib.sasb200_finish_runs(
+                n, runs, starts_ptr, table_ptr, q.data_ptr(), out.data_ptr(),
+                None if g is None else g.data_ptr(), self.y_std, self.y_mean, self.g_std,
+                self.g_mean, thr, qlo, qhi, result.data_ptr(), result.data_ptr() + 8*n, st),
+                "finish_runs")
+            host = result.cpu().numpy()
+        return host[:n], host[n:].view(np.bool_)[:n]
 
     def iq(self, cols, tol=None, device=None, form="float32c"):
         """I(q) for flat inputs: the network where its predicted error is
