@@ -18,6 +18,7 @@ every theory (``csrc/resolution.cu``).  ``weight_matrix`` is still available for
 that read it, built on the host on first access.
 """
 
+import contextlib
 import ctypes as ct
 import os
 
@@ -166,6 +167,32 @@ def _device(device):
 MAX_WEIGHTS = 1 << 25
 
 
+def _enter(dev, stream):
+    """Context in which allocations and copies go to *stream* of *dev*: none to
+    enter when they already do (each of torch's two contexts costs as much as a
+    launch)."""
+    import torch
+    if torch.cuda.current_device() == dev.index and torch.cuda.current_stream(dev) == stream:
+        return contextlib.nullcontext()
+    stack = contextlib.ExitStack()
+    stack.enter_context(torch.cuda.device(dev))
+    stack.enter_context(torch.cuda.stream(stream))
+    return stack
+
+
+def _on_device(theory, dev, n):
+    """(theory as a contiguous float64 tensor of n values on a GPU, whether it
+    came as one)."""
+    import torch
+    on_device = isinstance(theory, torch.Tensor) and theory.is_cuda
+    t = (theory if on_device else
+         torch.as_tensor(np.ascontiguousarray(theory, 'd'), device=dev))
+    t = t.to(torch.float64).contiguous()
+    if t.numel() != n:
+        raise ValueError("theory has %d points, q_calc %d" % (t.numel(), n))
+    return t, on_device
+
+
 def _band_plan(lo, hi, dev, form):
     """Weights of the bands [lo, hi) on the device, formed once by *form*
     (lo, hi, off, w, norm, stream), or None when they are too many.  Complete
@@ -262,16 +289,12 @@ class Pinhole1D:
         (enqueued on *stream*, default the current stream); a host array in,
         a host array out."""
         import torch
-        on_device = isinstance(theory, torch.Tensor) and theory.is_cuda
-        t = (theory if on_device else
-             torch.as_tensor(np.ascontiguousarray(theory, 'd'), device=self.device))
-        t = t.to(torch.float64).contiguous()
-        if t.numel() != len(self.q_calc):
-            raise ValueError("theory has %d points, q_calc %d" % (t.numel(), len(self.q_calc)))
+        dev = self.device
+        t, on_device = _on_device(theory, dev, len(self.q_calc))
         d = self._upload()
-        st = stream if stream is not None else torch.cuda.current_stream(self.device)
-        with torch.cuda.device(self.device), torch.cuda.stream(st):
-            out = torch.empty(len(d["q"]), dtype=torch.float64, device=self.device)
+        st = stream if stream is not None else torch.cuda.current_stream(dev)
+        with _enter(dev, st):
+            out = torch.empty(len(d["q"]), dtype=torch.float64, device=dev)
             if d["plan"] is not None:
                 _band_apply(d["plan"], 1, len(d["q"]), t.numel(), t, t.numel(), out, st)
             else:
@@ -293,8 +316,9 @@ class Pinhole1D:
             raise ValueError("theory must be [n_sets, %d] with contiguous rows" % len(self.q_calc))
         d = self._upload()
         nq = len(d["q"])
-        with torch.cuda.device(self.device), torch.cuda.stream(stream):
-            out = torch.empty((n_sets, nq), dtype=torch.float64, device=self.device)
+        dev = self.device
+        with _enter(dev, stream):
+            out = torch.empty((n_sets, nq), dtype=torch.float64, device=dev)
             if d["plan"] is not None:
                 _band_apply(d["plan"], n_sets, nq, n_calc, theory, theory.stride(0), out, stream)
             else:
@@ -400,16 +424,12 @@ class Slit1D:
         """Smeared I(q) from I(q_calc); CUDA tensor in -> CUDA tensor out,
         host array in -> host array out."""
         import torch
-        on_device = isinstance(theory, torch.Tensor) and theory.is_cuda
-        t = (theory if on_device else
-             torch.as_tensor(np.ascontiguousarray(theory, 'd'), device=self.device))
-        t = t.to(torch.float64).contiguous()
-        if t.numel() != len(self.q_calc):
-            raise ValueError("theory has %d points, q_calc %d" % (t.numel(), len(self.q_calc)))
+        dev = self.device
+        t, on_device = _on_device(theory, dev, len(self.q_calc))
         d = self._upload()
-        st = stream if stream is not None else torch.cuda.current_stream(self.device)
-        with torch.cuda.device(self.device), torch.cuda.stream(st):
-            out = torch.empty(len(self.q), dtype=torch.float64, device=self.device)
+        st = stream if stream is not None else torch.cuda.current_stream(dev)
+        with _enter(dev, st):
+            out = torch.empty(len(self.q), dtype=torch.float64, device=dev)
             if d["plan"] is not None:
                 _band_apply(d["plan"], 1, len(self.q), t.numel(), t, t.numel(), out, st)
             else:
@@ -502,21 +522,17 @@ class Pinhole2D:
         if self.q_calc_weights is None:
             return theory
         nq, nbins = len(self.qx_data), self.nr*self.nphi
-        on_device = isinstance(theory, torch.Tensor) and theory.is_cuda
-        t = (theory if on_device else
-             torch.as_tensor(np.ascontiguousarray(theory, 'd'), device=self.device))
-        t = t.to(torch.float64).contiguous()
-        if t.numel() != nq*nbins:
-            raise ValueError("theory has %d points, q_calc %d" % (t.numel(), nq*nbins))
+        dev = self.device
+        t, on_device = _on_device(theory, dev, nq*nbins)
         if self._w_dev is None:
             self._w_dev = torch.as_tensor(np.ascontiguousarray(self.q_calc_weights, 'd'),
-                                          device=self.device)
+                                          device=dev)
             # the normalisation formed exactly as np.average forms it
             wgt = np.broadcast_to(np.asarray(self.q_calc_weights, 'd'), (1, nbins))
             self._wsum = float(wgt.swapaxes(-1, 0).sum(axis=0)[0])
-        st = stream if stream is not None else torch.cuda.current_stream(self.device)
-        with torch.cuda.device(self.device), torch.cuda.stream(st):
-            out = torch.empty(nq, dtype=torch.float64, device=self.device)
+        st = stream if stream is not None else torch.cuda.current_stream(dev)
+        with _enter(dev, st):
+            out = torch.empty(nq, dtype=torch.float64, device=dev)
             _check(_lib().sasb200_pinhole2d_average(nq, nbins, t.data_ptr(),
                                                     self._w_dev.data_ptr(), self._wsum,
                                                     out.data_ptr(), st.cuda_stream),
@@ -534,13 +550,17 @@ def nllf_sets(theory, Iq, dIq, stream):
     import torch
     n_sets, nq = theory.shape
     dev = theory.device
-    with torch.cuda.device(dev), torch.cuda.stream(stream):
-        y = torch.as_tensor(np.ascontiguousarray(Iq, 'd'), device=dev)
-        dy = torch.as_tensor(np.ascontiguousarray(dIq, 'd'), device=dev)
-        if y.numel() != nq or dy.numel() != nq or theory.stride(1) != 1:
-            raise ValueError("data has %d points, theory %d" % (y.numel(), nq))
+    y, dy = np.ascontiguousarray(Iq, 'd'), np.ascontiguousarray(dIq, 'd')
+    if y.size != nq or dy.size != nq or theory.stride(1) != 1:
+        raise ValueError("data has %d points, theory %d" % (y.size, nq))
+    data = torch.from_numpy(np.concatenate([y.ravel(), dy.ravel()]))
+    with _enter(dev, stream):
+        # one copy, queued behind the theory instead of waiting for it (host
+        # memory that is not pinned has been read when the call returns; a
+        # captured copy would read it again later, so a capture refuses here)
+        data = data.to(dev, non_blocking=not torch.cuda.is_current_stream_capturing())
         out = torch.empty(n_sets, dtype=torch.float64, device=dev)
         _check(_lib().sasb200_nllf_sets(n_sets, nq, theory.data_ptr(), theory.stride(0),
-                                        y.data_ptr(), dy.data_ptr(), out.data_ptr(),
-                                        stream.cuda_stream), "nllf_sets")
+                                        data.data_ptr(), data.data_ptr() + 8*nq,
+                                        out.data_ptr(), stream.cuda_stream), "nllf_sets")
     return out

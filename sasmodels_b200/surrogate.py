@@ -45,7 +45,17 @@ PD_N = 35
 WARMUP_STEPS = 200
 
 
+_LIB = None
+
+
 def _lib():
+    global _LIB
+    if _LIB is None:
+        _LIB = _load()
+    return _LIB
+
+
+def _load():
     path = os.path.join(LIB_DIR, "libsasb200_mlp.so")
     if not os.path.exists(path):
         raise RuntimeError("surrogate library not built: %s" % path)
@@ -122,6 +132,7 @@ class MLP:
         self.w_out = torch.as_tensor(rng.uniform(-1, 1, HID)/math.sqrt(HID), **f32)
         self.b_out = torch.zeros(1, **f32)
         self.params = self.W + self.b + [self.w_out, self.b_out]
+        self._sizes = [p.numel() for p in self.params]
         self.m = [torch.zeros_like(p) for p in self.params]
         self.v = [torch.zeros_like(p) for p in self.params]
         self.step_count = 0
@@ -183,6 +194,14 @@ class MLP:
         self.gb = [torch.empty(HID, **f32) for _ in range(4)]
         self.gw = torch.empty(HID, **f32)
         self.gbo = torch.empty(1, **f32)
+        # their addresses, which change with them only
+        self._at = {k: getattr(self, k).data_ptr() for k in
+                    ("z_save", "h_save", "dz_save", "out", "dout", "row_sums", "gb_part",
+                     "gw_part")}
+        self._gW_at = self._ptrs(self.gW)
+        self._part_at = ([g.data_ptr() for g in self.gW]
+                         + [self._at["gb_part"] + 4*self.splits*HID*l for l in range(4)]
+                         + [self._at["gw_part"]])
         self._scratch_n = n_pad
 
     # ----------------------------------------------------------- kernels --
@@ -255,44 +274,38 @@ class MLP:
         self._pack()
         with torch.cuda.stream(self.stream):
             loss = torch.empty((), dtype=torch.float32, device=self.device)
-        self._gradient_kernels(x, x_lo, y, n, loss, self.gbo)
-        self._sum_partials(list(zip(self._vector_partials(), self.gb + [self.gw])))
+        self._gradient_kernels(x, x_lo, y, n, loss.data_ptr(), self.gbo.data_ptr())
+        self._sum_partials(4, [t.data_ptr() for t in self.gb + [self.gw]])
         return loss, self.gW, self.gb, self.gw, self.gbo
 
-    def _vector_partials(self):
-        """Partial sums of the four bias gradients and the output weights'."""
-        return [self.gb_part[l] for l in range(4)] + [self.gw_part]
-
-    def _sum_partials(self, pairs):
-        """Every (partials, out) pair summed over the splits, in one launch."""
-        n = len(pairs)
+    def _sum_partials(self, first, outs):
+        """The partial sums of the parameters from `first` on (in the order of
+        params, up to w_out) added over the splits into the addresses `outs`,
+        in one launch."""
+        n = 9 - first
         I32, VP = ct.c_int32*n, ct.c_void_p*n
         self._check(self.lib.sasb200_sum_partials(
-            n, I32(*[o.numel() for _, o in pairs]), I32(*[self.splits]*n),
-            VP(*[p.data_ptr() for p, _ in pairs]), VP(*[o.data_ptr() for _, o in pairs]),
-            self.stream.cuda_stream), "sum_partials")
+            n, I32(*self._sizes[first:9]), I32(*[self.splits]*n), VP(*self._part_at[first:]),
+            VP(*outs), self.stream.cuda_stream), "sum_partials")
 
     def _gradient_kernels(self, x, x_lo, y, n, loss, db_out):
         """Forward, backward and weight gradients of one batch: the loss and
         db_out as scalars, the other gradients as partial sums over
-        self.splits (gW, gb_part, gw_part)."""
+        self.splits (gW, gb_part, gw_part).  loss and db_out are addresses."""
         n_pad = x.shape[0]
-        st = self.stream.cuda_stream
-        lib = self.lib
-        err = self.err.data_ptr()
-        z, h, dz = (t.data_ptr() for t in (self.z_save, self.h_save, self.dz_save))
-        dout, sums = self.dout.data_ptr(), self.row_sums.data_ptr()
+        st, lib, at = self.stream.cuda_stream, self.lib, self._at
+        err, w_out = self.err.data_ptr(), self.w_out.data_ptr()
+        z, h, dz, dout, sums = (at[k] for k in ("z_save", "h_save", "dz_save", "dout",
+                                                "row_sums"))
         self._check(lib.sasb200_mlp_train_forward(
             n, n_pad, x.data_ptr(), x_lo.data_ptr(), self.img.data_ptr(), self._ptrs(self.b),
-            self.w_out.data_ptr(), self.b_out.data_ptr(), y.data_ptr(), float(self.huber),
-            self.out.data_ptr(), dout, sums, z, h, err, st), "forward")
-        self._check(lib.sasb200_mlp_train_backward(n_pad, self.img_t.data_ptr(),
-                                                   self.w_out.data_ptr(), dout, z, dz, err, st),
-                    "backward")
+            w_out, self.b_out.data_ptr(), y.data_ptr(), float(self.huber), at["out"], dout, sums,
+            z, h, err, st), "forward")
+        self._check(lib.sasb200_mlp_train_backward(n_pad, self.img_t.data_ptr(), w_out, dout, z,
+                                                   dz, err, st), "backward")
         self._check(lib.sasb200_mlp_weight_grads(
-            n, n_pad, self.splits, x.data_ptr(), h, dz, dout, sums, self._ptrs(self.gW),
-            self.gb_part.data_ptr(), self.gw_part.data_ptr(), loss.data_ptr(), db_out.data_ptr(),
-            err, st), "weight_grads")
+            n, n_pad, self.splits, x.data_ptr(), h, dz, dout, sums, self._gW_at, at["gb_part"],
+            at["gw_part"], loss, db_out, err, st), "weight_grads")
 
     def train_step(self, x, x_lo, y, n, lr, b1=0.9, b2=0.999, eps=1e-8, reduce=None):
         """One Adam step on one batch; returns the loss (a device scalar).
@@ -319,12 +332,13 @@ class MLP:
         torch = self.torch
         self._scratch(x.shape[0])
         self._pack()
-        sizes = [p.numel() for p in self.params]
+        sizes = self._sizes
         with torch.cuda.stream(self.stream):
             flat = torch.empty(sum(sizes) + 1, dtype=torch.float32, device=self.device)
+        ends = [flat.data_ptr() + 4*sum(sizes[:k]) for k in range(len(sizes) + 1)]
+        self._gradient_kernels(x, x_lo, y, n, ends[10], ends[9])
+        self._sum_partials(0, ends[:9])
         parts = flat.split(sizes + [1])
-        self._gradient_kernels(x, x_lo, y, n, parts[-1], parts[9])
-        self._sum_partials(list(zip(self.gW + self._vector_partials(), parts)))
         return [parts[-1]] + list(parts[:-1])
 
     def capture_training(self, x_all, x_lo_all, y_all, batch, lr, total, step0, warmup=200,
@@ -571,8 +585,9 @@ class TrainingGraph:
                 torch.index_select(x_lo_all, 0, self.idx, out=self.xlb)
                 torch.index_select(y_all, 0, self.idx, out=self.yb)
                 net._check(lib.sasb200_lr_schedule(*schedule, st), "lr_schedule")
-            net._gradient_kernels(self.xb, self.xlb, self.yb, batch, self.loss, net.gbo)
-            net._adam(net.gW + net._vector_partials() + [net.gbo], [net.splits]*9 + [1],
+            net._gradient_kernels(self.xb, self.xlb, self.yb, batch, self.loss.data_ptr(),
+                                  net.gbo.data_ptr())
+            net._adam(net.gW + list(net.gb_part) + [net.gw_part, net.gbo], [net.splits]*9 + [1],
                       self.sched, lr, b1, b2, eps)
         # what the graph reads and writes outlives the network's next, larger
         # scratch
