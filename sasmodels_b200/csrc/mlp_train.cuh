@@ -69,9 +69,11 @@ mlp_backward_t(int n_tiles, const uint8_t *__restrict__ img_t, const float *__re
         ready_seq = make_uint2(0u, 0u);
         tc::mbar_fence_init();
     }
+    tc::dependents_launch();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    tc::dependency_wait();
     const uint32_t tmem = tmem_slot;
 
     if (warp == SV_PROD_WARP) {
@@ -324,9 +326,11 @@ mlp_weight_grads(int n_tiles, int splits, WeightGrads prm, int *__restrict__ err
         tc::mbar_init(&done, 1);
         tc::mbar_fence_init();
     }
+    tc::dependents_launch();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    tc::dependency_wait();
     const uint32_t tmem = tmem_slot;
     bool ok = true;
 
@@ -504,6 +508,8 @@ struct SumTensors {
 __global__ void __launch_bounds__(256)
 sum_partials(SumTensors T)
 {
+    tc::dependents_launch();
+    tc::dependency_wait();
     const int k = blockIdx.y, size = T.size[k], splits = T.splits[k];
     const int i = blockIdx.x*256 + threadIdx.x;
     if (i >= size) return;
@@ -527,6 +533,8 @@ gather_batch(int n, long long rows, const int64_t *__restrict__ idx,
              float *__restrict__ y, int *__restrict__ counters, float *__restrict__ sched,
              int total, int warmup, float lr0, float b1, float b2, int *__restrict__ err)
 {
+    tc::dependents_launch();
+    tc::dependency_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0)
         schedule_step(counters, sched, total, warmup, lr0, b1, b2);
     const int i = blockIdx.x*256 + threadIdx.x, row = i >> 2, part = i & 3;
@@ -595,6 +603,8 @@ __global__ void __launch_bounds__(256)
 adam_pack(AdamPack A)
 {
     __shared__ __align__(16) __nv_bfloat16 tile[32*AP_LD];
+    tc::dependents_launch();
+    tc::dependency_wait();
     const int t = threadIdx.x, b = blockIdx.x;
     const float lr = A.sched ? A.sched[0] : A.lr, bc1 = A.sched ? A.sched[1] : A.bc1,
                 bc2 = A.sched ? A.sched[2] : A.bc2;

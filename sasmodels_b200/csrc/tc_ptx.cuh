@@ -153,6 +153,22 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
                  : "memory");
 }
 
+// ---- dependent launches ------------------------------------------------------
+// dependents_launch: the next kernel of the stream, when it was launched as a
+// dependent one (launch_dependent in mlp.cu), may take free SMs from now on.
+// dependency_wait: until every kernel before this one is complete and its writes
+// are visible; nothing that they touch may be accessed before it, and every CTA
+// has to come by here, so that a kernel's completion stands for all before it.
+// Both do nothing in an ordinary launch.
+__device__ __forceinline__ void dependents_launch()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void dependency_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ---- named barriers ----------------------------------------------------------
 // Barrier `id` among `count` threads (a multiple of 32) of the CTA.
 __device__ __forceinline__ void bar_sync(int id, int count)
