@@ -179,7 +179,8 @@ def build_support(force=False):
     """Libraries that do not depend on a model plugin."""
     return [build_plain("peaks.cu", "libsasb200_peaks.so", force),
             build_plain("mlp.cu", "libsasb200_mlp.so", force,
-                        extra_deps=("tc_ptx.cuh", "mlp_train.cuh", "mlp_pairs.cuh")),
+                        extra_deps=("tc_ptx.cuh", "mlp_train.cuh", "mlp_pairs.cuh",
+                                    "mlp_halves.cuh")),
             build_plain("resolution.cu", "libsasb200_resolution.so", force),
             build_plain("pack.cu", "libsasb200_pack.so", force)]
 

@@ -24,6 +24,7 @@
 //                  at once (a dedicated MMA warp, two TMEM accumulators,
 //                  layer l+1's MMAs under layer l's epilogue chunk by chunk);
 //                  serves inference and the training forward.
+//   mlp_serve_halves, mlp_backward_halves   few tiles: two SMs per tile
 //   mlp_serve_pairs   inference over many tiles: pairs of SMs (cta_group::2), two
 //                  tiles in flight on each (mlp_pairs.cuh).
 //   mlp_backward_t, mlp_weight_grads   the training step's backward and weight
@@ -37,6 +38,7 @@
 // report through *err (0 = ok).
 #include <cstdint>
 #include <cstdio>
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 
@@ -1079,7 +1081,8 @@ __device__ __forceinline__ uint64_t silu2(uint32_t a0, uint32_t a1, uint64_t bia
 
 // 8 columns of a row, from the accumulators r[at ..]: silu, then the hi and lo
 // halves (one 16-byte unit each)
-__device__ __forceinline__ void silu_columns(const uint32_t (&r)[16], int at, const float *bias,
+template <int N>
+__device__ __forceinline__ void silu_columns(const uint32_t (&r)[N], int at, const float *bias,
                                              uint4 &hi, uint4 &lo)
 {
     const ulonglong2 *b2 = reinterpret_cast<const ulonglong2 *>(bias + at);
@@ -1588,6 +1591,7 @@ mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
 
 #include "mlp_train.cuh"
 #include "mlp_pairs.cuh"
+#include "mlp_halves.cuh"
 
 // ---------------------------------------------------------------- backward --
 // mlp_backward_p: the backward pass through the three 256 x 256 layers as a
@@ -1870,12 +1874,12 @@ int32_t sasb200_mlp_infer(int32_t n, int32_t n_pad, const void *x, const void *x
 }
 
 // out[n] for x, x_lo [n_pad x 16] with the packed weights through the
-// overlapped kernels (mlp_serve; mlp_serve_pairs where a CTA has several tiles
-// and no planes are wanted: the same values), and, when z_save/h_save are given, the
-// pre-activations and activations of all four layers ([4][n_pad x 256] bf16
-// each, those of mlp_infer) for training; persistent grid of at most
-// `blocks` CTAs (0 = one per SM).  err receives 1, 2, 3 or 4 if a pipeline
-// wait ran out.
+// overlapped kernels (mlp_serve; where no planes are wanted, mlp_serve_halves for few
+// tiles and mlp_serve_pairs where a CTA has several: the same values), and, when
+// z_save/h_save are given, the pre-activations and activations of all four layers
+// ([4][n_pad x 256] bf16 each, those of mlp_infer) for training; grid of at most
+// `blocks` CTAs (0 = one per SM).  err receives 1, 2, 3 or 4 if a pipeline wait ran
+// out.
 int32_t sasb200_mlp_serve(int32_t n, int32_t n_pad, const void *x, const void *x_lo,
                           const void *img, const float *const *b, const float *w_out,
                           const float *b_out, float *out, void *z_save, void *h_save,
@@ -1907,6 +1911,18 @@ int32_t sasb200_mlp_serve(int32_t n, int32_t n_pad, const void *x, const void *x
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         blocks = sms > 0 ? sms : 1;
     }
+    const auto *xp = static_cast<const __nv_bfloat16 *>(x);
+    const auto *xlp = static_cast<const __nv_bfloat16 *>(x_lo);
+    // two CTAs per tile where all may run at once (74 tiles: 13.4 us, 18.0 with one);
+    // beyond, the second round would cost more than the halves save
+    CUtensorMap map;
+    if (!z_save && n_tiles <= blocks/2 && hv_map(map, img, IMG_BYTES/(8*HV_RUN))) {
+        const auto kernel = mlp_serve_halves<PLANES_NONE>;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HV_SMEM);
+        kernel<<<2*n_tiles, SP_THREADS, HV_SMEM, (cudaStream_t)stream>>>(n, n_tiles, xp, xlp, map, prm,
+                                                                         out, err);
+        return status("mlp_serve");
+    }
     if (blocks > n_tiles) blocks = n_tiles;
     // by pairs of CTAs, two tiles in flight, where a CTA has several tiles
     const bool in_pairs = !z_save && blocks > 1 && n_tiles > SP_TILES*blocks;
@@ -1915,19 +1931,19 @@ int32_t sasb200_mlp_serve(int32_t n, int32_t n_pad, const void *x, const void *x
                                : (in_pairs ? mlp_serve_pairs : mlp_serve<PLANES_NONE>);
     const int bytes = in_pairs ? SP_SMEM : SV_SMEM, threads = in_pairs ? SP_THREADS : SV_THREADS;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    kernel<<<blocks, threads, bytes, (cudaStream_t)stream>>>(
-        n, n_tiles, static_cast<const __nv_bfloat16 *>(x),
-        static_cast<const __nv_bfloat16 *>(x_lo), prm, out, err);
+    kernel<<<blocks, threads, bytes, (cudaStream_t)stream>>>(n, n_tiles, xp, xlp, prm, out, err);
     return status("mlp_serve");
 }
 
-// One CTA per SM, or per tile where there are fewer.
-static int tile_blocks(int n_tiles)
+// One CTA per SM, or per tile where there are fewer; map: whether two CTAs per tile
+// may run at once, and the map of the image for them.
+static int tile_blocks(int n_tiles, const void *img, int img_bytes, CUtensorMap &map, bool &halves)
 {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return n_tiles < sms || sms <= 0 ? n_tiles : sms;
+    halves = n_tiles <= sms/2 && hv_map(map, img, img_bytes/(8*HV_RUN));
+    return halves ? 2*n_tiles : (n_tiles < sms || sms <= 0 ? n_tiles : sms);
 }
 
 // The forward of a training step: out[n] as sasb200_mlp_serve, the tiled z and
@@ -1962,11 +1978,23 @@ int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const
     prm.dout = dout;
     prm.row_sums = row_sums;
     const int n_tiles = n_pad/TM;
-    const auto kernel = mlp_serve<PLANES_TILED>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
-    launch_dependent(kernel, dim3(tile_blocks(n_tiles)), SV_THREADS, SV_SMEM, (cudaStream_t)stream, n,
-                     n_tiles, static_cast<const __nv_bfloat16 *>(x),
-                     static_cast<const __nv_bfloat16 *>(x_lo), prm, out, err);
+    const auto *xp = static_cast<const __nv_bfloat16 *>(x);
+    const auto *xlp = static_cast<const __nv_bfloat16 *>(x_lo);
+    const auto st = (cudaStream_t)stream;
+    CUtensorMap map;
+    bool halves;
+    const int blocks = tile_blocks(n_tiles, img, IMG_BYTES, map, halves);
+    if (halves) {
+        const auto kernel = mlp_serve_halves<PLANES_TILED>;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HV_SMEM);
+        launch_dependent(kernel, dim3(blocks), SP_THREADS, HV_SMEM, st, n, n_tiles, xp, xlp, map, prm,
+                         out, err);
+    } else {
+        const auto kernel = mlp_serve<PLANES_TILED>;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
+        launch_dependent(kernel, dim3(blocks), SV_THREADS, SV_SMEM, st, n, n_tiles, xp, xlp, prm, out,
+                         err);
+    }
     return status("mlp_train_forward");
 }
 
@@ -1983,10 +2011,23 @@ int32_t sasb200_mlp_train_backward(int32_t n_pad, const void *img_t, const float
         return (std::snprintf(errbuf(), 256, "weights must be 16-byte aligned"), -1);
     if (n_pad == 0) return 0;
     const int n_tiles = n_pad/TM;
-    cudaFuncSetAttribute(mlp_backward_t, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM);
-    launch_dependent(mlp_backward_t, dim3(tile_blocks(n_tiles)), SV_THREADS, BT_SMEM,
-                     (cudaStream_t)stream, n_tiles, static_cast<const uint8_t *>(img_t), w_out, dout,
-                     static_cast<const __nv_bfloat16 *>(z), static_cast<__nv_bfloat16 *>(dz), err);
+    const auto *zp = static_cast<const __nv_bfloat16 *>(z);
+    auto *dzp = static_cast<__nv_bfloat16 *>(dz);
+    const auto st = (cudaStream_t)stream;
+    CUtensorMap map;
+    bool halves;
+    const int blocks = tile_blocks(n_tiles, img_t, WT_IMG_BYTES, map, halves);
+    if (halves) {
+        const auto kernel = mlp_backward_halves;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HV_BWD_SMEM);
+        launch_dependent(kernel, dim3(blocks), SP_THREADS, HV_BWD_SMEM, st, n_tiles, map, w_out, dout,
+                         zp, dzp, err);
+    } else {
+        const auto kernel = mlp_backward_t;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM);
+        launch_dependent(kernel, dim3(blocks), SV_THREADS, BT_SMEM, st, n_tiles,
+                         static_cast<const uint8_t *>(img_t), w_out, dout, zp, dzp, err);
+    }
     return status("mlp_train_backward");
 }
 

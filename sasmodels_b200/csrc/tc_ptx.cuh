@@ -101,6 +101,16 @@ __device__ __forceinline__ void cluster_sync()
     asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
                  "barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same in two steps (each by converged warps), where nothing but mbarriers set
+// up before (mbar_fence_init) has to be visible: the release took 1000 cycles.
+__device__ __forceinline__ void cluster_arrive_relaxed()
+{
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait()
+{
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // Arrive once on the barrier at this offset in CTA `rank` of the cluster.
 // Relaxed: see mlp_serve_pairs for what the count stands for.
 __device__ __forceinline__ void mbar_arrive_relaxed_cta(uint64_t *bar, uint32_t rank)
@@ -153,6 +163,17 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
                  : "memory");
 }
 
+// A 4-D box of a tensor map (innermost coordinate x; x times the element size a
+// multiple of 16 bytes) -> this CTA's shared memory, completion counted on *bar.
+__device__ __forceinline__ void box_load4(void *dst, const void *map, int x, int y, int z, int w,
+                                          uint64_t *bar)
+{
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                 " [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                 :: "r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w),
+                    "r"(smem_u32(bar)) : "memory");
+}
+
 // ---- dependent launches ------------------------------------------------------
 // dependents_launch: the next kernel of the stream, when it was launched as a
 // dependent one (launch_dependent in mlp.cu), may take free SMs from now on.
@@ -174,6 +195,12 @@ __device__ __forceinline__ void dependency_wait()
 __device__ __forceinline__ void bar_sync(int id, int count)
 {
     asm volatile("bar.sync %0, %1;" :: "r"(id), "r"(count) : "memory");
+}
+
+// This warp's part of it without waiting.
+__device__ __forceinline__ void bar_arrive(int id, int count)
+{
+    asm volatile("bar.arrive %0, %1;" :: "r"(id), "r"(count) : "memory");
 }
 
 // Barrier `id` among `count` threads that also ANDs `pred` over them.
