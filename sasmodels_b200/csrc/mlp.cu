@@ -1067,10 +1067,9 @@ __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c)
     return r;
 }
 
-// silu of two accumulator columns plus bias (see silu())
-__device__ __forceinline__ uint64_t silu2(uint32_t a0, uint32_t a1, uint64_t bias)
+// silu of two pre-activations (see silu())
+__device__ __forceinline__ uint64_t silu2(uint64_t z)
 {
-    const uint64_t z = f2_add(f2_pack(__uint_as_float(a0), __uint_as_float(a1)), bias);
     const uint64_t hz = f2_mul(z, f2_pack(0.5f, 0.5f));
     float x0, x1, t0, t1;
     f2_unpack(hz, x0, x1);
@@ -1078,12 +1077,23 @@ __device__ __forceinline__ uint64_t silu2(uint32_t a0, uint32_t a1, uint64_t bia
     asm("tanh.approx.f32 %0, %1;" : "=f"(t1) : "f"(x1));
     return f2_fma(hz, f2_pack(t0, t1), hz);
 }
+// two accumulator columns plus bias
+__device__ __forceinline__ uint64_t bias2(uint32_t a0, uint32_t a1, uint64_t bias)
+{
+    return f2_add(f2_pack(__uint_as_float(a0), __uint_as_float(a1)), bias);
+}
+__device__ __forceinline__ uint32_t pack2(uint64_t v)
+{
+    float x, y;
+    f2_unpack(v, x, y);
+    return pack2(x, y);
+}
 
 // 8 columns of a row, from the accumulators r[at ..]: silu, then the hi and lo
-// halves (one 16-byte unit each)
-template <int N>
+// halves (one 16-byte unit each), and the pre-activations if they are wanted
+template <bool Z = false, int N>
 __device__ __forceinline__ void silu_columns(const uint32_t (&r)[N], int at, const float *bias,
-                                             uint4 &hi, uint4 &lo)
+                                             uint4 &hi, uint4 &lo, uint4 *zq = nullptr)
 {
     const ulonglong2 *b2 = reinterpret_cast<const ulonglong2 *>(bias + at);
     const uint64_t minus1 = f2_pack(-1.0f, -1.0f);
@@ -1093,13 +1103,12 @@ __device__ __forceinline__ void silu_columns(const uint32_t (&r)[N], int at, con
         const ulonglong2 b = b2[e];
         #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            const uint64_t h = silu2(r[at + 4*e + 2*q], r[at + 4*e + 2*q + 1], q ? b.y : b.x);
-            float x, y, dx, dy;
-            f2_unpack(h, x, y);
-            const uint32_t u = pack2(x, y);
-            f2_unpack(f2_fma(f2_pack(bf_lo(u), bf_hi(u)), minus1, h), dx, dy);
+            const uint64_t z = bias2(r[at + 4*e + 2*q], r[at + 4*e + 2*q + 1], q ? b.y : b.x);
+            const uint64_t h = silu2(z);
+            const uint32_t u = pack2(h);
             hp[2*e + q] = u;
-            lp[2*e + q] = pack2(dx, dy);
+            lp[2*e + q] = pack2(f2_fma(f2_pack(bf_lo(u), bf_hi(u)), minus1, h));
+            if (Z) (&zq->x)[2*e + q] = pack2(z);
         }
     }
 }
@@ -1115,8 +1124,8 @@ __device__ __forceinline__ float dot8(const uint32_t (&r)[8], const float *bias,
         const ulonglong2 b = b2[e];
         const float4 w = w4[e];
         float h0, h1, h2, h3;
-        f2_unpack(silu2(r[4*e], r[4*e + 1], b.x), h0, h1);
-        f2_unpack(silu2(r[4*e + 2], r[4*e + 3], b.y), h2, h3);
+        f2_unpack(silu2(bias2(r[4*e], r[4*e + 1], b.x)), h0, h1);
+        f2_unpack(silu2(bias2(r[4*e + 2], r[4*e + 3], b.y)), h2, h3);
         dot = fmaf(h0, w.x, dot);
         dot = fmaf(h1, w.y, dot);
         dot = fmaf(h2, w.z, dot);

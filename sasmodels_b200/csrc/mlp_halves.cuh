@@ -276,6 +276,15 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         const int row = 32*q2 + lane, trow = rank*HV_ROWS + row;
         const int col0 = 32*half + 8*slot;
         const uint32_t lane_base = tmem_slot + ((uint32_t)(32*quad) << 16) + (uint32_t)(8*slot);
+        // z and h of this thread's columns, after they are handed over
+        auto save_planes = [&](int l, const uint4 (&z)[SP_CHUNKS], const uint4 (&h)[SP_CHUNKS]) {
+            #pragma unroll
+            for (int c = 0; c < SP_CHUNKS; ++c) {
+                const size_t at = tiled_at(l, n_tiles, tile, (col0 + 64*c)/8, trow);
+                *reinterpret_cast<uint4 *>(prm.z_save + at) = z[c];
+                *reinterpret_cast<uint4 *>(prm.h_save + at) = h[c];
+            }
+        };
         bool ok = true;
         #pragma unroll 1
         for (int l = 0; l < 3; ++l) {
@@ -289,26 +298,19 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             #pragma unroll
             for (int c = 0; c < SP_CHUNKS; ++c) tc::tmem_wait_ld8(r[c]);
             tc::fence_before_sync();
+            uint4 hi[SP_CHUNKS], z[SP_CHUNKS];
             #pragma unroll
             for (int c = 0; c < SP_CHUNKS; ++c) {
-                uint4 hi, lo;
-                if (PLANES == PLANES_NONE) {
-                    silu_columns(r[c], 0, bias + 64*c, hi, lo);
-                } else {
-                    float z[8], h[8];
-                    sv_silu8(r[c], 0, bias + 64*c, z, h);
-                    split8(h, hi, lo);
-                    const size_t at = tiled_at(l, n_tiles, tile, (col0 + 64*c)/8, trow);
-                    save8(prm.z_save + at, z);
-                    *reinterpret_cast<uint4 *>(prm.h_save + at) = hi;
-                }
+                uint4 lo;
+                silu_columns<PLANES == PLANES_TILED>(r[c], 0, bias + 64*c, hi[c], lo, &z[c]);
                 const uint32_t off = tc::kmajor_offset<HV_ROWS>(row, col0 + 64*c);
-                *reinterpret_cast<uint4 *>(act + off) = hi;
+                *reinterpret_cast<uint4 *>(act + off) = hi[c];
                 *reinterpret_cast<uint4 *>(act_lo + off) = lo;
                 tc::fence_async_smem();
                 __syncwarp();
                 if (lane == 0) arrive0(&ready[SP_CHUNKS*l + c]);
             }
+            if (PLANES == PLANES_TILED) save_planes(l, z, hi);
         }
         if (ok && (ok = warp_wait(&acc_full[3], 0u))) {
             // the output dot: the 8 columns at 8 (w/4) of every 32, summed in order as
@@ -317,6 +319,7 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             tc::fence_after_sync();
             const float *bias = par + 3*HID + col0, *wo = par + 4*HID + 8*slot;
             uint32_t r[SP_CHUNKS][8];
+            uint4 hq[SP_CHUNKS], zq[SP_CHUNKS];
             float h[SP_CHUNKS][8];
             #pragma unroll
             for (int c = 0; c < SP_CHUNKS; ++c) tc::tmem_ld8(lane_base + (uint32_t)(HV_ACC + 32*c), r[c]);
@@ -327,23 +330,30 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             float4 *over = reinterpret_cast<float4 *>(act) + slot*(2*SP_CHUNKS*HV_ROWS) + row;
             #pragma unroll
             for (int c = 0; c < SP_CHUNKS; ++c) {
-                float z[8];
-                sv_silu8(r[c], 0, bias + 64*c, z, h[c]);
+                const ulonglong2 *b2 = reinterpret_cast<const ulonglong2 *>(bias + 64*c);
+                #pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const ulonglong2 b = b2[e >> 1];
+                    const uint64_t z = bias2(r[c][2*e], r[c][2*e + 1], e & 1 ? b.y : b.x);
+                    const uint64_t v = silu2(z);
+                    f2_unpack(v, h[c][2*e], h[c][2*e + 1]);
+                    if (PLANES == PLANES_TILED) {
+                        (&zq[c].x)[e] = pack2(z);
+                        (&hq[c].x)[e] = pack2(v);
+                    }
+                }
                 if (half == 1) {
                     over[2*c*HV_ROWS] = make_float4(h[c][0], h[c][1], h[c][2], h[c][3]);
                     over[(2*c + 1)*HV_ROWS] = make_float4(h[c][4], h[c][5], h[c][6], h[c][7]);
                 }
-                if (PLANES == PLANES_TILED) {
-                    const size_t at = tiled_at(3, n_tiles, tile, (col0 + 64*c)/8, trow);
-                    save8(prm.z_save + at, z);
-                    save8(prm.h_save + at, h[c]);
-                }
             }
-            float dot = 0.0f;
             if (half == 1) {
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(&other_half[q2][slot]);
-            } else if ((ok = warp_wait(&other_half[q2][slot], 0u))) {
+            }
+            if (PLANES == PLANES_TILED) save_planes(3, zq, hq);
+            float dot = 0.0f;
+            if (half == 0 && (ok = warp_wait(&other_half[q2][slot], 0u))) {
                 #pragma unroll
                 for (int c = 0; c < SP_CHUNKS; ++c) {
                     const float4 o0 = over[2*c*HV_ROWS], o1 = over[(2*c + 1)*HV_ROWS];
@@ -513,18 +523,18 @@ mlp_backward_halves(int n_tiles, const __grid_constant__ CUtensorMap img_t,
                     }
                 }
             }
+            uint4 o[SP_CHUNKS];
             #pragma unroll
             for (int c = 0; c < SP_CHUNKS; ++c) {
-                uint4 o;
                 const uint32_t zu[4] = {z[c].x, z[c].y, z[c].z, z[c].w};
-                uint32_t *op = &o.x;
+                uint32_t *op = &o[c].x;
                 #pragma unroll
                 for (int e = 0; e < 4; ++e)
                     op[e] = pack2(__uint_as_float(r[c][2*e])*dsilu(bf_lo(zu[e])),
                                   __uint_as_float(r[c][2*e + 1])*dsilu(bf_hi(zu[e])));
                 if (s < 2) {
                     *reinterpret_cast<uint4 *>(
-                        act + tc::kmajor_offset<HV_ROWS>(row, col0 + 64*c)) = o;
+                        act + tc::kmajor_offset<HV_ROWS>(row, col0 + 64*c)) = o[c];
                     tc::fence_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -532,11 +542,15 @@ mlp_backward_halves(int n_tiles, const __grid_constant__ CUtensorMap img_t,
                         if (rank == 0) tc::mbar_arrive(bar);
                         else tc::mbar_arrive_relaxed_cta(bar, 0);
                     }
-                    // the next layer's z, in use one epilogue from now
-                    z[c] = z0[(size_t)(l - 1)*plane16 + 8*c*GROUP16];
                 }
-                dz0[(size_t)l*plane16 + 8*c*GROUP16] = o;
             }
+            // the next layer's z, in use one epilogue from now
+            if (s < 2) {
+                #pragma unroll
+                for (int c = 0; c < SP_CHUNKS; ++c) z[c] = z0[(size_t)(l - 1)*plane16 + 8*c*GROUP16];
+            }
+            #pragma unroll
+            for (int c = 0; c < SP_CHUNKS; ++c) dz0[(size_t)l*plane16 + 8*c*GROUP16] = o[c];
         }
         if (!ok && lane == 0) atomicExch(err, 1);
         __syncwarp();

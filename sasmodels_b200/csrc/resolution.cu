@@ -36,9 +36,9 @@ namespace res {
 constexpr unsigned FULL = 0xffffffffu;
 
 // band_apply (a warp per q and curve) up to this many (q, curve) pairs, then
-// band_apply_sets: 181 q x 61 curves 3.8 against 6.2 us and 400 x 61 5.7 against
-// 6.6, but 181 x 200 7.3 against 6.3 and 1000 x 61 12.1 against 8.4.
-constexpr long long BAND_WARP_LIMIT = 28000;
+// band_apply_sets: 181 q x 61 curves 3.8 against 4.3 us and 400 x 32 4.1 against
+// 4.7, but 181 x 100 4.9 against 4.2 and 400 x 61 5.8 against 4.6.
+constexpr long long BAND_WARP_LIMIT = 14000;
 
 // nllf_sets (a block per curve) up to this many curves, then nllf_rows: 800
 // curves of 1000 points 4.3 against 6.2 us, 1600 of 1000 6.8 against 6.7, 1600
@@ -329,76 +329,100 @@ __device__ __forceinline__ double quotient(double x, double d, double r)
     return r == 0.0 || !isfinite(q) ? x/d : fma(fma(-q, d, x), r, q);
 }
 
-// Many curves: a block takes 32 q and 64 curves; a warp holds 8 of the q, a
-// lane two of the curves, so one theory value in a register serves 8 sums and
-// one weight (read as a broadcast) serves 64: 16 multiply-adds per 6
-// shared-memory reads, the point where both pipes are as busy.  The points of
-// the 32 bands pass through shared memory 16 at a time, the next 16 on their
-// way meanwhile.  Sums over 16 points are added to the totals, which keeps the
-// rounding error below that of one long sum.  A warp runs over the union of its
-// 8 bands with weight 0 outside each; a sum that this leaves infinite or
-// undefined is formed again over its own band alone, so that such a theory value
-// reaches only the q that see it.  4096 curves of 1000 q, 5 % width: 48 us; with
-// the weights formed for every curve (pinhole_smear) 2868 us.
-constexpr int BQ = 32, BQW = 8, BJ = 16, BS = 64, BWARPS = BQ/BQW, BTHREADS = 32*BWARPS;
-constexpr int BW_LD = BQ + 2;                // even: pairs of weights are read as double2
-constexpr int BT_LD = BS + 1;                // odd: spreads a row of points over the banks
+// c = a b + c on the FP64 tensor pipe: a 16 x 4 (row-major), b 4 x 8, c 16 x 8, as
+// fused multiply-adds in the order of the 4 points.  Lane L holds rows L/4 and
+// L/4 + 8: of a the column L % 4, of c the columns 2 (L % 4) and the next; of b
+// row L % 4 and column L/4.
+__device__ __forceinline__ void mma_f64(double (&c)[4], double a0, double a1, double b)
+{
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6},"
+                 " {%0, %1, %2, %3};"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3]) : "d"(a0), "d"(a1), "d"(b));
+}
 
-__global__ void __launch_bounds__(BTHREADS, 4)
+// Many curves: a block takes 32 q and 32 curves, a warp 16 q and 16 curves as two
+// tiles of the FP64 tensor pipe, which has the rate of the plain one but takes a
+// third of the shared-memory reads and few instructions.  The points of the 32
+// bands pass through shared memory 16 at a time, the next 16 on their way
+// meanwhile.  Sums over 16 points are added to the totals, which keeps the
+// rounding error below that of one long sum.  A warp runs over the union of its
+// 16 bands, 4 points at a time, with weight 0 outside each; a sum that this leaves
+// infinite or undefined is formed again over its own band alone, so that such a
+// theory value reaches only the q that see it.
+//   Bound by latency: a band is 60 points, four chunks, so that a block is mostly
+// its start and the waits between chunks; six blocks per SM hide that best.
+// 4096 curves of 1000 q, 5 % width: 35 us (17 at the FP64 rate); 46 with
+// multiply-adds (8 q and 64 curves per warp), 38 with 32 curves per warp (four
+// blocks), 35-41 with blocks that go on to further curves, 37 with three stages,
+// 39 with chunks of 32.  200 curves of 181 q: 4.3 us, 6.2 with multiply-adds.
+constexpr int BQ = 32, BQW = 16, BJ = 16, BS = 32, BSW = 16, BWARPS = 4, BTHREADS = 32*BWARPS;
+constexpr int BR = BTHREADS/BJ;              // rows staged at once
+constexpr int B_LD = BJ + 4;                 // a fragment's 4 points x 8 rows hit all banks
+
+__global__ void __launch_bounds__(BTHREADS, 6)
 band_apply_sets(int n_sets, int nq, const int32_t *__restrict__ lo,
                 const int32_t *__restrict__ hi, const int64_t *__restrict__ off,
                 const double *__restrict__ w, const double *__restrict__ norm,
                 const double *__restrict__ theory, size_t theory_stride,
                 double *__restrict__ out, size_t out_stride)
 {
-    constexpr int TH = 2*BJ*BT_LD, OUT = BS*(BQ + 1);
-    __shared__ double th[TH > OUT ? TH : OUT];
-    __shared__ __align__(16) double ws[2*BJ*BW_LD];
+    constexpr int TH = 2*BS*B_LD, OUT = BS*(BQ + 1);
+    __shared__ double th[TH > OUT ? TH : OUT];       // [2][curve][point]
+    __shared__ double ws[2*BQ*B_LD];                 // [2][q][point]
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int q0 = blockIdx.x*BQ, s0 = blockIdx.y*BS;
+    const int wq = BQW*(warp & 1), wc = BSW*(warp >> 1);     // this warp's q and curves
     const int qs = q0 + lane;
     const int my_lo = qs < nq ? lo[qs] : 0x7fffffff, my_hi = qs < nq ? hi[qs] : 0;
     const int jmin = __reduce_min_sync(FULL, my_lo), jmax = __reduce_max_sync(FULL, my_hi);
     const int chunks = jmax > jmin ? (jmax - jmin + BJ - 1)/BJ : 0;
     // the union of this warp's bands
-    const bool mine = lane/BQW == warp;
+    const bool mine = lane/BQW == (warp & 1);
     const int ulo = __reduce_min_sync(FULL, mine ? my_lo : 0x7fffffff);
     const int uhi = __reduce_max_sync(FULL, mine ? my_hi : 0);
-    // staging: thread t copies point t % 16 of a chunk, of eight curves and of
-    // four q
+    // staging: thread t copies point t % 16 of a chunk, of four curves and of four q
     const int js = t & (BJ - 1), rs = t/BJ;
     const double *tsrc = theory + (size_t)min(s0 + rs, n_sets - 1)*theory_stride + jmin + js;
     const int t_rows = n_sets - s0 - rs;
-    int wlo[4], whi[4];
-    const double *wsrc[4];
+    int wlo[BQ/BR], whi[BQ/BR];
+    const double *wsrc[BQ/BR];
     #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int iq = q0 + rs + 8*r;
+    for (int r = 0; r < BQ/BR; ++r) {
+        const int iq = q0 + rs + BR*r;
         wlo[r] = iq < nq ? lo[iq] : 0;
         whi[r] = iq < nq ? hi[iq] : 0;
         wsrc[r] = w + (iq < nq ? off[iq] : 0) - wlo[r];
     }
     auto stage = [&](int c) {
         const int j = jmin + c*BJ + js;
-        double *tb = th + (c & 1)*BJ*BT_LD + js*BT_LD + rs;
-        double *wb = ws + (c & 1)*BJ*BW_LD + js*BW_LD + rs;
+        double *tb = th + (c & 1)*BS*B_LD + rs*B_LD + js;
+        double *wb = ws + (c & 1)*BQ*B_LD + rs*B_LD + js;
         const double *src = tsrc + c*BJ;
-        #pragma unroll
-        for (int r = 0; r < BS/8; ++r) {
-            const bool ok = 8*r < t_rows && j < jmax;
-            copy8(tb + 8*r, ok ? src : theory, ok);
-            src += 8*theory_stride;
+        if (n_sets - s0 >= BS && jmin + (c + 1)*BJ <= jmax) {
+            #pragma unroll
+            for (int r = 0; r < BS/BR; ++r) {
+                copy8(tb + BR*r*B_LD, src, true);
+                src += BR*theory_stride;
+            }
+        } else {
+            #pragma unroll
+            for (int r = 0; r < BS/BR; ++r) {
+                const bool ok = BR*r < t_rows && j < jmax;
+                copy8(tb + BR*r*B_LD, ok ? src : theory, ok);
+                src += BR*theory_stride;
+            }
         }
         #pragma unroll
-        for (int r = 0; r < 4; ++r) {
+        for (int r = 0; r < BQ/BR; ++r) {
             const bool ok = j >= wlo[r] && j < whi[r];
-            copy8(wb + 8*r, ok ? wsrc[r] + j : w, ok);
+            copy8(wb + BR*r*B_LD, ok ? wsrc[r] + j : w, ok);
         }
         copy_commit();
     };
-    double acc[BQW][2], part[BQW][2];
+    constexpr int NT = BSW/8;                        // tiles of 16 q x 8 curves
+    double acc[NT][4];
     #pragma unroll
-    for (int u = 0; u < BQW; ++u) acc[u][0] = acc[u][1] = part[u][0] = part[u][1] = 0.0;
+    for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0;
     if (chunks > 0) stage(0);
     for (int c = 0; c < chunks; ++c) {
         if (c + 1 < chunks) {
@@ -409,36 +433,33 @@ band_apply_sets(int n_sets, int nq, const int32_t *__restrict__ lo,
         }
         __syncthreads();
         const int jc = jmin + c*BJ;
-        const int first = max(ulo - jc, 0), last = min(BJ, uhi - jc);
-        const double *tb = th + (c & 1)*BJ*BT_LD + lane;
-        const double *wb = ws + (c & 1)*BJ*BW_LD + BQW*warp;
-        #pragma unroll 4
-        for (int jj = first; jj < last; ++jj) {
-            const double x0 = tb[jj*BT_LD], x1 = tb[jj*BT_LD + 32];
-            const double2 *wp = reinterpret_cast<const double2 *>(wb + jj*BW_LD);
+        const int first = ulo - jc, last = uhi - jc;
+        if (first < BJ && last > 0) {
+            const double *wb = ws + (c & 1)*BQ*B_LD + (wq + lane/4)*B_LD + lane % 4;
+            const double *tb = th + (c & 1)*BS*B_LD + (wc + lane/4)*B_LD + lane % 4;
+            double part[NT][4];
             #pragma unroll
-            for (int u = 0; u < BQW; u += 2) {
-                const double2 y = wp[u/2];
-                part[u][0] = fma(y.x, x0, part[u][0]);
-                part[u][1] = fma(y.x, x1, part[u][1]);
-                part[u + 1][0] = fma(y.y, x0, part[u + 1][0]);
-                part[u + 1][1] = fma(y.y, x1, part[u + 1][1]);
+            for (int n = 0; n < NT; ++n) part[n][0] = part[n][1] = part[n][2] = part[n][3] = 0.0;
+            #pragma unroll
+            for (int k = 0; k < BJ; k += 4) {
+                if (k + 4 <= first || k >= last) continue;
+                const double a0 = wb[k], a1 = wb[8*B_LD + k];
+                #pragma unroll
+                for (int n = 0; n < NT; ++n) mma_f64(part[n], a0, a1, tb[8*n*B_LD + k]);
             }
-        }
-        #pragma unroll
-        for (int u = 0; u < BQW; ++u) {
-            acc[u][0] += part[u][0];
-            acc[u][1] += part[u][1];
-            part[u][0] = part[u][1] = 0.0;
+            #pragma unroll
+            for (int n = 0; n < NT; ++n)
+                #pragma unroll
+                for (int e = 0; e < 4; ++e) acc[n][e] += part[n][e];
         }
         __syncthreads();
     }
     // through shared memory, so that rows of 32 q leave together
     #pragma unroll
-    for (int u = 0; u < BQW; ++u) {
-        th[lane*(BQ + 1) + BQW*warp + u] = acc[u][0];
-        th[(32 + lane)*(BQ + 1) + BQW*warp + u] = acc[u][1];
-    }
+    for (int n = 0; n < NT; ++n)
+        #pragma unroll
+        for (int e = 0; e < 4; ++e)
+            th[(wc + 8*n + 2*(lane % 4) + (e & 1))*(BQ + 1) + wq + lane/4 + 8*(e >> 1)] = acc[n][e];
     __syncthreads();
     if (qs < nq) {
         const double d = norm[qs], r = sr_of(d);

@@ -54,6 +54,28 @@ def test_band_apply_matches_matrix(cuda, nq, sets, shuffle):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nq, sets", [(15, 1000), (16, 1000), (17, 1025), (31, 500), (33, 479),
+                                      (500, 31), (500, 33), (875, 16), (875, 17)])
+def test_many_curves_at_the_tile_edges(cuda, nq, sets):
+    """Just beyond the rule for many curves, at the edges of its tiles of 16 and
+    32 q and 8, 16 and 32 curves; each curve's result is its own."""
+    import torch
+    from sasmodels_b200.resolution import Pinhole1D
+    assert 14000 <= nq*sets < 18000
+    q, qc = _grid(nq)
+    r = Pinhole1D(q, 0.05*q, q_calc=qc)
+    th = np.random.default_rng(nq).uniform(0.5, 2.0, (sets, len(qc)))
+    th[sets//2, len(qc)//2] = np.nan
+    got = r.apply_sets(torch.as_tensor(th, device="cuda"),
+                       torch.cuda.current_stream()).cpu().numpy()
+    th[sets//2, len(qc)//2] = 0.0
+    want = th @ r.weight_matrix
+    sees = (r.band_lo <= len(qc)//2) & (len(qc)//2 < r.band_hi)
+    want[sets//2, sees] = np.nan
+    np.testing.assert_allclose(got, want, rtol=1e-12, atol=0)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("sets", [1, 700])
 def test_infinite_theory_reaches_only_its_bands(cuda, sets):
     """A point where a model is undefined spoils the q that see it, no other."""
