@@ -2063,7 +2063,7 @@ int32_t sasb200_mlp_weight_grads(int32_t n, int32_t n_pad, int32_t splits, const
     prm.dout = dout;
     prm.row_sums = row_sums;
     for (int l = 0; l < 4; ++l) {
-        if (!dw[l] || reinterpret_cast<uintptr_t>(dw[l]) % 16)
+        if (!dw[l] || reinterpret_cast<uintptr_t>(dw[l]) % 32)
             return (std::snprintf(errbuf(), 256, "bad gradient pointer"), -1);
         prm.dw[l] = dw[l];
     }
