@@ -110,12 +110,26 @@ int32_t sasb200_adam(int32_t size, int32_t splits, const float *grad, float *p, 
  * each); the backward from dout; every gradient as partial sums over splits of
  * the rows (dw[l]: [splits][256 x (16 or 256)], db: [4][splits][256], dw_out:
  * [splits][256]), the mean loss and db_out as scalars; and outs[k][i] = sum of
- * parts[k][s*sizes[k] + i] over s for n <= 16 tensors (host arrays). */
+ * parts[k][s*sizes[k] + i] over s for n <= 16 tensors (host arrays).
+ * The forward of a captured step takes a batch (else NULL): x, x_lo and y then
+ * receive the rows idx[n] of the data set (x_all, x_lo_all [rows x 16] bf16,
+ * y_all[rows]) first, and the schedule advances as by sasb200_lr_schedule; an
+ * index outside the set leaves zeros and *err = 5. */
+typedef struct sasb200_mlp_batch {
+    const int64_t *idx;
+    int64_t rows;
+    const void *x_all, *x_lo_all;
+    const float *y_all;
+    int32_t *counters;
+    float *sched;
+    int32_t total, warmup;
+    float lr0, b1, b2;
+} sasb200_mlp_batch;
 int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const void *x_lo,
                                   const void *img, const float *const *b, const float *w_out,
                                   const float *b_out, const float *y, float delta, float *out,
-                                  float *dout, float *row_sums, void *z, void *h, int32_t *err,
-                                  void *stream);
+                                  float *dout, float *row_sums, void *z, void *h,
+                                  const sasb200_mlp_batch *batch, int32_t *err, void *stream);
 int32_t sasb200_mlp_train_backward(int32_t n_pad, const void *img_t, const float *w_out,
                                    const float *dout, const void *z, void *dz, int32_t *err,
                                    void *stream);
@@ -126,15 +140,6 @@ int32_t sasb200_mlp_weight_grads(int32_t n, int32_t n_pad, int32_t splits, const
                                  void *stream);
 int32_t sasb200_sum_partials(int32_t n, const int32_t *sizes, const int32_t *splits,
                              const float *const *parts, float *const *outs, void *stream);
-
-/* a captured step's batch and schedule in one launch: rows idx[n] of the data set
- * (x_all, x_lo_all [rows x 16] bf16, y_all[rows]) into x, x_lo, y, and the step
- * of sasb200_lr_schedule; an index outside the set leaves zeros and *err = 5. */
-int32_t sasb200_gather_batch(int32_t n, int64_t rows, const int64_t *idx, const void *x_all,
-                             const void *x_lo_all, const float *y_all, void *x, void *x_lo,
-                             float *y, int32_t *counters, float *sched, int32_t total,
-                             int32_t warmup, float lr0, float b1, float b2, int32_t *err,
-                             void *stream);
 
 /* Adam for the whole network in one launch (host arrays of 10 device pointers:
  * W0..W3, b0..b3, w_out, b_out, with splits[k] partial gradients each) with the

@@ -784,6 +784,21 @@ constexpr int INF_CONSUMERS = 256;               // 8 warps
 constexpr int INF_THREADS = INF_CONSUMERS + 32;  // + producer warp
 constexpr int INF_SMEM = 2*ACT_BYTES + STAGES*CHUNK_BYTES + W0_BYTES + 2*X_BYTES;
 
+// The batch of a captured training step: rows idx[n] of a data set of `rows` rows,
+// and the schedule to advance (see schedule_step).  idx null: none.
+struct Batch {
+    const int64_t *idx;
+    long long rows;
+    const __nv_bfloat16 *x_all, *xlo_all;
+    const float *y_all;
+    __nv_bfloat16 *x, *x_lo;      // where the batch goes
+    float *y;
+    int *counters;
+    float *sched;
+    int total, warmup;
+    float lr0, b1, b2;
+};
+
 struct InferParams {
     const uint8_t *img;           // packed weights (mlp_pack)
     const float *b[4];
@@ -796,6 +811,7 @@ struct InferParams {
     const float *y;
     float delta;
     float *dout, *row_sums;
+    Batch batch;                  // mlp_serve_halves: instead of x, x_lo and y
 };
 
 // W_l [out][in] bf16 -> the chunk image: W0 as one 256 x 16 canonical tile,
@@ -1777,6 +1793,18 @@ static cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, unsigned th
 
 extern "C" {
 
+// see Batch
+struct sasb200_mlp_batch {
+    const int64_t *idx;
+    int64_t rows;
+    const void *x_all, *x_lo_all;
+    const float *y_all;
+    int32_t *counters;
+    float *sched;
+    int32_t total, warmup;
+    float lr0, b1, b2;
+};
+
 const char *sasb200_mlp_last_error(void) { return errbuf(); }
 
 // Pack the bf16 weights [out][in] into the chunk image mlp_infer streams
@@ -1958,12 +1986,14 @@ static int tile_blocks(int n_tiles, const void *img, int img_bytes, CUtensorMap 
 // The forward of a training step: out[n] as sasb200_mlp_serve, the tiled z and
 // h planes ([4][n_pad x 256] bf16 each), dout[n_pad] of the mean Huber loss
 // (threshold delta; squared error for delta <= 0) against y[n], 0 on padding,
-// and row_sums[2][n_pad/32]: the loss and dout summed over 32 rows each.
+// and row_sums[2][n_pad/32]: the loss and dout summed over 32 rows each.  With a
+// batch, x, x_lo and y receive its rows of the data set first (err = 5 for a row
+// outside it) and the schedule advances as by sasb200_lr_schedule.
 int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const void *x_lo,
                                   const void *img, const float *const *b, const float *w_out,
                                   const float *b_out, const float *y, float delta, float *out,
-                                  float *dout, float *row_sums, void *z, void *h, int32_t *err,
-                                  void *stream)
+                                  float *dout, float *row_sums, void *z, void *h,
+                                  const sasb200_mlp_batch *batch, int32_t *err, void *stream)
 {
     errbuf()[0] = 0;
     if (n < 0 || n_pad % TM || n > n_pad || !x || !x_lo || !img || !b || !w_out || !b_out || !y
@@ -1976,6 +2006,21 @@ int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const
     for (int l = 0; l < 4; ++l) {
         if (!b[l]) return (std::snprintf(errbuf(), 256, "bad bias pointer"), -1);
         prm.b[l] = b[l];
+    }
+    if (batch) {
+        if (!batch->idx || batch->rows < 0 || !batch->x_all || !batch->x_lo_all || !batch->y_all
+            || !batch->counters || !batch->sched || batch->total <= 0 || batch->warmup <= 0
+            || n <= 0)
+            return (std::snprintf(errbuf(), 256, "bad batch"), -1);
+        if ((reinterpret_cast<uintptr_t>(batch->x_all) | reinterpret_cast<uintptr_t>(batch->x_lo_all)
+             | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(x_lo)) % 16)
+            return (std::snprintf(errbuf(), 256, "features must be 16-byte aligned"), -1);
+        prm.batch = {batch->idx, batch->rows, static_cast<const __nv_bfloat16 *>(batch->x_all),
+                     static_cast<const __nv_bfloat16 *>(batch->x_lo_all), batch->y_all,
+                     static_cast<__nv_bfloat16 *>(const_cast<void *>(x)),
+                     static_cast<__nv_bfloat16 *>(const_cast<void *>(x_lo)), const_cast<float *>(y),
+                     batch->counters, batch->sched, batch->total, batch->warmup, batch->lr0,
+                     batch->b1, batch->b2};
     }
     if (n_pad == 0) return 0;
     prm.w_out = w_out;
@@ -1999,6 +2044,9 @@ int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const
         launch_dependent(kernel, dim3(blocks), SP_THREADS, HV_SMEM, st, n, n_tiles, xp, xlp, map, prm,
                          out, err);
     } else {
+        if (batch)
+            launch_dependent(gather_batch, dim3((unsigned)((4ll*n + 255)/256)), 256, 0, st, n,
+                             prm.batch, err);
         const auto kernel = mlp_serve<PLANES_TILED>;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
         launch_dependent(kernel, dim3(blocks), SV_THREADS, SV_SMEM, st, n, n_tiles, xp, xlp, prm, out,
@@ -2076,30 +2124,6 @@ int32_t sasb200_mlp_weight_grads(int32_t n, int32_t n_pad, int32_t splits, const
     launch_dependent(mlp_weight_grads, dim3((WG_BIG + 2)*splits), WG_THREADS, WG_SMEM,
                      (cudaStream_t)stream, n_pad/TM, splits, prm, err);
     return status("mlp_weight_grads");
-}
-
-// The batch of a captured training step: rows idx[n] of the data set (x_all,
-// x_lo_all [rows x 16] bf16, y_all[rows]) into x, x_lo, y, and the schedule
-// step of sasb200_lr_schedule; err receives 5 for an index outside the set.
-int32_t sasb200_gather_batch(int32_t n, int64_t rows, const int64_t *idx, const void *x_all,
-                             const void *x_lo_all, const float *y_all, void *x, void *x_lo,
-                             float *y, int32_t *counters, float *sched, int32_t total,
-                             int32_t warmup, float lr0, float b1, float b2, int32_t *err,
-                             void *stream)
-{
-    errbuf()[0] = 0;
-    if (n <= 0 || rows < 0 || !idx || !x_all || !x_lo_all || !y_all || !x || !x_lo || !y
-        || !counters || !sched || total <= 0 || warmup <= 0 || !err)
-        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
-    if ((reinterpret_cast<uintptr_t>(x_all) | reinterpret_cast<uintptr_t>(x_lo_all)
-         | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(x_lo)) % 16)
-        return (std::snprintf(errbuf(), 256, "features must be 16-byte aligned"), -1);
-    launch_dependent(gather_batch, dim3((unsigned)((4ll*n + 255)/256)), 256, 0, (cudaStream_t)stream,
-                     n, rows, idx, static_cast<const uint4 *>(x_all),
-                     static_cast<const uint4 *>(x_lo_all), y_all, static_cast<uint4 *>(x),
-                     static_cast<uint4 *>(x_lo), y, counters, sched, total, warmup, lr0, b1, b2,
-                     err);
-    return status("gather_batch");
 }
 
 // Adam for the whole network (host arrays of 10 device pointers, in the order

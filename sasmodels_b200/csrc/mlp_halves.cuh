@@ -30,6 +30,10 @@
 // count crosses, what it stands for was handed to CTA 1's own tensor core before.
 // Both CTAs meet before either exits.
 //
+// In a captured training step the forward also gathers its batch and advances the
+// schedule: a step with a launch of its own for that (gather_batch) took 51.5 us, now
+// 50.6.
+//
 // Every value is that of the kernels of one tile per SM, bit for bit.  Bound by the
 // chain of a tile still: an MMA of a pair takes 103 cycles here (32 of them a layer),
 // an epilogue 700 cycles until its first hand-over, 170 from there to the MMAs.
@@ -110,6 +114,17 @@ __device__ __forceinline__ void hv_leave_together()
     __syncthreads();
     tc::cluster_arrive_relaxed();
     tc::cluster_wait();
+}
+
+// The data set's row of batch row r: -1 past the batch, and with err = 5 outside
+// the data set.
+__device__ __forceinline__ long long batch_row(const Batch &batch, int n, int r, int *err)
+{
+    if (r >= n) return -1;
+    const long long src = batch.idx[r];
+    if (src >= 0 && src < batch.rows) return src;
+    atomicExch(err, 5);
+    return -1;
 }
 
 // PLANES: none, or a training step's tiled planes with the loss gradient.
@@ -199,6 +214,10 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         __syncwarp();
         tc::cluster_wait();
         if (lane == 0) arrive0(&x_ready);
+        if (PLANES == PLANES_TILED && prm.batch.idx && blockIdx.x == 0 && lane == 0)
+            schedule_step(prm.batch.counters, prm.batch.sched, prm.batch.total, prm.batch.warmup,
+                          prm.batch.lr0, prm.batch.b1, prm.batch.b2);
+        __syncwarp();
         if (rank != 0 && !hv_relay(lane, ready) && lane == 0) atomicExch(err, 4);
         __syncwarp();
     } else if (warp == SP_X_WARP) {
@@ -207,8 +226,17 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         for (int j = 0; j < 4; ++j) {
             const int u = lane + 32*j;
             const size_t g = (size_t)(row0 + (u >> 1))*NIN + (u & 1)*8;
-            v[j] = *reinterpret_cast<const uint4 *>(x + g);
-            w[j] = *reinterpret_cast<const uint4 *>(x_lo + g);
+            if (PLANES == PLANES_TILED && prm.batch.idx) {
+                const long long src = batch_row(prm.batch, n, row0 + (u >> 1), err);
+                v[j] = w[j] = make_uint4(0, 0, 0, 0);
+                if (src >= 0) {
+                    v[j] = *reinterpret_cast<const uint4 *>(prm.batch.x_all + src*NIN + (u & 1)*8);
+                    w[j] = *reinterpret_cast<const uint4 *>(prm.batch.xlo_all + src*NIN + (u & 1)*8);
+                }
+            } else {
+                v[j] = *reinterpret_cast<const uint4 *>(x + g);
+                w[j] = *reinterpret_cast<const uint4 *>(x_lo + g);
+            }
         }
         #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -222,6 +250,15 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         tc::cluster_wait();
         if (lane == 0) arrive0(&x_ready);
         __syncwarp();
+        // the batch's features, for the weight gradients
+        if (PLANES == PLANES_TILED && prm.batch.idx) {
+            #pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const size_t g = (size_t)row0*NIN + (lane + 32*j)*8;
+                *reinterpret_cast<uint4 *>(prm.batch.x + g) = v[j];
+                *reinterpret_cast<uint4 *>(prm.batch.x_lo + g) = w[j];
+            }
+        }
     } else if (warp == SV_MMA_WARP) {
         tc::cluster_wait();
         tc::fence_after_sync();
@@ -276,6 +313,17 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         const int row = 32*q2 + lane, trow = rank*HV_ROWS + row;
         const int col0 = 32*half + 8*slot;
         const uint32_t lane_base = tmem_slot + ((uint32_t)(32*quad) << 16) + (uint32_t)(8*slot);
+        // the target of this row, for the warps that form the output
+        float target = 0.0f;
+        if (PLANES == PLANES_TILED && half == 0 && slot == 0) {
+            if (prm.batch.idx) {
+                const long long src = batch_row(prm.batch, n, row0 + row, err);
+                if (src >= 0) target = prm.batch.y_all[src];
+                if (row0 + row < n) prm.batch.y[row0 + row] = target;
+            } else if (row0 + row < n) {
+                target = prm.y[row0 + row];
+            }
+        }
         // z and h of this thread's columns, stored when all are handed over (each with
         // its chunk: 0.4 us more)
         auto save_planes = [&](int l, const uint4 (&z)[SP_CHUNKS], const uint4 (&h)[SP_CHUNKS]) {
@@ -378,7 +426,7 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 if (valid) out[row0 + row] = o;
                 if (PLANES == PLANES_TILED) {
                     float g, loss;
-                    loss_of(valid ? o - prm.y[row0 + row] : 0.0f, prm.delta, g, loss);
+                    loss_of(valid ? o - target : 0.0f, prm.delta, g, loss);
                     g = valid ? g/(float)n : 0.0f;
                     prm.dout[row0 + row] = g;
                     #pragma unroll

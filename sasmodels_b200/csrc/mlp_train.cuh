@@ -525,31 +525,29 @@ sum_partials(SumTensors T)
 }
 
 // ------------------------------------------------------ batch and schedule --
-// One launch at the head of a captured training step: the batch's rows of the
-// data set (idx, 32 bytes of x and of x_lo and one target each) and, by one
-// thread, the schedule.  Bound by the random 32-byte reads (0.8 MB of 8192 rows);
-// 5.6 us with cold caches, where three index_select launches and lr_schedule took
-// 29.  A row outside the data set leaves zeros and err = 5.
+// The batch of a captured training step for a forward of one tile per SM (that of
+// two SMs per tile gathers its own): the batch's rows of the data set (idx, 32 bytes
+// of x and of x_lo and one target each) and, by one thread, the schedule.  Bound by
+// the random 32-byte reads; 5.6 us with cold caches for 8192 rows, where three
+// index_select launches and lr_schedule took 29.  A row outside the data set leaves
+// zeros and err = 5.
 __global__ void __launch_bounds__(256)
-gather_batch(int n, long long rows, const int64_t *__restrict__ idx,
-             const uint4 *__restrict__ x_all, const uint4 *__restrict__ xlo_all,
-             const float *__restrict__ y_all, uint4 *__restrict__ x, uint4 *__restrict__ x_lo,
-             float *__restrict__ y, int *__restrict__ counters, float *__restrict__ sched,
-             int total, int warmup, float lr0, float b1, float b2, int *__restrict__ err)
+gather_batch(int n, Batch batch, int *__restrict__ err)
 {
     tc::dependents_launch();
     tc::dependency_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0)
-        schedule_step(counters, sched, total, warmup, lr0, b1, b2);
+        schedule_step(batch.counters, batch.sched, batch.total, batch.warmup, batch.lr0, batch.b1,
+                      batch.b2);
     const int i = blockIdx.x*256 + threadIdx.x, row = i >> 2, part = i & 3;
     if (row >= n) return;
-    const long long src = idx[row];
-    const bool in = src >= 0 && src < rows;
+    const long long src = batch.idx[row];
+    const bool in = src >= 0 && src < batch.rows;
     uint4 v = make_uint4(0, 0, 0, 0);
-    if (in) v = (part < 2 ? x_all : xlo_all)[2*src + (part & 1)];
-    (part < 2 ? x : x_lo)[2*row + (part & 1)] = v;
+    if (in) v = reinterpret_cast<const uint4 *>(part < 2 ? batch.x_all : batch.xlo_all)[2*src + (part & 1)];
+    reinterpret_cast<uint4 *>(part < 2 ? batch.x : batch.x_lo)[2*row + (part & 1)] = v;
     if (part == 0) {
-        y[row] = in ? y_all[src] : 0.0f;
+        batch.y[row] = in ? batch.y_all[src] : 0.0f;
         if (!in) atomicExch(err, 5);
     }
 }

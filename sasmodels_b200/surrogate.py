@@ -77,17 +77,16 @@ def _load():
     lib.sasb200_mlp_serve.argtypes = [I, I, P, P, P, P, P, P, P, P, P, P, I, P]
     lib.sasb200_mlp_pack_t.argtypes = [P, P, P, P, P]
     lib.sasb200_mlp_backward_p.argtypes = [I, I, P, P, P, P, P, P, I, P]
-    lib.sasb200_mlp_train_forward.argtypes = [I, I] + [P]*7 + [F] + [P]*7
+    lib.sasb200_mlp_train_forward.argtypes = [I, I] + [P]*7 + [F] + [P]*8
     lib.sasb200_mlp_train_backward.argtypes = [I] + [P]*7
     lib.sasb200_mlp_weight_grads.argtypes = [I, I, I] + [P]*12
     lib.sasb200_sum_partials.argtypes = [I] + [P]*5
-    lib.sasb200_gather_batch.argtypes = [I, ct.c_int64] + [P]*9 + [I, I, F, F, F, P, P]
     lib.sasb200_adam_pack.argtypes = [P]*10 + [F, I, F, F, F, P]
     D = ct.c_double
     lib.sasb200_features_runs.argtypes = [I, I, I] + [P]*6
     lib.sasb200_finish_runs.argtypes = [I, I] + [P]*5 + [D]*7 + [P]*3
     for name in ("sasb200_features_runs", "sasb200_finish_runs",
-                 "sasb200_gather_batch", "sasb200_adam_pack",
+                 "sasb200_adam_pack",
                  "sasb200_mlp_train_forward", "sasb200_mlp_train_backward",
                  "sasb200_mlp_weight_grads", "sasb200_sum_partials",
                  "sasb200_mlp_forward", "sasb200_mlp_backward", "sasb200_gemm_nt",
@@ -288,10 +287,11 @@ class MLP:
             n, I32(*self._sizes[first:9]), I32(*[self.splits]*n), VP(*self._part_at[first:]),
             VP(*outs), self.stream.cuda_stream), "sum_partials")
 
-    def _gradient_kernels(self, x, x_lo, y, n, loss, db_out):
+    def _gradient_kernels(self, x, x_lo, y, n, loss, db_out, batch=None):
         """Forward, backward and weight gradients of one batch: the loss and
         db_out as scalars, the other gradients as partial sums over
-        self.splits (gW, gb_part, gw_part).  loss and db_out are addresses."""
+        self.splits (gW, gb_part, gw_part).  loss and db_out are addresses.  With
+        `batch` (a _Batch), x, x_lo and y receive its rows first."""
         n_pad = x.shape[0]
         st, lib, at = self.stream.cuda_stream, self.lib, self._at
         err, w_out = self.err.data_ptr(), self.w_out.data_ptr()
@@ -300,7 +300,7 @@ class MLP:
         self._check(lib.sasb200_mlp_train_forward(
             n, n_pad, x.data_ptr(), x_lo.data_ptr(), self.img.data_ptr(), self._ptrs(self.b),
             w_out, self.b_out.data_ptr(), y.data_ptr(), float(self.huber), at["out"], dout, sums,
-            z, h, err, st), "forward")
+            z, h, None if batch is None else ct.byref(batch), err, st), "forward")
         self._check(lib.sasb200_mlp_train_backward(n_pad, self.img_t.data_ptr(), w_out, dout, z,
                                                    dz, err, st), "backward")
         self._check(lib.sasb200_mlp_weight_grads(
@@ -536,6 +536,15 @@ def gate_thresholds(r, err, tols, alpha):
     return np.maximum.accumulate(np.array(out, dtype=float))
 
 
+class _Batch(ct.Structure):
+    """The batch of a captured training step (sasb200_mlp_batch)."""
+
+    _fields_ = [("idx", ct.c_void_p), ("rows", ct.c_int64), ("x_all", ct.c_void_p),
+                ("x_lo_all", ct.c_void_p), ("y_all", ct.c_void_p), ("counters", ct.c_void_p),
+                ("sched", ct.c_void_p), ("total", ct.c_int32), ("warmup", ct.c_int32),
+                ("lr0", ct.c_float), ("b1", ct.c_float), ("b2", ct.c_float)]
+
+
 class TrainingGraph:
     """One training step of an :class:`MLP` captured as a CUDA graph: the
     batch gather (rows named by ``idx``) and the learning-rate schedule,
@@ -561,7 +570,7 @@ class TrainingGraph:
         self.loss = torch.zeros((), dtype=torch.float32, device=dev)
         net._scratch(batch)
         lib, st = net.lib, net.stream.cuda_stream
-        # the gather kernel takes 32-byte rows of bf16 and float targets, as
+        # the forward gathers 32-byte rows of bf16 and float targets, as
         # MLP.features and the surrogate lay them out
         direct = (all(t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[1] == NIN
                       for t in (x_all, x_lo_all))
@@ -574,19 +583,15 @@ class TrainingGraph:
         net.stream.synchronize()
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph, stream=net.stream):
-            if direct:
-                net._check(lib.sasb200_gather_batch(
-                    batch, len(y_all), self.idx.data_ptr(), x_all.data_ptr(),
-                    x_lo_all.data_ptr(), y_all.data_ptr(), self.xb.data_ptr(),
-                    self.xlb.data_ptr(), self.yb.data_ptr(), *schedule,
-                    net.err.data_ptr(), st), "gather_batch")
-            else:
+            if not direct:
                 torch.index_select(x_all, 0, self.idx, out=self.xb)
                 torch.index_select(x_lo_all, 0, self.idx, out=self.xlb)
                 torch.index_select(y_all, 0, self.idx, out=self.yb)
                 net._check(lib.sasb200_lr_schedule(*schedule, st), "lr_schedule")
-            net._gradient_kernels(self.xb, self.xlb, self.yb, batch, self.loss.data_ptr(),
-                                  net.gbo.data_ptr())
+            net._gradient_kernels(
+                self.xb, self.xlb, self.yb, batch, self.loss.data_ptr(), net.gbo.data_ptr(),
+                _Batch(self.idx.data_ptr(), len(y_all), x_all.data_ptr(), x_lo_all.data_ptr(),
+                       y_all.data_ptr(), *schedule) if direct else None)
             net._adam(net.gW + list(net.gb_part) + [net.gw_part, net.gbo], [net.splits]*9 + [1],
                       self.sched, lr, b1, b2, eps)
         # what the graph reads and writes outlives the network's next, larger

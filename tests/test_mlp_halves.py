@@ -47,3 +47,38 @@ def test_serve(cuda, rows):
 def test_training_step(cuda, extra):
     """The last batch that has two SMs per tile, and the first that has not."""
     train.test_training_step_kernels(cuda, _sms()//2*128 + extra)
+
+
+@pytest.mark.parametrize("tiles", [1, 0, "more"])
+def test_captured_batch(cuda, tiles):
+    """The forward that gathers its batch (tiles 0: the most it takes) and, from one
+    tile more on, the gathering launch, against index_select (strided data)."""
+    import torch
+    from sasmodels_b200.surrogate import MLP
+    B = 128*(_sms()//2 + 1 if tiles == "more" else tiles or _sms()//2)
+    n = B + 77
+    wide = torch.rand((n, 32), device="cuda").to(torch.bfloat16)
+    y = torch.randn(n, device="cuda")
+    idx = torch.randint(0, n, (B,), device="cuda")
+    done = []
+    for x in (wide[:, :16], wide[:, :16].contiguous()):
+        net = MLP(seed=4)
+        lo = torch.full_like(x, 2.0**-9)
+        torch.cuda.synchronize()
+        graph = net.capture_training(x, lo, y, B, 1e-3, 100, 1)
+        losses = [float(graph.step(idx).item()) for _ in range(2)]
+        net.stream.synchronize()
+        assert net.errors() == 0
+        done.append((net, losses, graph))
+    assert done[0][1] == done[1][1]
+    for u, v in zip(done[0][0].params, done[1][0].params):
+        assert torch.equal(u, v)
+    for name in ("xb", "xlb", "yb", "counters", "sched"):
+        assert torch.equal(getattr(done[0][2], name), getattr(done[1][2], name))
+    net, _, graph = done[1]
+    idx[B - 1] = -1
+    torch.cuda.synchronize()
+    graph.step(idx)
+    net.stream.synchronize()
+    assert net.errors() == 5
+    assert (graph.xb[B - 1] == 0).all() and graph.yb[B - 1] == 0
