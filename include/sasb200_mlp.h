@@ -103,18 +103,20 @@ int32_t sasb200_adam(int32_t size, int32_t splits, const float *grad, float *p, 
                      float *v, float lr, float b1, float b2, float eps, int32_t step, void *w,
                      void *wt, int32_t rows, int32_t cols, void *stream);
 
-/* a training step on tiled planes, [4 layers][n_pad/128 tiles][32 groups][128
- * rows][8] bf16 (group g holds columns 8g .. 8g + 7): the forward with the loss
- * gradient dout[n_pad] of the mean Huber loss (delta <= 0: squared error)
- * against y[n] and row_sums[2][n_pad/32] (loss and dout summed over 32 rows
- * each); the backward from dout; every gradient as partial sums over splits of
- * the rows (dw[l]: [splits][256 x (16 or 256)], db: [4][splits][256], dw_out:
- * [splits][256]), the mean loss and db_out as scalars; and outs[k][i] = sum of
- * parts[k][s*sizes[k] + i] over s for n <= 16 tensors (host arrays).
- * The forward of a captured step takes a batch (else NULL): x, x_lo and y then
- * receive the rows idx[n] of the data set (x_all, x_lo_all [rows x 16] bf16,
- * y_all[rows]) first, and the schedule advances as by sasb200_lr_schedule; an
- * index outside the set leaves zeros and *err = 5. */
+/* Loss and gradients of one batch, on tiled planes [4 layers][n_pad/128 tiles][32
+ * groups][128 rows][8] bf16 (group g holds columns 8g .. 8g + 7): the forward
+ * (out[n], z, h) with the loss gradient dout[n_pad] of the mean Huber loss (delta
+ * <= 0: squared error) against y[n] and row_sums[2][n_pad/32] (loss and dout
+ * summed over 32 rows each); the backward (dz); every gradient as partial sums
+ * over splits of the rows (dw[l]: [splits][256 x (16 or 256)], 32-byte aligned,
+ * db: [4][splits][256], dw_out: [splits][256]), the mean loss and db_out as
+ * scalars; then, for k < sums (at most 16), sum_outs[k][i] = sum of
+ * sum_parts[k][s*sum_sizes[k] + i] over s < sum_splits[k].
+ *
+ * A captured step takes a batch (else NULL): x, x_lo and y then receive the rows
+ * idx[n] of the data set (x_all, x_lo_all [rows x 16] bf16, y_all[rows]) first,
+ * and the schedule advances as by sasb200_lr_schedule; an index outside the set
+ * leaves zeros and *err = 5. */
 typedef struct sasb200_mlp_batch {
     const int64_t *idx;
     int64_t rows;
@@ -125,21 +127,26 @@ typedef struct sasb200_mlp_batch {
     int32_t total, warmup;
     float lr0, b1, b2;
 } sasb200_mlp_batch;
-int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const void *x_lo,
-                                  const void *img, const float *const *b, const float *w_out,
-                                  const float *b_out, const float *y, float delta, float *out,
-                                  float *dout, float *row_sums, void *z, void *h,
-                                  const sasb200_mlp_batch *batch, int32_t *err, void *stream);
-int32_t sasb200_mlp_train_backward(int32_t n_pad, const void *img_t, const float *w_out,
-                                   const float *dout, const void *z, void *dz, int32_t *err,
-                                   void *stream);
-int32_t sasb200_mlp_weight_grads(int32_t n, int32_t n_pad, int32_t splits, const void *x,
-                                 const void *h, const void *dz, const float *dout,
-                                 const float *row_sums, float *const *dw, float *db,
-                                 float *dw_out, float *loss, float *db_out, int32_t *err,
-                                 void *stream);
-int32_t sasb200_sum_partials(int32_t n, const int32_t *sizes, const int32_t *splits,
-                             const float *const *parts, float *const *outs, void *stream);
+typedef struct sasb200_mlp_pass {
+    int32_t n, n_pad, splits;
+    float delta;
+    const void *x, *x_lo;
+    const float *y;
+    const void *img, *img_t;       /* sasb200_mlp_pack, sasb200_mlp_pack_t */
+    const float *b[4];
+    const float *w_out, *b_out;
+    float *out, *dout, *row_sums;
+    void *z, *h, *dz;
+    float *dw[4];
+    float *db, *dw_out, *loss, *db_out;
+    const sasb200_mlp_batch *batch;
+    int32_t *err;
+    int32_t sums;
+    int32_t sum_sizes[16], sum_splits[16];
+    const float *sum_parts[16];
+    float *sum_outs[16];
+} sasb200_mlp_pass;
+int32_t sasb200_mlp_train_pass(const sasb200_mlp_pass *pass, void *stream);
 
 /* Adam for the whole network in one launch (host arrays of 10 device pointers:
  * W0..W3, b0..b3, w_out, b_out, with splits[k] partial gradients each) with the

@@ -1816,6 +1816,27 @@ struct sasb200_mlp_batch {
     float lr0, b1, b2;
 };
 
+// the operands of sasb200_mlp_train_pass
+struct sasb200_mlp_pass {
+    int32_t n, n_pad, splits;
+    float delta;
+    const void *x, *x_lo;
+    const float *y;
+    const void *img, *img_t;
+    const float *b[4];
+    const float *w_out, *b_out;
+    float *out, *dout, *row_sums;
+    void *z, *h, *dz;
+    float *dw[4];
+    float *db, *dw_out, *loss, *db_out;
+    const sasb200_mlp_batch *batch;
+    int32_t *err;
+    int32_t sums;
+    int32_t sum_sizes[16], sum_splits[16];
+    const float *sum_parts[16];
+    float *sum_outs[16];
+};
+
 const char *sasb200_mlp_last_error(void) { return errbuf(); }
 
 // Pack the bf16 weights [out][in] into the chunk image mlp_infer streams
@@ -2000,11 +2021,11 @@ static int tile_blocks(int n_tiles, const void *img, int img_bytes, CUtensorMap 
 // and row_sums[2][n_pad/32]: the loss and dout summed over 32 rows each.  With a
 // batch, x, x_lo and y receive its rows of the data set first (err = 5 for a row
 // outside it) and the schedule advances as by sasb200_lr_schedule.
-int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const void *x_lo,
-                                  const void *img, const float *const *b, const float *w_out,
-                                  const float *b_out, const float *y, float delta, float *out,
-                                  float *dout, float *row_sums, void *z, void *h,
-                                  const sasb200_mlp_batch *batch, int32_t *err, void *stream)
+static int32_t train_forward(int32_t n, int32_t n_pad, const void *x, const void *x_lo,
+                             const void *img, const float *const *b, const float *w_out,
+                             const float *b_out, const float *y, float delta, float *out,
+                             float *dout, float *row_sums, void *z, void *h,
+                             const sasb200_mlp_batch *batch, int32_t *err, void *stream)
 {
     errbuf()[0] = 0;
     if (n < 0 || n_pad % TM || n > n_pad || !x || !x_lo || !img || !b || !w_out || !b_out || !y
@@ -2068,9 +2089,9 @@ int32_t sasb200_mlp_train_forward(int32_t n, int32_t n_pad, const void *x, const
 
 // The backward of a training step: tiled dZ planes from dout[n_pad] and the
 // tiled z planes.
-int32_t sasb200_mlp_train_backward(int32_t n_pad, const void *img_t, const float *w_out,
-                                   const float *dout, const void *z, void *dz, int32_t *err,
-                                   void *stream)
+static int32_t train_backward(int32_t n_pad, const void *img_t, const float *w_out,
+                              const float *dout, const void *z, void *dz, int32_t *err,
+                              void *stream)
 {
     errbuf()[0] = 0;
     if (n_pad < 0 || n_pad % TM || !img_t || !w_out || !dout || !z || !dz || !err)
@@ -2102,11 +2123,11 @@ int32_t sasb200_mlp_train_backward(int32_t n_pad, const void *img_t, const float
 // Every gradient of a training step from its planes: dw[0..3] [splits][256 x (16
 // or 256)], db [4][splits][256] and dw_out [splits][256] as partial sums over
 // splits of the rows; the mean loss over n rows and db_out as scalars.
-int32_t sasb200_mlp_weight_grads(int32_t n, int32_t n_pad, int32_t splits, const void *x,
-                                 const void *h, const void *dz, const float *dout,
-                                 const float *row_sums, float *const *dw, float *db,
-                                 float *dw_out, float *loss, float *db_out, int32_t *err,
-                                 void *stream)
+static int32_t weight_grads(int32_t n, int32_t n_pad, int32_t splits, const void *x,
+                            const void *h, const void *dz, const float *dout,
+                            const float *row_sums, float *const *dw, float *db,
+                            float *dw_out, float *loss, float *db_out, int32_t *err,
+                            void *stream)
 {
     errbuf()[0] = 0;
     if (n < 0 || n > n_pad || n_pad <= 0 || n_pad % TM || splits <= 0 || splits > 4096 || !x || !h
@@ -2184,8 +2205,8 @@ int32_t sasb200_adam_pack(const float *const *grads, const int32_t *splits, floa
 
 // outs[k][i] = sum over s < splits[k] of parts[k][s*sizes[k] + i] for n (<= 16)
 // tensors (host arrays of device pointers).
-int32_t sasb200_sum_partials(int32_t n, const int32_t *sizes, const int32_t *splits,
-                             const float *const *parts, float *const *outs, void *stream)
+static int32_t sum_partials_of(int32_t n, const int32_t *sizes, const int32_t *splits,
+                               const float *const *parts, float *const *outs, void *stream)
 {
     errbuf()[0] = 0;
     if (n <= 0 || n > SUM_TENSORS || !sizes || !splits || !parts || !outs)
@@ -2203,6 +2224,27 @@ int32_t sasb200_sum_partials(int32_t n, const int32_t *sizes, const int32_t *spl
     }
     launch_dependent(sum_partials, dim3((most + 255)/256, n), 256, 0, (cudaStream_t)stream, T);
     return status("sum_partials");
+}
+
+// Loss and gradients of one batch: the forward, the backward and the weight
+// gradients above, then `sums` tensors added over the splits into their places.
+// One call, as the four cost a caller as long as the kernels take.
+int32_t sasb200_mlp_train_pass(const sasb200_mlp_pass *p, void *stream)
+{
+    errbuf()[0] = 0;
+    if (!p || p->sums < 0 || p->sums > SUM_TENSORS)
+        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
+    int32_t rc = train_forward(p->n, p->n_pad, p->x, p->x_lo, p->img, p->b, p->w_out, p->b_out, p->y,
+                               p->delta, p->out, p->dout, p->row_sums, p->z, p->h, p->batch, p->err,
+                               stream);
+    if (rc == 0)
+        rc = train_backward(p->n_pad, p->img_t, p->w_out, p->dout, p->z, p->dz, p->err, stream);
+    if (rc == 0)
+        rc = weight_grads(p->n, p->n_pad, p->splits, p->x, p->h, p->dz, p->dout, p->row_sums, p->dw,
+                          p->db, p->dw_out, p->loss, p->db_out, p->err, stream);
+    if (rc == 0 && p->sums > 0)
+        rc = sum_partials_of(p->sums, p->sum_sizes, p->sum_splits, p->sum_parts, p->sum_outs, stream);
+    return rc;
 }
 
 // out[n] (and z/h planes [4][n_pad x 256] when non-null) for x[n_pad x 16];

@@ -77,18 +77,14 @@ def _load():
     lib.sasb200_mlp_serve.argtypes = [I, I, P, P, P, P, P, P, P, P, P, P, I, P]
     lib.sasb200_mlp_pack_t.argtypes = [P, P, P, P, P]
     lib.sasb200_mlp_backward_p.argtypes = [I, I, P, P, P, P, P, P, I, P]
-    lib.sasb200_mlp_train_forward.argtypes = [I, I] + [P]*7 + [F] + [P]*8
-    lib.sasb200_mlp_train_backward.argtypes = [I] + [P]*7
-    lib.sasb200_mlp_weight_grads.argtypes = [I, I, I] + [P]*12
-    lib.sasb200_sum_partials.argtypes = [I] + [P]*5
+    lib.sasb200_mlp_train_pass.argtypes = [P, P]
     lib.sasb200_adam_pack.argtypes = [P]*10 + [F, I, F, F, F, P]
     D = ct.c_double
     lib.sasb200_features_runs.argtypes = [I, I, I] + [P]*6
     lib.sasb200_finish_runs.argtypes = [I, I] + [P]*5 + [D]*7 + [P]*3
     for name in ("sasb200_features_runs", "sasb200_finish_runs",
                  "sasb200_adam_pack",
-                 "sasb200_mlp_train_forward", "sasb200_mlp_train_backward",
-                 "sasb200_mlp_weight_grads", "sasb200_sum_partials",
+                 "sasb200_mlp_train_pass",
                  "sasb200_mlp_forward", "sasb200_mlp_backward", "sasb200_gemm_nt",
                  "sasb200_transpose_bf16", "sasb200_loss_grad",
                  "sasb200_adam", "sasb200_mlp_features", "sasb200_mlp_pack",
@@ -103,6 +99,30 @@ def _load():
 
 def pad128(n):
     return ((n + TM - 1)//TM)*TM
+
+
+class _Batch(ct.Structure):
+    """The batch of a captured training step (sasb200_mlp_batch)."""
+
+    _fields_ = [("idx", ct.c_void_p), ("rows", ct.c_int64), ("x_all", ct.c_void_p),
+                ("x_lo_all", ct.c_void_p), ("y_all", ct.c_void_p), ("counters", ct.c_void_p),
+                ("sched", ct.c_void_p), ("total", ct.c_int32), ("warmup", ct.c_int32),
+                ("lr0", ct.c_float), ("b1", ct.c_float), ("b2", ct.c_float)]
+
+
+class _Pass(ct.Structure):
+    """The operands of a gradient pass (sasb200_mlp_pass)."""
+
+    _fields_ = ([(k, ct.c_int32) for k in ("n", "n_pad", "splits")] + [("delta", ct.c_float)]
+                + [(k, ct.c_void_p) for k in ("x", "x_lo", "y", "img", "img_t")]
+                + [("b", ct.c_void_p*4)]
+                + [(k, ct.c_void_p) for k in ("w_out", "b_out", "out", "dout", "row_sums", "z",
+                                              "h", "dz")]
+                + [("dw", ct.c_void_p*4)]
+                + [(k, ct.c_void_p) for k in ("db", "dw_out", "loss", "db_out", "batch", "err")]
+                + [("sums", ct.c_int32), ("sum_sizes", ct.c_int32*16),
+                   ("sum_splits", ct.c_int32*16), ("sum_parts", ct.c_void_p*16),
+                   ("sum_outs", ct.c_void_p*16)])
 
 
 class MLP:
@@ -194,13 +214,14 @@ class MLP:
         self.gw = torch.empty(HID, **f32)
         self.gbo = torch.empty(1, **f32)
         # their addresses, which change with them only
-        self._at = {k: getattr(self, k).data_ptr() for k in
-                    ("z_save", "h_save", "dz_save", "out", "dout", "row_sums", "gb_part",
-                     "gw_part")}
-        self._gW_at = self._ptrs(self.gW)
-        self._part_at = ([g.data_ptr() for g in self.gW]
-                         + [self._at["gb_part"] + 4*self.splits*HID*l for l in range(4)]
-                         + [self._at["gw_part"]])
+        p = self._pass = _Pass(splits=self.splits, err=self.err.data_ptr())
+        for field, t in (("z", self.z_save), ("h", self.h_save), ("dz", self.dz_save),
+                         ("out", self.out), ("dout", self.dout), ("row_sums", self.row_sums),
+                         ("db", self.gb_part), ("dw_out", self.gw_part)):
+            setattr(p, field, t.data_ptr())
+        p.dw[:] = [g.data_ptr() for g in self.gW]
+        self._part_at = (list(p.dw) + [p.db + 4*self.splits*HID*l for l in range(4)]
+                         + [p.dw_out])
         self._scratch_n = n_pad
 
     # ----------------------------------------------------------- kernels --
@@ -273,39 +294,32 @@ class MLP:
         self._pack()
         with torch.cuda.stream(self.stream):
             loss = torch.empty((), dtype=torch.float32, device=self.device)
-        self._gradient_kernels(x, x_lo, y, n, loss.data_ptr(), self.gbo.data_ptr())
-        self._sum_partials(4, [t.data_ptr() for t in self.gb + [self.gw]])
+        self._gradient_kernels(x, x_lo, y, n, loss.data_ptr(), self.gbo.data_ptr(), 4,
+                               [t.data_ptr() for t in self.gb + [self.gw]])
         return loss, self.gW, self.gb, self.gw, self.gbo
 
-    def _sum_partials(self, first, outs):
-        """The partial sums of the parameters from `first` on (in the order of
-        params, up to w_out) added over the splits into the addresses `outs`,
-        in one launch."""
-        n = 9 - first
-        I32, VP = ct.c_int32*n, ct.c_void_p*n
-        self._check(self.lib.sasb200_sum_partials(
-            n, I32(*self._sizes[first:9]), I32(*[self.splits]*n), VP(*self._part_at[first:]),
-            VP(*outs), self.stream.cuda_stream), "sum_partials")
-
-    def _gradient_kernels(self, x, x_lo, y, n, loss, db_out, batch=None):
+    def _gradient_kernels(self, x, x_lo, y, n, loss, db_out, first=9, outs=(), batch=None):
         """Forward, backward and weight gradients of one batch: the loss and
         db_out as scalars, the other gradients as partial sums over
-        self.splits (gW, gb_part, gw_part).  loss and db_out are addresses.  With
-        `batch` (a _Batch), x, x_lo and y receive its rows first."""
-        n_pad = x.shape[0]
-        st, lib, at = self.stream.cuda_stream, self.lib, self._at
-        err, w_out = self.err.data_ptr(), self.w_out.data_ptr()
-        z, h, dz, dout, sums = (at[k] for k in ("z_save", "h_save", "dz_save", "dout",
-                                                "row_sums"))
-        self._check(lib.sasb200_mlp_train_forward(
-            n, n_pad, x.data_ptr(), x_lo.data_ptr(), self.img.data_ptr(), self._ptrs(self.b),
-            w_out, self.b_out.data_ptr(), y.data_ptr(), float(self.huber), at["out"], dout, sums,
-            z, h, None if batch is None else ct.byref(batch), err, st), "forward")
-        self._check(lib.sasb200_mlp_train_backward(n_pad, self.img_t.data_ptr(), w_out, dout, z,
-                                                   dz, err, st), "backward")
-        self._check(lib.sasb200_mlp_weight_grads(
-            n, n_pad, self.splits, x.data_ptr(), h, dz, dout, sums, self._gW_at, at["gb_part"],
-            at["gw_part"], loss, db_out, err, st), "weight_grads")
+        self.splits (gW, gb_part, gw_part); those of the parameters from
+        `first` on (in the order of params, up to w_out) added over the splits
+        into `outs`.  loss, db_out and outs are addresses.  With `batch` (a
+        _Batch), x, x_lo and y receive its rows first."""
+        p, sums = self._pass, len(outs)
+        p.n, p.n_pad, p.delta = n, x.shape[0], float(self.huber)
+        p.x, p.x_lo, p.y = x.data_ptr(), x_lo.data_ptr(), y.data_ptr()
+        p.img, p.img_t = self.img.data_ptr(), self.img_t.data_ptr()
+        p.b[:] = [t.data_ptr() for t in self.b]
+        p.w_out, p.b_out = self.w_out.data_ptr(), self.b_out.data_ptr()
+        p.loss, p.db_out, p.sums = loss, db_out, sums
+        if sums:
+            p.sum_sizes[:sums] = self._sizes[first:9]
+            p.sum_splits[:sums] = [self.splits]*sums
+            p.sum_parts[:sums] = self._part_at[first:]
+            p.sum_outs[:sums] = outs
+        p.batch = None if batch is None else ct.addressof(batch)
+        self._check(self.lib.sasb200_mlp_train_pass(ct.byref(p), self.stream.cuda_stream),
+                    "train_pass")
 
     def train_step(self, x, x_lo, y, n, lr, b1=0.9, b2=0.999, eps=1e-8, reduce=None):
         """One Adam step on one batch; returns the loss (a device scalar).
@@ -336,8 +350,7 @@ class MLP:
         with torch.cuda.stream(self.stream):
             flat = torch.empty(sum(sizes) + 1, dtype=torch.float32, device=self.device)
         ends = [flat.data_ptr() + 4*sum(sizes[:k]) for k in range(len(sizes) + 1)]
-        self._gradient_kernels(x, x_lo, y, n, ends[10], ends[9])
-        self._sum_partials(0, ends[:9])
+        self._gradient_kernels(x, x_lo, y, n, ends[10], ends[9], 0, ends[:9])
         parts = flat.split(sizes + [1])
         return [parts[-1]] + list(parts[:-1])
 
@@ -536,15 +549,6 @@ def gate_thresholds(r, err, tols, alpha):
     return np.maximum.accumulate(np.array(out, dtype=float))
 
 
-class _Batch(ct.Structure):
-    """The batch of a captured training step (sasb200_mlp_batch)."""
-
-    _fields_ = [("idx", ct.c_void_p), ("rows", ct.c_int64), ("x_all", ct.c_void_p),
-                ("x_lo_all", ct.c_void_p), ("y_all", ct.c_void_p), ("counters", ct.c_void_p),
-                ("sched", ct.c_void_p), ("total", ct.c_int32), ("warmup", ct.c_int32),
-                ("lr0", ct.c_float), ("b1", ct.c_float), ("b2", ct.c_float)]
-
-
 class TrainingGraph:
     """One training step of an :class:`MLP` captured as a CUDA graph: the
     batch gather (rows named by ``idx``) and the learning-rate schedule,
@@ -590,8 +594,8 @@ class TrainingGraph:
                 net._check(lib.sasb200_lr_schedule(*schedule, st), "lr_schedule")
             net._gradient_kernels(
                 self.xb, self.xlb, self.yb, batch, self.loss.data_ptr(), net.gbo.data_ptr(),
-                _Batch(self.idx.data_ptr(), len(y_all), x_all.data_ptr(), x_lo_all.data_ptr(),
-                       y_all.data_ptr(), *schedule) if direct else None)
+                batch=_Batch(self.idx.data_ptr(), len(y_all), x_all.data_ptr(), x_lo_all.data_ptr(),
+                             y_all.data_ptr(), *schedule) if direct else None)
             net._adam(net.gW + list(net.gb_part) + [net.gw_part, net.gbo], [net.splits]*9 + [1],
                       self.sched, lr, b1, b2, eps)
         # what the graph reads and writes outlives the network's next, larger
