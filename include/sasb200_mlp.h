@@ -58,12 +58,14 @@ int32_t sasb200_mlp_infer(int32_t n, int32_t n_pad, const void *x, const void *x
                           const float *b_out, float *out, void *z_save, void *h_save,
                           int32_t *err, int32_t blocks, void *stream);
 
-/* the same forward through the overlapped kernel (a dedicated MMA warp, two
- * TMEM accumulators, layer l+1's MMAs running under layer l's epilogue chunk
- * by chunk), same image and arguments.  Hidden activations and the z/h
- * planes bitwise those of sasb200_mlp_infer; out differs only by the order
- * of the output dot's sums.  Used for inference (planes NULL) and for the
- * training forward. */
+/* the same forward through the overlapped kernels (a dedicated MMA warp, layer
+ * l+1's MMAs running under layer l's epilogue chunk by chunk), same image and
+ * arguments: two SMs per tile of 128 rows while 2 n_pad/128 CTAs may run at
+ * once, then a tile per SM, then pairs of SMs with two tiles each in flight;
+ * with planes always a tile per SM.  The values do not depend on the choice.
+ * Hidden activations and the z/h planes bitwise those of sasb200_mlp_infer; out
+ * differs only by the order of the output dot's sums.  *err receives 1, 2, 3 or
+ * 4 if a pipeline wait ran out. */
 int32_t sasb200_mlp_serve(int32_t n, int32_t n_pad, const void *x, const void *x_lo,
                           const void *img, const float *const *b, const float *w_out,
                           const float *b_out, float *out, void *z_save, void *h_save,

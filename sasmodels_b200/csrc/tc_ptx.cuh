@@ -146,10 +146,6 @@ __device__ __forceinline__ uint32_t spin_acquire_until(const uint32_t *p, uint32
     for (uint32_t i = 0; i < WAIT_LIMIT && v < target; ++i) v = ld_acquire_shared(p);
     return v;
 }
-__device__ __forceinline__ bool spin_acquire_ge(const uint32_t *p, uint32_t target)
-{
-    return spin_acquire_until(p, target) >= target;
-}
 
 // ---- bulk copy (TMA engine, untiled, no multicast) --------------------------
 // global -> this CTA's shared memory, completion counted on *bar.  Both

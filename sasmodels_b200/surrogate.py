@@ -342,7 +342,7 @@ class MLP:
     def reduced_gradients(self, x, x_lo, y, n):
         """[loss (1 element), dW_1..dW_4, db_1..db_4, dw_out, db_out] of one
         batch as fp32 device tensors, the weight gradients summed over their
-        split-K partials: the ≈200k numbers a data-parallel step exchanges."""
+        partials: the ≈200k numbers a data-parallel step exchanges."""
         torch = self.torch
         self._scratch(x.shape[0])
         self._pack()
