@@ -24,7 +24,8 @@
 //                  at once (a dedicated MMA warp, two TMEM accumulators,
 //                  layer l+1's MMAs under layer l's epilogue chunk by chunk);
 //                  serves inference and the training forward.
-//   mlp_serve_halves, mlp_backward_halves   few tiles: two SMs per tile
+//   mlp_halves     few tiles: two SMs per tile; serving, or forward and backward of
+//                  a training step (mlp_halves.cuh)
 //   mlp_serve_pairs   inference over many tiles: pairs of SMs (cta_group::2), two
 //                  tiles in flight on each (mlp_pairs.cuh).
 //   mlp_backward_t, mlp_weight_grads   the training step's backward and weight
@@ -822,7 +823,7 @@ struct InferParams {
     const float *y;
     float delta;
     float *dout, *row_sums;
-    Batch batch;                  // mlp_serve_halves: instead of x, x_lo and y
+    Batch batch;                  // mlp_halves: instead of x, x_lo and y
 };
 
 // W_l [out][in] bf16 -> the chunk image: W0 as one 256 x 16 canonical tile,
@@ -1943,7 +1944,7 @@ int32_t sasb200_mlp_infer(int32_t n, int32_t n_pad, const void *x, const void *x
 }
 
 // out[n] for x, x_lo [n_pad x 16] with the packed weights through the
-// overlapped kernels (mlp_serve; where no planes are wanted, mlp_serve_halves for few
+// overlapped kernels (mlp_serve; where no planes are wanted, mlp_halves for few
 // tiles and mlp_serve_pairs where a CTA has several: the same values), and, when
 // z_save/h_save are given, the pre-activations and activations of all four layers
 // ([4][n_pad x 256] bf16 each, those of mlp_infer) for training; grid of at most
@@ -1986,10 +1987,10 @@ int32_t sasb200_mlp_serve(int32_t n, int32_t n_pad, const void *x, const void *x
     // beyond, the second round would cost more than the halves save
     CUtensorMap map;
     if (!z_save && n_tiles <= blocks/2 && hv_map(map, img, IMG_BYTES/(8*HV_RUN))) {
-        const auto kernel = mlp_serve_halves<PLANES_NONE>;
+        const auto kernel = mlp_halves<false>;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HV_SMEM);
-        kernel<<<2*n_tiles, SP_THREADS, HV_SMEM, (cudaStream_t)stream>>>(n, n_tiles, xp, xlp, map, prm,
-                                                                         out, err);
+        kernel<<<2*n_tiles, SP_THREADS, HV_SMEM, (cudaStream_t)stream>>>(n, n_tiles, xp, xlp, map, map,
+                                                                         prm, out, nullptr, err);
         return status("mlp_serve");
     }
     if (blocks > n_tiles) blocks = n_tiles;
@@ -2004,120 +2005,79 @@ int32_t sasb200_mlp_serve(int32_t n, int32_t n_pad, const void *x, const void *x
     return status("mlp_serve");
 }
 
-// One CTA per SM, or per tile where there are fewer; map: whether two CTAs per tile
-// may run at once, and the map of the image for them.
-static int tile_blocks(int n_tiles, const void *img, int img_bytes, CUtensorMap &map, bool &halves)
+// The forward and the backward of a gradient pass: out[n] as sasb200_mlp_serve, the
+// tiled z and h planes, dout[n_pad] of the mean Huber loss (threshold delta; squared
+// error for delta <= 0) against y[n], 0 on padding, row_sums[2][n_pad/32]: the loss
+// and dout summed over 32 rows each; and the dZ planes.  With a batch, x, x_lo and y
+// receive its rows of the data set first (err = 5 for a row outside it) and the
+// schedule advances as by sasb200_lr_schedule.
+static int32_t forward_backward(const sasb200_mlp_pass &p, cudaStream_t st)
 {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    halves = n_tiles <= sms/2 && hv_map(map, img, img_bytes/(8*HV_RUN));
-    return halves ? 2*n_tiles : (n_tiles < sms || sms <= 0 ? n_tiles : sms);
-}
-
-// The forward of a training step: out[n] as sasb200_mlp_serve, the tiled z and
-// h planes ([4][n_pad x 256] bf16 each), dout[n_pad] of the mean Huber loss
-// (threshold delta; squared error for delta <= 0) against y[n], 0 on padding,
-// and row_sums[2][n_pad/32]: the loss and dout summed over 32 rows each.  With a
-// batch, x, x_lo and y receive its rows of the data set first (err = 5 for a row
-// outside it) and the schedule advances as by sasb200_lr_schedule.
-static int32_t train_forward(int32_t n, int32_t n_pad, const void *x, const void *x_lo,
-                             const void *img, const float *const *b, const float *w_out,
-                             const float *b_out, const float *y, float delta, float *out,
-                             float *dout, float *row_sums, void *z, void *h,
-                             const sasb200_mlp_batch *batch, int32_t *err, void *stream)
-{
-    errbuf()[0] = 0;
-    if (n < 0 || n_pad % TM || n > n_pad || !x || !x_lo || !img || !b || !w_out || !b_out || !y
-        || !out || !dout || !row_sums || !z || !h || !err)
+    const int n = p.n, n_pad = p.n_pad;
+    if (n < 0 || n_pad < 0 || n_pad % TM || n > n_pad || !p.x || !p.x_lo || !p.img || !p.img_t
+        || !p.w_out || !p.b_out || !p.y || !p.out || !p.dout || !p.row_sums || !p.z || !p.h || !p.dz
+        || !p.err)
         return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
-    if (reinterpret_cast<uintptr_t>(img) % 16)
-        return (std::snprintf(errbuf(), 256, "weight image must be 16-byte aligned"), -1);
+    if ((reinterpret_cast<uintptr_t>(p.img) | reinterpret_cast<uintptr_t>(p.img_t)
+         | reinterpret_cast<uintptr_t>(p.w_out)) % 16)
+        return (std::snprintf(errbuf(), 256, "weights must be 16-byte aligned"), -1);
     InferParams prm = {};
-    prm.img = static_cast<const uint8_t *>(img);
+    prm.img = static_cast<const uint8_t *>(p.img);
     for (int l = 0; l < 4; ++l) {
-        if (!b[l]) return (std::snprintf(errbuf(), 256, "bad bias pointer"), -1);
-        prm.b[l] = b[l];
+        if (!p.b[l]) return (std::snprintf(errbuf(), 256, "bad bias pointer"), -1);
+        prm.b[l] = p.b[l];
     }
-    if (batch) {
+    const auto *xp = static_cast<const __nv_bfloat16 *>(p.x);
+    const auto *xlp = static_cast<const __nv_bfloat16 *>(p.x_lo);
+    if (const sasb200_mlp_batch *batch = p.batch) {
         if (!batch->idx || batch->rows < 0 || !batch->x_all || !batch->x_lo_all || !batch->y_all
             || !batch->counters || !batch->sched || batch->total <= 0 || batch->warmup <= 0
             || n <= 0)
             return (std::snprintf(errbuf(), 256, "bad batch"), -1);
         if ((reinterpret_cast<uintptr_t>(batch->x_all) | reinterpret_cast<uintptr_t>(batch->x_lo_all)
-             | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(x_lo)) % 16)
+             | reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.x_lo)) % 16)
             return (std::snprintf(errbuf(), 256, "features must be 16-byte aligned"), -1);
         prm.batch = {batch->idx, batch->rows, static_cast<const __nv_bfloat16 *>(batch->x_all),
                      static_cast<const __nv_bfloat16 *>(batch->x_lo_all), batch->y_all,
-                     static_cast<__nv_bfloat16 *>(const_cast<void *>(x)),
-                     static_cast<__nv_bfloat16 *>(const_cast<void *>(x_lo)), const_cast<float *>(y),
-                     batch->counters, batch->sched, batch->total, batch->warmup, batch->lr0,
-                     batch->b1, batch->b2};
+                     const_cast<__nv_bfloat16 *>(xp), const_cast<__nv_bfloat16 *>(xlp),
+                     const_cast<float *>(p.y), batch->counters, batch->sched, batch->total,
+                     batch->warmup, batch->lr0, batch->b1, batch->b2};
     }
     if (n_pad == 0) return 0;
-    prm.w_out = w_out;
-    prm.b_out = b_out;
-    prm.z_save = static_cast<__nv_bfloat16 *>(z);
-    prm.h_save = static_cast<__nv_bfloat16 *>(h);
-    prm.y = y;
-    prm.delta = delta;
-    prm.dout = dout;
-    prm.row_sums = row_sums;
+    prm.w_out = p.w_out;
+    prm.b_out = p.b_out;
+    prm.z_save = static_cast<__nv_bfloat16 *>(p.z);
+    prm.h_save = static_cast<__nv_bfloat16 *>(p.h);
+    prm.y = p.y;
+    prm.delta = p.delta;
+    prm.dout = p.dout;
+    prm.row_sums = p.row_sums;
+    auto *dz = static_cast<__nv_bfloat16 *>(p.dz);
     const int n_tiles = n_pad/TM;
-    const auto *xp = static_cast<const __nv_bfloat16 *>(x);
-    const auto *xlp = static_cast<const __nv_bfloat16 *>(x_lo);
-    const auto st = (cudaStream_t)stream;
-    CUtensorMap map;
-    bool halves;
-    const int blocks = tile_blocks(n_tiles, img, IMG_BYTES, map, halves);
-    if (halves) {
-        const auto kernel = mlp_serve_halves<PLANES_TILED>;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // two CTAs per tile where all may run at once (see sasb200_mlp_serve)
+    CUtensorMap map, map_t;
+    if (n_tiles <= sms/2 && hv_map(map, p.img, IMG_BYTES/(8*HV_RUN))
+        && hv_map(map_t, p.img_t, WT_IMG_BYTES/(8*HV_RUN))) {
+        const auto kernel = mlp_halves<true>;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HV_SMEM);
-        launch_dependent(kernel, dim3(blocks), SP_THREADS, HV_SMEM, st, n, n_tiles, xp, xlp, map, prm,
-                         out, err);
-    } else {
-        if (batch)
-            launch_dependent(gather_batch, dim3((unsigned)((4ll*n + 255)/256)), 256, 0, st, n,
-                             prm.batch, err);
-        const auto kernel = mlp_serve<PLANES_TILED>;
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
-        launch_dependent(kernel, dim3(blocks), SV_THREADS, SV_SMEM, st, n, n_tiles, xp, xlp, prm, out,
-                         err);
+        launch_dependent(kernel, dim3(2*n_tiles), SP_THREADS, HV_SMEM, st, n, n_tiles, xp, xlp, map,
+                         map_t, prm, p.out, dz, p.err);
+        return status("mlp_halves");
     }
-    return status("mlp_train_forward");
-}
-
-// The backward of a training step: tiled dZ planes from dout[n_pad] and the
-// tiled z planes.
-static int32_t train_backward(int32_t n_pad, const void *img_t, const float *w_out,
-                              const float *dout, const void *z, void *dz, int32_t *err,
-                              void *stream)
-{
-    errbuf()[0] = 0;
-    if (n_pad < 0 || n_pad % TM || !img_t || !w_out || !dout || !z || !dz || !err)
-        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
-    if (reinterpret_cast<uintptr_t>(img_t) % 16 || reinterpret_cast<uintptr_t>(w_out) % 16)
-        return (std::snprintf(errbuf(), 256, "weights must be 16-byte aligned"), -1);
-    if (n_pad == 0) return 0;
-    const int n_tiles = n_pad/TM;
-    const auto *zp = static_cast<const __nv_bfloat16 *>(z);
-    auto *dzp = static_cast<__nv_bfloat16 *>(dz);
-    const auto st = (cudaStream_t)stream;
-    CUtensorMap map;
-    bool halves;
-    const int blocks = tile_blocks(n_tiles, img_t, WT_IMG_BYTES, map, halves);
-    if (halves) {
-        const auto kernel = mlp_backward_halves;
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HV_BWD_SMEM);
-        launch_dependent(kernel, dim3(blocks), SP_THREADS, HV_BWD_SMEM, st, n_tiles, map, w_out, dout,
-                         zp, dzp, err);
-    } else {
-        const auto kernel = mlp_backward_t;
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM);
-        launch_dependent(kernel, dim3(blocks), SV_THREADS, BT_SMEM, st, n_tiles,
-                         static_cast<const uint8_t *>(img_t), w_out, dout, zp, dzp, err);
-    }
-    return status("mlp_train_backward");
+    if (p.batch)
+        launch_dependent(gather_batch, dim3((unsigned)((4ll*n + 255)/256)), 256, 0, st, n, prm.batch,
+                         p.err);
+    const dim3 blocks(n_tiles < sms || sms <= 0 ? n_tiles : sms);
+    const auto forward = mlp_serve<PLANES_TILED>;
+    cudaFuncSetAttribute(forward, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
+    launch_dependent(forward, blocks, SV_THREADS, SV_SMEM, st, n, n_tiles, xp, xlp, prm, p.out, p.err);
+    cudaFuncSetAttribute(mlp_backward_t, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM);
+    launch_dependent(mlp_backward_t, blocks, SV_THREADS, BT_SMEM, st, n_tiles,
+                     static_cast<const uint8_t *>(p.img_t), p.w_out, p.dout, prm.z_save, dz, p.err);
+    return status("mlp_backward_t");
 }
 
 // Every gradient of a training step from its planes: dw[0..3] [splits][256 x (16
@@ -2226,19 +2186,15 @@ static int32_t sum_partials_of(int32_t n, const int32_t *sizes, const int32_t *s
     return status("sum_partials");
 }
 
-// Loss and gradients of one batch: the forward, the backward and the weight
-// gradients above, then `sums` tensors added over the splits into their places.
+// Loss and gradients of one batch: the forward and the backward, the weight
+// gradients, then `sums` tensors added over the splits into their places.
 // One call, as the four cost a caller as long as the kernels take.
 int32_t sasb200_mlp_train_pass(const sasb200_mlp_pass *p, void *stream)
 {
     errbuf()[0] = 0;
     if (!p || p->sums < 0 || p->sums > SUM_TENSORS)
         return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
-    int32_t rc = train_forward(p->n, p->n_pad, p->x, p->x_lo, p->img, p->b, p->w_out, p->b_out, p->y,
-                               p->delta, p->out, p->dout, p->row_sums, p->z, p->h, p->batch, p->err,
-                               stream);
-    if (rc == 0)
-        rc = train_backward(p->n_pad, p->img_t, p->w_out, p->dout, p->z, p->dz, p->err, stream);
+    int32_t rc = forward_backward(*p, (cudaStream_t)stream);
     if (rc == 0)
         rc = weight_grads(p->n, p->n_pad, p->splits, p->x, p->h, p->dz, p->dout, p->row_sums, p->dw,
                           p->db, p->dw_out, p->loss, p->db_out, p->err, stream);

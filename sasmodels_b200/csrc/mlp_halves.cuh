@@ -1,4 +1,4 @@
-// mlp_serve_halves and mlp_backward_halves: the forward and the backward of few
+// mlp_halves: serving, or the forward and the backward of a training step, of few
 // tiles, each tile on two SMs.  Included by mlp.cu.
 //
 // With one tile per SM (mlp_serve, mlp_backward_t) a small batch takes the chain of
@@ -22,34 +22,35 @@
 //   warp 16     the TMEM allocation; CTA 0, lane 0: issues the MMAs, a chunk as soon
 //               as its barrier says that inputs and weights are there.
 //   warp 17     producer of this CTA's half of the weights, a box copy per chunk.
-//   warp 18     layer 0's weights (forward).  CTA 1: passes on to CTA 0 that its
-//               weights have landed.
-//   warp 19     the features (forward).
+//   warp 18     layer 0's weights.  CTA 1: passes on to CTA 0 that its weights have
+//               landed.
+//   warp 19     the features.
 // A cluster has one tile and every barrier one phase: all waits are for parity 0,
 // bounded.  CTA 1's arrivals in CTA 0 are relaxed, as in mlp_serve_pairs: only the
 // count crosses, what it stands for was handed to CTA 1's own tensor core before.
 // Both CTAs meet before either exits.
 //
-// In a captured training step the forward also gathers its batch and advances the
-// schedule: a step with a launch of its own for that (gather_batch) took 51.5 us, now
-// 50.6.
+// Training goes on in the same launch: the rows of a CTA have their loss gradient
+// when their output is known, so dZ3 forms from the z that the warps still hold, and
+// the transposed weights follow the others through the ring.  In a captured step the
+// features are gathered here and the schedule advances.  A step of 8192 rows with
+// launches of their own for the backward 50.5 us and for the gathering 51.5, now 47.1.
 //
 // Every value is that of the kernels of one tile per SM, bit for bit.  Bound by the
 // chain of a tile still: an MMA of a pair takes 103 cycles here (32 of them a layer),
 // an epilogue 700 cycles until its first hand-over, 170 from there to the MMAs.
-// Serving 8 tiles 17.5 -> 12.3 us, 64 tiles 17.9 -> 13.3; the captured training step
-// of 8192 rows 65.5 -> 52.7 us with both kernels.
+// Serving 8 tiles 17.5 -> 12.3 us, 64 tiles 17.9 -> 13.2.
 #pragma once
 
 constexpr int HV_RELAY_WARP = SV_EPI_WARPS + 2;
 constexpr int HV_ROWS = TM/2;                      // rows of a CTA
-constexpr int HV_CHUNKS = 3*SP_CHUNKS;             // of 64 inputs, layers 1-3
+constexpr int HV_CHUNKS = 3*SP_CHUNKS;             // of 64 inputs: layers 1-3, then W3, W2,
+                                                   // W1 transposed
 constexpr int HV_ACT = ACT_BYTES/2;
 constexpr int HV_X = X_BYTES/2;
 constexpr int HV_ACC = HID/2;                      // TMEM columns of an accumulator
-constexpr int HV_STAGES = 8;                       // forward: two layers of weights
+constexpr int HV_STAGES = 8;                       // of the ring: two layers of weights
 constexpr int HV_SMEM = 2*HV_ACT + HV_STAGES*SP_HALF + W0_BYTES/2 + 2*HV_X + 4*SV_PARAMS;
-constexpr int HV_BWD_SMEM = HV_ACT + HV_CHUNKS*SP_HALF;        // all of them
 // Arrivals of a chunk in CTA 0: its inputs, by the warps of both CTAs, and its
 // weights, by both producers (with the bytes) -- one barrier, because each that the
 // MMA thread looks at costs it 100 cycles.  In CTA 1 its own weights.
@@ -97,9 +98,9 @@ __device__ __forceinline__ bool hv_spin(uint64_t *bar)
 }
 
 // CTA 1: passes on to CTA 0 that its weights have landed (whole warp).
-__device__ __forceinline__ bool hv_relay(int lane, uint64_t *ready)
+__device__ __forceinline__ bool hv_relay(int lane, int chunks, uint64_t *ready)
 {
-    for (int c = 0; c < HV_CHUNKS; ++c) {
+    for (int c = 0; c < chunks; ++c) {
         if (!warp_wait(&ready[c], 0u)) return false;
         if (lane == 0) tc::mbar_arrive_relaxed_cta(&ready[c], 0);
     }
@@ -127,15 +128,15 @@ __device__ __forceinline__ long long batch_row(const Batch &batch, int n, int r,
     return -1;
 }
 
-// PLANES: none, or a training step's tiled planes with the loss gradient.
-template <int PLANES>
+// TRAIN: with the tiled planes, the loss gradient and the backward.
+template <bool TRAIN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SP_THREADS, 1)
-mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
-                 const __nv_bfloat16 *__restrict__ x_lo,
-                 const __grid_constant__ CUtensorMap img, InferParams prm,
-                 float *__restrict__ out, int *__restrict__ err)
+mlp_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
+           const __nv_bfloat16 *__restrict__ x_lo, const __grid_constant__ CUtensorMap img,
+           const __grid_constant__ CUtensorMap img_t, InferParams prm, float *__restrict__ out,
+           __nv_bfloat16 *__restrict__ dz_save, int *__restrict__ err)
 {
-    static_assert(PLANES == PLANES_NONE || PLANES == PLANES_TILED, "no row-major planes here");
+    constexpr int CHUNKS = TRAIN ? 2*HV_CHUNKS : HV_CHUNKS, LAYERS = TRAIN ? 7 : 4;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *act = smem;
     uint8_t *act_lo = smem + HV_ACT;
@@ -143,22 +144,23 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
     uint8_t *w0 = ring + HV_STAGES*SP_HALF;
     uint8_t *xs = w0 + W0_BYTES/2;                // [hi, lo] x HV_X
     float *par = reinterpret_cast<float *>(xs + 2*HV_X);
-    __shared__ __align__(8) uint64_t ready[HV_CHUNKS], acc_full[4];
+    __shared__ __align__(8) uint64_t ready[CHUNKS], acc_full[LAYERS];
     __shared__ __align__(8) uint64_t stage_free[SP_CHUNKS];
-    __shared__ __align__(8) uint64_t other_half[2][4], dot_bar[2], x_ready, drain;
+    __shared__ __align__(8) uint64_t other_half[2][4], dot_bar[2], dout_bar[2], x_ready, drain;
     __shared__ uint32_t tmem_slot;
-    __shared__ float dot_part[3][HV_ROWS];
+    __shared__ float dot_part[3][HV_ROWS], dout_s[HV_ROWS];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int rank = (int)tc::cluster_rank(), tile = blockIdx.x >> 1;
     const int row0 = tile*TM + rank*HV_ROWS;
 
     if (t == 0) {
-        for (int c = 0; c < HV_CHUNKS; ++c) tc::mbar_init(&ready[c], rank == 0 ? HV_ARRIVALS : 1);
-        for (int l = 0; l < 4; ++l) tc::mbar_init(&acc_full[l], 1);
+        for (int c = 0; c < CHUNKS; ++c) tc::mbar_init(&ready[c], rank == 0 ? HV_ARRIVALS : 1);
+        for (int l = 0; l < LAYERS; ++l) tc::mbar_init(&acc_full[l], 1);
         for (int c = 0; c < SP_CHUNKS; ++c) tc::mbar_init(&stage_free[c], 1);
         for (int q = 0; q < 2; ++q) {
             for (int s = 0; s < 4; ++s) tc::mbar_init(&other_half[q][s], 1);
             tc::mbar_init(&dot_bar[q], SV_EPI_WARPS/4 - 1);
+            tc::mbar_init(&dout_bar[q], 1);
         }
         tc::mbar_init(&x_ready, 4);
         tc::mbar_init(&drain, 1);
@@ -190,11 +192,17 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         tc::cluster_wait();
         if (lane == 0) {
             int issued = HV_STAGES;
-            // layer 3's take the places of layer 1's
-            for (; issued < HV_CHUNKS; ++issued) {
+            // layer 3's take the places of layer 1's chunk by chunk, the later ones
+            // those of the layer two before
+            for (; issued < CHUNKS; ++issued) {
                 const int c = issued - HV_STAGES;
-                if (!(ok = tc::mbar_wait(&stage_free[c], 0u))) break;
-                hv_load_chunk(ring + c*SP_HALF, img, first + issued*(SP_K/8), rank, &ready[issued]);
+                if (!(ok = tc::mbar_wait(c < SP_CHUNKS ? &stage_free[c] : &acc_full[1 + c/SP_CHUNKS],
+                                         0u)))
+                    break;
+                const bool back = issued >= HV_CHUNKS;
+                hv_load_chunk(ring + (issued % HV_STAGES)*SP_HALF, back ? img_t : img,
+                              back ? (issued - HV_CHUNKS)*(SP_K/8) : first + issued*(SP_K/8), rank,
+                              &ready[issued]);
             }
             // every issued copy has landed before the CTA may exit
             for (int c = 0; c < issued; ++c) ok = tc::mbar_wait(&ready[c], 0u) && ok;
@@ -214,11 +222,11 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         __syncwarp();
         tc::cluster_wait();
         if (lane == 0) arrive0(&x_ready);
-        if (PLANES == PLANES_TILED && prm.batch.idx && blockIdx.x == 0 && lane == 0)
+        if (TRAIN && prm.batch.idx && blockIdx.x == 0 && lane == 0)
             schedule_step(prm.batch.counters, prm.batch.sched, prm.batch.total, prm.batch.warmup,
                           prm.batch.lr0, prm.batch.b1, prm.batch.b2);
         __syncwarp();
-        if (rank != 0 && !hv_relay(lane, ready) && lane == 0) atomicExch(err, 4);
+        if (rank != 0 && !hv_relay(lane, CHUNKS, ready) && lane == 0) atomicExch(err, 4);
         __syncwarp();
     } else if (warp == SP_X_WARP) {
         uint4 v[4], w[4];
@@ -226,7 +234,7 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         for (int j = 0; j < 4; ++j) {
             const int u = lane + 32*j;
             const size_t g = (size_t)(row0 + (u >> 1))*NIN + (u & 1)*8;
-            if (PLANES == PLANES_TILED && prm.batch.idx) {
+            if (TRAIN && prm.batch.idx) {
                 const long long src = batch_row(prm.batch, n, row0 + (u >> 1), err);
                 v[j] = w[j] = make_uint4(0, 0, 0, 0);
                 if (src >= 0) {
@@ -251,7 +259,7 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         if (lane == 0) arrive0(&x_ready);
         __syncwarp();
         // the batch's features, for the weight gradients
-        if (PLANES == PLANES_TILED && prm.batch.idx) {
+        if (TRAIN && prm.batch.idx) {
             #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const size_t g = (size_t)row0*NIN + (lane + 32*j)*8;
@@ -292,6 +300,20 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 if (c == SP_CHUNKS - 1) tc::mma_commit_pair(&acc_full[l]);
                 if (l == 1) tc::mma_commit_pair(&stage_free[c]);
             }
+            // the backward: dZ3 W3, dZ2 W2, dZ1 W1 into acc[0], acc[1], acc[0]
+            for (int i = HV_CHUNKS; i < CHUNKS && ok; ++i) {
+                const int s = i/SP_CHUNKS - 3, c = i % SP_CHUNKS;
+                if (!(ok = hv_spin(&ready[i]))) break;
+                tc::fence_after_sync();
+                const uint32_t d = tmem + (uint32_t)(HV_ACC*(s & 1));
+                const uint32_t b_addr = tc::smem_u32(ring + (i % HV_STAGES)*SP_HALF);
+                #pragma unroll
+                for (int st = 0; st < SP_K/16; ++st)
+                    tc::mma_bf16_pair(d, tc::kmajor_desc<HV_ROWS>(a_hi, c*(SP_K/16) + st),
+                                      tc::kmajor_desc<HID/2>(b_addr, st), idesc,
+                                      (c > 0 || st > 0) ? 1u : 0u);
+                if (c == SP_CHUNKS - 1) tc::mma_commit_pair(&acc_full[4 + s]);
+            }
             // every MMA issued has completed before TMEM is released
             tc::mma_commit_pair(&drain);
             ok = tc::mbar_wait(&drain, 0u) && ok;
@@ -315,7 +337,7 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         const uint32_t lane_base = tmem_slot + ((uint32_t)(32*quad) << 16) + (uint32_t)(8*slot);
         // the target of this row, for the warps that form the output
         float target = 0.0f;
-        if (PLANES == PLANES_TILED && half == 0 && slot == 0) {
+        if (TRAIN && half == 0 && slot == 0) {
             if (prm.batch.idx) {
                 const long long src = batch_row(prm.batch, n, row0 + row, err);
                 if (src >= 0) target = prm.batch.y_all[src];
@@ -335,6 +357,7 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             }
         };
         bool ok = true;
+        uint4 zq[SP_CHUNKS];                           // layer 3's z, later the next needed
         #pragma unroll 1
         for (int l = 0; l < 3; ++l) {
             if (!(ok = warp_wait(&acc_full[l], 0u))) break;
@@ -351,7 +374,7 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             #pragma unroll
             for (int c = 0; c < SP_CHUNKS; ++c) {
                 uint4 lo;
-                silu_columns<PLANES == PLANES_TILED>(r[c], 0, bias + 64*c, hi[c], lo, &z[c]);
+                silu_columns<TRAIN>(r[c], 0, bias + 64*c, hi[c], lo, &z[c]);
                 const uint32_t off = tc::kmajor_offset<HV_ROWS>(row, col0 + 64*c);
                 *reinterpret_cast<uint4 *>(act + off) = hi[c];
                 *reinterpret_cast<uint4 *>(act_lo + off) = lo;
@@ -359,16 +382,17 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 __syncwarp();
                 if (lane == 0) arrive0(&ready[SP_CHUNKS*l + c]);
             }
-            if (PLANES == PLANES_TILED) save_planes(l, z, hi);
+            if (TRAIN) save_planes(l, z, hi);
         }
         if (ok && (ok = warp_wait(&acc_full[3], 0u))) {
             // the output dot: the 8 columns at 8 (w/4) of every 32, summed in order as
             // in mlp_serve by the warps that hold the first of each pair of 32; the
-            // others leave their activations in the place of the inputs, all read
+            // others leave their activations in the place of the inputs' lo halves, all
+            // read (the hi halves' place is for dZ)
             tc::fence_after_sync();
             const float *bias = par + 3*HID + col0, *wo = par + 4*HID + 8*slot;
             uint32_t r[SP_CHUNKS][8];
-            uint4 hq[SP_CHUNKS], zq[SP_CHUNKS];
+            uint4 hq[SP_CHUNKS];
             float h[SP_CHUNKS][8];
             #pragma unroll
             for (int c = 0; c < SP_CHUNKS; ++c) tc::tmem_ld8(lane_base + (uint32_t)(HV_ACC + 32*c), r[c]);
@@ -376,7 +400,7 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             for (int c = 0; c < SP_CHUNKS; ++c) tc::tmem_wait_ld8(r[c]);
             tc::fence_before_sync();
             // [slot][chunk][4 columns][row] of 16 bytes
-            float4 *over = reinterpret_cast<float4 *>(act) + slot*(2*SP_CHUNKS*HV_ROWS) + row;
+            float4 *over = reinterpret_cast<float4 *>(act_lo) + slot*(2*SP_CHUNKS*HV_ROWS) + row;
             #pragma unroll
             for (int c = 0; c < SP_CHUNKS; ++c) {
                 const ulonglong2 *b2 = reinterpret_cast<const ulonglong2 *>(bias + 64*c);
@@ -386,7 +410,7 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                     const uint64_t z = bias2(r[c][2*e], r[c][2*e + 1], e & 1 ? b.y : b.x);
                     const uint64_t v = silu2(z);
                     f2_unpack(v, h[c][2*e], h[c][2*e + 1]);
-                    if (PLANES == PLANES_TILED) {
+                    if (TRAIN) {
                         (&zq[c].x)[e] = pack2(z);
                         (&hq[c].x)[e] = pack2(v);
                     }
@@ -400,7 +424,7 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(&other_half[q2][slot]);
             }
-            if (PLANES == PLANES_TILED) save_planes(3, zq, hq);
+            if (TRAIN) save_planes(3, zq, hq);
             float dot = 0.0f;
             if (half == 0 && (ok = warp_wait(&other_half[q2][slot], 0u))) {
                 #pragma unroll
@@ -424,11 +448,14 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 const float o = ((dot + dot_part[0][row]) + dot_part[1][row])
                                 + dot_part[2][row] + b_out;
                 if (valid) out[row0 + row] = o;
-                if (PLANES == PLANES_TILED) {
+                if (TRAIN) {
                     float g, loss;
                     loss_of(valid ? o - target : 0.0f, prm.delta, g, loss);
                     g = valid ? g/(float)n : 0.0f;
                     prm.dout[row0 + row] = g;
+                    dout_s[row] = g;
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&dout_bar[q2]);
                     #pragma unroll
                     for (int o2 = 16; o2 > 0; o2 >>= 1) {
                         g += __shfl_xor_sync(0xffffffffu, g, o2);
@@ -442,169 +469,63 @@ mlp_serve_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 }
             }
         }
-        if (!ok && lane == 0) atomicExch(err, 1);
-        __syncwarp();
-    }
-    hv_leave_together();
-    if (warp == SV_MMA_WARP) tc::tmem_dealloc2(tmem_slot, 2*HID);
-}
-
-// The values of mlp_backward_t.  All weights fit beside the gradients of 64 rows, so
-// the producer fetches them at once.
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SP_THREADS, 1)
-mlp_backward_halves(int n_tiles, const __grid_constant__ CUtensorMap img_t,
-                    const float *__restrict__ w_out,
-                    const float *__restrict__ dout, const __nv_bfloat16 *__restrict__ z_save,
-                    __nv_bfloat16 *__restrict__ dz_save, int *__restrict__ err)
-{
-    extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t *act = smem;
-    uint8_t *weights = smem + HV_ACT;
-    __shared__ __align__(8) uint64_t ready[HV_CHUNKS], acc_full[3], drain;
-    __shared__ uint32_t tmem_slot;
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const int rank = (int)tc::cluster_rank(), tile = blockIdx.x >> 1;
-
-    if (t == 0) {
-        for (int c = 0; c < HV_CHUNKS; ++c) tc::mbar_init(&ready[c], rank == 0 ? HV_ARRIVALS : 1);
-        for (int s = 0; s < 3; ++s) tc::mbar_init(&acc_full[s], 1);
-        tc::mbar_init(&drain, 1);
-        tc::mbar_fence_init();
-    }
-    tc::dependents_launch();
-    __syncthreads();
-    if (warp == SV_MMA_WARP) {
-        tc::tmem_alloc2(&tmem_slot, 2*HID);
-        tc::fence_before_sync();
-        tc::bar_arrive(1, SV_EPI + 32);
-    }
-    tc::cluster_arrive_relaxed();
-    tc::dependency_wait();
-
-    if (warp == SV_PROD_WARP) {
-        if (lane == 0)
-            for (int c = 0; c < HV_CHUNKS; ++c)
-                hv_load_chunk(weights + c*SP_HALF, img_t, c*(SP_K/8), rank, &ready[c]);
-        __syncwarp();
-        tc::cluster_wait();
-        if (lane == 0) {
-            bool ok = true;
-            for (int c = 0; c < HV_CHUNKS; ++c) ok = tc::mbar_wait(&ready[c], 0u) && ok;
-            if (!ok) atomicExch(err, 2);
-        }
-        __syncwarp();
-    } else if (warp == HV_RELAY_WARP) {
-        tc::cluster_wait();
-        if (rank != 0 && !hv_relay(lane, ready) && lane == 0) atomicExch(err, 4);
-        __syncwarp();
-    } else if (warp == SV_MMA_WARP) {
-        tc::cluster_wait();
-        tc::fence_after_sync();
-        const uint32_t tmem = tmem_slot;
-        if (lane == 0 && rank == 0) {
-            constexpr uint32_t idesc = tc::idesc_bf16(TM, HID);
-            const uint32_t a_addr = tc::smem_u32(act);
-            bool ok = true;
-            for (int i = 0; i < HV_CHUNKS && ok; ++i) {
-                const int s = i/SP_CHUNKS, c = i % SP_CHUNKS;
-                if (!(ok = hv_spin(&ready[i]))) break;
-                tc::fence_after_sync();
-                const uint32_t d = tmem + (uint32_t)(HV_ACC*(s & 1));
-                const uint32_t b_addr = tc::smem_u32(weights + i*SP_HALF);
-                #pragma unroll
-                for (int st = 0; st < SP_K/16; ++st)
-                    tc::mma_bf16_pair(d, tc::kmajor_desc<HV_ROWS>(a_addr, c*(SP_K/16) + st),
-                                      tc::kmajor_desc<HID/2>(b_addr, st), idesc,
-                                      (c > 0 || st > 0) ? 1u : 0u);
-                if (c == SP_CHUNKS - 1) tc::mma_commit_pair(&acc_full[s]);
-            }
-            tc::mma_commit_pair(&drain);
-            ok = tc::mbar_wait(&drain, 0u) && ok;
-            if (!ok) atomicExch(err, 3);
-        } else if (lane == 0) {
-            if (!tc::mbar_wait(&drain, 0u)) atomicExch(err, 3);
-        }
-        __syncwarp();
-    } else if (warp < SV_EPI_WARPS) {
-        const int quad = warp & 3, slot = warp >> 2;
-        const int half = quad >> 1, row = 32*(quad & 1) + lane, trow = rank*HV_ROWS + row;
-        const int col0 = 32*half + 8*slot;
-        const float d = dout[tile*TM + trow];
-        // this thread's 8 columns of each 64
-        const size_t at0 = tiled_at(0, n_tiles, tile, col0/8, trow);
-        const uint4 *z0 = reinterpret_cast<const uint4 *>(z_save + at0);
-        uint4 *dz0 = reinterpret_cast<uint4 *>(dz_save + at0);
-        const size_t plane16 = (size_t)n_tiles*TILE_ELEMS/8;   // a plane in 16-byte units
-        constexpr int GROUP16 = GROUP_ELEMS/8;
-        uint4 z[SP_CHUNKS];
-        #pragma unroll
-        for (int c = 0; c < SP_CHUNKS; ++c) z[c] = z0[3*plane16 + 8*c*GROUP16];
-        tc::bar_sync(1, SV_EPI + 32);                  // tmem_slot
-        tc::fence_after_sync();
-        tc::cluster_wait();
-        const uint32_t lane_base = tmem_slot + ((uint32_t)(32*quad) << 16) + (uint32_t)(8*slot);
-        bool ok = true;
-        // s = -1: dZ3 from dout; s = 0, 1, 2: the epilogues of W3, W2, W1
-        #pragma unroll 1
-        for (int s = -1; s < 3; ++s) {
-            const int l = 2 - s;
-            uint32_t r[SP_CHUNKS][8];
-            if (s >= 0) {
-                if (!(ok = warp_wait(&acc_full[s], 0u))) break;
-                tc::fence_after_sync();
-                #pragma unroll
-                for (int c = 0; c < SP_CHUNKS; ++c)
-                    tc::tmem_ld8(lane_base + (uint32_t)(HV_ACC*(s & 1) + 32*c), r[c]);
-                #pragma unroll
-                for (int c = 0; c < SP_CHUNKS; ++c) tc::tmem_wait_ld8(r[c]);
-                tc::fence_before_sync();
-            } else {
+        // ---- backward: dZ3 from dout, then the epilogues of W3, W2, W1 ----
+        if (TRAIN && ok && (ok = warp_wait(&dout_bar[q2], 0u))) {
+            const size_t plane16 = (size_t)n_tiles*TILE_ELEMS/8;       // in 16-byte units
+            constexpr int GROUP16 = GROUP_ELEMS/8;
+            const size_t at0 = tiled_at(0, n_tiles, tile, col0/8, trow);
+            const uint4 *z0 = reinterpret_cast<const uint4 *>(prm.z_save + at0);
+            uint4 *dz0 = reinterpret_cast<uint4 *>(dz_save + at0);
+            const float d = dout_s[row];
+            #pragma unroll 1
+            for (int s = -1; s < 3; ++s) {
+                const int l = 2 - s;
+                uint32_t r[SP_CHUNKS][8];
+                if (s >= 0) {
+                    if (!(ok = warp_wait(&acc_full[4 + s], 0u))) break;
+                    tc::fence_after_sync();
+                    #pragma unroll
+                    for (int c = 0; c < SP_CHUNKS; ++c)
+                        tc::tmem_ld8(lane_base + (uint32_t)(HV_ACC*(s & 1) + 32*c), r[c]);
+                    #pragma unroll
+                    for (int c = 0; c < SP_CHUNKS; ++c) tc::tmem_wait_ld8(r[c]);
+                    tc::fence_before_sync();
+                } else {
+                    #pragma unroll
+                    for (int c = 0; c < SP_CHUNKS; ++c)
+                        #pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            r[c][e] = __float_as_uint(d*par[4*HID + col0 + 64*c + e]);
+                }
+                uint4 o[SP_CHUNKS];
                 #pragma unroll
                 for (int c = 0; c < SP_CHUNKS; ++c) {
-                    const float4 *wp = reinterpret_cast<const float4 *>(w_out + col0 + 64*c);
+                    const uint32_t zu[4] = {zq[c].x, zq[c].y, zq[c].z, zq[c].w};
+                    uint32_t *op = &o[c].x;
                     #pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const float4 w = __ldg(wp + e);
-                        r[c][4*e] = __float_as_uint(d*w.x);
-                        r[c][4*e + 1] = __float_as_uint(d*w.y);
-                        r[c][4*e + 2] = __float_as_uint(d*w.z);
-                        r[c][4*e + 3] = __float_as_uint(d*w.w);
+                    for (int e = 0; e < 4; ++e)
+                        op[e] = pack2(__uint_as_float(r[c][2*e])*dsilu(bf_lo(zu[e])),
+                                      __uint_as_float(r[c][2*e + 1])*dsilu(bf_hi(zu[e])));
+                    if (s < 2) {
+                        *reinterpret_cast<uint4 *>(
+                            act + tc::kmajor_offset<HV_ROWS>(row, col0 + 64*c)) = o[c];
+                        tc::fence_async_smem();
+                        __syncwarp();
+                        if (lane == 0) arrive0(&ready[HV_CHUNKS + SP_CHUNKS*(s + 1) + c]);
                     }
                 }
-            }
-            uint4 o[SP_CHUNKS];
-            #pragma unroll
-            for (int c = 0; c < SP_CHUNKS; ++c) {
-                const uint32_t zu[4] = {z[c].x, z[c].y, z[c].z, z[c].w};
-                uint32_t *op = &o[c].x;
-                #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    op[e] = pack2(__uint_as_float(r[c][2*e])*dsilu(bf_lo(zu[e])),
-                                  __uint_as_float(r[c][2*e + 1])*dsilu(bf_hi(zu[e])));
+                // the next layer's z (this thread stored it), in use one epilogue from now
                 if (s < 2) {
-                    *reinterpret_cast<uint4 *>(
-                        act + tc::kmajor_offset<HV_ROWS>(row, col0 + 64*c)) = o[c];
-                    tc::fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0) {
-                        uint64_t *bar = &ready[SP_CHUNKS*(s + 1) + c];
-                        if (rank == 0) tc::mbar_arrive(bar);
-                        else tc::mbar_arrive_relaxed_cta(bar, 0);
-                    }
+                    #pragma unroll
+                    for (int c = 0; c < SP_CHUNKS; ++c)
+                        zq[c] = z0[(size_t)(l - 1)*plane16 + 8*c*GROUP16];
                 }
-            }
-            // the next layer's z, in use one epilogue from now
-            if (s < 2) {
                 #pragma unroll
-                for (int c = 0; c < SP_CHUNKS; ++c) z[c] = z0[(size_t)(l - 1)*plane16 + 8*c*GROUP16];
+                for (int c = 0; c < SP_CHUNKS; ++c) dz0[(size_t)l*plane16 + 8*c*GROUP16] = o[c];
             }
-            #pragma unroll
-            for (int c = 0; c < SP_CHUNKS; ++c) dz0[(size_t)l*plane16 + 8*c*GROUP16] = o[c];
         }
         if (!ok && lane == 0) atomicExch(err, 1);
         __syncwarp();
-    } else {
-        tc::cluster_wait();
     }
     hv_leave_together();
     if (warp == SV_MMA_WARP) tc::tmem_dealloc2(tmem_slot, 2*HID);
