@@ -28,11 +28,11 @@ __device__ __forceinline__ float warp_sum8(float (&v)[8], int lane)
 // mlp_backward.  Built as mlp_serve: sixteen epilogue warps (quadrant w % 4, 16
 // columns of every 64 at 16(w / 4)), one MMA warp, a bulk-copy producer and the two
 // counting warps, two TMEM accumulators, so that the MMAs of the next layer start on the
-// first columns while the epilogue works on the last.  A
-// training batch of 8192 rows is one tile for 64 CTAs, so the kernel is bound by
-// the latency of one tile's chain: the ring holds a whole layer of weights
-// (fetched while dZ3 forms), and each warp loads the z of its eight chunks one
-// layer ahead.  8192 rows: 18.5 us (mlp_backward_p 38 us).
+// first columns while the epilogue works on the last.  For batches of more tiles
+// than half the SMs (fewer: mlp_halves).  Bound by the latency of one tile's
+// chain: the ring holds a whole layer of weights (fetched while dZ3 forms), and each
+// warp loads the z of its eight chunks one layer ahead.  64 tiles on as many SMs:
+// 16.5 us (mlp_backward_p 38 us).
 constexpr int BT_STAGES = 8;
 constexpr int BT_SMEM = ACT_BYTES + BT_STAGES*CHUNK_BYTES;
 
