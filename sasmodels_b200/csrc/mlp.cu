@@ -1169,7 +1169,7 @@ __device__ __forceinline__ float dot8(const uint32_t (&r)[8], const float *bias,
 // hidden activations are bitwise those of mlp_infer; the output dot sums
 // the 256 columns in another order (four partial sums per row).
 //
-// Roles, 19 warps per CTA (one CTA per SM, persistent over 128-row tiles):
+// Roles, 20 warps per CTA (one CTA per SM, persistent over 128-row tiles):
 //   warps 0-15  epilogue.  Warp w reads the TMEM lanes of its quadrant
 //               (rows 32(w%4) .. +31) and the 16 columns at 16(w/4) of every 64,
 //               all of them before the first is used (which frees the
