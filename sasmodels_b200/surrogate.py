@@ -848,6 +848,10 @@ class Surrogate:
         net, dev = self.net, self.net.device
         sid = np.asarray(cols["set"])
         n = len(sid)
+        q = np.ascontiguousarray(cols["q"], 'd')
+        # the kernels take addresses: q has a value for each of the n points
+        if sid.ndim != 1 or q.shape != sid.shape:
+            raise ValueError("q has shape %s, set %s" % (q.shape, sid.shape))
         if n == 0:
             return np.zeros(0), np.zeros(0, bool)
         starts = np.concatenate([[0], np.flatnonzero(sid[1:] != sid[:-1]) + 1])
@@ -869,7 +873,7 @@ class Surrogate:
         n_pad = pad128(n)
         with torch.cuda.stream(net.stream):
             rows = torch.as_tensor(rows, device=dev)
-            q = torch.as_tensor(np.ascontiguousarray(cols["q"], 'd'), device=dev)
+            q = torch.as_tensor(q, device=dev)
             feats = torch.empty((2, n_pad, NIN), dtype=torch.bfloat16, device=dev)
             result = torch.empty(n + (n + 7)//8, dtype=torch.float64, device=dev)
             st = net.stream.cuda_stream

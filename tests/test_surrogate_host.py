@@ -1,0 +1,33 @@
+"""
+What the surrogate's entry points refuse before anything reaches the GPU.
+"""
+
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+
+from sasmodels_b200.surrogate import Surrogate, sample_sets
+
+
+def _surrogate():
+    """A surrogate whose network is never reached."""
+    S = Surrogate.__new__(Surrogate)
+    S.torch, S.net, S.gate = None, SimpleNamespace(device=None), None
+    return S
+
+
+@pytest.mark.parametrize("q_shape", [(9,), (11,), (0,), (10, 1), (1, 10), ()])
+def test_iq_refuses_q_of_another_length(q_shape):
+    """Shorter, longer and two-dimensional q against ten points."""
+    cols = sample_sets(10, np.random.default_rng(0))
+    cols.update(set=np.arange(10), q=np.full(q_shape, 0.1))
+    with pytest.raises(ValueError, match="q has shape"):
+        _surrogate().iq(cols)
+
+
+def test_iq_refuses_q_without_points():
+    cols = {k: v[:0] for k, v in sample_sets(1, np.random.default_rng(0)).items()}
+    cols.update(set=np.zeros(0, int), q=np.full(3, 0.1))
+    with pytest.raises(ValueError, match="q has shape"):
+        _surrogate().iq(cols)
