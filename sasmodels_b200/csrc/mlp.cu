@@ -1224,6 +1224,11 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity)
 {
     return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity)) != 0;
 }
+// The same for a barrier that both CTAs of a pair arrive on, or their MMAs complete.
+__device__ __forceinline__ bool warp_wait_cluster(uint64_t *bar, uint32_t parity)
+{
+    return __all_sync(0xffffffffu, tc::mbar_wait_cluster(bar, parity)) != 0;
+}
 
 // z = acc + bias and h = silu(z) for 8 columns, accumulators r[at ..].
 template <int N>

@@ -26,9 +26,8 @@
 //               landed.
 //   warp 19     the features.
 // A cluster has one tile and every barrier one phase: all waits are for parity 0,
-// bounded.  CTA 1's arrivals in CTA 0 are relaxed, as in mlp_serve_pairs: only the
-// count crosses, what it stands for was handed to CTA 1's own tensor core before.
-// Both CTAs meet before either exits.
+// bounded.  CTA 1's arrivals in CTA 0 release what they stand for, as in
+// mlp_serve_pairs.  Both CTAs meet before either exits.
 //
 // Training goes on in the same launch: the rows of a CTA have their loss gradient
 // when their output is known, so dZ3 forms from the z that the warps still hold, and
@@ -93,7 +92,10 @@ __device__ __forceinline__ void hv_load_chunk(uint8_t *to, const CUtensorMap &ma
 __device__ __forceinline__ bool hv_spin(uint64_t *bar)
 {
     for (uint32_t i = 0; i < tc::WAIT_LIMIT; ++i)
-        if (tc::mbar_test(bar, 0u)) return true;
+        if (tc::mbar_test_relaxed(bar, 0u)) {
+            tc::cluster_acquire();
+            return true;
+        }
     return false;
 }
 
@@ -102,7 +104,7 @@ __device__ __forceinline__ bool hv_relay(int lane, int chunks, uint64_t *ready)
 {
     for (int c = 0; c < chunks; ++c) {
         if (!warp_wait(&ready[c], 0u)) return false;
-        if (lane == 0) tc::mbar_arrive_relaxed_cta(&ready[c], 0);
+        if (lane == 0) tc::mbar_arrive_cta(&ready[c], 0);
     }
     return true;
 }
@@ -178,7 +180,7 @@ mlp_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
     tc::dependency_wait();
     auto arrive0 = [&](uint64_t *bar) {
         if (rank == 0) tc::mbar_arrive(bar);
-        else tc::mbar_arrive_relaxed_cta(bar, 0);
+        else tc::mbar_arrive_cta(bar, 0);
     };
 
     if (warp == SV_PROD_WARP) {
@@ -196,8 +198,8 @@ mlp_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             // those of the layer two before
             for (; issued < CHUNKS; ++issued) {
                 const int c = issued - HV_STAGES;
-                if (!(ok = tc::mbar_wait(c < SP_CHUNKS ? &stage_free[c] : &acc_full[1 + c/SP_CHUNKS],
-                                         0u)))
+                if (!(ok = tc::mbar_wait_cluster(
+                          c < SP_CHUNKS ? &stage_free[c] : &acc_full[1 + c/SP_CHUNKS], 0u)))
                     break;
                 const bool back = issued >= HV_CHUNKS;
                 hv_load_chunk(ring + (issued % HV_STAGES)*SP_HALF, back ? img_t : img,
@@ -316,10 +318,10 @@ mlp_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             }
             // every MMA issued has completed before TMEM is released
             tc::mma_commit_pair(&drain);
-            ok = tc::mbar_wait(&drain, 0u) && ok;
+            ok = tc::mbar_wait_cluster(&drain, 0u) && ok;
             if (!ok) atomicExch(err, 3);
         } else if (lane == 0) {
-            if (!tc::mbar_wait(&drain, 0u)) atomicExch(err, 3);
+            if (!tc::mbar_wait_cluster(&drain, 0u)) atomicExch(err, 3);
         }
         __syncwarp();
     } else {
@@ -360,7 +362,7 @@ mlp_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         uint4 zq[SP_CHUNKS];                           // layer 3's z, later the next needed
         #pragma unroll 1
         for (int l = 0; l < 3; ++l) {
-            if (!(ok = warp_wait(&acc_full[l], 0u))) break;
+            if (!(ok = warp_wait_cluster(&acc_full[l], 0u))) break;
             tc::fence_after_sync();
             const float *bias = par + l*HID + col0;
             uint32_t r[SP_CHUNKS][8];
@@ -384,7 +386,7 @@ mlp_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             }
             if (TRAIN) save_planes(l, z, hi);
         }
-        if (ok && (ok = warp_wait(&acc_full[3], 0u))) {
+        if (ok && (ok = warp_wait_cluster(&acc_full[3], 0u))) {
             // the output dot: the 8 columns at 8 (w/4) of every 32, summed in order as
             // in mlp_serve by the warps that hold the first of each pair of 32; the
             // others leave their activations in the place of the inputs' lo halves, all
@@ -482,7 +484,7 @@ mlp_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 const int l = 2 - s;
                 uint32_t r[SP_CHUNKS][8];
                 if (s >= 0) {
-                    if (!(ok = warp_wait(&acc_full[4 + s], 0u))) break;
+                    if (!(ok = warp_wait_cluster(&acc_full[4 + s], 0u))) break;
                     tc::fence_after_sync();
                     #pragma unroll
                     for (int c = 0; c < SP_CHUNKS; ++c)

@@ -50,11 +50,12 @@
 // step s - 1 done, whose inputs come from epilogues before it.  Both CTAs meet
 // before either exits.
 //
-// CTA 1's arrivals in CTA 0 are relaxed: only the count crosses.  Its activations,
-// weights and features stay in its own shared memory, are read by its own tensor
-// core, and were handed to that (fence.proxy.async, or a bulk copy's completion)
-// before the count is sent.  Releases at cluster scope took over a thousand
-// cycles each and doubled the kernel's time.
+// CTA 1's arrivals in CTA 0 stand for its activations, features and weights, which its
+// own tensor core reads for an MMA that CTA 0 issues: each writer hands them to the
+// async proxy (fence.proxy.async, or a bulk copy's completion), the arrival releases
+// them at cluster scope, and who polls the barrier acquires them before the count goes
+// on.  Both fences are restricted to shared memory (see mbar_arrive_cta).  An
+// accumulator that has been read is handed over as tcgen05.fence asks.
 //
 // The hidden activations and the output are those of mlp_serve bit for bit (the
 // paired FP32 operations round each half as the scalar ones).  4,000,000 rows 3.10
@@ -159,7 +160,7 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
     // one arrival on a barrier of CTA 0
     auto arrive0 = [&](uint64_t *bar) {
         if (rank == 0) tc::mbar_arrive(bar);
-        else tc::mbar_arrive_relaxed_cta(bar, 0);
+        else tc::mbar_arrive_cta(bar, 0);
     };
 
     if (warp == SV_PROD_WARP) {
@@ -179,7 +180,8 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 // chunk c of a step has stage c, last read by chunk c of the step
                 // before
                 for (int c = 0; c < SP_CHUNKS; ++c) {
-                    if (i > 0 && !(ok = tc::mbar_wait(&chunk_done[c], (uint32_t)((i - 1) & 1)))) break;
+                    if (i > 0 && !(ok = tc::mbar_wait_cluster(&chunk_done[c], (uint32_t)((i - 1) & 1))))
+                        break;
                     tc::mbar_arrive_expect_tx(&full[c], SP_HALF);
                     const uint8_t *src = img + W0_BYTES + (size_t)(l - 1)*HID*HID*2
                                        + (size_t)c*(SP_K/8)*2*SP_GROUP;
@@ -208,7 +210,8 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             uint32_t unit = 0;
             ok = warp_wait(&w0_bar, 0u);
             for (int p = 0; p < 2 && p < mine && ok; ++p) {
-                ok = warp_wait(&x_ready[p], 0u);
+                ok = warp_wait_cluster(&x_ready[p], 0u);
+                __syncwarp();
                 ++unit;
                 if (lane == 0 && ok) tc::st_release_shared(&ready_seq, unit);
             }
@@ -232,7 +235,7 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 int done = 0;
                 for (uint32_t n_try = 0; done < units && n_try < tc::WAIT_LIMIT; ++n_try) {
                     const bool on = (need & ~seen & (1u << lane)) != 0;
-                    seen |= __ballot_sync(0xffffffffu, on && tc::mbar_test(bar, parity));
+                    seen |= __ballot_sync(0xffffffffu, on && tc::mbar_test_relaxed(bar, parity));
                     // units in order, the layer 0 in the middle
                     uint32_t r = seen & (seen >> 8) & all;
                     if (z >= 0)
@@ -241,6 +244,7 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                     const int here = (seen >> 16) & 1u ? __ffs(~r) - 1 : 0;
                     if (here > done) {
                         done = here;
+                        tc::cluster_acquire();
                         __syncwarp();
                         if (lane == 0) tc::st_release_shared(&ready_seq, unit + (uint32_t)done);
                     }
@@ -293,7 +297,7 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         for (int i = 0; 2*i < mine && ok; ++i) {
             for (int p = 0; p < 2 && 2*i + p < mine; ++p) {
                 // the buffer's last reader, layer 0 of the tile before
-                if (i > 0 && !(ok = warp_wait(&x_free[p], (uint32_t)((i - 1) & 1)))) break;
+                if (i > 0 && !(ok = warp_wait_cluster(&x_free[p], (uint32_t)((i - 1) & 1)))) break;
                 load_x(p, i);
                 if (lane == 0) arrive0(&x_ready[p]);
             }
@@ -349,7 +353,7 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
             }
             // every MMA issued has completed before TMEM is released
             tc::mma_commit_pair(&drain);
-            ok = tc::mbar_wait(&drain, 0u) && ok;
+            ok = tc::mbar_wait_cluster(&drain, 0u) && ok;
             if (!ok) atomicExch(err, 3);
         }
         __syncwarp();
@@ -367,7 +371,7 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
         for (int j = SP_FIRST; j < turns && ok; ++j) {
             int p, l, i;
             if (!sp_turn(j, mine, p, l, i)) continue;
-            if (!(ok = warp_wait(&acc_full[p], (uint32_t)(l & 1)))) break;
+            if (!(ok = warp_wait_cluster(&acc_full[p], (uint32_t)(l & 1)))) break;
             tc::fence_after_sync();
             if (l < 3) {
                 // 16 columns of every 64
@@ -385,7 +389,8 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 // chunk c of step s takes the place of chunk c of step s - 1
                 // (completion s - 1); the last one done means that all are
                 const uint32_t before = (uint32_t)((s - 1) & 1);
-                const bool free_all = s == 0 || tc::mbar_test(&chunk_done[SP_CHUNKS - 1], before);
+                const bool free_all = s == 0 || tc::mbar_test_relaxed(&chunk_done[SP_CHUNKS - 1], before);
+                tc::cluster_acquire();
                 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     constexpr int RU = SP_K/64;
@@ -399,7 +404,7 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                         if (lane == 0) arrive0(&act_ready[c - 1]);
                     }
                     silu_columns(r[q], 8, bias + 64*q, hi[1], lo[1]);
-                    if (q % RU == 0 && !free_all && !tc::mbar_wait(&chunk_done[c], before)) ok = false;
+                    if (q % RU == 0 && !free_all && !tc::mbar_wait_cluster(&chunk_done[c], before)) ok = false;
                     #pragma unroll
                     for (int g = 0; g < 2; ++g) {
                         const uint32_t off = tc::kmajor_offset<TM>(row, 64*q + 16*slot + 8*g);
@@ -409,6 +414,7 @@ mlp_serve_pairs(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
                 }
                 tc::fence_async_smem();
                 ok = __all_sync(0xffffffffu, ok) != 0;
+                __syncwarp();
                 if (lane == 0) arrive0(&act_ready[SP_CHUNKS - 1]);
                 if (!ok) break;
                 ++s;

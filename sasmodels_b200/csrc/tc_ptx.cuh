@@ -54,17 +54,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
     return done != 0;
 }
 
-// Whether the phase with the given parity is complete, without suspending.
-__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity)
-{
-    uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return done != 0;
-}
-
 // Bounded wait for the phase with the given parity to complete.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity)
 {
@@ -111,14 +100,51 @@ __device__ __forceinline__ void cluster_wait()
 {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Arrive once on the barrier at this offset in CTA `rank` of the cluster.
-// Relaxed: see mlp_serve_pairs for what the count stands for.
-__device__ __forceinline__ void mbar_arrive_relaxed_cta(uint64_t *bar, uint32_t rank)
+// Arrive once on the barrier at this offset in CTA `rank` of the cluster: releases,
+// at cluster scope, what this thread wrote to shared memory or has seen written there
+// by others (bulk copies included).  The fence orders accesses to this CTA's shared
+// memory only; a release of everything (mbarrier.arrive.release.cluster) also waits for the
+// thread's accesses to global memory and took over 1000 cycles.
+__device__ __forceinline__ void mbar_arrive_cta(uint64_t *bar, uint32_t rank)
 {
-    asm volatile("{\n\t.reg .b32 remote;\n\t"
+    asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n\t"
+                 "{\n\t.reg .b32 remote;\n\t"
                  "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
                  "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [remote];\n\t}"
                  :: "r"(smem_u32(bar)), "r"(rank) : "memory");
+}
+// Its other side: makes what such arrivals released visible to this thread, after a
+// test or wait of cluster scope saw the phase complete.
+__device__ __forceinline__ void cluster_acquire()
+{
+    asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+}
+// Whether the phase with the given parity of a barrier that the other CTA arrives on is
+// complete, without suspending; cluster_acquire has to follow.
+__device__ __forceinline__ bool mbar_test_relaxed(uint64_t *bar, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "mbarrier.test_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return done != 0;
+}
+// mbar_wait for such a barrier, or one that a pair's MMAs complete.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity)
+{
+    for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (done) {
+            cluster_acquire();
+            return true;
+        }
+    }
+    return false;
 }
 
 // ---- release/acquire flags in shared memory ------------------------------
