@@ -1301,8 +1301,7 @@ struct ReadyCounts {
 enum { PLANES_NONE, PLANES_ROWS, PLANES_TILED };
 template <int PLANES>
 __global__ void __launch_bounds__(SV_THREADS, 1)
-mlp_serve(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
-          const __nv_bfloat16 *__restrict__ x_lo, InferParams prm, float *__restrict__ out,
+mlp_serve(int n, int n_tiles, const __nv_bfloat16 *x, const __nv_bfloat16 *x_lo, InferParams prm, float *__restrict__ out,
           int *__restrict__ err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];

@@ -133,8 +133,7 @@ __device__ __forceinline__ long long batch_row(const Batch &batch, int n, int r,
 // TRAIN: with the tiled planes, the loss gradient and the backward.
 template <bool TRAIN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SP_THREADS, 1)
-mlp_halves(int n, int n_tiles, const __nv_bfloat16 *__restrict__ x,
-           const __nv_bfloat16 *__restrict__ x_lo, const __grid_constant__ CUtensorMap img,
+mlp_halves(int n, int n_tiles, const __nv_bfloat16 *x, const __nv_bfloat16 *x_lo, const __grid_constant__ CUtensorMap img,
            const __grid_constant__ CUtensorMap img_t, InferParams prm, float *__restrict__ out,
            __nv_bfloat16 *__restrict__ dz_save, int *__restrict__ err)
 {

@@ -37,9 +37,8 @@ constexpr int BT_STAGES = 8;
 constexpr int BT_SMEM = ACT_BYTES + BT_STAGES*CHUNK_BYTES;
 
 __global__ void __launch_bounds__(SV_THREADS, 1)
-mlp_backward_t(int n_tiles, const uint8_t *__restrict__ img_t, const float *__restrict__ w_out,
-               const float *__restrict__ dout, const __nv_bfloat16 *__restrict__ z_save,
-               __nv_bfloat16 *__restrict__ dz_save, int *__restrict__ err)
+mlp_backward_t(int n_tiles, const uint8_t *img_t, const float *w_out, const float *dout,
+               const __nv_bfloat16 *z_save, __nv_bfloat16 *__restrict__ dz_save, int *__restrict__ err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *act = smem;
@@ -203,7 +202,7 @@ mlp_backward_t(int n_tiles, const uint8_t *__restrict__ img_t, const float *__re
                         const float4 *wp = reinterpret_cast<const float4 *>(w_out + 64*q + 16*slot);
                         #pragma unroll
                         for (int e = 0; e < 4; ++e) {
-                            const float4 w = __ldg(wp + e);
+                            const float4 w = wp[e];
                             ra[4*e] = __float_as_uint(d*w.x);
                             ra[4*e + 1] = __float_as_uint(d*w.y);
                             ra[4*e + 2] = __float_as_uint(d*w.z);

@@ -201,7 +201,9 @@ __device__ __forceinline__ void box_load4(void *dst, const void *map, int x, int
 // dependent one (launch_dependent in mlp.cu), may take free SMs from now on.
 // dependency_wait: until every kernel before this one is complete and its writes
 // are visible; nothing that they touch may be accessed before it, and every CTA
-// has to come by here, so that a kernel's completion stands for all before it.
+// has to come by here, so that a kernel's completion stands for all before it.  Their
+// writes fall into this kernel's lifetime, so no pointer to them may be const
+// __restrict__, nor be read by __ldg.
 // Both do nothing in an ordinary launch.
 __device__ __forceinline__ void dependents_launch()
 {
