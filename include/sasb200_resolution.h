@@ -28,7 +28,8 @@
  *   sasb200_slit_weights       formed once (the reference's weight_matrix, its
  *                              bands only): those of q i at w[off[i] + j -
  *                              lo[i]] for lo[i] <= j < hi[i], to be divided
- *                              by norm[i];
+ *                              by norm[i]; -0.0 for a point inside the band
+ *                              that is not part of the sum;
  *   sasb200_band_apply         apply_resolution_matrix with them, for n_sets
  *                              curves.
  * All arrays are device pointers; the calls are asynchronous on *stream*.

@@ -211,7 +211,10 @@ slit_smear(int nq, int n_calc, const double *__restrict__ q, const double *__res
 // while its weights never change, so they are formed once (pinhole_weights,
 // slit_weights) and each application is a banded product.  Weights of q i:
 // w[off[i] + j - lo[i]] for the calculated points lo[i] <= j < hi[i], divided
-// by norm[i] after the sum.
+// by norm[i] after the sum.  A weight of -0.0 marks a point that is not part of
+// the sum, whatever the theory there (the steps across a wide slit with a short
+// length leave such points between them); no sum forms one by itself.
+constexpr long long NO_WEIGHT = 0x8000000000000000ll;        // the bits of -0.0
 
 // One warp per q: the bin masses of pinhole_smear and their sum, in its order.
 __global__ void __launch_bounds__(256)
@@ -244,8 +247,8 @@ pinhole_weights(int nq, const double *__restrict__ q, const double *__restrict__
 // shared memory.  A warp takes 31 bins at a time: lane L forms sqrt(u) at edge
 // L of the group and gets the next edge's from lane L + 1, so each (edge,
 // step) costs one square root instead of slit_smear's two and its two binary
-// searches per step.  A step that does not reach a bin has equal u at both of
-// its edges and adds 0.
+// searches per step.  A step that does not reach a bin (see slit_smear's searches)
+// has equal u at both of its edges and adds 0.
 constexpr int SLIT_BATCH = 128;
 __global__ void __launch_bounds__(256)
 slit_weights(const double *__restrict__ q, const double *__restrict__ width,
@@ -263,7 +266,8 @@ slit_weights(const double *__restrict__ q, const double *__restrict__ width,
     if (wi == 0.0 && li == 0.0) {
         // perfect resolution: the theory at q_calc == q
         if (t == 0) norm[i] = 1.0;
-        for (int j = a + t; j < b; j += (int)blockDim.x) out[j - a] = q_calc[j] == qi ? 1.0 : 0.0;
+        for (int j = a + t; j < b; j += (int)blockDim.x)
+            out[j - a] = q_calc[j] == qi ? 1.0 : __longlong_as_double(NO_WEIGHT);
         return;
     }
     const int kmax = wi == 0.0 ? 0 : n_length;
@@ -280,15 +284,18 @@ slit_weights(const double *__restrict__ q, const double *__restrict__ width,
         __syncthreads();
         for (int j0 = a + 31*warp; j0 < b; j0 += 31*warps) {
             const double edge = edges[min(j0 + lane, b)];
+            const double above = __shfl_down_sync(FULL, edge, 1);
             double acc = 0.0;
+            bool reached = false;
             #pragma unroll 4
             for (int k = 0; k < nk; ++k) {
                 const double r = sqrt(slit_u(edge, sq[k], sl[k]));
                 acc += __dsub_rn(__shfl_down_sync(FULL, r, 1), r);
+                reached = reached || (above >= fabs(sq[k]) && edge <= sl[k]);
             }
             const int j = j0 + lane;
             if (lane < 31 && j < b) {
-                const double part = acc/li;
+                const double part = reached ? acc/li : __longlong_as_double(NO_WEIGHT);
                 out[j - a] = k0 == 0 ? part : out[j - a] + part;
             }
         }
@@ -310,7 +317,10 @@ band_apply(int nq, const int32_t *__restrict__ lo, const int32_t *__restrict__ h
     const double *wi = w + off[i], *th = theory + blockIdx.y*theory_stride + a;
     double acc = 0.0;
     #pragma unroll 4
-    for (int j = lane; j < n; j += 32) acc += wi[j]*th[j];
+    for (int j = lane; j < n; j += 32) {
+        const double m = wi[j], x = th[j];
+        if (__double_as_longlong(m) != NO_WEIGHT) acc += m*x;
+    }
     #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
     if (lane == 0) out[blockIdx.y*out_stride + i] = acc/norm[i];
