@@ -172,16 +172,23 @@ class MLP:
 
     # bf16 copies used by the kernels
     def _sync_bf16(self):
+        """Refresh the bf16 copies from weights that were set on the current
+        stream; in order with the work on self.stream and on the current one."""
         torch = self.torch
+        current = torch.cuda.current_stream(self.device)
         self._wversion = getattr(self, "_wversion", 0) + 1
         if not hasattr(self, "Wb"):
             self.Wb = [torch.empty_like(w, dtype=torch.bfloat16) for w in self.W]
             self.WTb = [torch.empty_like(w.t(), dtype=torch.bfloat16,
                                          memory_format=torch.contiguous_format) for w in self.W]
-        # in place: a captured training step holds their addresses
-        for w, wb, wtb in zip(self.W, self.Wb, self.WTb):
-            wb.copy_(w)
-            wtb.copy_(w.t())
+        # in place: a captured training step holds their addresses, and kernels
+        # on self.stream may still read or write them
+        self.stream.wait_stream(current)
+        with torch.cuda.stream(self.stream):
+            for w, wb, wtb in zip(self.W, self.Wb, self.WTb):
+                wb.copy_(w)
+                wtb.copy_(w.t())
+        current.wait_stream(self.stream)
 
     def _ptrs(self, tensors):
         arr = (ct.c_void_p*len(tensors))(*[t.data_ptr() for t in tensors])
@@ -413,7 +420,10 @@ class MLP:
                              ("b_out", self.b_out))}
 
     def load_state(self, st):
+        """Set the weights (arrays or tensors ready on the current stream), behind
+        the work queued on self.stream and ahead of what follows there."""
         torch = self.torch
+        torch.cuda.current_stream(self.device).wait_stream(self.stream)
         for l in range(4):
             self.W[l].copy_(torch.as_tensor(st["W"][l]))
             self.b[l].copy_(torch.as_tensor(st["b"][l]))
