@@ -582,6 +582,7 @@ class TrainingGraph:
         self.xlb = torch.empty_like(self.xb)
         self.yb = torch.empty(batch, dtype=y_all.dtype, device=dev)
         self.loss = torch.zeros((), dtype=torch.float32, device=dev)
+        self._done = torch.cuda.Event()
         net._scratch(batch)
         lib, st = net.lib, net.stream.cuda_stream
         # the forward gathers 32-byte rows of bf16 and float targets, as
@@ -616,12 +617,16 @@ class TrainingGraph:
     def step(self, idx):
         """One training step on rows `idx` (int64 device tensor of `batch`
         entries); returns the loss (a device scalar, overwritten by the
-        next step)."""
-        net = self.net
+        next step) for the current stream, which waits for the step."""
+        net, torch = self.net, self.net.torch
         net._pack()          # current unless the weights were set from outside
-        with net.torch.cuda.stream(net.stream):
+        current = torch.cuda.current_stream(net.device)
+        with torch.cuda.stream(net.stream):
             self.idx.copy_(idx)
             self.graph.replay()
+        if current != net.stream:
+            self._done.record(net.stream)
+            current.wait_event(self._done)
         net.step_count += 1
         net._packed = (net.step_count, net._wversion)
         return self.loss
@@ -701,6 +706,7 @@ class Surrogate:
         use_graph = nranks == 1 and (batch//nranks) % TM == 0
         for ep in range(epochs):
             perm = torch.randperm(n, device=net.device, generator=gen)
+            net.stream.wait_stream(torch.cuda.current_stream(net.device))
             for s in range(steps):
                 lo, hi = batch_slice(s*batch, batch, rank, nranks)
                 idx = perm[lo:hi]

@@ -71,3 +71,23 @@ def test_load_state_between_steps(cuda, batch):
                                          + [net.img, net.img_t]])
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("batch", [128, 128*80])
+def test_loss_of_a_captured_step_on_the_callers_stream(cuda, batch):
+    """The loss is read while the step is still to come on the network's stream."""
+    import torch
+    from sasmodels_b200.surrogate import MLP
+    x = torch.rand((batch, 16), device="cuda").to(torch.bfloat16)
+    lo, y = torch.zeros_like(x), torch.randn(batch, device="cuda")
+    idx = torch.arange(batch, device="cuda")
+    net = MLP(seed=1)
+    torch.cuda.synchronize()
+    graph = net.capture_training(x, lo, y, batch, 1e-3, 100, 1)
+    torch.cuda.synchronize()
+    for _ in range(2):
+        with torch.cuda.stream(net.stream):
+            torch.cuda._sleep(CYCLES)
+        got = float(graph.step(idx).item())
+        torch.cuda.synchronize()
+        assert got == float(graph.loss.item()) and got > 0
