@@ -117,8 +117,10 @@ int32_t sasb200_adam(int32_t size, int32_t splits, const float *grad, float *p, 
  *
  * A captured step takes a batch (else NULL): x, x_lo and y then receive the rows
  * idx[n] of the data set (x_all, x_lo_all [rows x 16] bf16, y_all[rows]) first,
- * and the schedule advances as by sasb200_lr_schedule; an index outside the set
- * leaves zeros and *err = 5. */
+ * and the schedule advances as by sasb200_lr_schedule.  An index outside the set
+ * leaves zeros, *err = 5, sched[3] = 1 (sched has four floats, the last 0 before the
+ * first step), *refused = 1 (memory that the host reads, page-locked) and an undefined
+ * loss; see sasb200_adam_pack. */
 typedef struct sasb200_mlp_batch {
     const int64_t *idx;
     int64_t rows;
@@ -126,6 +128,7 @@ typedef struct sasb200_mlp_batch {
     const float *y_all;
     int32_t *counters;
     float *sched;
+    int32_t *refused;
     int32_t total, warmup;
     float lr0, b1, b2;
 } sasb200_mlp_batch;
@@ -154,7 +157,7 @@ int32_t sasb200_mlp_train_pass(const sasb200_mlp_pass *pass, void *stream);
  * W0..W3, b0..b3, w_out, b_out, with splits[k] partial gradients each) with the
  * bf16 weights w[4], transposes wt[4] and both weight images; lr and the bias
  * corrections from sched (sasb200_lr_schedule), or from lr and step when it is
- * NULL. */
+ * NULL.  Where the fourth float of sched is not 0, nothing is updated. */
 int32_t sasb200_adam_pack(const float *const *grads, const int32_t *splits, float *const *p,
                           float *const *m, float *const *v, void *const *w, void *const *wt,
                           void *img, void *img_t, const float *sched, float lr, int32_t step,

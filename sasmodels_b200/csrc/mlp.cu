@@ -806,10 +806,24 @@ struct Batch {
     __nv_bfloat16 *x, *x_lo;      // where the batch goes
     float *y;
     int *counters;
-    float *sched;
+    float *sched;                 // sched[3] != 0: a row was outside, nothing is updated any more
+    int *refused;                 // the same for the host (its memory)
     int total, warmup;
     float lr0, b1, b2;
 };
+
+// The data set's row of batch row r, or -1 outside the data set.  Such a step may
+// not train: its loss is undefined and adam_pack leaves everything as it is, in
+// this step and all that follow with this schedule.
+__device__ __forceinline__ long long batch_row(const Batch &batch, int r, int *err)
+{
+    const long long src = batch.idx[r];
+    if (src >= 0 && src < batch.rows) return src;
+    atomicExch(err, 5);
+    batch.sched[3] = 1.0f;
+    *(volatile int *)batch.refused = 1;
+    return -1;
+}
 
 struct InferParams {
     const uint8_t *img;           // packed weights (mlp_pack)
@@ -1817,6 +1831,7 @@ struct sasb200_mlp_batch {
     const float *y_all;
     int32_t *counters;
     float *sched;
+    int32_t *refused;
     int32_t total, warmup;
     float lr0, b1, b2;
 };
@@ -2013,7 +2028,7 @@ int32_t sasb200_mlp_serve(int32_t n, int32_t n_pad, const void *x, const void *x
 // tiled z and h planes, dout[n_pad] of the mean Huber loss (threshold delta; squared
 // error for delta <= 0) against y[n], 0 on padding, row_sums[2][n_pad/32]: the loss
 // and dout summed over 32 rows each; and the dZ planes.  With a batch, x, x_lo and y
-// receive its rows of the data set first (err = 5 for a row outside it) and the
+// receive its rows of the data set first (a row outside it: see batch_row) and the
 // schedule advances as by sasb200_lr_schedule.
 static int32_t forward_backward(const sasb200_mlp_pass &p, cudaStream_t st)
 {
@@ -2035,7 +2050,7 @@ static int32_t forward_backward(const sasb200_mlp_pass &p, cudaStream_t st)
     const auto *xlp = static_cast<const __nv_bfloat16 *>(p.x_lo);
     if (const sasb200_mlp_batch *batch = p.batch) {
         if (!batch->idx || batch->rows < 0 || !batch->x_all || !batch->x_lo_all || !batch->y_all
-            || !batch->counters || !batch->sched || batch->total <= 0 || batch->warmup <= 0
+            || !batch->counters || !batch->sched || !batch->refused || batch->total <= 0 || batch->warmup <= 0
             || n <= 0)
             return (std::snprintf(errbuf(), 256, "bad batch"), -1);
         if ((reinterpret_cast<uintptr_t>(batch->x_all) | reinterpret_cast<uintptr_t>(batch->x_lo_all)
@@ -2044,8 +2059,8 @@ static int32_t forward_backward(const sasb200_mlp_pass &p, cudaStream_t st)
         prm.batch = {batch->idx, batch->rows, static_cast<const __nv_bfloat16 *>(batch->x_all),
                      static_cast<const __nv_bfloat16 *>(batch->x_lo_all), batch->y_all,
                      const_cast<__nv_bfloat16 *>(xp), const_cast<__nv_bfloat16 *>(xlp),
-                     const_cast<float *>(p.y), batch->counters, batch->sched, batch->total,
-                     batch->warmup, batch->lr0, batch->b1, batch->b2};
+                     const_cast<float *>(p.y), batch->counters, batch->sched, batch->refused,
+                     batch->total, batch->warmup, batch->lr0, batch->b1, batch->b2};
     }
     if (n_pad == 0) return 0;
     prm.w_out = p.w_out;
@@ -2086,12 +2101,13 @@ static int32_t forward_backward(const sasb200_mlp_pass &p, cudaStream_t st)
 
 // Every gradient of a training step from its planes: dw[0..3] [splits][256 x (16
 // or 256)], db [4][splits][256] and dw_out [splits][256] as partial sums over
-// splits of the rows; the mean loss over n rows and db_out as scalars.
+// splits of the rows; the mean loss over n rows and db_out as scalars.  refused: null,
+// or nonzero there for an undefined loss.
 static int32_t weight_grads(int32_t n, int32_t n_pad, int32_t splits, const void *x,
                             const void *h, const void *dz, const float *dout,
                             const float *row_sums, float *const *dw, float *db,
-                            float *dw_out, float *loss, float *db_out, int32_t *err,
-                            void *stream)
+                            float *dw_out, float *loss, float *db_out, const float *refused,
+                            int32_t *err, void *stream)
 {
     errbuf()[0] = 0;
     if (n < 0 || n > n_pad || n_pad <= 0 || n_pad % TM || splits <= 0 || splits > 4096 || !x || !h
@@ -2116,6 +2132,7 @@ static int32_t weight_grads(int32_t n, int32_t n_pad, int32_t splits, const void
     prm.loss = loss;
     prm.db_out = db_out;
     prm.n = (float)n;
+    prm.refused = refused;
     cudaFuncSetAttribute(mlp_weight_grads, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
     launch_dependent(mlp_weight_grads, dim3((WG_BIG + 2)*splits), WG_THREADS, WG_SMEM,
                      (cudaStream_t)stream, n_pad/TM, splits, prm, err);
@@ -2125,7 +2142,8 @@ static int32_t weight_grads(int32_t n, int32_t n_pad, int32_t splits, const void
 // Adam for the whole network (host arrays of 10 device pointers, in the order
 // W0..W3, b0..b3, w_out, b_out; splits partial gradients each) refreshing the
 // bf16 weights w[4], their transposes wt[4] and both weight images; lr and the
-// bias corrections from sched when it is not NULL, else lr and step (>= 1).
+// bias corrections from sched when it is not NULL (nothing is updated where sched[3] is
+// set), else lr and step (>= 1).
 int32_t sasb200_adam_pack(const float *const *grads, const int32_t *splits, float *const *p,
                           float *const *m, float *const *v, void *const *w, void *const *wt,
                           void *img, void *img_t, const float *sched, float lr, int32_t step,
@@ -2201,7 +2219,8 @@ int32_t sasb200_mlp_train_pass(const sasb200_mlp_pass *p, void *stream)
     int32_t rc = forward_backward(*p, (cudaStream_t)stream);
     if (rc == 0)
         rc = weight_grads(p->n, p->n_pad, p->splits, p->x, p->h, p->dz, p->dout, p->row_sums, p->dw,
-                          p->db, p->dw_out, p->loss, p->db_out, p->err, stream);
+                          p->db, p->dw_out, p->loss, p->db_out,
+                          p->batch ? p->batch->sched + 3 : nullptr, p->err, stream);
     if (rc == 0 && p->sums > 0)
         rc = sum_partials_of(p->sums, p->sum_sizes, p->sum_splits, p->sum_parts, p->sum_outs, stream);
     return rc;

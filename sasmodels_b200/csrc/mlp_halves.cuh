@@ -119,17 +119,6 @@ __device__ __forceinline__ void hv_leave_together()
     tc::cluster_wait();
 }
 
-// The data set's row of batch row r: -1 past the batch, and with err = 5 outside
-// the data set.
-__device__ __forceinline__ long long batch_row(const Batch &batch, int n, int r, int *err)
-{
-    if (r >= n) return -1;
-    const long long src = batch.idx[r];
-    if (src >= 0 && src < batch.rows) return src;
-    atomicExch(err, 5);
-    return -1;
-}
-
 // TRAIN: with the tiled planes, the loss gradient and the backward.
 template <bool TRAIN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SP_THREADS, 1)
@@ -236,7 +225,8 @@ mlp_halves(int n, int n_tiles, const __nv_bfloat16 *x, const __nv_bfloat16 *x_lo
             const int u = lane + 32*j;
             const size_t g = (size_t)(row0 + (u >> 1))*NIN + (u & 1)*8;
             if (TRAIN && prm.batch.idx) {
-                const long long src = batch_row(prm.batch, n, row0 + (u >> 1), err);
+                const int r = row0 + (u >> 1);
+                const long long src = r < n ? batch_row(prm.batch, r, err) : -1;
                 v[j] = w[j] = make_uint4(0, 0, 0, 0);
                 if (src >= 0) {
                     v[j] = *reinterpret_cast<const uint4 *>(prm.batch.x_all + src*NIN + (u & 1)*8);
@@ -340,7 +330,7 @@ mlp_halves(int n, int n_tiles, const __nv_bfloat16 *x, const __nv_bfloat16 *x_lo
         float target = 0.0f;
         if (TRAIN && half == 0 && slot == 0) {
             if (prm.batch.idx) {
-                const long long src = batch_row(prm.batch, n, row0 + row, err);
+                const long long src = row0 + row < n ? batch_row(prm.batch, row0 + row, err) : -1;
                 if (src >= 0) target = prm.batch.y_all[src];
                 if (row0 + row < n) prm.batch.y[row0 + row] = target;
             } else if (row0 + row < n) {

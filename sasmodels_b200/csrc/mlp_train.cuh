@@ -293,6 +293,7 @@ struct WeightGrads {
     float *dw_out;                   // [S][256]
     float *loss, *db_out;            // scalars
     float n;                         // rows of the mean loss
+    const float *refused;            // null, or nonzero there: the loss is undefined
 };
 
 __global__ void __launch_bounds__(WG_THREADS, 1)
@@ -461,7 +462,9 @@ mlp_weight_grads(int n_tiles, int splits, WeightGrads prm, int *__restrict__ err
             for (int j = lane; j < 4*n_tiles; j += 32) v += part[j];
             #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) *(warp == 0 ? prm.loss : prm.db_out) = warp == 0 ? v/prm.n : v;
+            if (warp == 0) v = prm.refused && *prm.refused != 0.0f ? __int_as_float(0x7fffffff)
+                                                                   : v/prm.n;
+            if (lane == 0) *(warp == 0 ? prm.loss : prm.db_out) = v;
         }
         // ---- the accumulators: warps 0-3 the first 64 columns, 4-7 the rest ----
         if (mma && ok) {
@@ -529,7 +532,7 @@ sum_partials(SumTensors T)
 // of x and of x_lo and one target each) and, by one thread, the schedule.  Bound by
 // the random 32-byte reads; 5.6 us with cold caches for 8192 rows, where three
 // index_select launches and lr_schedule took 29.  A row outside the data set leaves
-// zeros and err = 5.
+// zeros (see batch_row).
 __global__ void __launch_bounds__(256)
 gather_batch(int n, Batch batch, int *__restrict__ err)
 {
@@ -540,15 +543,12 @@ gather_batch(int n, Batch batch, int *__restrict__ err)
                       batch.b2);
     const int i = blockIdx.x*256 + threadIdx.x, row = i >> 2, part = i & 3;
     if (row >= n) return;
-    const long long src = batch.idx[row];
-    const bool in = src >= 0 && src < batch.rows;
+    const long long src = batch_row(batch, row, err);
+    const bool in = src >= 0;
     uint4 v = make_uint4(0, 0, 0, 0);
     if (in) v = reinterpret_cast<const uint4 *>(part < 2 ? batch.x_all : batch.xlo_all)[2*src + (part & 1)];
     reinterpret_cast<uint4 *>(part < 2 ? batch.x : batch.x_lo)[2*row + (part & 1)] = v;
-    if (part == 0) {
-        batch.y[row] = in ? batch.y_all[src] : 0.0f;
-        if (!in) atomicExch(err, 5);
-    }
+    if (part == 0) batch.y[row] = in ? batch.y_all[src] : 0.0f;
 }
 
 // -------------------------------------------------------------------- Adam --
@@ -567,7 +567,7 @@ struct AdamPack {
     float *p[10], *m[10], *v[10];
     __nv_bfloat16 *w[4], *wt[4];
     uint8_t *img, *img_t;
-    const float *sched;              // {lr, bc1, bc2}, or null and the values below
+    const float *sched;              // {lr, bc1, bc2, refused}, or null and the values below
     float lr, bc1, bc2, b1, b2, eps;
 };
 constexpr int AP_TILES = (HID/32)*(HID/32);
@@ -607,6 +607,7 @@ adam_pack(AdamPack A)
     tc::dependents_launch();
     tc::dependency_wait();
     const int t = threadIdx.x, b = blockIdx.x;
+    if (A.sched && A.sched[3] != 0.0f) return;           // see batch_row
     const float lr = A.sched ? A.sched[0] : A.lr, bc1 = A.sched ? A.sched[1] : A.bc1,
                 bc2 = A.sched ? A.sched[2] : A.bc2;
     if (b < 3*AP_TILES) {

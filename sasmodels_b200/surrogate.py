@@ -97,6 +97,11 @@ def _load():
     return lib
 
 
+#: code of a captured step whose batch names a row that the data set lacks
+ROW_OUTSIDE = 5
+OUTSIDE = "a row index outside the training data"
+
+
 def pad128(n):
     return ((n + TM - 1)//TM)*TM
 
@@ -106,7 +111,7 @@ class _Batch(ct.Structure):
 
     _fields_ = [("idx", ct.c_void_p), ("rows", ct.c_int64), ("x_all", ct.c_void_p),
                 ("x_lo_all", ct.c_void_p), ("y_all", ct.c_void_p), ("counters", ct.c_void_p),
-                ("sched", ct.c_void_p), ("total", ct.c_int32), ("warmup", ct.c_int32),
+                ("sched", ct.c_void_p), ("refused", ct.c_void_p), ("total", ct.c_int32), ("warmup", ct.c_int32),
                 ("lr0", ct.c_float), ("b1", ct.c_float), ("b2", ct.c_float)]
 
 
@@ -169,6 +174,9 @@ class MLP:
         self._infer_out = None
         self._sync_bf16()
         self._scratch_n = 0
+        # host flags of the training graphs: a queued replay may still set one
+        # when its graph is gone
+        self._refused = []
 
     # bf16 copies used by the kernels
     def _sync_bf16(self):
@@ -593,20 +601,26 @@ class TrainingGraph:
                   and len(x_all) == len(x_lo_all) == len(y_all)
                   and all(t.is_contiguous() and t.data_ptr() % 16 == 0
                           for t in (x_all, x_lo_all, y_all)))
-        schedule = (self.counters.data_ptr(), self.sched.data_ptr(), int(total), int(warmup),
-                    float(lr), b1, b2)
+        rates = (int(total), int(warmup), float(lr), b1, b2)
+        schedule = (self.counters.data_ptr(), self.sched.data_ptr())
+        refused = torch.zeros(1, dtype=torch.int32).pin_memory()
+        net._refused.append(refused)
+        self._refused = refused.numpy()
         net.stream.synchronize()
+        if net.errors() == ROW_OUTSIDE:
+            net.err.zero_()          # of a graph before, which stays refused
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph, stream=net.stream):
             if not direct:
                 torch.index_select(x_all, 0, self.idx, out=self.xb)
                 torch.index_select(x_lo_all, 0, self.idx, out=self.xlb)
                 torch.index_select(y_all, 0, self.idx, out=self.yb)
-                net._check(lib.sasb200_lr_schedule(*schedule, st), "lr_schedule")
+                net._check(lib.sasb200_lr_schedule(*schedule, *rates, st), "lr_schedule")
             net._gradient_kernels(
                 self.xb, self.xlb, self.yb, batch, self.loss.data_ptr(), net.gbo.data_ptr(),
                 batch=_Batch(self.idx.data_ptr(), len(y_all), x_all.data_ptr(), x_lo_all.data_ptr(),
-                             y_all.data_ptr(), *schedule) if direct else None)
+                             y_all.data_ptr(), *schedule, refused.data_ptr(), *rates)
+                if direct else None)
             net._adam(net.gW + list(net.gb_part) + [net.gw_part, net.gbo], [net.splits]*9 + [1],
                       self.sched, lr, b1, b2, eps)
         # what the graph reads and writes outlives the network's next, larger
@@ -617,8 +631,15 @@ class TrainingGraph:
     def step(self, idx):
         """One training step on rows `idx` (int64 device tensor of `batch`
         entries); returns the loss (a device scalar, overwritten by the
-        next step) for the current stream, which waits for the step."""
+        next step) for the current stream, which waits for the step.
+
+        A row outside the data set ends the training of this graph, as it
+        cannot be known before the kernels read it: the loss is NaN, weights
+        and moments stay those of the step before, ``net.errors()`` is 5, and
+        calls raise once the host has seen it."""
         net, torch = self.net, self.net.torch
+        if self._refused[0]:
+            raise RuntimeError(OUTSIDE)
         net._pack()          # current unless the weights were set from outside
         current = torch.cuda.current_stream(net.device)
         with torch.cuda.stream(net.stream):
@@ -733,7 +754,7 @@ class Surrogate:
         graph = None
         code = net.errors()
         if code:
-            raise RuntimeError("a row index outside the training data" if code == 5 else
+            raise RuntimeError(OUTSIDE if code == ROW_OUTSIDE else
                                "tensor-core kernel reported a timeout")
         return losses
 
