@@ -581,6 +581,9 @@ class TrainingGraph:
         dev = net.device
         if batch % TM:
             raise ValueError("batch must be a multiple of %d" % TM)
+        # the kernels take addresses
+        if any(t.device != dev for t in (x_all, x_lo_all, y_all)):
+            raise ValueError("the data set must be on %s" % dev)
         self.batch = batch
         self.idx = torch.zeros(batch, dtype=torch.int64, device=dev)
         self.counters = torch.tensor([int(step0), int(net.step_count)], dtype=torch.int32,

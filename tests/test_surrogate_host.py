@@ -7,7 +7,7 @@ from types import SimpleNamespace
 import numpy as np
 import pytest
 
-from sasmodels_b200.surrogate import Surrogate, sample_sets
+from sasmodels_b200.surrogate import Surrogate, TrainingGraph, sample_sets
 
 
 def _surrogate():
@@ -31,3 +31,17 @@ def test_iq_refuses_q_without_points():
     cols.update(set=np.zeros(0, int), q=np.full(3, 0.1))
     with pytest.raises(ValueError, match="q has shape"):
         _surrogate().iq(cols)
+
+
+@pytest.mark.parametrize("place", [("cpu", "meta", "meta"), ("meta", "cpu", "meta"),
+                                   ("meta", "meta", "cpu")])
+def test_capture_refuses_a_data_set_elsewhere(place):
+    """Features, their low halves or targets on another device than the network
+    (here the meta device, which has no memory that a kernel could reach)."""
+    import torch
+    shapes = ((256, 16), (256, 16), (256,))
+    types = (torch.bfloat16, torch.bfloat16, torch.float32)
+    data = [torch.zeros(s, dtype=t, device=d) for s, t, d in zip(shapes, types, place)]
+    net = SimpleNamespace(torch=torch, device=torch.device("meta"))
+    with pytest.raises(ValueError, match="must be on"):
+        TrainingGraph(net, *data, 128, 1e-3, 10, 0, 1, 0.9, 0.999, 1e-8)
