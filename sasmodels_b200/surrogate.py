@@ -597,11 +597,12 @@ class TrainingGraph:
         net._scratch(batch)
         lib, st = net.lib, net.stream.cuda_stream
         # the forward gathers 32-byte rows of bf16 and float targets, as
-        # MLP.features and the surrogate lay them out
-        direct = (all(t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[1] == NIN
+        # MLP.features (whose rows are padded to whole tiles) and the surrogate
+        # lay them out
+        direct = self.direct = (all(t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[1] == NIN
                       for t in (x_all, x_lo_all))
                   and y_all.dtype == torch.float32 and y_all.dim() == 1
-                  and len(x_all) == len(x_lo_all) == len(y_all)
+                  and len(y_all) <= min(len(x_all), len(x_lo_all))
                   and all(t.is_contiguous() and t.data_ptr() % 16 == 0
                           for t in (x_all, x_lo_all, y_all)))
         rates = (int(total), int(warmup), float(lr), b1, b2)

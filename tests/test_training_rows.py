@@ -1,6 +1,7 @@
 """
 A captured training step whose batch names a row outside the data set trains
-nothing and says so, in the step itself and in those that follow.
+nothing and says so, in the step itself and in those that follow; features
+padded to whole tiles are gathered like others.
 """
 
 import pytest
@@ -49,3 +50,36 @@ def test_row_outside_trains_nothing(cuda, batch, row, huber):
     torch.cuda.synchronize()
     assert torch.isfinite(loss) and net.errors() == 0
     assert not torch.equal(kept[0], net.params[0])
+
+
+@pytest.mark.parametrize("batch", [128, 128*80])
+@pytest.mark.parametrize("n", [1, 1000, 1024])
+def test_padded_features_are_gathered(cuda, batch, n):
+    """n targets with the padded features of MLP.features, as the surrogate trains,
+    against index_select (strided data); the padding is outside the data set."""
+    import torch
+    from sasmodels_b200.surrogate import MLP, pad128
+    wide = torch.rand((pad128(n), 32), device="cuda").to(torch.bfloat16)
+    y = torch.randn(n, device="cuda")
+    idx = torch.randint(0, n, (batch,), device="cuda")
+    results = []
+    for x in (wide[:, :16].contiguous(), wide[:n, :16]):
+        net = MLP(seed=4)
+        lo = torch.full_like(x, 2.0**-9)
+        torch.cuda.synchronize()
+        graph = net.capture_training(x, lo, y, batch, 1e-3, 100, 1)
+        assert graph.direct == x.is_contiguous()
+        for _ in range(2):
+            loss = graph.step(idx)
+        torch.cuda.synchronize()
+        assert net.errors() == 0
+        results.append([loss.clone()] + [t.clone() for t in net.params + net.m + net.v])
+        if graph.direct and n < len(x):
+            idx_pad = idx.clone()
+            idx_pad[0] = n
+            torch.cuda.synchronize()
+            loss = graph.step(idx_pad)
+            torch.cuda.synchronize()
+            assert torch.isnan(loss) and net.errors() == 5
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
