@@ -39,6 +39,7 @@
 // report through *err (0 = ok).
 #include <cstdint>
 #include <cstdio>
+#include <type_traits>
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
@@ -2133,9 +2134,14 @@ static int32_t weight_grads(int32_t n, int32_t n_pad, int32_t splits, const void
     prm.db_out = db_out;
     prm.n = (float)n;
     prm.refused = refused;
-    cudaFuncSetAttribute(mlp_weight_grads, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
-    launch_dependent(mlp_weight_grads, dim3((WG_BIG + 2)*splits), WG_THREADS, WG_SMEM,
-                     (cudaStream_t)stream, n_pad/TM, splits, prm, err);
+    // the tensor core's sums lose about half an ulp of the sum per step of 16 rows,
+    // always towards zero, so a chain is no longer than those of a batch split 32
+    // ways, and 256 rows at most; chains are added in FP32
+    const auto kernel = n_pad <= 2048 ? mlp_weight_grads<1>
+                      : n_pad <= 6144 ? mlp_weight_grads<2> : mlp_weight_grads<4>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
+    launch_dependent(kernel, dim3((WG_BIG + 2)*splits), WG_THREADS, WG_SMEM, (cudaStream_t)stream,
+                     n_pad/TM, splits, prm, err);
     return status("mlp_weight_grads");
 }
 

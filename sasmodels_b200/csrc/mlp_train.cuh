@@ -269,12 +269,16 @@ mlp_backward_t(int n_tiles, const uint8_t *img_t, const float *w_out, const floa
 //                   of them also adds the loss and dout sums of the forward.
 // The rows are the K dimension of both operands, so the 32 KB halves of the tile
 // images are MN-major operands as they lie in memory: each half is one bulk
-// copy into a three-stage ring.  Bound by those copies (64 KB per 512-cycle
-// tile of MMAs); eight warps add the columns from the same stages meanwhile.
-// 14 S <= 148 blocks are one wave: S = 10.  Partial sums leave per split, added
-// by whoever reads them (Adam, sum_partials).  8192 rows: 9.7 us, 3001 rows 6.4
-// (14 with cold caches, for eight transposes, four split-K GEMMs, 28 us the larger,
-// and five column sums on four streams).
+// copy into a three-stage ring.  An accumulation chain in TMEM is 64 to 256 rows (the
+// tensor core's sums round towards zero: with a split's 819 rows in one chain the
+// gradients of 8192 rows were off by 8e-7 and are by 2.3e-7, at 131,072 rows 1.4e-5
+// and 2.4e-7); eight warps add the chains, which alternate between two buffers, in
+// FP32 registers, and the columns from the same stages meanwhile.  Bound by the copies
+// (64 KB per 512-cycle tile of MMAs) and, in layer 0, the hand-over of the features.
+// 14 S <= 148 blocks are one wave: S = 10.  Partial sums leave per split, added by
+// whoever reads them (Adam, sum_partials).  8192 rows: 9.7 us (14 with cold caches, for
+// eight transposes, four split-K GEMMs, 28 us the larger, and five column sums on four
+// streams).
 constexpr int WG_STAGES = 3;
 constexpr int WG_HALF = ACT_BYTES/2;                   // 32 KB: 128 columns of a tile
 constexpr int WG_STAGE_BYTES = 2*WG_HALF;
@@ -282,6 +286,12 @@ constexpr int WG_SUM_WARPS = 8;
 constexpr int WG_THREADS = 32*(WG_SUM_WARPS + 2);      // + producer, MMA
 constexpr int WG_SMEM = WG_STAGES*(WG_STAGE_BYTES + X_BYTES);
 constexpr int WG_BIG = 12;
+// 112 registers a thread, so that two blocks of adam_pack (48 registers, 256 threads)
+// fit beside a block and all are set up when the last gradients leave: a captured step
+// of 8192 rows 48.7 us, with 128 registers 50.7, with 160 49.8, with 102 49.1.
+constexpr int WG_BOUND = 576;
+constexpr int WG_PART = TM/2;                          // rows by which chains grow
+constexpr int WG_ACC = 128;                            // TMEM columns of an accumulator
 
 struct WeightGrads {
     const __nv_bfloat16 *x;          // [n_pad x 16] features (high halves)
@@ -296,12 +306,16 @@ struct WeightGrads {
     const float *refused;            // null, or nonzero there: the loss is undefined
 };
 
-__global__ void __launch_bounds__(WG_THREADS, 1)
+// CHAIN: parts of an accumulation chain (1, 2 or 4)
+template <int CHAIN>
+__global__ void __launch_bounds__(WG_BOUND, 1)
 mlp_weight_grads(int n_tiles, int splits, WeightGrads prm, int *__restrict__ err)
 {
+    constexpr int PARTS = TM/WG_PART;                  // of a tile
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *xs = smem + WG_STAGES*WG_STAGE_BYTES;
     __shared__ __align__(8) uint64_t full[WG_STAGES], empty[WG_STAGES], x_full[WG_STAGES], done;
+    __shared__ __align__(8) uint64_t acc_full[2], acc_free[2];
     __shared__ uint32_t tmem_slot;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int b = blockIdx.x;
@@ -314,7 +328,7 @@ mlp_weight_grads(int n_tiles, int splits, WeightGrads prm, int *__restrict__ err
     const int tiles = (int)((long long)n_tiles*(split + 1)/splits) - t0;
 
     if (warp == 0) {
-        tc::tmem_alloc(&tmem_slot, 128);
+        tc::tmem_alloc(&tmem_slot, 2*WG_ACC);
         tc::tmem_relinquish();
     }
     if (t == 0) {
@@ -322,6 +336,10 @@ mlp_weight_grads(int n_tiles, int splits, WeightGrads prm, int *__restrict__ err
             tc::mbar_init(&full[s], 1);
             tc::mbar_init(&empty[s], (mma ? 1 : 0) + (sums ? WG_SUM_WARPS : 0));
             tc::mbar_init(&x_full[s], WG_SUM_WARPS);
+        }
+        for (int a = 0; a < 2; ++a) {
+            tc::mbar_init(&acc_full[a], 1);
+            tc::mbar_init(&acc_free[a], WG_SUM_WARPS);
         }
         tc::mbar_init(&done, 1);
         tc::mbar_fence_init();
@@ -360,145 +378,182 @@ mlp_weight_grads(int n_tiles, int splits, WeightGrads prm, int *__restrict__ err
         }
     } else if (warp == WG_SUM_WARPS + 1) {
         // ---- MMA issue ----
-        if (lane == 0) {
-            if (mma) {
-                for (int i = 0; i < tiles; ++i) {
-                    const int s = i % WG_STAGES;
-                    const uint32_t parity = (uint32_t)((i/WG_STAGES) & 1);
-                    if (!(ok = tc::mbar_wait(&full[s], parity)
-                               && (big || tc::mbar_wait(&x_full[s], parity))))
-                        break;
-                    tc::fence_after_sync();
-                    const uint32_t a = tc::smem_u32(smem + s*WG_STAGE_BYTES);
-                    if (big) {
-                        constexpr uint32_t idesc = tc::idesc_bf16_mn(TM, 128);
-                        #pragma unroll
-                        for (int st = 0; st < TM/16; ++st)
-                            tc::mma_bf16(tmem, tc::mnmajor_desc<TM>(a, st),
-                                         tc::mnmajor_desc<TM>(a + WG_HALF, st), idesc,
-                                         (i > 0 || st > 0) ? 1u : 0u);
-                    } else {
-                        constexpr uint32_t idesc = tc::idesc_bf16_mn(TM, NIN);
-                        const uint32_t bx = tc::smem_u32(xs + s*X_BYTES);
-                        #pragma unroll
-                        for (int st = 0; st < TM/16; ++st) {
-                            const uint64_t bd = tc::mnmajor_desc<TM>(bx, st);
-                            const uint32_t acc = (i > 0 || st > 0) ? 1u : 0u;
-                            tc::mma_bf16(tmem, tc::mnmajor_desc<TM>(a, st), bd, idesc, acc);
-                            tc::mma_bf16(tmem + 64u, tc::mnmajor_desc<TM>(a + WG_HALF, st), bd,
-                                         idesc, acc);
-                        }
+        // Nothing but the first MMA of a tile asks whether it starts a chain: what
+        // this thread works out between two MMAs is time without them.
+        auto issue = [&](auto is_big) {
+            constexpr bool BIG = decltype(is_big)::value;
+            constexpr uint32_t idesc = tc::idesc_bf16_mn(TM, BIG ? 128 : NIN);
+            for (int i = 0; i < tiles; ++i) {
+                const int s = i % WG_STAGES;
+                const uint32_t parity = (uint32_t)((i/WG_STAGES) & 1);
+                if (!(ok = tc::mbar_wait(&full[s], parity)
+                           && (BIG || tc::mbar_wait(&x_full[s], parity))))
+                    break;
+                tc::fence_after_sync();
+                const uint32_t a = tc::smem_u32(smem + s*WG_STAGE_BYTES);
+                const uint32_t bm = BIG ? a + WG_HALF : tc::smem_u32(xs + s*X_BYTES);
+                #pragma unroll
+                for (int k = 0; k < PARTS; ++k) {
+                    // the chain, and whether it starts here: its buffer was read
+                    // two chains ago (completion u/2 - 1)
+                    const int u = CHAIN <= PARTS ? PARTS/CHAIN*i + k/CHAIN : i/(CHAIN/PARTS);
+                    const bool starts = k % CHAIN == 0 && (CHAIN <= PARTS || i % (CHAIN/PARTS) == 0);
+                    const uint32_t d = tmem + (uint32_t)(WG_ACC*(u & 1));
+                    if (starts && u >= 2) {
+                        if (!(ok = tc::mbar_wait(&acc_free[u & 1], (uint32_t)((u/2 - 1) & 1)))) break;
+                        tc::fence_after_sync();
                     }
-                    tc::mma_commit(&empty[s]);
+                    #pragma unroll
+                    for (int st = 0; st < WG_PART/16; ++st) {
+                        const int ks = k*(WG_PART/16) + st;
+                        const uint64_t bd = tc::mnmajor_desc<TM>(bm, ks);
+                        const uint32_t acc = (st > 0 || !starts) ? 1u : 0u;
+                        tc::mma_bf16(d, tc::mnmajor_desc<TM>(a, ks), bd, idesc, acc);
+                        if (!BIG) tc::mma_bf16(d + WG_ACC/2, tc::mnmajor_desc<TM>(a + WG_HALF, ks), bd,
+                                               idesc, acc);
+                    }
+                    if (CHAIN <= PARTS ? (k + 1) % CHAIN == 0
+                                       : k + 1 == PARTS && ((i + 1) % (CHAIN/PARTS) == 0 || i + 1 == tiles))
+                        tc::mma_commit(&acc_full[u & 1]);
                 }
+                if (!ok) break;
+                tc::mma_commit(&empty[s]);
             }
+        };
+        if (lane == 0) {
+            if (big) issue(std::true_type());
+            else if (mma) issue(std::false_type());
             tc::mma_commit(&done);
             ok = tc::mbar_wait(&done, 0u) && ok;
             if (!ok) atomicExch(err, 3);
         }
         __syncwarp();
     } else {
-        // ---- column sums: lane = row (mod 32), a warp 2 or 4 groups of 8 columns ----
-        const int groups = big ? 2 : 4;
-        float acc[4][8];
-        #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        // ---- column sums (lane = row (mod 32), a warp 2 or 4 groups of 8 columns)
+        // and the sums of the chains: warps 0-3 the first 64 columns of the
+        // accumulators, 4-7 the rest, lane = row.  By the kind of block, so that
+        // neither keeps the other's registers: what they leave lets the next
+        // kernel's blocks in early ----
+        auto add_up = [&](auto is_big) {
+            constexpr bool BIG = decltype(is_big)::value;
+            constexpr int GROUPS = BIG ? 2 : 4, COLUMNS = BIG ? WG_ACC/2 : NIN;
+            float acc[GROUPS][8];
             #pragma unroll
-            for (int e = 0; e < 8; ++e) acc[q][e] = 0.0f;
-        }
-        if (sums) {
+            for (int q = 0; q < GROUPS; ++q) {
+                #pragma unroll
+                for (int e = 0; e < 8; ++e) acc[q][e] = 0.0f;
+            }
+            const int quad = warp & 3, part = warp >> 2;
+            const uint32_t at = tmem + ((uint32_t)(32*quad) << 16) + (uint32_t)(WG_ACC/2*part);
+            float g[COLUMNS];
+            #pragma unroll
+            for (int j = 0; j < COLUMNS; ++j) g[j] = 0.0f;
+            // the features of a tile: one 16-byte unit per thread, a tile ahead
+            const int xr = t >> 1, xc = (t & 1)*8;
+            const uint4 *xsrc = reinterpret_cast<const uint4 *>(prm.x + ((size_t)t0*TM + xr)*NIN + xc);
+            uint4 xv = make_uint4(0, 0, 0, 0);
+            if (!BIG && first && tiles > 0) xv = *xsrc;
+            int u = 0;                                       // chain
             for (int i = 0; i < tiles && ok; ++i) {
                 const int s = i % WG_STAGES;
-                if (first) {
-                    // the features of the tile: one 16-byte unit per thread
+                if (!BIG && first) {
                     if (i >= WG_STAGES
                         && !(ok = warp_wait(&empty[s], (uint32_t)((i/WG_STAGES - 1) & 1))))
                         break;
-                    const int r = t >> 1, c = (t & 1)*8;
-                    *reinterpret_cast<uint4 *>(xs + s*X_BYTES + tc::kmajor_offset<TM>(r, c)) =
-                        *reinterpret_cast<const uint4 *>(prm.x + ((size_t)(t0 + i)*TM + r)*NIN + c);
+                    *reinterpret_cast<uint4 *>(xs + s*X_BYTES + tc::kmajor_offset<TM>(xr, xc)) = xv;
                     tc::fence_async_smem();
                     __syncwarp();
                     if (lane == 0) tc::mbar_arrive(&x_full[s]);
+                    if (i + 1 < tiles) xv = xsrc[(size_t)(i + 1)*(TM*NIN/8)];
                 }
-                float w[4] = {1.0f, 1.0f, 1.0f, 1.0f};
-                if (layer == 4) {
-                    #pragma unroll
-                    for (int r = 0; r < 4; ++r) w[r] = prm.dout[(t0 + i)*TM + 32*r + lane];
-                }
-                if (!(ok = warp_wait(&full[s], (uint32_t)((i/WG_STAGES) & 1)))) break;
-                const uint8_t *from = smem + s*WG_STAGE_BYTES + warp*groups*(2*GROUP_ELEMS) + 16*lane;
-                #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (q >= groups) break;
-                    #pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        const uint4 u = *reinterpret_cast<const uint4 *>(from + q*(2*GROUP_ELEMS)
-                                                                         + 512*r);
-                        const uint32_t v[4] = {u.x, u.y, u.z, u.w};
+                if (sums) {
+                    float w[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+                    if (!BIG && layer == 4) {
                         #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            acc[q][2*e] = fmaf(bf_lo(v[e]), w[r], acc[q][2*e]);
-                            acc[q][2*e + 1] = fmaf(bf_hi(v[e]), w[r], acc[q][2*e + 1]);
+                        for (int r = 0; r < 4; ++r) w[r] = prm.dout[(t0 + i)*TM + 32*r + lane];
+                    }
+                    if (!(ok = warp_wait(&full[s], (uint32_t)((i/WG_STAGES) & 1)))) break;
+                    const uint8_t *from = smem + s*WG_STAGE_BYTES + warp*GROUPS*(2*GROUP_ELEMS)
+                                        + 16*lane;
+                    #pragma unroll
+                    for (int q = 0; q < GROUPS; ++q) {
+                        #pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            const uint4 z = *reinterpret_cast<const uint4 *>(
+                                from + q*(2*GROUP_ELEMS) + 512*r);
+                            const uint32_t v[4] = {z.x, z.y, z.z, z.w};
+                            #pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                acc[q][2*e] = fmaf(bf_lo(v[e]), w[r], acc[q][2*e]);
+                                acc[q][2*e + 1] = fmaf(bf_hi(v[e]), w[r], acc[q][2*e + 1]);
+                            }
                         }
                     }
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&empty[s]);
                 }
-                __syncwarp();
-                if (lane == 0) tc::mbar_arrive(&empty[s]);
+                if (!mma) continue;
+                // the chains that end in this tile
+                if (CHAIN > PARTS && (i + 1) % (CHAIN/PARTS) != 0 && i + 1 < tiles) continue;
+                #pragma unroll 1
+                for (int k = 0; k < (CHAIN < PARTS ? PARTS/CHAIN : 1); ++k, ++u) {
+                    if (!(ok = warp_wait(&acc_full[u & 1], (uint32_t)((u/2) & 1)))) break;
+                    tc::fence_after_sync();
+                    #pragma unroll
+                    for (int c0 = 0; c0 < COLUMNS; c0 += 16) {
+                        uint32_t r[16];
+                        tc::tmem_ld16(at + (uint32_t)(WG_ACC*(u & 1) + c0), r);
+                        tc::tmem_wait_ld();
+                        tc::tmem_tie16(r);
+                        #pragma unroll
+                        for (int j = 0; j < 16; ++j) g[c0 + j] += __uint_as_float(r[j]);
+                    }
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&acc_free[u & 1]);
+                }
             }
-            float *to = layer == 4 ? prm.dw_out + (size_t)split*HID
-                                   : prm.db + ((size_t)layer*splits + split)*HID + mh*128;
-            #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (q >= groups) break;
-                const float v = warp_sum8(acc[q], lane);
-                if ((lane & 3) == 0) to[8*(warp*groups + q) + (lane >> 2)] = v;
+            if (sums) {
+                float *to = layer == 4 ? prm.dw_out + (size_t)split*HID
+                                       : prm.db + ((size_t)layer*splits + split)*HID + mh*128;
+                #pragma unroll
+                for (int q = 0; q < GROUPS; ++q) {
+                    const float v = warp_sum8(acc[q], lane);
+                    if ((lane & 3) == 0) to[8*(warp*GROUPS + q) + (lane >> 2)] = v;
+                }
             }
-        }
+            if (mma) {
+                const int m = 32*quad + lane;
+                float *crow = prm.dw[layer]
+                            + (BIG ? (size_t)split*HID*HID + (size_t)(mh*128 + m)*HID + nh*128 + 64*part
+                                   : (size_t)split*HID*NIN + (size_t)(128*part + m)*NIN);
+                // a whole 32-byte sector per store (in halves: 0.9 us more per launch)
+                #pragma unroll
+                for (int j = 0; j < COLUMNS; j += 8)
+                    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                                 :: "l"(crow + j), "f"(g[j]), "f"(g[j + 1]), "f"(g[j + 2]),
+                                    "f"(g[j + 3]), "f"(g[j + 4]), "f"(g[j + 5]), "f"(g[j + 6]),
+                                    "f"(g[j + 7]) : "memory");
+            }
+        };
+        if (big) add_up(std::true_type());
+        else add_up(std::false_type());
         if (layer == 4 && split == 0 && warp < 2) {
             // warp 0 the loss, warp 1 the output bias: sums of 4 n_tiles partials
             const float *part = prm.row_sums + (size_t)warp*4*n_tiles;
-            float v = 0.0f;
-            for (int j = lane; j < 4*n_tiles; j += 32) v += part[j];
+            double sum = 0.0;
+            for (int j = lane; j < 4*n_tiles; j += 32) sum += (double)part[j];
             #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (warp == 0) v = prm.refused && *prm.refused != 0.0f ? __int_as_float(0x7fffffff)
-                                                                   : v/prm.n;
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            float v = (float)(warp == 0 ? sum/(double)prm.n : sum);
+            if (warp == 0 && prm.refused && *prm.refused != 0.0f) v = __int_as_float(0x7fffffff);
             if (lane == 0) *(warp == 0 ? prm.loss : prm.db_out) = v;
-        }
-        // ---- the accumulators: warps 0-3 the first 64 columns, 4-7 the rest ----
-        if (mma && ok) {
-            ok = warp_wait(&done, 0u);
-            tc::fence_after_sync();
-            const int quad = warp & 3, part = warp >> 2;
-            const uint32_t at = tmem + ((uint32_t)(32*quad) << 16) + (uint32_t)(64*part);
-            const int m = 32*quad + lane;
-            const int ld = big ? HID : NIN;
-            float *crow = prm.dw[layer] + (size_t)split*HID*ld
-                        + (big ? (size_t)(mh*128 + m)*HID + nh*128 + 64*part
-                               : (size_t)(128*part + m)*NIN);
-            for (int c0 = 0; c0 < (big ? 64 : NIN); c0 += 16) {
-                uint32_t r[16];
-                tc::tmem_ld16(at + (uint32_t)c0, r);
-                tc::tmem_wait_ld();
-                if (tiles == 0) {
-                    #pragma unroll
-                    for (int j = 0; j < 16; ++j) r[j] = 0u;
-                }
-                // a whole 32-byte sector per store (in halves: 0.9 us more per launch)
-                #pragma unroll
-                for (int j = 0; j < 16; j += 8)
-                    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                                 :: "l"(crow + c0 + j), "r"(r[j]), "r"(r[j + 1]), "r"(r[j + 2]),
-                                    "r"(r[j + 3]), "r"(r[j + 4]), "r"(r[j + 5]), "r"(r[j + 6]),
-                                    "r"(r[j + 7]) : "memory");
-            }
-            tc::fence_before_sync();
         }
         if (!ok && lane == 0) atomicExch(err, 1);
     }
+    tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, 128);
+    if (warp == 0) tc::tmem_dealloc(tmem, 2*WG_ACC);
 }
 
 // out[k][i] = the sum over its splits of part[k][s*size + i], in split order, for
@@ -520,10 +575,10 @@ sum_partials(SumTensors T)
     const int i = blockIdx.x*256 + threadIdx.x;
     if (i >= size) return;
     const float *p = T.part[k] + i;
-    float v = 0.0f;
+    double v = 0.0;
     #pragma unroll 8
-    for (int s = 0; s < splits; ++s) v += p[(size_t)s*size];
-    T.out[k][i] = v;
+    for (int s = 0; s < splits; ++s) v += (double)p[(size_t)s*size];
+    T.out[k][i] = (float)v;
 }
 
 // ------------------------------------------------------ batch and schedule --
@@ -656,8 +711,9 @@ adam_pack(AdamPack A)
     } else {
         const int k = 4 + b - 3*AP_TILES - AP_W0, size = k < 9 ? HID : 1;
         if (t >= size) return;
-        float g = 0.0f;
-        for (int s = 0; s < A.splits[k]; ++s) g += A.grad[k][s*size + t];
+        double sum = 0.0;
+        for (int s = 0; s < A.splits[k]; ++s) sum += (double)A.grad[k][s*size + t];
+        const float g = (float)sum;
         float p = A.p[k][t], m = A.m[k][t], v = A.v[k][t];
         adam_update(g, p, m, v, lr, A.b1, A.b2, A.eps, bc1, bc2);
         A.p[k][t] = p;
