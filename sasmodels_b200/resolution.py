@@ -221,6 +221,12 @@ def _band_apply(plan, n_sets, nq, n_calc, theory, stride, out, stream):
         theory.data_ptr(), stride, out.data_ptr(), nq, stream.cuda_stream), "band_apply")
 
 
+def _without_plan(self):
+    """State of a copy or a pickle: without what is kept on the device, whose
+    addresses are those of this object's tensors; the copy forms its own."""
+    return dict(self.__dict__, _dev=None)
+
+
 class Perfect1D:
     """No smearing (``resolution.py:52-63``)."""
 
@@ -259,6 +265,8 @@ class Pinhole1D:
         self._device_arg = device
         self._dev = None
         self._weight_matrix = None
+
+    __getstate__ = _without_plan
 
     @property
     def device(self):
@@ -378,6 +386,8 @@ class Slit1D:
         self.q_calc = abs(q_calc)
         self._device_arg = device
         self._dev = None
+
+    __getstate__ = _without_plan
 
     @property
     def device(self):
