@@ -31,7 +31,8 @@
  *                              by norm[i]; -0.0 for a point inside the band
  *                              that is not part of the sum;
  *   sasb200_band_apply         apply_resolution_matrix with them, for n_sets
- *                              curves.
+ *                              curves; _ordered: q i goes to out[order[i]], for
+ *                              q whose bands are in no order of their own.
  * All arrays are device pointers; the calls are asynchronous on *stream*.
  * Return 0, -1 for a bad argument, -3 for a launch error;
  * sasb200_resolution_last_error() describes the last failure.
@@ -83,6 +84,11 @@ int32_t sasb200_band_apply(int32_t n_sets, int32_t nq, int32_t n_calc, const int
                            const int32_t *hi, const int64_t *off, const double *w,
                            const double *norm, const double *theory, int64_t theory_stride,
                            double *out, int64_t out_stride, void *stream);
+int32_t sasb200_band_apply_ordered(int32_t n_sets, int32_t nq, int32_t n_calc,
+                                   const int32_t *order, const int32_t *lo, const int32_t *hi,
+                                   const int64_t *off, const double *w, const double *norm,
+                                   const double *theory, int64_t theory_stride, double *out,
+                                   int64_t out_stride, void *stream);
 
 #ifdef __cplusplus
 }

@@ -303,9 +303,10 @@ slit_weights(const double *__restrict__ q, const double *__restrict__ width,
 }
 
 // One warp per (q, curve): bound by latency and the two streams of doubles;
-// taken for one curve and for few (see sasb200_band_apply).
+// taken for one curve and for few (see sasb200_band_apply).  order: the place of each
+// q in the output (null: its own).
 __global__ void __launch_bounds__(128)
-band_apply(int nq, const int32_t *__restrict__ lo, const int32_t *__restrict__ hi,
+band_apply(int nq, const int32_t *__restrict__ order, const int32_t *__restrict__ lo, const int32_t *__restrict__ hi,
            const int64_t *__restrict__ off, const double *__restrict__ w,
            const double *__restrict__ norm, const double *__restrict__ theory,
            size_t theory_stride, double *__restrict__ out, size_t out_stride)
@@ -323,7 +324,7 @@ band_apply(int nq, const int32_t *__restrict__ lo, const int32_t *__restrict__ h
     }
     #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
-    if (lane == 0) out[blockIdx.y*out_stride + i] = acc/norm[i];
+    if (lane == 0) out[blockIdx.y*out_stride + (order ? order[i] : i)] = acc/norm[i];
 }
 
 // x/d from r = 1/d: one Newton step on the quotient's residual, which rounds as
@@ -370,7 +371,8 @@ constexpr int BR = BTHREADS/BJ;              // rows staged at once
 constexpr int B_LD = BJ + 4;                 // a fragment's 4 points x 8 rows hit all banks
 
 __global__ void __launch_bounds__(BTHREADS, 6)
-band_apply_sets(int n_sets, int nq, const int32_t *__restrict__ lo,
+band_apply_sets(int n_sets, int nq, const int32_t *__restrict__ order,
+                const int32_t *__restrict__ lo,
                 const int32_t *__restrict__ hi, const int64_t *__restrict__ off,
                 const double *__restrict__ w, const double *__restrict__ norm,
                 const double *__restrict__ theory, size_t theory_stride,
@@ -474,6 +476,7 @@ band_apply_sets(int n_sets, int nq, const int32_t *__restrict__ lo,
     if (qs < nq) {
         const double d = norm[qs], r = sr_of(d);
         const int64_t o = off[qs];
+        const int at = order ? order[qs] : qs;
         for (int k = warp; k < BS && s0 + k < n_sets; k += BWARPS) {
             double v = th[k*(BQ + 1) + lane];
             if (!isfinite(v)) {
@@ -481,7 +484,7 @@ band_apply_sets(int n_sets, int nq, const int32_t *__restrict__ lo,
                 const double *src = theory + (s0 + k)*theory_stride;
                 for (int j = my_lo; j < my_hi; ++j) v = fma(w[o + (j - my_lo)], src[j], v);
             }
-            out[(s0 + k)*out_stride + qs] = quotient(v, d, r);
+            out[(s0 + k)*out_stride + at] = quotient(v, d, r);
         }
     }
 }
@@ -647,11 +650,15 @@ int32_t sasb200_slit_weights(int32_t nq, const double *q, const double *width,
 }
 
 // out[s*out_stride + i] = sum_j w[off[i] + j - lo[i]] theory[s*theory_stride + j]/norm[i]
-// over lo[i] <= j < hi[i], for n_sets curves.
-int32_t sasb200_band_apply(int32_t n_sets, int32_t nq, int32_t n_calc, const int32_t *lo,
-                           const int32_t *hi, const int64_t *off, const double *w,
-                           const double *norm, const double *theory, int64_t theory_stride,
-                           double *out, int64_t out_stride, void *stream)
+// over lo[i] <= j < hi[i], for n_sets curves; to out[s*out_stride + order[i]] where order is
+// not NULL.  Neighbouring i should have neighbouring bands: a block of many curves
+// reads all points between the first and the last of its 32 (1000 curves and q of 20,000
+// points, 1 % width: 82 us in order of q, 2064 in any).
+int32_t sasb200_band_apply_ordered(int32_t n_sets, int32_t nq, int32_t n_calc,
+                                   const int32_t *order, const int32_t *lo, const int32_t *hi,
+                                   const int64_t *off, const double *w, const double *norm,
+                                   const double *theory, int64_t theory_stride, double *out,
+                                   int64_t out_stride, void *stream)
 {
     res::errbuf()[0] = 0;
     if (n_sets < 0 || n_sets > 65535 || nq < 0 || n_calc < 0 || theory_stride < n_calc
@@ -664,13 +671,22 @@ int32_t sasb200_band_apply(int32_t n_sets, int32_t nq, int32_t n_calc, const int
     const unsigned qb = (unsigned)((nq + res::BQ - 1)/res::BQ);
     if ((long long)nq*n_sets <= res::BAND_WARP_LIMIT) {
         const dim3 grid((unsigned)((nq + 3)/4), (unsigned)n_sets);
-        res::band_apply<<<grid, 128, 0, st>>>(nq, lo, hi, off, w, norm, theory, ts, out, os);
+        res::band_apply<<<grid, 128, 0, st>>>(nq, order, lo, hi, off, w, norm, theory, ts, out, os);
     } else {
         const dim3 grid(qb, (unsigned)((n_sets + res::BS - 1)/res::BS));
-        res::band_apply_sets<<<grid, res::BTHREADS, 0, st>>>(n_sets, nq, lo, hi, off, w, norm,
+        res::band_apply_sets<<<grid, res::BTHREADS, 0, st>>>(n_sets, nq, order, lo, hi, off, w, norm,
                                                              theory, ts, out, os);
     }
     return res::status("band_apply");
+}
+
+int32_t sasb200_band_apply(int32_t n_sets, int32_t nq, int32_t n_calc, const int32_t *lo,
+                           const int32_t *hi, const int64_t *off, const double *w,
+                           const double *norm, const double *theory, int64_t theory_stride,
+                           double *out, int64_t out_stride, void *stream)
+{
+    return sasb200_band_apply_ordered(n_sets, nq, n_calc, nullptr, lo, hi, off, w, norm, theory,
+                                      theory_stride, out, out_stride, stream);
 }
 
 // out[s] = 0.5 sum_i ((theory[s*theory_stride + i] - y[i])/dy[i])^2.

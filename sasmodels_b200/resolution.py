@@ -64,6 +64,8 @@ def _lib():
         lib.sasb200_slit_weights.restype = I
         lib.sasb200_band_apply.argtypes = [I, I, I, P, P, P, P, P, P, L, P, L, P]
         lib.sasb200_band_apply.restype = I
+        lib.sasb200_band_apply_ordered.argtypes = [I, I, I, P, P, P, P, P, P, P, L, P, L, P]
+        lib.sasb200_band_apply_ordered.restype = I
         lib.sasb200_resolution_last_error.restype = ct.c_char_p
         _LIB = lib
     return _LIB
@@ -193,10 +195,20 @@ def _on_device(theory, dev, n):
     return t, on_device
 
 
-def _band_plan(lo, hi, dev, form):
+def _band_order(q):
+    """Order in which the bands of the measured points lie side by side, or
+    None where they do already."""
+    step = np.diff(q)
+    if np.all(step >= 0) or np.all(step <= 0):
+        return None
+    return np.argsort(q, kind="stable").astype(np.int32)
+
+
+def _band_plan(lo, hi, dev, form, order=None):
     """Weights of the bands [lo, hi) on the device, formed once by *form*
     (lo, hi, off, w, norm, stream), or None when they are too many.  Complete
-    on return, so that any stream may use them."""
+    on return, so that any stream may use them.  Band i is that of measured
+    point order[i] (None: of point i)."""
     import torch
     off = np.hstack([0, np.cumsum(np.maximum(hi.astype(np.int64) - lo, 0))])
     if off[-1] > MAX_WEIGHTS:
@@ -211,11 +223,20 @@ def _band_plan(lo, hi, dev, form):
                     hi=index[3*n:].data_ptr(), norm=weights.data_ptr(),
                     w=weights[n:].data_ptr())
         form(plan["lo"], plan["hi"], plan["off"], plan["w"], plan["norm"], st.cuda_stream)
+        if order is not None:
+            plan["order"] = torch.as_tensor(order, device=dev)
         st.synchronize()
     return plan
 
 
 def _band_apply(plan, n_sets, nq, n_calc, theory, stride, out, stream):
+    order = plan.get("order")
+    if order is not None:
+        _check(_lib().sasb200_band_apply_ordered(
+            n_sets, nq, n_calc, order.data_ptr(), plan["lo"], plan["hi"], plan["off"], plan["w"],
+            plan["norm"], theory.data_ptr(), stride, out.data_ptr(), nq, stream.cuda_stream),
+            "band_apply")
+        return
     _check(_lib().sasb200_band_apply(
         n_sets, nq, n_calc, plan["lo"], plan["hi"], plan["off"], plan["w"], plan["norm"],
         theory.data_ptr(), stride, out.data_ptr(), nq, stream.cuda_stream), "band_apply")
@@ -276,19 +297,25 @@ class Pinhole1D:
         if self._dev is None:
             import torch
             dev = self.device
-            d = dict(
-                q=torch.as_tensor(np.ascontiguousarray(self.q, 'd'), device=dev),
-                width=torch.as_tensor(self._width, device=dev),
-                edges=torch.as_tensor(self.edges, device=dev))
+            q, width = np.ascontiguousarray(self.q, 'd'), self._width
+            lo, hi = self.band_lo, self.band_hi
+            d = dict(edges=torch.as_tensor(self.edges, device=dev))
+            order = _band_order(q)
+
+            def upload(k):
+                d.update(q=torch.as_tensor(q[k], device=dev),
+                         width=torch.as_tensor(width[k], device=dev))
 
             def form(lo, hi, off, w, norm, stream):
                 _check(_lib().sasb200_pinhole_weights(
                     len(d["q"]), d["q"].data_ptr(), d["width"].data_ptr(), lo, hi, off,
                     d["edges"].data_ptr(), w, norm, stream), "pinhole_weights")
-            d["plan"] = _band_plan(self.band_lo, self.band_hi, dev, form)
+            k = slice(None) if order is None else order
+            upload(k)
+            d["plan"] = _band_plan(lo[k], hi[k], dev, form, order)
             if d["plan"] is None:
-                d.update(lo=torch.as_tensor(self.band_lo, device=dev),
-                         hi=torch.as_tensor(self.band_hi, device=dev))
+                upload(slice(None))
+                d.update(lo=torch.as_tensor(lo, device=dev), hi=torch.as_tensor(hi, device=dev))
             self._dev = d
         return self._dev
 
