@@ -327,9 +327,11 @@ band_apply(int nq, const int32_t *__restrict__ order, const int32_t *__restrict_
     if (lane == 0) out[blockIdx.y*out_stride + (order ? order[i] : i)] = acc/norm[i];
 }
 
-// x/d from r = 1/d: one Newton step on the quotient's residual, which rounds as
-// the division does for the normal range that sr_of admits; an infinite
-// quotient has no residual and r = 0 marks the divisors that sr_of refuses.
+// x/d from r = 1/d, correctly rounded, by one correction of x r with its residual
+// (Markstein 1990), which rounds as the division does.  That wants a residual
+// without rounding of its own: the division itself where the numerator or the
+// quotient is so small that the residual's last bits fall below the smallest number,
+// where the quotient is infinite, and for divisors that sr_of refuses (r = 0).
 __device__ __forceinline__ double sr_of(double d)
 {
     return fabs(d) > 1e-290 && fabs(d) < 1e290 ? 1.0/d : 0.0;
@@ -337,7 +339,8 @@ __device__ __forceinline__ double sr_of(double d)
 __device__ __forceinline__ double quotient(double x, double d, double r)
 {
     const double q = x*r;
-    return r == 0.0 || !isfinite(q) ? x/d : fma(fma(-q, d, x), r, q);
+    const bool normal = fabs(x) > 1e-290 && fabs(q) > 1e-290 && fabs(q) <= 1.7e308;
+    return r != 0.0 && normal ? fma(fma(-q, d, x), r, q) : x/d;
 }
 
 // c = a b + c on the FP64 tensor pipe: a 16 x 4 (row-major), b 4 x 8, c 16 x 8, as
