@@ -83,8 +83,7 @@ int32_t sasb200_mlp_backward_p(int32_t n, int32_t n_pad, const void *img_t, cons
 
 /* training: forward with saved pre-activations and activations
  * (z_save, h_save: [4][n_pad x 256] bf16 each, or both NULL), backward
- * through the hidden layers (wt: transposed bf16 weights), weight
- * gradients as split-K partial GEMMs C[splits][M x nb] = A[M x K] B[nb x K]^T,
+ * through the hidden layers (wt: transposed bf16 weights),
  * Huber loss gradient, Adam (also refreshing the bf16
  * copies w and, if non-NULL, the transposed wt). */
 int32_t sasb200_mlp_forward(int32_t n, int32_t n_pad, const void *x, const void *x_lo,
@@ -94,11 +93,6 @@ int32_t sasb200_mlp_forward(int32_t n, int32_t n_pad, const void *x, const void 
 int32_t sasb200_mlp_backward(int32_t n, int32_t n_pad, const void *const *wt,
                              const float *w_out, const float *dout, const void *z_save,
                              void *dz_save, int32_t *err, void *stream);
-int32_t sasb200_gemm_nt(int32_t M, int32_t nb, int32_t K, int32_t lda, int32_t ldb,
-                        const void *A, const void *B, int32_t splits, float *C, int32_t *err,
-                        void *stream);
-int32_t sasb200_transpose_bf16(int32_t rows, int32_t cols, const void *src, void *dst,
-                               void *stream);
 int32_t sasb200_loss_grad(int32_t n, int32_t n_pad, const float *out, const float *y,
                           float delta, float *dout, float *loss, void *stream);
 int32_t sasb200_adam(int32_t size, int32_t splits, const float *grad, float *p, float *m,
@@ -170,16 +164,6 @@ int32_t sasb200_adam_pack(const float *const *grads, const int32_t *splits, floa
  * whole training step replays with these. */
 int32_t sasb200_lr_schedule(int32_t *counters, float *sched, int32_t total, int32_t warmup,
                             float lr0, float b1, float b2, void *stream);
-
-/* Adam for all n (<= 16) parameter tensors in one launch, lr and bias
- * corrections from sched (sasb200_lr_schedule): host arrays of n entries
- * (device pointers; w[k], wt[k] may be NULL), each tensor updated as by
- * sasb200_adam */
-int32_t sasb200_adam_multi(int32_t n, const int32_t *sizes, const int32_t *splits,
-                           const float *const *grads, float *const *p, float *const *m,
-                           float *const *v, void *const *w, void *const *wt, const int32_t *rows,
-                           const int32_t *cols, const float *sched, float b1, float b2, float eps,
-                           void *stream);
 
 /* out[c] = sum over r of M[r][c] (times v[r] when v is non-NULL) for a
  * row-major bf16 [rows x cols] matrix, in a fixed order: partial sums of

@@ -30,10 +30,8 @@
 //                  tiles in flight on each (mlp_pairs.cuh).
 //   mlp_backward_t, mlp_weight_grads   the training step's backward and weight
 //                  gradients on tiled planes (mlp_train.cuh).
-//   gemm_nt        C_split = A[M x K] B[N x K]^T over a K range (split-K).
-//   + transpose, column sums (bias gradients), loss gradient, the learning
-//     rate schedule, Adam (one tensor, or every tensor in one launch),
-//     feature packing.
+//   + the learning rate schedule, Adam, feature packing; column sums, loss
+//     gradient and Adam of one tensor, which tests compare with.
 //
 // All launches return an error code; device-side waits are bounded and
 // report through *err (0 = ok).
@@ -56,7 +54,6 @@ constexpr int THREADS = 128;
 constexpr int ACT_BYTES = TM*HID*2;                // one 128 x 256 bf16 tile
 constexpr int FWD_SMEM = 2*ACT_BYTES + HID*KC*2;   // act hi + lo + 32 KB weights
 constexpr int BWD_SMEM = ACT_BYTES + HID*KC*2;     // dZ tile + 32 KB weights
-constexpr int GEMM_SMEM = 100*1024;                // keeps <= 2 CTAs per SM (TMEM)
 
 struct Weights {
     const __nv_bfloat16 *w[4];    // w[0]: 256 x 16, w[1..3]: 256 x 256, [out][in]
@@ -380,88 +377,8 @@ mlp_backward(int n, WeightsT wts, const float *__restrict__ dout,
     if (!pp.ok && t == 0) atomicExch(err, 1);
 }
 
-// C[split][M x NB] = A[M x K] B[NB x K]^T restricted to this split's K range
-// (multiples of 64).  grid = (M/128, splits).
-template <int NB>
-__global__ void __launch_bounds__(THREADS, 1)
-gemm_nt(int K, int lda, int ldb, const __nv_bfloat16 *__restrict__ A,
-        const __nv_bfloat16 *__restrict__ B, int k_per_split, float *__restrict__ C,
-        int M, int *__restrict__ err)
-{
-    extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t *abuf = smem;
-    uint8_t *bbuf = smem + TM*KC*2;
-    __shared__ __align__(8) uint64_t bar;
-    __shared__ uint32_t tmem_slot;
-    constexpr uint32_t NCOL = NB < 32 ? 32 : NB;
-    const int t = threadIdx.x;
-    const int m0 = blockIdx.x*TM;
-    const int k_begin = blockIdx.y*k_per_split;
-    const int k_end = min(K, k_begin + k_per_split);
-
-    if (t < 32) {
-        tc::tmem_alloc(&tmem_slot, NCOL);
-        tc::tmem_relinquish();
-    }
-    if (t == 0) {
-        tc::mbar_init(&bar, 1);
-        tc::mbar_fence_init();
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    const uint32_t tmem = tmem_slot;
-    Pipe pp{&bar, 0u, true};
-    bool any = false;
-    for (int k0 = k_begin; k0 < k_end && pp.ok; k0 += KC) {
-        load_tile<TM, KC>(abuf, A + (size_t)m0*lda, lda, k0, M - m0);
-        load_tile<NB, KC>(bbuf, B, ldb, k0, NB);
-        mma_chunk<NB, KC/16>(pp, tmem, tc::smem_u32(abuf), 0, tc::smem_u32(bbuf), any);
-        any = true;
-    }
-    if (pp.ok) {
-        float *crow = C + ((size_t)blockIdx.y*M + m0 + t)*NB;
-        const bool valid = m0 + t < M;
-        for (int c0 = 0; c0 < NB; c0 += 16) {
-            float v[16];
-            tmem_row16(tmem, c0, v);
-            if (!any) {
-                #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = 0.0f;
-            }
-            if (valid) {
-                #pragma unroll
-                for (int j = 0; j < 16; j += 4)
-                    *reinterpret_cast<float4 *>(crow + c0 + j) = make_float4(v[j], v[j+1], v[j+2], v[j+3]);
-            }
-        }
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    if (t < 32) tc::tmem_dealloc(tmem, NCOL);
-    if (!pp.ok && t == 0) atomicExch(err, 1);
-}
-
 // ---- small CUDA-core kernels ------------------------------------------------
 
-// dst[c][r] = src[r][c]  (bf16), 32x32 tiles through shared memory
-__global__ void transpose_bf16(int rows, int cols, const __nv_bfloat16 *__restrict__ src,
-                               __nv_bfloat16 *__restrict__ dst)
-{
-    __shared__ __nv_bfloat16 tile[32][33];
-    const int bx = blockIdx.x*32, by = blockIdx.y*32;
-    for (int j = threadIdx.y; j < 32; j += 8) {
-        const int r = by + j, c = bx + threadIdx.x;
-        if (r < rows && c < cols) tile[j][threadIdx.x] = src[(size_t)r*cols + c];
-    }
-    __syncthreads();
-    for (int j = threadIdx.y; j < 32; j += 8) {
-        const int c = bx + j, r = by + threadIdx.x;
-        if (r < rows && c < cols) dst[(size_t)c*rows + r] = tile[threadIdx.x][j];
-    }
-}
-
-// out[r] = sum_c M[r][c] * (v ? v[c] : 1), one warp per row, fixed order
 // Column sums of a row-major [rows x cols] bf16 matrix, each row weighted
 // by v[row] when v is given (the bias gradients from the dZ planes, the
 // output-layer gradient from the last h plane with v = dout).  Pass 1: one
@@ -547,18 +464,15 @@ __device__ __forceinline__ void adam_update(float g, float &p, float &m, float &
     p = p - lr*(mi/bc1)/(sqrtf(vi/bc2) + eps);
 }
 
-// Adam on one FP32 master tensor; grad = sum of `splits` partial gradients.
-// Writes the BF16 copy (and its transpose if wt != nullptr, rows x cols).
-// Adam update of element i: the gradient summed over its `splits` split-K
-// partials, moments, parameter, and its bf16 copies (w; wt transposed).
-__device__ __forceinline__ void adam_element(int i, int size, int splits,
-                                             const float *__restrict__ grad,
-                                             float *__restrict__ p, float *__restrict__ m,
-                                             float *__restrict__ v, float lr, float b1, float b2,
-                                             float eps, float bc1, float bc2,
-                                             __nv_bfloat16 *__restrict__ w,
-                                             __nv_bfloat16 *__restrict__ wt, int rows, int cols)
+// Adam on one FP32 master tensor; the gradient is the sum of its `splits` partials.
+// Writes the BF16 copy and, if wt is given, its transpose (rows x cols).
+__global__ void adam_step(int size, int splits, const float *__restrict__ grad, float *__restrict__ p,
+                          float *__restrict__ m, float *__restrict__ v, float lr, float b1,
+                          float b2, float eps, float bc1, float bc2, __nv_bfloat16 *__restrict__ w,
+                          __nv_bfloat16 *__restrict__ wt, int rows, int cols)
 {
+    const int i = blockIdx.x*blockDim.x + threadIdx.x;
+    if (i >= size) return;
     float g = 0.0f;
     for (int s = 0; s < splits; ++s) g += grad[(size_t)s*size + i];
     float pi = p[i];
@@ -569,41 +483,6 @@ __device__ __forceinline__ void adam_element(int i, int size, int splits,
         const int r = i/cols, c = i % cols;
         wt[(size_t)c*rows + r] = __float2bfloat16_rn(pi);
     }
-}
-
-__global__ void adam_step(int size, int splits, const float *__restrict__ grad, float *__restrict__ p,
-                          float *__restrict__ m, float *__restrict__ v, float lr, float b1,
-                          float b2, float eps, float bc1, float bc2, __nv_bfloat16 *__restrict__ w,
-                          __nv_bfloat16 *__restrict__ wt, int rows, int cols)
-{
-    const int i = blockIdx.x*blockDim.x + threadIdx.x;
-    if (i >= size) return;
-    adam_element(i, size, splits, grad, p, m, v, lr, b1, b2, eps, bc1, bc2, w, wt, rows, cols);
-}
-
-// Every parameter tensor of the network in one launch (blockIdx.y = tensor),
-// the update of adam_step with lr and the bias corrections read from the
-// device (sched = {lr, bc1, bc2}, written by lr_schedule on the same stream,
-// so a CUDA graph of a training step replays with the schedule advancing).
-constexpr int ADAM_MAX_TENSORS = 16;
-struct AdamTensors {
-    int n;
-    int size[ADAM_MAX_TENSORS], splits[ADAM_MAX_TENSORS];
-    int rows[ADAM_MAX_TENSORS], cols[ADAM_MAX_TENSORS];
-    const float *grad[ADAM_MAX_TENSORS];
-    float *p[ADAM_MAX_TENSORS], *m[ADAM_MAX_TENSORS], *v[ADAM_MAX_TENSORS];
-    __nv_bfloat16 *w[ADAM_MAX_TENSORS], *wt[ADAM_MAX_TENSORS];
-};
-
-__global__ void adam_multi(AdamTensors T, float b1, float b2, float eps,
-                           const float *__restrict__ sched)
-{
-    const int k = blockIdx.y;
-    if (k >= T.n) return;
-    const int i = blockIdx.x*blockDim.x + threadIdx.x;
-    if (i >= T.size[k]) return;
-    adam_element(i, T.size[k], T.splits[k], T.grad[k], T.p[k], T.m[k], T.v[k], sched[0], b1, b2,
-                 eps, sched[1], sched[2], T.w[k], T.wt[k], T.rows[k], T.cols[k]);
 }
 
 // One training step's learning rate and Adam bias corrections from two
@@ -2278,44 +2157,6 @@ int32_t sasb200_mlp_backward(int32_t n, int32_t n_pad, const void *const *wt, co
     return status("mlp_backward");
 }
 
-// C[splits][M x nb] partial products of A[M x K] (row stride lda) and
-// B[nb x K] (row stride ldb); M % 128 == 0, K % 64 == 0, nb in {16, 256}.
-int32_t sasb200_gemm_nt(int32_t M, int32_t nb, int32_t K, int32_t lda, int32_t ldb,
-                        const void *A, const void *B, int32_t splits, float *C, int32_t *err,
-                        void *stream)
-{
-    errbuf()[0] = 0;
-    if (M <= 0 || M % TM || K <= 0 || K % KC || splits <= 0 || !A || !B || !C || !err
-        || lda < K || ldb < K || lda % 8 || ldb % 8)
-        return (std::snprintf(errbuf(), 256, "bad arguments"), -1);
-    int per = (K + splits - 1)/splits;
-    per = ((per + KC - 1)/KC)*KC;
-    dim3 grid(M/TM, splits);
-    const __nv_bfloat16 *a = static_cast<const __nv_bfloat16 *>(A);
-    const __nv_bfloat16 *bb = static_cast<const __nv_bfloat16 *>(B);
-    cudaStream_t st = (cudaStream_t)stream;
-    if (nb == 256) {
-        cudaFuncSetAttribute(gemm_nt<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
-        gemm_nt<256><<<grid, THREADS, GEMM_SMEM, st>>>(K, lda, ldb, a, bb, per, C, M, err);
-    } else if (nb == 16) {
-        cudaFuncSetAttribute(gemm_nt<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
-        gemm_nt<16><<<grid, THREADS, GEMM_SMEM, st>>>(K, lda, ldb, a, bb, per, C, M, err);
-    } else {
-        return (std::snprintf(errbuf(), 256, "nb must be 16 or 256"), -1);
-    }
-    return status("gemm_nt");
-}
-
-int32_t sasb200_transpose_bf16(int32_t rows, int32_t cols, const void *src, void *dst, void *stream)
-{
-    if (rows < 0 || cols < 0 || !src || !dst) return -1;
-    if (!rows || !cols) return 0;
-    dim3 grid((cols + 31)/32, (rows + 31)/32), block(32, 8);
-    transpose_bf16<<<grid, block, 0, (cudaStream_t)stream>>>(
-        rows, cols, static_cast<const __nv_bfloat16 *>(src), static_cast<__nv_bfloat16 *>(dst));
-    return status("transpose_bf16");
-}
-
 int32_t sasb200_loss_grad(int32_t n, int32_t n_pad, const float *out, const float *y, float delta,
                           float *dout, float *loss, void *stream)
 {
@@ -2337,37 +2178,6 @@ int32_t sasb200_adam(int32_t size, int32_t splits, const float *grad, float *p, 
         size, splits, grad, p, m, v, lr, b1, b2, eps, bc1, bc2,
         static_cast<__nv_bfloat16 *>(w), static_cast<__nv_bfloat16 *>(wt), rows, cols);
     return status("adam_step");
-}
-
-int32_t sasb200_adam_multi(int32_t n, const int32_t *sizes, const int32_t *splits,
-                           const float *const *grads, float *const *p, float *const *m,
-                           float *const *v, void *const *w, void *const *wt, const int32_t *rows,
-                           const int32_t *cols, const float *sched, float b1, float b2, float eps,
-                           void *stream)
-{
-    if (n <= 0 || n > ADAM_MAX_TENSORS || !sizes || !splits || !grads || !p || !m || !v || !w
-        || !wt || !rows || !cols || !sched)
-        return -1;
-    AdamTensors T;
-    T.n = n;
-    int most = 0;
-    for (int k = 0; k < n; ++k) {
-        if (sizes[k] <= 0 || splits[k] <= 0 || !grads[k] || !p[k] || !m[k] || !v[k]) return -1;
-        if (wt[k] && rows[k]*cols[k] != sizes[k]) return -1;
-        T.size[k] = sizes[k];
-        T.splits[k] = splits[k];
-        T.rows[k] = rows[k];
-        T.cols[k] = cols[k];
-        T.grad[k] = grads[k];
-        T.p[k] = p[k];
-        T.m[k] = m[k];
-        T.v[k] = v[k];
-        T.w[k] = static_cast<__nv_bfloat16 *>(w[k]);
-        T.wt[k] = static_cast<__nv_bfloat16 *>(wt[k]);
-        most = sizes[k] > most ? sizes[k] : most;
-    }
-    adam_multi<<<dim3((most + 255)/256, n), 256, 0, (cudaStream_t)stream>>>(T, b1, b2, eps, sched);
-    return status("adam_multi");
 }
 
 int32_t sasb200_col_sums(int32_t rows, int32_t cols, const void *M, const float *v, float *part,

@@ -2,6 +2,9 @@
 What the surrogate's entry points refuse before anything reaches the GPU.
 """
 
+import glob
+import os
+import re
 from types import SimpleNamespace
 
 import numpy as np
@@ -45,3 +48,16 @@ def test_capture_refuses_a_data_set_elsewhere(place):
     net = SimpleNamespace(torch=torch, device=torch.device("meta"))
     with pytest.raises(ValueError, match="must be on"):
         TrainingGraph(net, *data, 128, 1e-3, 10, 0, 1, 0.9, 0.999, 1e-8)
+
+
+def test_every_entry_of_the_library_has_a_caller():
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    with open(os.path.join(root, "sasmodels_b200", "csrc", "mlp.cu")) as f:
+        entries = re.findall(r"^(?:int32_t|const char \*) ?(sasb200_\w+)\(", f.read(), re.M)
+    calls = ""
+    for path in (glob.glob(os.path.join(root, "sasmodels_b200", "*.py"))
+                 + glob.glob(os.path.join(root, "tests", "*.py"))):
+        with open(path) as f:
+            calls += f.read()
+    assert len(entries) > 15
+    assert [e for e in entries if "." + e + "(" not in calls] == []
