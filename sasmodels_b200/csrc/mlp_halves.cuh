@@ -33,12 +33,13 @@
 // when their output is known, so dZ3 forms from the z that the warps still hold, and
 // the transposed weights follow the others through the ring.  In a captured step the
 // features are gathered here and the schedule advances.  A step of 8192 rows with
-// launches of their own for the backward 50.5 us and for the gathering 51.5, now 47.1.
+// launches of their own for the backward 50.5 us and for the gathering 51.5, in one
+// 47.1; 48.7 with hand-overs that release what they stand for (mbar_arrive_cta).
 //
 // Every value is that of the kernels of one tile per SM, bit for bit.  Bound by the
 // chain of a tile still: an MMA of a pair takes 103 cycles here (32 of them a layer),
 // an epilogue 700 cycles until its first hand-over, 170 from there to the MMAs.
-// Serving 8 tiles 17.5 -> 12.3 us, 64 tiles 17.9 -> 13.2.
+// Serving 8 tiles 16.6 us with one SM each, 12.1 with two; 64 tiles 16.9 and 13.2.
 #pragma once
 
 constexpr int HV_RELAY_WARP = SV_EPI_WARPS + 2;

@@ -59,9 +59,10 @@
 //
 // The hidden activations and the output are those of mlp_serve bit for bit (the
 // paired FP32 operations round each half as the scalar ones).  4,000,000 rows 3.10
-// -> 2.12 ms (1.52 PFLOP/s of MMA, both halves counted: 0.94 of the measured
-// BF16 peak), 500,000 rows 411 -> 269 us, 50,021 rows 51.8 -> 39.1 us.  Chunks of
-// 32 inputs: 2.18 ms, of 128: 2.42 ms.
+// -> 2.14 ms (1.50 PFLOP/s of MMA, both halves counted: 0.93 of the measured
+// BF16 peak), 500,000 rows 411 -> 275 us, 50,021 rows 51.8 -> 38.4 us; without the
+// fences of the hand-overs 2.13 ms, 269 and 37.6 us.  Chunks of 32 inputs took 3 % more,
+// of 128 14 %.
 #pragma once
 
 constexpr int SP_POLL_WARP = SV_EPI_WARPS + 2;

@@ -31,8 +31,8 @@ __device__ __forceinline__ float warp_sum8(float (&v)[8], int lane)
 // first columns while the epilogue works on the last.  For batches of more tiles
 // than half the SMs (fewer: mlp_halves).  Bound by the latency of one tile's
 // chain: the ring holds a whole layer of weights (fetched while dZ3 forms), and each
-// warp loads the z of its eight chunks one layer ahead.  64 tiles on as many SMs:
-// 16.5 us (mlp_backward_p 38 us).
+// warp loads the z of its eight chunks one layer ahead.  100 tiles: 20.4 us with cold
+// caches.
 constexpr int BT_STAGES = 8;
 constexpr int BT_SMEM = ACT_BYTES + BT_STAGES*CHUNK_BYTES;
 
@@ -276,9 +276,8 @@ mlp_backward_t(int n_tiles, const uint8_t *img_t, const float *w_out, const floa
 // FP32 registers, and the columns from the same stages meanwhile.  Bound by the copies
 // (64 KB per 512-cycle tile of MMAs) and, in layer 0, the hand-over of the features.
 // 14 S <= 148 blocks are one wave: S = 10.  Partial sums leave per split, added by
-// whoever reads them (Adam, sum_partials).  8192 rows: 9.7 us (14 with cold caches, for
-// eight transposes, four split-K GEMMs, 28 us the larger, and five column sums on four
-// streams).
+// whoever reads them (Adam, sum_partials).  With cold caches 15.7 us for 8192 rows (15.4
+// with a split in one chain), 11.7 for 3001.
 constexpr int WG_STAGES = 3;
 constexpr int WG_HALF = ACT_BYTES/2;                   // 32 KB: 128 columns of a tile
 constexpr int WG_STAGE_BYTES = 2*WG_HALF;
@@ -286,9 +285,10 @@ constexpr int WG_SUM_WARPS = 8;
 constexpr int WG_THREADS = 32*(WG_SUM_WARPS + 2);      // + producer, MMA
 constexpr int WG_SMEM = WG_STAGES*(WG_STAGE_BYTES + X_BYTES);
 constexpr int WG_BIG = 12;
-// 112 registers a thread, so that two blocks of adam_pack (48 registers, 256 threads)
-// fit beside a block and all are set up when the last gradients leave: a captured step
-// of 8192 rows 48.7 us, with 128 registers 50.7, with 160 49.8, with 102 49.1.
+// Threads by which the registers are bounded (to 96), so that two blocks of adam_pack
+// (48 registers, 256 threads) fit beside a block and all are set up when the last
+// gradients leave: a quarter of the SM holds 3 warps of one and 4 of the others.  A captured
+// step of 8192 rows 48.7 us, with 128 registers 50.7, with up to 168 49.8.
 constexpr int WG_BOUND = 576;
 constexpr int WG_PART = TM/2;                          // rows by which chains grow
 constexpr int WG_ACC = 128;                            // TMEM columns of an accumulator
@@ -558,7 +558,8 @@ mlp_weight_grads(int n_tiles, int splits, WeightGrads prm, int *__restrict__ err
 
 // out[k][i] = the sum over its splits of part[k][s*size + i], in split order, for
 // up to 16 tensors in one launch (blockIdx.y = tensor): a step's gradients as
-// one set of plain tensors.  Bound by the bytes of the partials (8 MB, in L2).
+// one set of plain tensors.  In double precision, so that the sum rounds once.  Bound by
+// the bytes of the partials (8 MB, in L2): 6.3 us with cold caches.
 constexpr int SUM_TENSORS = 16;
 struct SumTensors {
     int size[SUM_TENSORS], splits[SUM_TENSORS];
