@@ -1679,6 +1679,14 @@ mlp_backward_p(int n, int n_tiles, const uint8_t *__restrict__ img_t,
 
 using namespace mlp;
 
+// A kernel lets its dependents in before it has allocated its tensor memory, so a
+// dependent that allocates some must not come to the same SM: it would wait there for
+// the kernel, which would wait for the memory.  No two of these fit one SM's shared memory.
+constexpr int SM_SHARED = 227*1024;
+constexpr int LEAST_TMEM_SMEM = BT_SMEM < WG_SMEM ? BT_SMEM : WG_SMEM;
+static_assert(LEAST_TMEM_SMEM <= SV_SMEM && LEAST_TMEM_SMEM <= HV_SMEM
+              && 2*LEAST_TMEM_SMEM > SM_SHARED, "two kernels with tensor memory on one SM");
+
 // A launch whose CTAs may be placed while the kernels before it on the stream still
 // run; the kernel waits for them by itself (tc::dependency_wait).  Hides the
 // launch and the set-up of each kernel of a training step behind the one before:

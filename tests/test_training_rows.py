@@ -34,7 +34,7 @@ def test_row_outside_trains_nothing(cuda, batch, row, huber):
             + [net.img, net.img_t]]
     torch.cuda.synchronize()
     with torch.cuda.stream(net.stream):
-        torch.cuda._sleep(20_000_000)
+        torch.cuda._sleep(200_000_000)
     graph.step(bad)
     loss = graph.step(idx)           # queued before the host can know
     torch.cuda.synchronize()
